@@ -2,10 +2,11 @@
 
 ``libgcb200_host.so``  -- CPU oracles and host-side native helpers (g++, no CUDA needed)
 ``libgcb200_cuda.so``  -- every sm_100a kernel (nvcc ``-gencode arch=compute_100a,code=sm_100a``)
+``gcb200_ext.so``      -- CPython extension module: the reducers' native front end (g++ with torch's headers)
 
-Both land in ``gradient_compression_b200/_lib/`` next to the sources they are built from, and are
+All land in ``gradient_compression_b200/_lib/`` next to the sources they are built from.  The first two are
 bound with ctypes (plain C ABI: raw pointers + a ``cudaStream_t``), so a rebuild takes seconds and
-needs neither libtorch headers nor pybind.  Run ``python -m gradient_compression_b200.build``.
+needs neither libtorch headers nor pybind; the third reads ``torch.Tensor`` objects natively.  Run ``python -m gradient_compression_b200.build``.
 """
 from __future__ import annotations
 
@@ -20,7 +21,8 @@ CSRC = os.path.join(HERE, "csrc")
 LIBDIR = os.path.join(HERE, "_lib")
 
 HOST_SOURCES = ["host_oracle.cpp"]
-CUDA_SOURCES = ["gc_kernels.cu", "gc_fused.cu", "gc_noalloc.cu", "gc_bn.cu", "gc_head.cu", "gc_powersgd.cu", "gc_topk.cu", "gc_gemm_tc.cu", "gc_conv_tc.cu", "gc_varpack.cu", "gc_augment.cu"]
+EXT_SOURCES = ["pyext.cpp"]
+CUDA_SOURCES = ["gc_kernels.cu", "gc_fused.cu", "gc_solo.cu", "gc_noalloc.cu", "gc_bn.cu", "gc_head.cu", "gc_powersgd.cu", "gc_topk.cu", "gc_gemm_tc.cu", "gc_conv_tc.cu", "gc_varpack.cu", "gc_augment.cu"]
 NVCC_ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
 
@@ -192,8 +194,40 @@ def build_cuda(force=False, verbose=False, ptxas_info=False, debug_bounds=False)
     return lib
 
 
+def ext_path():
+    return os.path.join(LIBDIR, "gcb200_ext.so")
+
+
+def build_ext(force=False, verbose=False):
+    """The extension module.  It links torch's libraries by name only: torch is imported before it is loaded."""
+    import sysconfig
+
+    import torch
+
+    os.makedirs(LIBDIR, exist_ok=True)
+    srcs = _sources(EXT_SOURCES)
+    root = os.path.dirname(torch.__file__)
+    cuda_home = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+    flags = ["-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
+    cmd = (["g++"] + flags + ["-I", sysconfig.get_paths()["include"], "-isystem", os.path.join(root, "include"), "-isystem",
+                              os.path.join(root, "include", "torch", "csrc", "api", "include"), "-isystem", os.path.join(cuda_home, "include"),
+                              "-o", ext_path()] + srcs + ["-L", os.path.join(root, "lib"), "-ltorch_python", "-ltorch_cpu", "-lc10", "-lc10_cuda"])
+    digest = _digest(srcs, _flags_only(cmd) + torch.__version__ + sys.version)
+    if not force and not _stale(ext_path(), digest):
+        return ext_path()
+    if shutil.which("g++") is None:
+        raise RuntimeError("g++ not found: cannot build gcb200_ext.so")
+    with _BuildLock():
+        if force or _stale(ext_path(), digest):
+            if verbose:
+                print(" ".join(cmd))
+            _compile(cmd, ext_path())
+            _finish(ext_path(), digest)
+    return ext_path()
+
+
 def build_all(force=False, verbose=False):
-    return build_host(force, verbose), build_cuda(force, verbose)
+    return build_host(force, verbose), build_cuda(force, verbose), build_ext(force, verbose)
 
 
 if __name__ == "__main__":
@@ -206,3 +240,4 @@ if __name__ == "__main__":
     force = "--force" in sys.argv
     print(build_host(force, verbose=True))
     print(build_cuda(force, verbose=True, ptxas_info="--ptxas" in sys.argv))
+    print(build_ext(force, verbose=True))

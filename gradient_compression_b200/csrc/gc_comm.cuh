@@ -35,7 +35,10 @@ struct ArenaHeader {
   uint32_t epoch;                          // epoch of the last fused launch on this rank (device-resident so that
                                            // a replayed CUDA graph still advances it)
   uint32_t calls;                          // launches so far; optional source of the Philox step
-  uint32_t pad0[1];
+  uint32_t solo_max[2];                    // single-worker kernels: grid-wide maximum (float bits), used in turn
+  uint32_t solo_arrived;                   // their grid barrier: arrivals since the arena was made (never reset) ...
+  uint32_t solo_passed;                    // ... and how many of them earlier launches account for
+  uint32_t solo_turn;                      // which of the two maxima the next launch uses (low bit)
   float partial[MAX_PARTIALS];             // per-block partial maxima
   float reduced[8];                        // small per-step results (local norm, ...)
 };
@@ -48,6 +51,17 @@ struct RankView {
   const void* aux;        // optional second input (index list of the sparse exchange)
   int rank;
   int pad;
+};
+
+// Host side of one rank's arena.
+struct CommCtx {
+  int world, rank, device;
+  int64_t bytes;
+  uint8_t* local;
+  uint8_t* peers[MAXW];
+  bool ipc_opened[MAXW];
+  int step_from_device;
+  int sm_count;
 };
 
 // Up to MAXW virtual ranks per launch: real multi-GPU runs use exactly one (its own rank); the

@@ -16,6 +16,7 @@
 
 #include "gc_comm.cuh"
 #include "gc_perm.h"
+#include "gc_solo.h"
 
 using namespace gc;
 
@@ -220,36 +221,10 @@ __global__ void __maxnreg__(GC_FUSED_MAXNREG) qsgd_fused_kernel(LaunchViews lv, 
   // P0: global max-norm
   float m = rank_max(w, local_absmax(c, v.in, n, al_in), c.bid, c.nblocks, smem, 0x20);
   commit_epoch(c.hdr, epoch, c.bid);
-  float norm = (world > 1) ? exchange_max(w, v, world, epoch, m, c.bid == 0, smem) : m;
+  float norm = exchange_max(w, v, world, epoch, m, c.bid == 0, smem);
   float scale = (norm > 0.0f) ? (float)p.s / norm : 0.0f;
   float dq = dequant_scale(norm, p.s, world);
   RngKey key = rng_key(p.c, rng_step, v.rank, PURPOSE_ROUND);
-
-  if (world == 1) {
-    // single worker: quantise and dequantise in registers, one pass, four rows per warp in flight
-    for (int64_t row0 = c.warp; row0 < rows; row0 += 4 * c.nwarps) {
-      float4 x[4];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        int64_t row = row0 + u * c.nwarps;
-        x[u] = (row < rows) ? load_quad(v.in, row * 128 + c.lane * 4, n, al_in) : make_float4(0.f, 0.f, 0.f, 0.f);
-      }
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        int64_t row = row0 + u * c.nwarps;
-        if (row >= rows) break;
-        int64_t e0 = row * 128 + c.lane * 4;
-        U4 r = philox_block(key, (uint64_t)(e0 >> 2));
-        float4 y;
-        y.x = mul_rn(dq, (float)quantize_level(x[u].x, scale, p.s, r.x));
-        y.y = mul_rn(dq, (float)quantize_level(x[u].y, scale, p.s, r.y));
-        y.z = mul_rn(dq, (float)quantize_level(x[u].z, scale, p.s, r.z));
-        y.w = mul_rn(dq, (float)quantize_level(x[u].w, scale, p.s, r.w));
-        store_quad(v.out, e0, n, al_out, y);
-      }
-    }
-    return;
-  }
 
   // P1: quantise + pack into this rank's arena (four rows per warp in flight)
   uint8_t* my = v.arena[v.rank];
@@ -328,28 +303,26 @@ __global__ void __maxnreg__(GC_FUSED_MAXNREG) twoscale_fused_kernel(LaunchViews 
 
   float m = rank_max(w, local_absmax(c, v.in, n, al_in), c.bid, c.nblocks, smem, 0x30);
   commit_epoch(c.hdr, epoch, c.bid);
-  float norm = (world > 1) ? exchange_max(w, v, world, epoch, m, c.bid == 0, smem) : m;
+  float norm = exchange_max(w, v, world, epoch, m, c.bid == 0, smem);
   float sc_lo = (norm > 0.0f) ? (float)p.s_lo / norm : 0.0f;
   float sc_hi = (norm > 0.0f) ? (float)p.s_hi / norm : 0.0f;
   float dq_lo = dequant_scale(norm, p.s_lo, world), dq_hi = dequant_scale(norm, p.s_hi, world);
   RngKey k_lo = rng_key(p.c, rng_step, v.rank, PURPOSE_ROUND), k_hi = rng_key(p.c, rng_step, v.rank, PURPOSE_ROUND_HI);
 
   // P1a: which elements' rounded high-scale level still fits the low range (this rank's vote)
-  if (world > 1) {
-    for (int64_t row = c.warp; row < rows; row += c.nwarps) {
-      int64_t e0 = row * 128 + c.lane * 4;
-      float4 x = load_quad(v.in, e0, n, al_in);
-      U4 r = philox_block(k_hi, (uint64_t)(e0 >> 2));
-      bool fit[4] = {abs(quantize_level(x.x, sc_hi, p.s_hi, r.x)) <= p.s_lo,
-                     abs(quantize_level(x.y, sc_hi, p.s_hi, r.y)) <= p.s_lo,
-                     abs(quantize_level(x.z, sc_hi, p.s_hi, r.z)) <= p.s_lo,
-                     abs(quantize_level(x.w, sc_hi, p.s_hi, r.w)) <= p.s_lo};
-      store_row_plane(reinterpret_cast<uint32_t*>(my + p.off_mask_local), row, c.lane, fit);
-    }
-    grid_barrier(w, c.nblocks, 0x31);
-    if (c.bid == 0) signal_all(v, world, PH_MASK, epoch);
-    wait_all(w, world, PH_MASK, epoch);
+  for (int64_t row = c.warp; row < rows; row += c.nwarps) {
+    int64_t e0 = row * 128 + c.lane * 4;
+    float4 x = load_quad(v.in, e0, n, al_in);
+    U4 r = philox_block(k_hi, (uint64_t)(e0 >> 2));
+    bool fit[4] = {abs(quantize_level(x.x, sc_hi, p.s_hi, r.x)) <= p.s_lo,
+                   abs(quantize_level(x.y, sc_hi, p.s_hi, r.y)) <= p.s_lo,
+                   abs(quantize_level(x.z, sc_hi, p.s_hi, r.z)) <= p.s_lo,
+                   abs(quantize_level(x.w, sc_hi, p.s_hi, r.w)) <= p.s_lo};
+    store_row_plane(reinterpret_cast<uint32_t*>(my + p.off_mask_local), row, c.lane, fit);
   }
+  grid_barrier(w, c.nblocks, 0x31);
+  if (c.bid == 0) signal_all(v, world, PH_MASK, epoch);
+  wait_all(w, world, PH_MASK, epoch);
 
   // P1b: AND of all votes (one-shot read of every peer's bit plane), pick the scale, quantise
   for (int64_t row = c.warp; row < rows; row += c.nwarps) {
@@ -362,41 +335,26 @@ __global__ void __maxnreg__(GC_FUSED_MAXNREG) twoscale_fused_kernel(LaunchViews 
     int ql[4] = {quantize_level(x.x, sc_lo, p.s_lo, rl.x), quantize_level(x.y, sc_lo, p.s_lo, rl.y),
                  quantize_level(x.z, sc_lo, p.s_lo, rl.z), quantize_level(x.w, sc_lo, p.s_lo, rl.w)};
     bool use_hi[4];
-    if (world > 1) {
-      uint32_t mine = load_plane_all_ranks(v, world, p.off_mask_local, row, c.lane);
-      uint32_t andw[4] = {0xffffffffu, 0xffffffffu, 0xffffffffu, 0xffffffffu};
+    uint32_t mine = load_plane_all_ranks(v, world, p.off_mask_local, row, c.lane);
+    uint32_t andw[4] = {0xffffffffu, 0xffffffffu, 0xffffffffu, 0xffffffffu};
 #pragma unroll
-      for (int src = 0; src < MAXW; ++src)
+    for (int src = 0; src < MAXW; ++src)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          uint32_t t = __shfl_sync(FULL, mine, src * 4 + j);
-          if (src < world) andw[j] &= t;
-        }
+      for (int j = 0; j < 4; ++j) {
+        uint32_t t = __shfl_sync(FULL, mine, src * 4 + j);
+        if (src < world) andw[j] &= t;
+      }
 #pragma unroll
-      for (int j = 0; j < 4; ++j) use_hi[j] = (andw[j] >> c.lane) & 1u;
-    } else {
-#pragma unroll
-      for (int j = 0; j < 4; ++j) use_hi[j] = abs(qh[j]) <= p.s_lo;
-    }
+    for (int j = 0; j < 4; ++j) use_hi[j] = (andw[j] >> c.lane) & 1u;
     int q[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) q[j] = use_hi[j] ? qh[j] : ql[j];
-    if (world == 1) {
-      float4 y;
-      y.x = mul_rn(use_hi[0] ? dq_hi : dq_lo, (float)q[0]);
-      y.y = mul_rn(use_hi[1] ? dq_hi : dq_lo, (float)q[1]);
-      y.z = mul_rn(use_hi[2] ? dq_hi : dq_lo, (float)q[2]);
-      y.w = mul_rn(use_hi[3] ? dq_hi : dq_lo, (float)q[3]);
-      store_quad(v.out, e0, n, al_out, y);
-    } else {
-      int mg[4] = {abs(q[0]), abs(q[1]), abs(q[2]), abs(q[3])};
-      bool sg[4] = {q[0] < 0, q[1] < 0, q[2] < 0, q[3] < 0};
-      store_row_mags<MW>(my + p.off_mags, row, c.lane, mg);
-      store_row_plane(reinterpret_cast<uint32_t*>(my + p.off_signs), row, c.lane, sg);
-      store_row_plane(reinterpret_cast<uint32_t*>(my + p.off_mask_final), row, c.lane, use_hi);
-    }
+    int mg[4] = {abs(q[0]), abs(q[1]), abs(q[2]), abs(q[3])};
+    bool sg[4] = {q[0] < 0, q[1] < 0, q[2] < 0, q[3] < 0};
+    store_row_mags<MW>(my + p.off_mags, row, c.lane, mg);
+    store_row_plane(reinterpret_cast<uint32_t*>(my + p.off_signs), row, c.lane, sg);
+    store_row_plane(reinterpret_cast<uint32_t*>(my + p.off_mask_final), row, c.lane, use_hi);
   }
-  if (world == 1) return;
   grid_barrier(w, c.nblocks, 0x32);
   if (c.bid == 0) signal_all(v, world, PH_READY, epoch);
   wait_all(w, world, PH_READY, epoch);
@@ -571,11 +529,6 @@ __global__ void __maxnreg__(GC_FUSED_MAXNREG) allreduce_fused_kernel(LaunchViews
   const int64_t nq = (n + 3) / 4;
   const int64_t stride = (int64_t)c.nblocks * THREADS;
   const int64_t tid = (int64_t)c.bid * THREADS + threadIdx.x;
-  if (world == 1) {
-    if (v.in != v.out)
-      for (int64_t q = tid; q < nq; q += stride) store_quad(v.out, q * 4, n, al_out, load_quad(v.in, q * 4, n, al_in));
-    return;
-  }
   float4* stage = reinterpret_cast<float4*>(v.arena[v.rank] + p.off_stage);
   {
     int64_t q = tid;
@@ -841,16 +794,6 @@ __global__ void __launch_bounds__(THREADS, 2) sparse_fused_kernel(LaunchViews lv
 }
 
 // ------------------------------------------------------------------------------------------ host side
-struct CommCtx {
-  int world, rank, device;
-  int64_t bytes;
-  uint8_t* local;
-  uint8_t* peers[MAXW];
-  bool ipc_opened[MAXW];
-  int step_from_device;
-  int sm_count;
-};
-
 int max_coresident(const void* kernel, int sm_count) {
   int per_sm = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, THREADS, 0);
@@ -926,6 +869,13 @@ Common make_common(CommCtx** ctxs, int n_virtual, int64_t n, uint64_t seed, uint
   c.seed_hi = (uint32_t)(seed >> 32);
   c.step = step;
   return c;
+}
+
+// A flat vector on a single worker: the kernels of gc_solo.cu.
+int solo_flat(CommCtx* c, const float* in, float* out, int64_t n, int bits_lo, int bits_hi, uint64_t seed, uint32_t step, int timeout_ms,
+              int max_blocks, void* cs) {
+  const SegDesc seg{in, out, 0};
+  return gc_solo_maxnorm(c, &seg, 1, n, bits_lo, bits_hi, seed, step, timeout_ms, max_blocks, cs);
 }
 
 inline int64_t align_up(int64_t x, int64_t a) { return (x + a - 1) / a * a; }
@@ -1046,7 +996,9 @@ int gc_comm_clear_status(void* ctx, void* cs) {
   ArenaHeader* h = (ArenaHeader*)c->local;
   // status, status_detail, abort are adjacent; the barrier words are reset too (a timed-out barrier
   // may have left arrivals behind)
-  return (int)cudaMemsetAsync(&h->bar_count, 0, 5 * sizeof(uint32_t), (cudaStream_t)cs);   // bar_count .. abort
+  cudaError_t e = cudaMemsetAsync(&h->bar_count, 0, 5 * sizeof(uint32_t), (cudaStream_t)cs);   // bar_count .. abort
+  if (e != cudaSuccess) return (int)e;
+  return (int)cudaMemsetAsync(&h->solo_max[0], 0, 4 * sizeof(uint32_t), (cudaStream_t)cs);     // solo_max .. solo_passed
 }
 
 int gc_comm_destroy(void* ctx) {
@@ -1091,6 +1043,7 @@ int gc_fused_qsgd(void** ctxs_, int n_virtual, const float* const* ins, float* c
                   uint64_t seed, uint32_t step, int timeout_ms, int max_blocks, void* cs) {
   CommCtx** ctxs = (CommCtx**)ctxs_;
   int world = ctxs[0]->world;
+  if (world == 1) return solo_flat(ctxs[0], ins[0], outs[0], n, bits, 0, seed, step, timeout_ms, max_blocks, cs);
   int s = (1 << bits) - 1, mw = mag_width(bits), sumb = sum_container_bytes(s, world);
   int64_t npad = pad128(n);
   QsgdParams p;
@@ -1114,6 +1067,7 @@ int gc_fused_twoscale(void** ctxs_, int n_virtual, const float* const* ins, floa
                       int bits_hi, uint64_t seed, uint32_t step, int timeout_ms, int max_blocks, void* cs) {
   CommCtx** ctxs = (CommCtx**)ctxs_;
   int world = ctxs[0]->world;
+  if (world == 1) return solo_flat(ctxs[0], ins[0], outs[0], n, bits_lo, bits_hi, seed, step, timeout_ms, max_blocks, cs);
   int s_lo = (1 << bits_lo) - 1, s_hi = (1 << bits_hi) - 1, mw = mag_width(bits_lo);
   int sumb = sum_container_bytes(s_lo, world);
   int64_t npad = pad128(n);
@@ -1157,7 +1111,7 @@ int gc_fused_multiscale(void** ctxs_, int n_virtual, const float* const* ins, fl
   p.off_idx_final[0] = take(plane_bytes(npad));
   p.off_idx_final[1] = take(plane_bytes(npad));
   p.off_sums = take(npad * sumb);
-  if (off > ctxs[0]->bytes) return (int)cudaErrorMemoryAllocation;
+  if (world > 1 && off > ctxs[0]->bytes) return (int)cudaErrorMemoryAllocation;      // (one rank writes nothing behind the header)
   int64_t rows = npad / 128;
   p.chunk_rows = (rows + world - 1) / world;
   const void* kern = multiscale_kernel_for(mw, sumb);
@@ -1173,11 +1127,15 @@ int gc_fused_allreduce(void** ctxs_, int n_virtual, const float* const* ins, flo
                        int timeout_ms, int max_blocks, void* cs) {
   CommCtx** ctxs = (CommCtx**)ctxs_;
   int world = ctxs[0]->world;
+  if (world == 1) {
+    const SegDesc seg{ins[0], outs[0], 0};
+    return ins[0] == outs[0] ? 0 : gc_solo_copy(ctxs[0], &seg, 1, n, cs);
+  }
   int64_t npad = pad128(n);
   AllreduceParams p;
   p.off_stage = ARENA_HEADER_BYTES;
   p.off_result = align_up(p.off_stage + npad * 4, 256);
-  if (world > 1 && p.off_result + npad * 4 > ctxs[0]->bytes) return (int)cudaErrorMemoryAllocation;
+  if (p.off_result + npad * 4 > ctxs[0]->bytes) return (int)cudaErrorMemoryAllocation;
   int64_t nq = npad / 4;
   p.chunk_quads = (nq + world - 1) / world;
   p.alpha = 1.0f / (float)world;

@@ -1,0 +1,12 @@
+// Entry points of the single-worker reducers (gc_solo.cu).  `segs`: n_seg SegDesc (gc_segs.cuh) of n elements in all.
+#pragma once
+#include <stdint.h>
+
+#include "gc_segs.cuh"
+
+extern "C" {
+int gc_solo_max_segs();
+int gc_solo_maxnorm(void* ctx, const void* segs, int n_seg, int64_t n, int bits_lo, int bits_hi, uint64_t seed, uint32_t step, int timeout_ms,
+                    int max_blocks, void* cs);
+int gc_solo_copy(void* ctx, const void* segs, int n_seg, int64_t n, void* cs);
+}

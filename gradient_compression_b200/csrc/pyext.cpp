@@ -1,0 +1,228 @@
+// The reducers' way from Python into the kernels: a CPython extension module.
+//
+// A reduce of a whole model hands over some hundred tensors, and what it computes takes a few dozen microseconds; looking at
+// the tensors through the Python interpreter (dtype, layout, address, adjacency) takes ten times that.  This module reads
+// them natively, merges neighbours, and calls the C ABI of the kernel library, whose entry points it is given as addresses
+// (`bind`), so that the regular and the bounds-checking build are served by the same module.
+#define PY_SSIZE_T_CLEAN
+#include <Python.h>
+
+#include <ATen/ATen.h>
+#include <c10/cuda/CUDAFunctions.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/autograd/python_variable.h>
+
+#include <algorithm>
+#include <cstring>
+#include <string>
+#include <unordered_map>
+#include <vector>
+
+namespace {
+
+struct SegDesc {            // csrc/gc_segs.cuh
+  const float* in;
+  float* out;
+  int64_t start;
+};
+
+// Entry points of the kernel library.
+struct Api {
+  int (*solo_max_segs)();
+  int (*solo_maxnorm)(void*, const void*, int, int64_t, int, int, uint64_t, uint32_t, int, int, void*);
+  int (*solo_copy)(void*, const void*, int, int64_t, void*);
+} api;
+int max_segs = 0;
+
+struct Entry { const char* name; void** slot; };
+const Entry entries[] = {
+    {"gc_solo_max_segs", (void**)&api.solo_max_segs},
+    {"gc_solo_maxnorm", (void**)&api.solo_maxnorm},
+    {"gc_solo_copy", (void**)&api.solo_copy},
+};
+
+// What one reducer saw last: its segment table, and the fact that its inputs and outputs do not overlap in an unsafe way
+// (checked once per set of addresses).
+struct Plan {
+  std::vector<SegDesc> segs, checked;
+  int64_t n = 0;
+  int device = -1;
+};
+
+void plan_free(PyObject* cap) { delete (Plan*)PyCapsule_GetPointer(cap, "gcb200.plan"); }
+Plan* plan_of(PyObject* o) { return (Plan*)PyCapsule_GetPointer(o, "gcb200.plan"); }
+
+PyObject* plan_new(PyObject*, PyObject*) { return PyCapsule_New(new Plan(), "gcb200.plan", plan_free); }
+
+// Address of a dense fp32 CUDA tensor in one of the two memory orders reducers take (contiguous, or channels-last for four
+// dimensions); nullptr for anything else.  `order`: 0 contiguous, 1 channels-last.
+float* dense_ptr(PyObject* o, int64_t* n, int* device, int* order) {
+  if (!THPVariable_Check(o)) return nullptr;
+  const at::Tensor& t = THPVariable_Unpack(o);
+  if (!t.is_cuda() || t.scalar_type() != at::kFloat || t.layout() != at::kStrided) return nullptr;
+  if (t.is_contiguous()) *order = 0;
+  else if (t.dim() == 4 && t.is_contiguous(at::MemoryFormat::ChannelsLast)) *order = 1;
+  else return nullptr;
+  *n = t.numel();
+  *device = t.device().index();
+  return (float*)t.data_ptr();
+}
+
+// Inputs are read again after outputs have been written: an output may be its own input, but must not touch another one.
+bool overlap_free(const std::vector<SegDesc>& segs, int64_t n) {
+  struct Range { uintptr_t lo, hi; int seg; bool out; };
+  std::vector<Range> r;
+  r.reserve(segs.size() * 2);
+  for (size_t i = 0; i < segs.size(); ++i) {
+    const int64_t len = (i + 1 < segs.size() ? segs[i + 1].start : n) - segs[i].start;
+    if (len <= 0) continue;
+    const uintptr_t a = (uintptr_t)segs[i].in, b = (uintptr_t)segs[i].out;
+    r.push_back({a, a + (uintptr_t)len * 4, (int)i, false});
+    r.push_back({b, b + (uintptr_t)len * 4, (int)i, true});
+  }
+  std::sort(r.begin(), r.end(), [](const Range& x, const Range& y) { return x.lo < y.lo || (x.lo == y.lo && x.seg < y.seg); });
+  // sweep: the furthest end of any input / output seen so far, and whose it is
+  uintptr_t in_hi = 0, out_hi = 0;
+  int in_seg = -1, out_seg = -1;
+  for (const Range& x : r) {
+    const bool same_in = in_seg == x.seg && segs[x.seg].in == segs[x.seg].out, same_out = out_seg == x.seg && segs[x.seg].in == segs[x.seg].out;
+    if (x.lo < out_hi && !same_out) return false;
+    if (x.out && x.lo < in_hi && !same_in) return false;
+    if (x.out) { if (x.hi > out_hi) { out_hi = x.hi; out_seg = x.seg; } }
+    else if (x.hi > in_hi) { in_hi = x.hi; in_seg = x.seg; }
+  }
+  return true;
+}
+
+// Fills the plan from two lists of tensors.  False: not a case for the segment kernels (the caller takes the general path).
+bool collect(Plan& p, PyObject* ins, PyObject* outs) {
+  PyObject* fa = PySequence_Fast(ins, "reduce() takes lists of tensors");
+  if (!fa) return false;
+  PyObject* fb = ins == outs ? (Py_INCREF(fa), fa) : PySequence_Fast(outs, "reduce() takes lists of tensors");
+  if (!fb) { Py_DECREF(fa); return false; }
+  const Py_ssize_t k = PySequence_Fast_GET_SIZE(fa);
+  bool ok = k > 0 && PySequence_Fast_GET_SIZE(fb) == k;
+  p.segs.clear();
+  p.n = 0;
+  p.device = -1;
+  for (Py_ssize_t i = 0; ok && i < k; ++i) {
+    int64_t na = 0, nb = 0;
+    int da = 0, db = 0, oa = 0, ob = 0;
+    PyObject *pa = PySequence_Fast_GET_ITEM(fa, i), *pb = PySequence_Fast_GET_ITEM(fb, i);
+    float* a = dense_ptr(pa, &na, &da, &oa);
+    float* b = a;
+    if (pa == pb) { nb = na; db = da; ob = oa; }
+    else b = dense_ptr(pb, &nb, &db, &ob);
+    if (na == 0 && nb == 0 && THPVariable_Check(pa) && THPVariable_Check(pb)) continue;
+    if (a == nullptr || b == nullptr || na != nb || da != db || oa != ob || (p.device >= 0 && da != p.device)) { ok = false; break; }
+    if (oa == 1 && pa != pb && THPVariable_Unpack(pa).sizes() != THPVariable_Unpack(pb).sizes()) { ok = false; break; }
+    p.device = da;
+    if (!p.segs.empty()) {
+      const SegDesc& last = p.segs.back();
+      const int64_t len = p.n - last.start;
+      if (a == last.in + len && b == last.out + len) { p.n += na; continue; }
+    }
+    p.segs.push_back({a, b, p.n});
+    p.n += na;
+  }
+  Py_DECREF(fa);
+  Py_DECREF(fb);
+  if (PyErr_Occurred()) return false;
+  if (!ok || p.segs.empty() || (int)p.segs.size() > max_segs) return false;
+  const bool known = p.checked.size() == p.segs.size() + 1 && p.checked.back().start == p.n &&
+                     memcmp(p.checked.data(), p.segs.data(), p.segs.size() * sizeof(SegDesc)) == 0;
+  if (!known) {
+    p.checked.clear();
+    if (!overlap_free(p.segs, p.n)) return false;
+    p.checked = p.segs;
+    p.checked.push_back({nullptr, nullptr, p.n});
+  }
+  return true;
+}
+
+void* stream_on(int device) { return (void*)c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)device).stream(); }
+
+PyObject* cuda_error(const char* what, int err) {
+  PyErr_Format(PyExc_RuntimeError, "%s: CUDA error %d", what, err);
+  return nullptr;
+}
+
+int64_t as_int(PyObject* o) { return PyLong_AsLongLong(o); }
+
+bool want(Py_ssize_t nargs, Py_ssize_t n, const char* name) {
+  if (nargs == n) return true;
+  PyErr_Format(PyExc_TypeError, "%s takes %zd arguments (%zd given)", name, n, nargs);
+  return false;
+}
+
+// solo_maxnorm(plan, ctx, grad_in, grad_out, bits_lo, bits_hi, seed, step, timeout_ms, max_blocks) -> elements, or None
+PyObject* solo_maxnorm(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
+  if (!want(nargs, 10, "solo_maxnorm")) return nullptr;
+  Plan* p = plan_of(a[0]);
+  if (!p) return nullptr;
+  if (!collect(*p, a[2], a[3])) { if (PyErr_Occurred()) return nullptr; Py_RETURN_NONE; }
+  void* ctx = (void*)PyLong_AsUnsignedLongLong(a[1]);
+  const int lo = (int)as_int(a[4]), hi = (int)as_int(a[5]), timeout = (int)as_int(a[8]), blocks = (int)as_int(a[9]);
+  const uint64_t seed = PyLong_AsUnsignedLongLongMask(a[6]);
+  const uint32_t step = (uint32_t)PyLong_AsUnsignedLongLongMask(a[7]);
+  if (PyErr_Occurred()) return nullptr;
+  c10::cuda::OptionalCUDAGuard guard(c10::Device(c10::kCUDA, (c10::DeviceIndex)p->device));
+  const int err = api.solo_maxnorm(ctx, p->segs.data(), (int)p->segs.size(), p->n, lo, hi, seed, step, timeout, blocks, stream_on(p->device));
+  if (err) return cuda_error("solo_maxnorm", err);
+  return PyLong_FromLongLong(p->n);
+}
+
+// solo_copy(plan, ctx, grad_in, grad_out) -> elements, or None
+PyObject* solo_copy(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
+  if (!want(nargs, 4, "solo_copy")) return nullptr;
+  Plan* p = plan_of(a[0]);
+  if (!p) return nullptr;
+  if (!collect(*p, a[2], a[3])) { if (PyErr_Occurred()) return nullptr; Py_RETURN_NONE; }
+  void* ctx = (void*)PyLong_AsUnsignedLongLong(a[1]);
+  if (PyErr_Occurred()) return nullptr;
+  bool moves = false;
+  for (const SegDesc& s : p->segs) moves = moves || s.in != s.out;
+  if (moves) {
+    c10::cuda::OptionalCUDAGuard guard(c10::Device(c10::kCUDA, (c10::DeviceIndex)p->device));
+    const int err = api.solo_copy(ctx, p->segs.data(), (int)p->segs.size(), p->n, stream_on(p->device));
+    if (err) return cuda_error("solo_copy", err);
+  }
+  return PyLong_FromLongLong(p->n);
+}
+
+// bind({name: address}): the kernel library's entry points
+PyObject* bind(PyObject*, PyObject* table) {
+  for (const Entry& e : entries) {
+    PyObject* v = PyDict_GetItemString(table, e.name);
+    if (!v) { PyErr_Format(PyExc_KeyError, "%s", e.name); return nullptr; }
+    *e.slot = (void*)PyLong_AsUnsignedLongLong(v);
+    if (PyErr_Occurred()) return nullptr;
+  }
+  max_segs = api.solo_max_segs();
+  Py_RETURN_NONE;
+}
+
+PyObject* names(PyObject*, PyObject*) {
+  PyObject* l = PyList_New(0);
+  for (const Entry& e : entries) {
+    PyObject* s = PyUnicode_FromString(e.name);
+    PyList_Append(l, s);
+    Py_DECREF(s);
+  }
+  return l;
+}
+
+PyMethodDef methods[] = {
+    {"bind", bind, METH_O, "bind(table): addresses of the kernel library's entry points by name"},
+    {"names", names, METH_NOARGS, "names() -> the entry points bind() needs"},
+    {"plan_new", plan_new, METH_NOARGS, "plan_new() -> a plan, one per reducer"},
+    {"solo_maxnorm", (PyCFunction)(void (*)(void))solo_maxnorm, METH_FASTCALL, "QSGD-MaxNorm reduce of a single worker"},
+    {"solo_copy", (PyCFunction)(void (*)(void))solo_copy, METH_FASTCALL, "plain mean of a single worker"},
+    {nullptr, nullptr, 0, nullptr}};
+
+PyModuleDef module = {PyModuleDef_HEAD_INIT, "gcb200_ext", "native front end of the reducers", -1, methods};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit_gcb200_ext() { return PyModule_Create(&module); }

@@ -209,6 +209,30 @@ def cuda():
     return _cuda
 
 
+_ext = None
+
+
+def ext():
+    """The extension module (``csrc/pyext.cpp``), bound to the loaded kernel library."""
+    global _ext
+    if _ext is None:
+        lib = cuda()
+        try:
+            path = _build.build_ext()      # no-op when up to date
+        except Exception as exc:
+            path = _build.ext_path()
+            if not os.path.exists(path):
+                raise NativeError(f"gcb200_ext.so is missing and could not be built: {exc}") from exc
+        import importlib.util
+
+        spec = importlib.util.spec_from_file_location("gcb200_ext", path)
+        mod = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(mod)
+        mod.bind({name: ctypes.cast(getattr(lib, name), c_void_p).value for name in mod.names()})
+        _ext = mod
+    return _ext
+
+
 _launches = 0
 
 

@@ -146,6 +146,9 @@ class FusedEngine:
         self.ops = None             # FusedOps of the family used last (what status checks look at)
         self._ops = {}              # family -> FusedOps
         self._n = 0
+        self.ext = None             # extension module, loaded with the first single-worker reduce
+        self.plan = None            # native view of the tensors a single worker's reduce was called with
+        self._solo = None           # (registry key, arena, handle) behind it
 
     @classmethod
     def for_reducer(cls, reducer):
@@ -161,17 +164,38 @@ class FusedEngine:
         if oneshot_region_bytes is None:
             # an owner that knows its largest gradient (a bucketed reducer: its largest bucket) says so, and the arena is
             # sized once instead of being replaced when a larger bucket shows up
-            family, nbytes = "twoshot", comm.required_bytes(max(n, int(getattr(self._owner, "fused_arena_elements", 0) or 0)))
+            # (a single worker has nobody to exchange a payload with: the header words are all its kernels use)
+            most = max(n, int(getattr(self._owner, "fused_arena_elements", 0) or 0)) if self._owner.n_workers > 1 else 0
+            family, nbytes = "twoshot", comm.required_bytes(most)
         else:
             family, nbytes = "oneshot", max(comm.oneshot_bytes(oneshot_region_bytes), ONESHOT_MIN_BYTES)
         arena = shared_arena(nbytes, self.device, self.group, family)
         ops = self._ops.get(family)
         if ops is None or ops.arena is not arena:
             ops = self._ops[family] = FusedOps(arena)
-        ops.max_blocks = int(getattr(self._owner, "fused_max_blocks", 0) or 0)
+        ops.max_blocks = self.max_blocks()
         self.ops = ops
         self._n = max(self._n, n)
         return ops
+
+    def max_blocks(self):
+        return int(getattr(self._owner, "fused_max_blocks", 0) or 0)
+
+    def solo_handle(self):
+        """Context handle for the single-worker kernels (``csrc/gc_solo.cu``): they need the header words of an arena, not its
+        payload.  The registry is asked every time, as another reducer may have had the arena replaced by a larger one.  None when
+        the engine's arena belongs to a group of several ranks."""
+        solo = self._solo
+        if solo is None or _shared_arena.get(solo[0]) is not solo[1]:
+            ops = self._ensure(0)
+            if ops.arena.ctxs[0].world != 1:
+                return None
+            if self.plan is None:
+                self.ext = nat.ext()
+                self.plan = self.ext.plan_new()
+            solo = self._solo = ((str(self.device), id(self.group), "twoshot"), ops.arena, ops.arena.ctxs[0].handle.value)
+        self.ops = self._ops["twoshot"]
+        return solo[2]
 
     def arenas(self):
         """Every arena this engine has launched on (status words to check, graphs to arm)."""
@@ -348,6 +372,33 @@ def _engine(reducer):
         eng = FusedEngine.for_reducer(reducer)
         reducer._fused = eng if eng is not None else False
     return eng or None
+
+
+def solo_maxnorm(reducer, grad_in, grad_out, bits_lo, bits_hi):
+    """A single worker's QSGD-MaxNorm reduce (``bits_hi``: two scales) on the tensors as they are: elements reduced, or None
+    where the tensors are not the kernels' case (other dtypes or layouts, more tensors than a table holds)."""
+    eng = reducer._fused or _engine(reducer)
+    handle, noise = eng.solo_handle(), reducer._noise
+    if handle is None:
+        return None
+    with reducer._timer("reduce.fused", verbosity=2):
+        n = eng.ext.solo_maxnorm(eng.plan, handle, grad_in, grad_out, bits_lo, bits_hi, noise.seed, noise.step, eng.ops.timeout_ms,
+                                 eng.max_blocks())
+    if n is not None:
+        noise.step += 1
+        nat.count_launch()
+    return n
+
+
+def solo_copy(reducer, grad_in, grad_out):
+    eng = reducer._fused or _engine(reducer)
+    handle = eng.solo_handle()
+    if handle is None:
+        return None
+    n = eng.ext.solo_copy(eng.plan, handle, grad_in, grad_out)
+    if n is not None:
+        nat.count_launch()
+    return n
 
 
 def allreduce_mean(reducer, flat, grad_out):

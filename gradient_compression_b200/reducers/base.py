@@ -107,9 +107,15 @@ def physical(t):
     return t
 
 
-def _physical_args(reduce_fn):
+def _physical_args(reduce_fn, solo_fn=None):
+    """``reduce_fn`` with its tensors in memory order.  ``solo_fn`` (the ``_solo_reduce`` of the class that defines
+    ``reduce_fn``) is asked first: a single worker's reduce straight on the lists, or None to take the general path."""
     @functools.wraps(reduce_fn)
     def reduce(self, grad_in, grad_out):
+        if solo_fn is not None and self.n_workers == 1 and self._use_fused():
+            bits = solo_fn(self, grad_in, grad_out)
+            if bits is not None:
+                return bits
         return reduce_fn(self, [physical(t) for t in grad_in], [physical(t) for t in grad_out])
 
     reduce._physical_wrapped = True
@@ -130,7 +136,7 @@ class Reducer:
         super().__init_subclass__(**kwargs)
         fn = cls.__dict__.get("reduce")
         if fn is not None and not getattr(fn, "_physical_wrapped", False):
-            cls.reduce = _physical_args(fn)         # every reduce() sees contiguous tensors in memory order
+            cls.reduce = _physical_args(fn, cls.__dict__.get("_solo_reduce"))   # reduce() sees contiguous tensors in memory order
 
     def __init__(self, device, timer=None, backend="auto", seed=0, group=None, reference_compat=False):
         if _dist_on():

@@ -3,6 +3,7 @@ from __future__ import annotations
 
 import torch
 
+from ..parallel import engine as fused
 from .base import Reducer, TensorBuffer, n_bits
 
 
@@ -11,6 +12,13 @@ class NoneAllReducer(Reducer):
 
     fused_capable = True
 
+    def _solo_reduce(self, grad_in, grad_out):
+        n = fused.solo_copy(self, grad_in, grad_out)
+        if n is None:
+            return None
+        self.last_wire_bits = 32 * n
+        return 32 * n
+
     def reduce(self, grad_in, grad_out):
         with self._timer("reduce.flat_pack"):
             flat = TensorBuffer(grad_in)
@@ -18,7 +26,6 @@ class NoneAllReducer(Reducer):
         self.last_wire_bits = bits
         with self._timer("reduce.allreduce", verbosity=2):
             if self._use_fused():
-                from ..parallel import engine as fused
                 if fused.allreduce_mean(self, flat, grad_out):
                     return bits
             self._all_reduce(flat.buffer)

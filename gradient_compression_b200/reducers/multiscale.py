@@ -6,6 +6,7 @@ import torch.distributed as dist
 
 from .. import compressors as C
 from .. import ops
+from ..parallel import engine as fused
 from .base import Reducer, TensorBuffer, n_bits
 from .qsgd import _write_flat
 
@@ -46,11 +47,15 @@ class QSGDMaxNormTwoScaleReducer(Reducer):
             out = self._compressor.decompress(max_norm, levels, mask, self.n_workers)
         return out, bits
 
+    def _solo_reduce(self, grad_in, grad_out):
+        lo = self._lower_quantization_level
+        n = fused.solo_maxnorm(self, grad_in, grad_out, lo, self._higher_quantization_level)
+        return None if n is None else 32 + 8 * n + (8 if lo < 8 else 32) * n
+
     def reduce(self, grad_in, grad_out):
         with self._timer("reduce.flat_pack"):
             flat = TensorBuffer(grad_in)
         if self._use_fused():
-            from ..parallel import engine as fused
             bits = fused.qsgd_twoscale(self, flat, grad_out)
             if bits is not None:
                 return bits
@@ -83,7 +88,6 @@ class QSGDMaxNormMultiScaleReducer(Reducer):
         with self._timer("reduce.flat_pack"):
             flat = TensorBuffer(grad_in)
         if self._use_fused():
-            from ..parallel import engine as fused
             bits = fused.qsgd_multiscale(self, flat, grad_out)
             if bits is not None:
                 return bits

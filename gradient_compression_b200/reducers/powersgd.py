@@ -16,6 +16,7 @@ import torch
 
 from .. import ops
 from ..ops import philox
+from ..parallel import engine as fused
 from .base import Reducer, TensorBuffer, n_bits
 
 
@@ -80,7 +81,6 @@ class RankKReducer(Reducer):
             if self._memory is None:
                 self._memory = torch.zeros_like(flat.buffer)
         if self._use_fused():
-            from ..parallel import engine as fused
             bits = fused.powersgd(self, flat, grad_out, plan, fresh)   # adds the error memory inside its first kernel
             if bits is not None:
                 self._step += 1

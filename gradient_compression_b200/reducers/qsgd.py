@@ -10,6 +10,7 @@ import torch
 
 from .. import compressors as C
 from .. import ops
+from ..parallel import engine as fused
 from .base import Reducer, TensorBuffer, n_bits
 
 
@@ -46,6 +47,16 @@ class _MaxNormReducer(Reducer):
         mb, pb = ops.packed_sizes(n, self._quantization_level)
         return 32 + 8 * (mb + pb)
 
+    def _solo_reduce(self, grad_in, grad_out):
+        if self.error_feedback:
+            return None
+        b = self._quantization_level
+        n = fused.solo_maxnorm(self, grad_in, grad_out, b, 0)
+        if n is None:
+            return None
+        self.last_wire_bits = self._wire_bits(n)
+        return 32 + (8 if b < 8 else 32) * n
+
     def reduce(self, grad_in, grad_out):
         with self._timer("reduce.flat_pack"):
             flat = TensorBuffer(grad_in)
@@ -56,7 +67,6 @@ class _MaxNormReducer(Reducer):
                 else:
                     flat.buffer.add_(self._memory)
         if self._use_fused() and not self.error_feedback:
-            from ..parallel import engine as fused
             bits = fused.qsgd_maxnorm(self, flat, grad_out)
             if bits is not None:
                 return bits

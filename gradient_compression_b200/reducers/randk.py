@@ -12,6 +12,7 @@ from __future__ import annotations
 
 from .. import compressors as C
 from .. import ops
+from ..parallel import engine as fused
 from .base import Reducer, TensorBuffer, n_bits
 from .multiscale import QSGDMaxNormTwoScaleReducer
 
@@ -74,7 +75,6 @@ class GlobalRandKMaxNormReducer(Reducer):
         n = flat.buffer.numel()
         start, k, npass = self._queue.next_window(n)
         if self._use_fused():
-            from ..parallel import engine as fused
             bits = fused.randk(self, flat, grad_out, start, k, npass)
             if bits is not None:
                 return bits

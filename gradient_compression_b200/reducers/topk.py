@@ -13,6 +13,7 @@ from __future__ import annotations
 import torch
 
 from ..ops.topk import TopKSelector
+from ..parallel import engine as fused
 from .base import Reducer, TensorBuffer
 
 
@@ -51,7 +52,6 @@ class _TopKBase(Reducer):
         bits = sel.total * (32 + self.position_bits)
         self.last_wire_bits = sel.total * 64
         if self._use_fused():
-            from ..parallel import engine as fused
             if fused.sparse(self, flat, grad_out, idx, vals):
                 return bits
         with self._timer("reduce.gather", verbosity=2):

@@ -17,7 +17,7 @@ from __future__ import annotations
 
 import json
 import time
-from contextlib import contextmanager
+from contextlib import contextmanager, nullcontext
 from io import StringIO
 
 import numpy as np
@@ -175,9 +175,10 @@ class Timer:
 class NullTimer(Timer):
     """A timer that measures nothing; used inside graph-captured or fused hot paths."""
 
+    _nothing = nullcontext()      # re-usable and re-entrant: entering it costs no generator
+
     def __init__(self):
         super().__init__(verbosity_level=-1, on_cuda=False, quiet=True)
 
-    @contextmanager
     def __call__(self, label, epoch=-1.0, verbosity=1):
-        yield
+        return self._nothing

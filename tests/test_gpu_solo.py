@@ -1,0 +1,76 @@
+"""Single-worker reducers on lists of tensors as they are: bit for bit what the same reducer computes on the CPU."""
+import pytest
+import torch
+
+from gradient_compression_b200 import make_reducer
+
+pytestmark = pytest.mark.gpu
+
+TILE = 4096        # elements of one tile of the segment kernels
+
+SIZES = {
+    "one": [1], "tail": [5], "tile": [TILE], "tile+1": [TILE + 1], "one-block": [4 * TILE], "two-blocks": [4 * TILE + 1],
+    "kept": [148 * TILE * 2 + 77], "re-read": [148 * TILE * 13 + 3],                        # beyond the tiles kept in shared memory
+    "many": [64, 3, 4097, 1, 10, 127, 36864, 2, 8191, 512 * 10], "odd starts": [1, TILE, 2, TILE, 3, TILE, 4 * TILE + 1],
+    "most": [7] * 320, "too many": [7] * 321,
+}
+
+
+def _values(sizes, seed):
+    gen = torch.Generator().manual_seed(seed)
+    return [torch.randn(n, generator=gen) * 10.0 ** (-(i % 3)) for i, n in enumerate(sizes)]
+
+
+def _on_gpu(host, layout):
+    """flat: views of one buffer (neighbours merge); separate: an allocation each; shifted: none of them 16-byte aligned."""
+    if layout == "flat":
+        buf, out, off = torch.cat(host).cuda(), [], 0
+        for t in host:
+            out.append(buf[off: off + t.numel()])
+            off += t.numel()
+        return out
+    if layout == "separate":
+        return [t.cuda() for t in host]
+    return [torch.cat([torch.zeros(1), t]).cuda()[1:] for t in host]
+
+
+@pytest.mark.parametrize("layout", ["flat", "separate", "shifted"])
+@pytest.mark.parametrize("sizes", list(SIZES))
+@pytest.mark.parametrize("name,config", [("QSGDMaxNormReducer", {"quantization_level": 8}), ("QSGDMaxNormReducer", {"quantization_level": 1}),
+                                         ("QSGDMaxNormTwoScaleReducer", {"quantization_level": 2, "higher_quantization_level": 6}),
+                                         ("NoneAllReducer", {})])
+def test_matches_the_cpu(name, config, sizes, layout):
+    host = _values(SIZES[sizes], 3)
+    send, outs = _on_gpu(host, layout), _on_gpu([torch.zeros_like(t) for t in host], layout)
+    cpu, gpu = (make_reducer(name, d, None, dict(config, seed=11)) for d in ("cpu", "cuda"))
+    for step in range(2):
+        in_place = step == 1
+        want = [torch.empty_like(t) for t in host]
+        bits = cpu.reduce([t.clone() for t in host], want)
+        got = send if in_place else outs
+        assert gpu.reduce(send, got) == bits
+        for w, g in zip(want, got):
+            assert torch.equal(w, g.cpu())
+
+
+@pytest.mark.parametrize("value", [0.0, float("nan"), float("inf"), -float("inf"), 1e-38])
+def test_special_values(value):
+    host = [torch.full((6,), value), torch.tensor([-1e-3, 0.5, value, -0.25])]
+    cpu, gpu = (make_reducer("QSGDMaxNormReducer", d, None, {"quantization_level": 4, "seed": 1}) for d in ("cpu", "cuda"))
+    want, got = [torch.empty_like(t) for t in host], [torch.empty_like(t).cuda() for t in host]
+    cpu.reduce([t.clone() for t in host], want)
+    gpu.reduce([t.cuda() for t in host], got)
+    for w, g in zip(want, got):
+        assert torch.equal(torch.nan_to_num(w, nan=7.0), torch.nan_to_num(g.cpu(), nan=7.0))
+
+
+def test_overlapping_tensors_take_the_general_path():
+    buf = torch.randn(64, device="cuda")
+    send, outs = [buf[:32].clone(), buf[8:40]], [buf[8:40], buf[40:72] if buf.numel() > 72 else torch.zeros(32, device="cuda")]
+    host = [t.cpu().clone() for t in send]
+    want = [torch.empty_like(t) for t in host]
+    cpu, gpu = (make_reducer("QSGDMaxNormReducer", d, None, {"quantization_level": 4, "seed": 1}) for d in ("cpu", "cuda"))
+    cpu.reduce([t.clone() for t in host], want)
+    gpu.reduce(send, outs)
+    for w, g in zip(want, outs):
+        assert torch.equal(w, g.cpu())
