@@ -97,20 +97,20 @@ struct SegCursor {
   // N further tiles at once, all of them whole (N <= run)
   template <int N>
   __device__ __forceinline__ void skip() {
-    tile += DIR * N;
+    tile += (uint32_t)(DIR * N);
     run -= N;
     in += DIR * N * 4 * SEG_TILE;
     out += DIR * N * 4 * SEG_TILE;
-    quad += (int64_t)DIR * N * SEG_TILE;
+    quad += (uint64_t)((int64_t)DIR * N * SEG_TILE);
   }
   __device__ __forceinline__ void step(const SegTable<CAP>& t) {
     if (DIR < 0 && tile == 0) return;
-    tile += DIR;
+    tile += (uint32_t)DIR;
     if (run > 0) {
       --run;
       in += DIR * 4 * SEG_TILE;
       out += DIR * 4 * SEG_TILE;
-      quad += (int64_t)DIR * SEG_TILE;
+      quad += (uint64_t)((int64_t)DIR * SEG_TILE);
       return;
     }
     if (tile >= t.tile0[t.n]) return;

@@ -1,195 +1,603 @@
-// Top-K selection by |value| for many segments (tensors) of one flat buffer at once: exact radix select on
-// the IEEE bit pattern of |a| (3 passes of 11 + 11 + 10 bits), then compaction into (index, value) lists.
-// Error feedback is fused: pass 0 forms a = g + e and stores it in e; compaction zeroes the selected
-// entries of e, so afterwards e is exactly the memory the reference keeps (reducer.py:1161,1186-1189), and
-// the reference's per-tensor torch.topk calls (reducer.py:1180; 161 launches + sorts for ResNet-50) become
-// 7 launches that each stream the gradient once.
-// Segment table: int64 rows of {start, len, k, out_off, chunk_start, 0}.
+// Top-K selection by |value| for many tensors at once (reference: reducer.py:1144-1451, there one torch.topk per tensor), with
+// the error feedback folded in: a = g + e; the k largest |a| of every group are selected; e becomes a with the selected
+// entries zeroed.  A group is one tensor, or all of them together.
+//
+//   topk_fold_kernel     a = g + e -> e, and a histogram of the top 13 bits of |a| per group                 (12 bytes an element)
+//   topk_pick_kernel     per group: the bin that holds the k-th largest (groups of up to 4096 elements: the whole selection)
+//   topk_split_kernel    above that bin: selected.  In it: put on the group's candidate list.  Below: not selected.
+//   topk_refine_kernel   per group: exact selection among the candidates by the remaining 18 bits, in two steps of 9
+//
+// Two outputs.  LISTS (several workers): index and value of the selected entries, for the exchange.  DENSE (a single
+// worker, whose exchange is the identity): the selected entries in an otherwise zero gradient, written by the split
+// kernel where it reads, straight into the gradient tensors.
+//
+// What bounds it: fold reads g and e and writes e, split reads e and writes the gradient: 20 bytes an element against the 16 no
+// implementation can avoid.  Thirteen bits (five of the mantissa, so a bin spans three percent in value) make that second
+// reading the last one: a bin near the threshold holds about 0.2 % of normally distributed values (some percent once error
+// feedback has piled values up below it), few enough for a cluster of blocks per group to finish.  Split walks the tiles backwards: what fold wrote last is read from L2.  Counts and
+// candidates are gathered in shared memory and leave it in one atomic per warp and some hundred entries.
+// Groups whose bin holds more candidates than their list has room for (one value repeated over much of a tensor) are
+// refined by reading the tensor again instead (split then leaves the error memory to refine, which still has to tell the
+// selected entries from the candidates).
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
 #include "gc_device.cuh"
+#include "gc_segs.cuh"
 
 using namespace gc;
+namespace cg = cooperative_groups;
 
 namespace {
 
-constexpr int SEG_FIELDS = 6;
-constexpr int CHUNK = 4096;
-constexpr int BINS = 2048;
-constexpr int TK_THREADS = 256;
+constexpr int THREADS = SEG_TILE;
+constexpr int WARPS = THREADS / 32;
+constexpr int LOW_BITS = 18, HIGH_BITS = 13;
+constexpr int BINS = 1 << HIGH_BITS;
+constexpr int SMALL = 4 * THREADS;         // groups of at most this many elements are selected from by one block, in registers
+constexpr int WARP_ROOM = 256;             // candidates a warp holds back; a quad per lane adds at most 128
+constexpr int SUB_BITS = 9, SUB_BINS = 1 << SUB_BITS;
 
-struct SegState {          // per segment, device resident
-  uint32_t prefix;         // selected high bits so far
-  int32_t k_rem;           // how many still to take among the elements that match the prefix
-  uint32_t gt_count;       // compaction: slots handed to keys > threshold
-  uint32_t eq_count;       // compaction: keys == threshold seen
+struct GroupState {        // device resident, all zero between runs except what pick writes
+  int32_t bin;             // -1: everything is selected
+  int32_t k_rem;           // how many of the bin's entries are selected
+  uint32_t in_bin;         // entries in the bin
+  uint32_t taken;          // LISTS: slots handed to selected entries
+  uint32_t listed;         // candidates on the list
+  uint32_t pad[3];
 };
 
-__device__ __forceinline__ int find_seg(const int64_t* __restrict__ tab, int n_seg, int64_t chunk) {
-  int lo = 0, hi = n_seg - 1;
-  while (lo < hi) {
-    int mid = (lo + hi + 1) >> 1;
-    if (tab[(int64_t)mid * SEG_FIELDS + 4] <= chunk) lo = mid; else hi = mid - 1;
-  }
-  return lo;
-}
+struct Cand {
+  float a;
+  int32_t at;
+  __device__ __forceinline__ uint32_t key() const { return __float_as_uint(a) & 0x7fffffffu; }
+};
+
+template <int CAP>
+struct TopkParams {
+  SegTable<CAP> t;
+  int k[CAP];              // per group
+  int64_t room0[CAP + 1];  // candidate lists: first entry per group
+  int64_t slot0[CAP];      // LISTS: first output slot per group
+  uint16_t large[CAP];     // groups of more than SMALL elements
+  int n_groups, n_large, per_tensor;
+  float* e;                // error memory by flat element (nullptr: none, a = g)
+  GroupState* state;
+  uint32_t* hist;
+  Cand* cands;
+  int32_t* out_idx;
+  float* out_val;
+  __device__ __forceinline__ int group(int s) const { return CAP == 1 || per_tensor ? s : 0; }
+  __device__ __forceinline__ bool small(int g) const { return per_tensor && t.start[g + 1] - t.start[g] <= SMALL; }
+  __device__ __forceinline__ int64_t len(int g) const { return per_tensor ? t.start[g + 1] - t.start[g] : t.start[t.n] - t.start[0]; }
+};
 
 __device__ __forceinline__ uint32_t key_of(float a) { return __float_as_uint(a) & 0x7fffffffu; }
 
-// pass: 0, 1, 2.  Pass 0 also folds the error memory: e <- g + e.
-template <int PASS>
-__global__ void __launch_bounds__(TK_THREADS) topk_hist_kernel(const float* __restrict__ g, float* __restrict__ e,
-                                                               const int64_t* __restrict__ tab, int n_seg,
-                                                               const SegState* __restrict__ state,
-                                                               uint32_t* __restrict__ hist) {
-  __shared__ uint32_t sh[BINS];
-  int seg = find_seg(tab, n_seg, (int64_t)blockIdx.x);
-  const int64_t* t = tab + (int64_t)seg * SEG_FIELDS;
-  int64_t start = t[0], len = t[1], k = t[2];
-  int64_t c0 = ((int64_t)blockIdx.x - t[4]) * CHUNK;
-  int64_t c1 = c0 + CHUNK < len ? c0 + CHUNK : len;
-  bool skip = k >= len;       // everything is taken: no threshold needed
-  for (int i = threadIdx.x; i < BINS; i += TK_THREADS) sh[i] = 0;
+template <int CAP>
+__device__ __forceinline__ void fold_flush(const TopkParams<CAP>& p, uint32_t* sh, int g) {
   __syncthreads();
-  uint32_t prefix = PASS == 0 ? 0u : state[seg].prefix;
-  for (int64_t i = c0 + threadIdx.x; i < c1; i += TK_THREADS) {
-    float a;
-    if (PASS == 0) {
-      a = g[start + i] + (e != nullptr ? e[start + i] : 0.0f);
-      if (e != nullptr) e[start + i] = a;
-    } else {
-      a = e != nullptr ? e[start + i] : g[start + i];
-    }
-    if (skip) continue;
-    uint32_t key = key_of(a);
-    if (PASS == 0) atomicAdd(&sh[key >> 21], 1u);
-    else if (PASS == 1) { if ((key >> 21) == prefix) atomicAdd(&sh[(key >> 10) & 0x7ffu], 1u); }
-    else { if ((key >> 10) == prefix) atomicAdd(&sh[key & 0x3ffu], 1u); }
-  }
+  for (int i = threadIdx.x; i < BINS; i += THREADS)
+    if (sh[i]) { atomicAdd(&p.hist[(int64_t)g * BINS + i], sh[i]); sh[i] = 0; }
   __syncthreads();
-  if (skip) return;
-  for (int i = threadIdx.x; i < BINS; i += TK_THREADS)
-    if (sh[i]) atomicAdd(&hist[(int64_t)seg * BINS + i], sh[i]);
 }
 
-// One block per segment: pick the bin that holds the k_rem-th largest key, refine prefix / k_rem, clear hist.
-template <int PASS>
-__global__ void __launch_bounds__(TK_THREADS) topk_select_kernel(const int64_t* __restrict__ tab, SegState* __restrict__ state,
-                                                                 uint32_t* __restrict__ hist) {
-  __shared__ uint32_t part[TK_THREADS];
-  __shared__ int chosen;
-  __shared__ uint32_t above;
-  int seg = blockIdx.x;
-  const int64_t* t = tab + (int64_t)seg * SEG_FIELDS;
-  int64_t len = t[1], k = t[2];
-  uint32_t* h = hist + (int64_t)seg * BINS;
-  constexpr int PER = BINS / TK_THREADS;     // 8 consecutive bins per thread, thread 0 owns the TOP bins
-  int top = BINS - 1 - threadIdx.x * PER;
+// a quad of which only elements [a, b) belong to the tensor
+__device__ __forceinline__ void quad_store_part(float* p, const float4& v, int a, int b) {
+  if (b - a == 4 && (reinterpret_cast<uintptr_t>(p) & 15u) == 0) { *reinterpret_cast<float4*>(p) = v; return; }
+  if (a <= 0 && b > 0) p[0] = v.x;
+  if (a <= 1 && b > 1) p[1] = v.y;
+  if (a <= 2 && b > 2) p[2] = v.z;
+  if (a <= 3 && b > 3) p[3] = v.w;
+}
+__device__ __forceinline__ float4 quad_load_part(const float* p, int a, int b) {
+  if (b - a == 4 && (reinterpret_cast<uintptr_t>(p) & 15u) == 0) return __ldcg(reinterpret_cast<const float4*>(p));
+  float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (a <= 0 && b > 0) v.x = p[0];
+  if (a <= 1 && b > 1) v.y = p[1];
+  if (a <= 2 && b > 2) v.z = p[2];
+  if (a <= 3 && b > 3) v.w = p[3];
+  return v;
+}
+
+template <int CAP>
+__global__ void __launch_bounds__(THREADS, 1) topk_fold_kernel(const __grid_constant__ TopkParams<CAP> p) {
+  __shared__ uint32_t sh[BINS];
+  const SegTable<CAP>& t = p.t;
+  for (int i = threadIdx.x; i < BINS; i += THREADS) sh[i] = 0;
+  __syncthreads();
+  const uint32_t tiles = t.tile0[t.n], per = (tiles + gridDim.x - 1) / gridDim.x, first = blockIdx.x * per;
+  if (first >= tiles) return;
+  uint32_t left = tiles - first < per ? tiles - first : per;
+  auto count = [&](const float4& a) {
+    atomicAdd(&sh[key_of(a.x) >> LOW_BITS], 1u);
+    atomicAdd(&sh[key_of(a.y) >> LOW_BITS], 1u);
+    atomicAdd(&sh[key_of(a.z) >> LOW_BITS], 1u);
+    atomicAdd(&sh[key_of(a.w) >> LOW_BITS], 1u);
+  };
+  const bool mem = p.e != nullptr, al_e = (reinterpret_cast<uintptr_t>(p.e) & 15u) == 0;
+  SegCursor<CAP, 1> c(t, first);
+  int g = p.group(c.s);
+  while (left > 0) {
+    if (p.group(c.s) != g) { fold_flush(p, sh, g); g = p.group(c.s); }
+    const bool counts = p.k[g] < p.len(g) && !p.small(g);          // (everything is selected: no threshold to find)
+    if (left >= 4 && c.fast_in && al_e && c.run >= 3) {
+      // four whole tiles at a time: 128 KB in flight per SM
+      float4 a[4];
+      float4* e = reinterpret_cast<float4*>(p.e) + c.quad;
+#pragma unroll
+      for (int u = 0; u < 4; ++u) a[u] = __ldcs(reinterpret_cast<const float4*>(c.in) + u * SEG_TILE);
+      if (mem) {
+        float4 b[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) b[u] = __ldcg(e + u * SEG_TILE);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          a[u].x += b[u].x; a[u].y += b[u].y; a[u].z += b[u].z; a[u].w += b[u].w;
+          e[u * SEG_TILE] = a[u];
+        }
+      }
+      if (counts) {
+#pragma unroll
+        for (int u = 0; u < 4; ++u) count(a[u]);
+      }
+      left -= 4;
+      c.template skip<3>();
+      if (left > 0) c.step(t);
+      continue;
+    }
+    if (!c.empty(t)) {
+      const int a0 = c.whole ? 0 : c.first(t), b0 = c.whole ? 4 : c.last(t);
+      float4 a = c.load(t);
+      if (mem) {
+        float* e = p.e + c.quad * 4;
+        const float4 b = quad_load_part(e, a0, b0);
+        a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w;
+        quad_store_part(e, a, a0, b0);
+      }
+      if (counts) {
+        if (b0 - a0 == 4) count(a);
+        else {
+          const float v[4] = {a.x, a.y, a.z, a.w};
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            if (j >= a0 && j < b0) atomicAdd(&sh[key_of(v[j]) >> LOW_BITS], 1u);
+        }
+      }
+    }
+    --left;
+    if (left > 0) c.step(t);
+  }
+  fold_flush(p, sh, g);
+}
+
+// Thread i of the block holds sum; returns the total of the threads before it.
+__device__ __forceinline__ uint32_t block_exclusive(uint32_t sum, uint32_t* warp_sums) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  uint32_t incl = sum;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t up = __shfl_up_sync(FULL, incl, o);
+    if (lane >= o) incl += up;
+  }
+  __syncthreads();
+  if (lane == 31) warp_sums[wid] = incl;
+  __syncthreads();
+  if (wid == 0) {
+    uint32_t w = lane < (int)(blockDim.x >> 5) ? warp_sums[lane] : 0u, s = w;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t up = __shfl_up_sync(FULL, s, o);
+      if (lane >= o) s += up;
+    }
+    warp_sums[lane] = s - w;
+  }
+  __syncthreads();
+  return warp_sums[wid] + incl - sum;
+}
+
+// Appends to the output lists, `n` entries per call of a warp's lanes (n is 0 or 1 per lane).
+template <int CAP>
+__device__ __forceinline__ void list_take(const TopkParams<CAP>& p, int g, bool take, int64_t at, float a) {
+  const unsigned m = __ballot_sync(FULL, take);
+  if (m == 0) return;
+  const int lane = threadIdx.x & 31;
+  uint32_t base = 0;
+  if (lane == 0) base = atomicAdd(&p.state[g].taken, (uint32_t)__popc(m));
+  base = __shfl_sync(FULL, base, 0);
+  if (take) {
+    const int64_t slot = p.slot0[g] + base + __popc(m & ((1u << lane) - 1u));
+    p.out_idx[slot] = (int32_t)at;
+    p.out_val[slot] = a;
+  }
+}
+
+// A small group, whole: its elements in registers, the threshold found eight bits at a time.
+template <int CAP, bool LISTS>
+__device__ __forceinline__ void select_small(const TopkParams<CAP>& p, int g, uint32_t* hist, uint32_t* warp_sums, int* found) {
+  const SegTable<CAP>& t = p.t;
+  const int64_t lo = t.start[g], len = t.start[g + 1] - lo, k = p.k[g];
+  float v[4];
+  uint32_t key[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const int64_t i = threadIdx.x + j * THREADS;
+    v[j] = i < len ? (p.e != nullptr ? p.e[lo + i] : t.in[g][i]) : 0.0f;
+    key[j] = key_of(v[j]);
+  }
+  uint32_t prefix = 0;
+  int rem = (int)k;
+  if (k < len) {
+#pragma unroll
+    for (int part = 0; part < 4; ++part) {             // 8 + 8 + 8 + 7 bits
+      const int shift = part == 3 ? 0 : 23 - 8 * part, bits = part == 3 ? 7 : 8;
+      if (threadIdx.x < 256) hist[threadIdx.x] = 0;
+      __syncthreads();
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (threadIdx.x + j * THREADS < len && (part == 0 || (key[j] >> (shift + bits)) == prefix)) atomicAdd(&hist[(key[j] >> shift) & ((1u << bits) - 1u)], 1u);
+      __syncthreads();
+      const uint32_t mine = threadIdx.x < 256 ? hist[255 - threadIdx.x] : 0u;
+      const uint32_t above = block_exclusive(mine, warp_sums);
+      if (above < (uint32_t)rem && above + mine >= (uint32_t)rem) { found[0] = 255 - threadIdx.x; found[1] = rem - (int)above; }
+      __syncthreads();
+      prefix = (prefix << bits) | (uint32_t)found[0];
+      rem = found[1];
+      __syncthreads();
+    }
+  }
+  if (threadIdx.x == 0) found[0] = 0;                  // entries equal to the threshold taken so far
+  __syncthreads();
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const int64_t i = threadIdx.x + j * THREADS;
+    bool take = i < len && k > 0 && (k >= len || key[j] > prefix);
+    if (i < len && k > 0 && k < len && key[j] == prefix) take = atomicAdd(found, 1) < rem;
+    if (LISTS) list_take(p, g, take, lo + i, v[j]);
+    else if (i < len) t.out[g][i] = take ? v[j] : 0.0f;
+    if (take && p.e != nullptr) p.e[lo + i] = 0.0f;
+  }
+}
+
+// One block per group; thread 0 owns the top bins.
+template <int CAP, bool LISTS>
+__global__ void __launch_bounds__(THREADS) topk_pick_kernel(const __grid_constant__ TopkParams<CAP> p) {
+  __shared__ uint32_t warp_sums[32], hist[256];
+  __shared__ int found[2];
+  const int g = blockIdx.x;
+  const int64_t k = p.k[g], len = p.len(g);
+  GroupState* st = p.state + g;
+  if (threadIdx.x == 0) { st->taken = 0; st->listed = 0; }
+  __syncthreads();
+  if (p.small(g)) { select_small<CAP, LISTS>(p, g, hist, warp_sums, found); return; }
+  constexpr int PER = BINS / THREADS;
+  const int top = BINS - 1 - threadIdx.x * PER;
+  uint32_t* h = p.hist + (int64_t)g * BINS + (top - PER + 1);
   uint32_t local[PER], sum = 0;
 #pragma unroll
-  for (int j = 0; j < PER; ++j) { local[j] = h[top - j]; sum += local[j]; h[top - j] = 0; }
-  part[threadIdx.x] = sum;
-  if (threadIdx.x == 0) { chosen = -1; above = 0; }
-  __syncthreads();
-  if (k >= len) {
-    if (threadIdx.x == 0 && PASS == 0) { state[seg].prefix = 0; state[seg].k_rem = (int32_t)k; state[seg].gt_count = 0; state[seg].eq_count = 0; }
+  for (int j = 0; j < PER; j += 4) {
+    const uint4 v = *reinterpret_cast<const uint4*>(h + j);
+    *reinterpret_cast<uint4*>(h + j) = make_uint4(0, 0, 0, 0);
+    local[j] = v.x; local[j + 1] = v.y; local[j + 2] = v.z; local[j + 3] = v.w;
+    sum += v.x + v.y + v.z + v.w;
+  }
+  if (k >= len || k <= 0) {
+    if (threadIdx.x == 0) { st->bin = k <= 0 ? BINS : -1; st->k_rem = 0; st->in_bin = 0; }
     return;
   }
-  // exclusive prefix over threads (= number of keys in higher bins than this thread's first bin)
-  uint32_t excl = 0;
-  for (int i = 0; i < (int)threadIdx.x; ++i) excl += part[i];
-  int32_t k_rem = PASS == 0 ? (int32_t)k : state[seg].k_rem;
-  uint32_t run = excl;
+  uint32_t run = block_exclusive(sum, warp_sums);
 #pragma unroll
-  for (int j = 0; j < PER; ++j) {
-    if (run < (uint32_t)k_rem && run + local[j] >= (uint32_t)k_rem) { chosen = top - j; above = run; }
+  for (int j = PER - 1; j >= 0; --j) {               // local[PER - 1] is this thread's top bin
+    if (run < (uint32_t)k && run + local[j] >= (uint32_t)k) {
+      st->bin = top - (PER - 1) + j;
+      st->k_rem = (int32_t)((uint32_t)k - run);
+      st->in_bin = local[j];
+    }
     run += local[j];
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int b = chosen < 0 ? 0 : chosen;
-    uint32_t prev = PASS == 0 ? 0u : state[seg].prefix;
-    state[seg].prefix = PASS == 0 ? (uint32_t)b : (PASS == 1 ? ((prev << 11) | (uint32_t)b) : ((prev << 10) | (uint32_t)b));
-    state[seg].k_rem = k_rem - (int32_t)above;
-    if (PASS == 0) { state[seg].gt_count = 0; state[seg].eq_count = 0; }
   }
 }
 
-// Compaction: (global index, value) of the selected entries -> out lists; selected entries of e are zeroed.
-__global__ void __launch_bounds__(TK_THREADS) topk_compact_kernel(const float* __restrict__ g, float* __restrict__ e,
-                                                                  const int64_t* __restrict__ tab, int n_seg,
-                                                                  SegState* __restrict__ state, int32_t* __restrict__ out_idx,
-                                                                  float* __restrict__ out_val) {
-  int seg = find_seg(tab, n_seg, (int64_t)blockIdx.x);
-  const int64_t* t = tab + (int64_t)seg * SEG_FIELDS;
-  int64_t start = t[0], len = t[1], k = t[2], out_off = t[3];
-  int64_t c0 = ((int64_t)blockIdx.x - t[4]) * CHUNK;
-  int64_t c1 = c0 + CHUNK < len ? c0 + CHUNK : len;
-  bool all = k >= len;
-  uint32_t thr = state[seg].prefix;
-  int32_t need_eq = state[seg].k_rem;
-  int64_t n_gt = k - need_eq;
+template <int CAP, bool LISTS>
+__global__ void __launch_bounds__(THREADS, 1) topk_split_kernel(const __grid_constant__ TopkParams<CAP> p) {
+  extern __shared__ Cand held_all[];       // [WARPS][WARP_ROOM]
+  __shared__ int held_count[WARPS];
+  const SegTable<CAP>& t = p.t;
   const int lane = threadIdx.x & 31;
-  for (int64_t ib = c0; ib < c1; ib += TK_THREADS) {       // uniform trip count: the ballots below need whole warps
-    int64_t i = ib + threadIdx.x;
-    bool valid = i < c1;
-    float a = 0.f;
-    if (valid) a = e != nullptr ? e[start + i] : g[start + i];
-    int64_t slot = -1;
-    if (all) {
-      if (valid) slot = i;
-    } else {
-      uint32_t key = key_of(a);
-      bool gt = valid && key > thr, eq = valid && key == thr;
-      // warp-aggregated slot allocation: one atomic per warp and class instead of one per selected element
-      unsigned mgt = __ballot_sync(0xffffffffu, gt), meq = __ballot_sync(0xffffffffu, eq);
-      uint32_t base_gt = 0, base_eq = 0;
-      if (lane == 0) {
-        if (mgt) base_gt = atomicAdd(&state[seg].gt_count, (uint32_t)__popc(mgt));
-        if (meq) base_eq = atomicAdd(&state[seg].eq_count, (uint32_t)__popc(meq));
-      }
-      base_gt = __shfl_sync(0xffffffffu, base_gt, 0);
-      base_eq = __shfl_sync(0xffffffffu, base_eq, 0);
-      unsigned below = (1u << lane) - 1u;
-      if (gt) slot = (int64_t)base_gt + __popc(mgt & below);
-      else if (eq) {
-        uint32_t q = base_eq + (uint32_t)__popc(meq & below);
-        if ((int32_t)q < need_eq) slot = n_gt + q;
-      }
+  Cand* held = held_all + (threadIdx.x >> 5) * WARP_ROOM;
+  int* count = held_count + (threadIdx.x >> 5);
+  if (lane == 0) *count = 0;
+  __syncwarp();
+  const uint32_t tiles = t.tile0[t.n], per = (tiles + gridDim.x - 1) / gridDim.x, first = blockIdx.x * per;
+  if (first >= tiles) return;
+  uint32_t left = tiles - first < per ? tiles - first : per;
+  const bool mem = p.e != nullptr, al_e = (reinterpret_cast<uintptr_t>(p.e) & 15u) == 0;
+
+  auto flush = [&](int g) {
+    __syncwarp();
+    const int n = *count;
+    if (n > 0) {
+      uint32_t base = 0;
+      if (lane == 0) base = atomicAdd(&p.state[g].listed, (uint32_t)n);
+      base = __shfl_sync(FULL, base, 0);
+      Cand* list = p.cands + p.room0[g] + base;
+      for (int i = lane; i < n; i += 32) list[i] = held[i];          // fits: the bin's count was checked against the room
     }
-    if (slot >= 0) {
-      out_idx[out_off + slot] = (int32_t)(start + i);
-      out_val[out_off + slot] = a;
-      if (e != nullptr) e[start + i] = 0.0f;
+    __syncwarp();
+    if (lane == 0) *count = 0;
+    __syncwarp();
+  };
+  int g = -1;
+  uint32_t from = 0, above = 0;              // keys of the bin: [from, above)
+  bool listing = false;
+  // one quad: a (elements [a0, b0) of it) at flat element `at`; y: what goes into the gradient; true when `a` changed
+  auto quad = [&](float4& a, int64_t at, int a0, int b0, float4& y) {
+    float* v = &a.x;
+    float* o = &y.x;
+    uint32_t key[4];
+    unsigned cand = 0;
+    bool changed = false;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      key[j] = key_of(v[j]);
+      const bool mine = j >= a0 && j < b0;
+      const bool sure = mine && key[j] >= above;
+      if (mine && !sure && key[j] >= from) cand |= 1u << j;
+      if (LISTS) list_take(p, g, sure, at + j, v[j]);
+      o[j] = sure ? v[j] : 0.0f;
+      changed = changed || sure;
     }
+    if (changed && listing) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (o[j] != 0.0f) v[j] = 0.0f;       // (a selected zero is a zero either way)
+    }
+    if (listing && __any_sync(FULL, cand != 0)) {
+      if (cand != 0) {
+        int to = atomicAdd(count, __popc(cand));
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          if ((cand >> j) & 1u) held[to++] = Cand{v[j], (int32_t)(at + j)};
+      }
+      __syncwarp();
+      if (*count > WARP_ROOM - 128) flush(g);
+    }
+    return changed && listing;
+  };
+
+  SegCursor<CAP, -1> c(t, first + left - 1);
+  while (left > 0) {
+    if (p.group(c.s) != g) {
+      if (g >= 0) flush(g);
+      g = p.group(c.s);
+      if (p.small(g)) {                      // done by the pick kernel
+        g = -1;
+        if (--left > 0) c.step(t);
+        continue;
+      }
+      const int bin = p.state[g].bin;                                 // -1: everything is above it
+      from = bin < 0 ? 0u : (uint32_t)bin << LOW_BITS;
+      above = (uint32_t)(bin + 1) << LOW_BITS;
+      listing = (int64_t)p.state[g].in_bin <= p.room0[g + 1] - p.room0[g];
+    }
+    if (left >= 4 && c.fast_in && (LISTS || c.fast_out) && al_e && c.run >= 3) {
+      float4 a[4];
+      const float4* src = mem ? reinterpret_cast<const float4*>(p.e) + c.quad : reinterpret_cast<const float4*>(c.in);
+#pragma unroll
+      for (int u = 0; u < 4; ++u) a[u] = __ldcg(src - u * SEG_TILE);
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        float4 y;
+        const bool changed = quad(a[u], (int64_t)(c.quad - u * SEG_TILE) * 4, 0, 4, y);
+        if (mem && changed) *(reinterpret_cast<float4*>(p.e) + c.quad - u * SEG_TILE) = a[u];
+        if (!LISTS) __stcs(reinterpret_cast<float4*>(c.out) - u * SEG_TILE, y);
+      }
+      left -= 4;
+      c.template skip<3>();
+      if (left > 0) c.step(t);
+      continue;
+    }
+    {
+      const int a0 = c.whole ? 0 : c.first(t), b0 = c.whole ? 4 : c.last(t);
+      float* e = p.e + c.quad * 4;
+      float4 a = mem ? quad_load_part(e, a0, b0) : (a0 < b0 ? c.load(t) : make_float4(0.f, 0.f, 0.f, 0.f));
+      float4 y;
+      const bool changed = quad(a, (int64_t)c.quad * 4, a0, b0, y);
+      if (mem && changed) quad_store_part(e, a, a0, b0);
+      if (!LISTS && a0 < b0) c.store(t, y);
+    }
+    --left;
+    if (left > 0) c.step(t);
   }
+  if (g >= 0) flush(g);
+}
+
+// One cluster of blocks per group; the blocks share the group's candidates and add their counts up in rank 0's shared memory.
+template <int CAP, bool LISTS>
+__global__ void __launch_bounds__(THREADS) topk_refine_kernel(const __grid_constant__ TopkParams<CAP> p) {
+  __shared__ uint32_t hist[SUB_BINS], warp_sums[32];
+  __shared__ int chosen, need;
+  __shared__ uint32_t equal_seen;
+  cg::cluster_group cluster = cg::this_cluster();
+  const unsigned rank = cluster.block_rank(), ranks = cluster.num_blocks();
+  const SegTable<CAP>& t = p.t;
+  const int g = p.large[blockIdx.x / ranks];
+  GroupState* st = p.state + g;
+  const int k_rem = st->k_rem;
+  const uint32_t in_bin = st->in_bin;
+  if (k_rem <= 0) return;                  // (the whole cluster)
+  const int bin = st->bin;
+  const bool listed = (int64_t)in_bin <= p.room0[g + 1] - p.room0[g];
+  const int64_t lo = p.per_tensor ? t.start[g] : t.start[0];
+  const int64_t count = listed ? (int64_t)in_bin : p.len(g);
+  const int64_t from = (int64_t)rank * THREADS, stride = (int64_t)ranks * THREADS;
+  const Cand* list = p.cands + p.room0[g];
+  // entry i of the list; without one, element i of the group
+  auto entry = [&](int64_t i) {
+    if (listed) return list[i];
+    const int64_t at = lo + i;
+    if (p.e != nullptr) return Cand{p.e[at], (int32_t)at};
+    const int s = seg_of_elem(t, at);
+    return Cand{t.in[s][at - t.start[s]], (int32_t)at};
+  };
+  auto in_it = [&](const Cand& c) { return listed || (int)(c.key() >> LOW_BITS) == bin; };
+  uint32_t prefix = 0;
+  int rem = k_rem;
+  const bool all = (uint32_t)k_rem >= in_bin;
+  if (threadIdx.x == 0) equal_seen = 0;
+  if (!all) {
+#pragma unroll
+    for (int part = 0; part < 2; ++part) {
+      if (threadIdx.x < SUB_BINS) hist[threadIdx.x] = 0;
+      __syncthreads();
+      auto tally = [&](const Cand& c) {
+        const uint32_t low = c.key() & ((1u << LOW_BITS) - 1u);
+        if (part == 0) atomicAdd(&hist[low >> SUB_BITS], 1u);
+        else if ((low >> SUB_BITS) == prefix) atomicAdd(&hist[low & (SUB_BINS - 1)], 1u);
+      };
+      int64_t i = from + threadIdx.x;
+      if (listed)
+        for (; i + 3 * stride < count; i += 4 * stride) {
+          const Cand c0 = list[i], c1 = list[i + stride], c2 = list[i + 2 * stride], c3 = list[i + 3 * stride];
+          tally(c0); tally(c1); tally(c2); tally(c3);
+        }
+      for (; i < count; i += stride) {
+        const Cand c = entry(i);
+        if (in_it(c)) tally(c);
+      }
+      cluster.sync();
+      if (rank != 0 && threadIdx.x < SUB_BINS && hist[threadIdx.x]) atomicAdd(cluster.map_shared_rank(&hist[threadIdx.x], 0), hist[threadIdx.x]);
+      cluster.sync();
+      if (rank == 0) {
+        const uint32_t mine = threadIdx.x < SUB_BINS ? hist[SUB_BINS - 1 - threadIdx.x] : 0u;
+        const uint32_t above = block_exclusive(mine, warp_sums);
+        if (above < (uint32_t)rem && above + mine >= (uint32_t)rem) { chosen = SUB_BINS - 1 - threadIdx.x; need = rem - (int)above; }
+      }
+      cluster.sync();
+      const uint32_t got = (uint32_t)*cluster.map_shared_rank(&chosen, 0);
+      prefix = part == 0 ? got : (prefix << SUB_BITS) | got;
+      rem = *cluster.map_shared_rank(&need, 0);
+      cluster.sync();
+    }
+  } else {
+    cluster.sync();
+  }
+  uint32_t* equal = cluster.map_shared_rank(&equal_seen, 0);
+  auto settle = [&](const Cand& c, bool there) {
+    const bool valid = there && in_it(c), taken = there && !listed && (int)(c.key() >> LOW_BITS) > bin;
+    const uint32_t low = c.key() & ((1u << LOW_BITS) - 1u);
+    bool take = valid && (all || low > prefix);
+    if (valid && !all && low == prefix) take = (int)atomicAdd(equal, 1u) < rem;
+    if (LISTS) list_take(p, g, take, c.at, c.a);
+    if (take && !LISTS) {
+      const int s = p.per_tensor ? g : seg_of_elem(t, (int64_t)c.at);
+      t.out[s][c.at - t.start[s]] = c.a;
+    }
+    if ((take || taken) && p.e != nullptr) p.e[c.at] = 0.0f;
+  };
+  int64_t base = from;
+  for (; listed && base + 3 * stride + THREADS <= count; base += 4 * stride) {
+    const Cand* l = list + base + threadIdx.x;
+    const Cand c0 = l[0], c1 = l[stride], c2 = l[2 * stride], c3 = l[3 * stride];
+    settle(c0, true); settle(c1, true); settle(c2, true); settle(c3, true);
+  }
+  for (; base < count; base += stride) {
+    const bool there = base + threadIdx.x < count;
+    settle(there ? entry(base + threadIdx.x) : Cand{0.0f, 0}, there);
+  }
+  cluster.sync();                          // rank 0's shared memory stays until every block is done with it
+}
+
+int64_t list_room(int64_t len) { return len / 8 + 1024; }
+
+template <int CAP>
+int run(const SegDesc* segs, int n_seg, int64_t end, const int64_t* k, int per_tensor, float* e, void* state, void* list, int32_t* out_idx, float* out_val,
+        cudaStream_t st) {
+  TopkParams<CAP> p;
+  if (!seg_table(p.t, segs, n_seg, end)) return (int)cudaErrorInvalidValue;
+  if (p.t.tile0[n_seg] == 0) return 0;
+  p.n_groups = per_tensor ? n_seg : 1;
+  p.per_tensor = per_tensor || n_seg == 1;
+  p.n_large = 0;
+  int64_t room = 0, slot = 0, longest = 0;
+  for (int g = 0; g < p.n_groups; ++g) {
+    const int64_t len = p.per_tensor ? p.t.start[g + 1] - p.t.start[g] : end - p.t.start[0];
+    const int64_t kk = k[g] < len ? k[g] : len;
+    p.k[g] = (int)kk;
+    p.room0[g] = room;
+    p.slot0[g] = slot;
+    room += list_room(len);
+    longest = len > longest ? len : longest;
+    if (!p.per_tensor || len > SMALL) p.large[p.n_large++] = (uint16_t)g;
+    slot += kk;
+  }
+  p.room0[p.n_groups] = room;
+  p.e = e;
+  p.state = (GroupState*)state;
+  p.hist = (uint32_t*)((uint8_t*)state + (int64_t)p.n_groups * sizeof(GroupState));
+  p.cands = (Cand*)list;
+  p.out_idx = out_idx;
+  p.out_val = out_val;
+  int dev = 0, sms = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const uint32_t tiles = p.t.tile0[n_seg];
+  const unsigned grid = tiles < (uint32_t)sms ? tiles : (unsigned)sms;
+  constexpr int held = WARPS * WARP_ROOM * (int)sizeof(Cand);
+  const bool lists = out_idx != nullptr;
+  const void* split = lists ? (const void*)topk_split_kernel<CAP, true> : (const void*)topk_split_kernel<CAP, false>;
+  cudaError_t err = cudaFuncSetAttribute(split, cudaFuncAttributeMaxDynamicSharedMemorySize, held);
+  if (err != cudaSuccess) return (int)err;
+  topk_fold_kernel<CAP><<<grid, THREADS, 0, st>>>(p);
+  if (lists) topk_pick_kernel<CAP, true><<<p.n_groups, THREADS, 0, st>>>(p);
+  else topk_pick_kernel<CAP, false><<<p.n_groups, THREADS, 0, st>>>(p);
+  if (p.n_large == 0) return (int)cudaGetLastError();
+  void* args[1] = {&p};
+  err = cudaLaunchKernel(split, dim3(grid), dim3(THREADS), args, held, st);
+  if (err != cudaSuccess) return (int)err;
+  // Blocks per group: what the longest group can fill with a few thousand candidates each (with error feedback, values pile up
+  // below the threshold and the bin holds some percent of the group), as long as all groups fit on the chip at once, two blocks
+  // an SM; clusters of sixteen only for a few groups, as they take whole GPU clusters to place (ResNet-50's 55 groups: 23 us
+  // with eight blocks each, 48 us with sixteen; one group of 64 M elements: 210 us with eight, 84 us with sixteen).
+  int ranks = 1;
+  while (ranks < (p.n_large <= 4 ? 16 : 8) && longest / 32 > (int64_t)ranks * 4 * THREADS && p.n_large * ranks * 2 <= 2 * sms) ranks *= 2;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(p.n_large * ranks));
+  cfg.blockDim = dim3(THREADS);
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)ranks;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  if (ranks > 8) {
+    const void* refine = lists ? (const void*)topk_refine_kernel<CAP, true> : (const void*)topk_refine_kernel<CAP, false>;
+    err = cudaFuncSetAttribute(refine, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (err != cudaSuccess) return (int)err;
+  }
+  return (int)(lists ? cudaLaunchKernelEx(&cfg, topk_refine_kernel<CAP, true>, p) : cudaLaunchKernelEx(&cfg, topk_refine_kernel<CAP, false>, p));
 }
 
 }  // namespace
 
 extern "C" {
 
-int64_t gc_cuda_topk_state_bytes(int n_seg) { return (int64_t)n_seg * (sizeof(SegState) + BINS * 4); }
-int gc_cuda_topk_chunk() { return CHUNK; }
+// Tensors one run takes.
+int gc_cuda_topk_max_segs() { return SEG_CAP_MANY; }
+// Scratch of a run: state is zeroed once after allocation (every run leaves it ready for the next), lists need no initialisation.
+int64_t gc_cuda_topk_state_bytes(int n_groups) { return (int64_t)n_groups * ((int64_t)sizeof(GroupState) + BINS * 4); }
+int64_t gc_cuda_topk_list_bytes(int64_t len) { return list_room(len) * (int64_t)sizeof(Cand); }
 
-// g: gradient (read only); e: error memory (updated in place; NULL = no error feedback, selection on g).
-// state: gc_cuda_topk_state_bytes(n_seg) bytes, zeroed once after allocation.  out_idx / out_val: sum of k entries.
-int gc_cuda_topk_select(const float* g, float* e, const int64_t* tab, int n_seg, int64_t total_chunks, void* state_,
-                        int32_t* out_idx, float* out_val, void* cs) {
-  if (n_seg <= 0 || total_chunks <= 0) return 0;
-  cudaStream_t st = (cudaStream_t)cs;
-  SegState* state = (SegState*)state_;
-  uint32_t* hist = (uint32_t*)((uint8_t*)state_ + (int64_t)n_seg * sizeof(SegState));
-  unsigned grid = (unsigned)total_chunks;
-  topk_hist_kernel<0><<<grid, TK_THREADS, 0, st>>>(g, e, tab, n_seg, state, hist);
-  topk_select_kernel<0><<<n_seg, TK_THREADS, 0, st>>>(tab, state, hist);
-  topk_hist_kernel<1><<<grid, TK_THREADS, 0, st>>>(g, e, tab, n_seg, state, hist);
-  topk_select_kernel<1><<<n_seg, TK_THREADS, 0, st>>>(tab, state, hist);
-  topk_hist_kernel<2><<<grid, TK_THREADS, 0, st>>>(g, e, tab, n_seg, state, hist);
-  topk_select_kernel<2><<<n_seg, TK_THREADS, 0, st>>>(tab, state, hist);
-  topk_compact_kernel<<<grid, TK_THREADS, 0, st>>>(g, e, tab, n_seg, state, out_idx, out_val);
-  return (int)cudaGetLastError();
+// segs: n_seg SegDesc, consecutive in the flat vector, the last one ending at flat element `end`.  k: one count per group
+// (per_tensor: a group per segment, otherwise one group).  e: error memory by flat element (NULL: selection on g itself).
+// out_idx / out_val: sum of k entries, group after group; NULL: the selected entries go into the segments' outputs, which
+// are zero elsewhere.
+int gc_cuda_topk_run(const void* segs, int n_seg, int64_t end, const int64_t* k, int per_tensor, float* e, void* state, void* list, int32_t* out_idx,
+                     float* out_val, void* cs) {
+  if (n_seg < 1 || n_seg > SEG_CAP_MANY || end > 0x7fffffffll) return (int)cudaErrorInvalidValue;
+  if (n_seg == 1) return run<1>((const SegDesc*)segs, 1, end, k, per_tensor, e, state, list, out_idx, out_val, (cudaStream_t)cs);
+  return run<SEG_CAP_MANY>((const SegDesc*)segs, n_seg, end, k, per_tensor, e, state, list, out_idx, out_val, (cudaStream_t)cs);
 }
 
 }  // extern "C"

@@ -32,6 +32,7 @@ struct Api {
   int (*solo_max_segs)();
   int (*solo_maxnorm)(void*, const void*, int, int64_t, int, int, uint64_t, uint32_t, int, int, void*);
   int (*solo_copy)(void*, const void*, int, int64_t, void*);
+  int (*topk_run)(const void*, int, int64_t, const int64_t*, int, float*, void*, void*, int32_t*, float*, void*);
 } api;
 int max_segs = 0;
 
@@ -40,13 +41,16 @@ const Entry entries[] = {
     {"gc_solo_max_segs", (void**)&api.solo_max_segs},
     {"gc_solo_maxnorm", (void**)&api.solo_maxnorm},
     {"gc_solo_copy", (void**)&api.solo_copy},
+    {"gc_cuda_topk_run", (void**)&api.topk_run},
 };
 
 // What one reducer saw last: its segment table, and the fact that its inputs and outputs do not overlap in an unsafe way
 // (checked once per set of addresses).
 struct Plan {
   std::vector<SegDesc> segs, checked;
+  std::vector<int64_t> starts;     // the sizes behind `generation`
   int64_t n = 0;
+  int64_t generation = 0;          // counts changes of the tensors' sizes
   int device = -1;
 };
 
@@ -96,7 +100,8 @@ bool overlap_free(const std::vector<SegDesc>& segs, int64_t n) {
 }
 
 // Fills the plan from two lists of tensors.  False: not a case for the segment kernels (the caller takes the general path).
-bool collect(Plan& p, PyObject* ins, PyObject* outs) {
+// `merge`: neighbours in memory become one segment (otherwise a segment per non-empty tensor).
+bool collect(Plan& p, PyObject* ins, PyObject* outs, bool merge = true) {
   PyObject* fa = PySequence_Fast(ins, "reduce() takes lists of tensors");
   if (!fa) return false;
   PyObject* fb = ins == outs ? (Py_INCREF(fa), fa) : PySequence_Fast(outs, "reduce() takes lists of tensors");
@@ -118,7 +123,7 @@ bool collect(Plan& p, PyObject* ins, PyObject* outs) {
     if (a == nullptr || b == nullptr || na != nb || da != db || oa != ob || (p.device >= 0 && da != p.device)) { ok = false; break; }
     if (oa == 1 && pa != pb && THPVariable_Unpack(pa).sizes() != THPVariable_Unpack(pb).sizes()) { ok = false; break; }
     p.device = da;
-    if (!p.segs.empty()) {
+    if (merge && !p.segs.empty()) {
       const SegDesc& last = p.segs.back();
       const int64_t len = p.n - last.start;
       if (a == last.in + len && b == last.out + len) { p.n += na; continue; }
@@ -191,6 +196,38 @@ PyObject* solo_copy(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   return PyLong_FromLongLong(p->n);
 }
 
+// collect(plan, grad_in, grad_out, merge) -> (elements, generation of the tensors' sizes), or None
+PyObject* collect_py(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
+  if (!want(nargs, 4, "collect")) return nullptr;
+  Plan* p = plan_of(a[0]);
+  if (!p) return nullptr;
+  if (!collect(*p, a[1], a[2], PyObject_IsTrue(a[3]) == 1)) { if (PyErr_Occurred()) return nullptr; Py_RETURN_NONE; }
+  bool same = p->starts.size() == p->segs.size() + 1 && p->starts.back() == p->n;
+  for (size_t i = 0; same && i < p->segs.size(); ++i) same = p->starts[i] == p->segs[i].start;
+  if (!same) {
+    p->starts.clear();
+    for (const SegDesc& s : p->segs) p->starts.push_back(s.start);
+    p->starts.push_back(p->n);
+    ++p->generation;
+  }
+  return Py_BuildValue("LL", (long long)p->n, (long long)p->generation);
+}
+
+// solo_topk(plan, counts (address of int64 per group), per_tensor, memory, state, lists: addresses): on what collect() found
+PyObject* solo_topk(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
+  if (!want(nargs, 6, "solo_topk")) return nullptr;
+  Plan* p = plan_of(a[0]);
+  if (!p) return nullptr;
+  uint64_t v[6] = {};
+  for (int i = 1; i < 6; ++i) v[i] = PyLong_AsUnsignedLongLong(a[i]);
+  if (PyErr_Occurred()) return nullptr;
+  c10::cuda::OptionalCUDAGuard guard(c10::Device(c10::kCUDA, (c10::DeviceIndex)p->device));
+  const int err = api.topk_run(p->segs.data(), (int)p->segs.size(), p->n, (const int64_t*)v[1], (int)v[2], (float*)v[3], (void*)v[4], (void*)v[5], nullptr,
+                               nullptr, stream_on(p->device));
+  if (err) return cuda_error("solo_topk", err);
+  Py_RETURN_NONE;
+}
+
 // bind({name: address}): the kernel library's entry points
 PyObject* bind(PyObject*, PyObject* table) {
   for (const Entry& e : entries) {
@@ -219,6 +256,8 @@ PyMethodDef methods[] = {
     {"plan_new", plan_new, METH_NOARGS, "plan_new() -> a plan, one per reducer"},
     {"solo_maxnorm", (PyCFunction)(void (*)(void))solo_maxnorm, METH_FASTCALL, "QSGD-MaxNorm reduce of a single worker"},
     {"solo_copy", (PyCFunction)(void (*)(void))solo_copy, METH_FASTCALL, "plain mean of a single worker"},
+    {"collect", (PyCFunction)(void (*)(void))collect_py, METH_FASTCALL, "reads two lists of tensors into a plan"},
+    {"solo_topk", (PyCFunction)(void (*)(void))solo_topk, METH_FASTCALL, "top-k with error feedback of a single worker"},
     {nullptr, nullptr, 0, nullptr}};
 
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "gcb200_ext", "native front end of the reducers", -1, methods};

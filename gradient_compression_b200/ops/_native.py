@@ -23,6 +23,12 @@ class NativeError(RuntimeError):
     pass
 
 
+class SegDesc(ctypes.Structure):
+    """One tensor of a segment table (``SegDesc`` in ``csrc/gc_segs.cuh``)."""
+
+    _fields_ = [("inp", ctypes.c_void_p), ("out", ctypes.c_void_p), ("start", ctypes.c_int64)]
+
+
 class BnFinArgs(ctypes.Structure):
     """Host-side argument block of the GEMM / convolution kernels that finish batch-norm statistics themselves
     (``BnFinHost`` in ``csrc/gc_tc.cuh``)."""
@@ -143,9 +149,10 @@ def cuda():
         _declare(lib, "gc_cuda_psgd_q_blocks", c_i64, [c_int, c_int])
         _declare(lib, "gc_cuda_psgd_q", c_int, [P, P, c_int, c_i64, P, P, c_i64, c_int, P])
         _declare(lib, "gc_cuda_psgd_out", c_int, [P, P, P, c_int, c_i64, P, P, P, c_int, P, c_float, P])
+        _declare(lib, "gc_cuda_topk_max_segs", c_int, [])
         _declare(lib, "gc_cuda_topk_state_bytes", c_i64, [c_int])
-        _declare(lib, "gc_cuda_topk_chunk", c_int, [])
-        _declare(lib, "gc_cuda_topk_select", c_int, [P, P, P, c_int, c_i64, P, P, P, P])
+        _declare(lib, "gc_cuda_topk_list_bytes", c_i64, [c_i64])
+        _declare(lib, "gc_cuda_topk_run", c_int, [P, c_int, c_i64, P, c_int, P, P, P, P, P, P])
         _declare(lib, "gc_cuda_batched_transpose", c_int, [P, c_int, c_i64, P])
         _declare(lib, "gc_cuda_gemm_tf32_supported", c_int, [P, P, c_int, c_int, c_int, c_i64, c_i64])
         _declare(lib, "gc_cuda_gemm_tf32", c_int, [P, P, P, P, c_int, c_int, c_int, c_i64, c_i64, c_i64, c_int, P, P, P, P])

@@ -401,6 +401,19 @@ def solo_copy(reducer, grad_in, grad_out):
     return n
 
 
+def solo_collect(reducer, grad_in, grad_out, merge):
+    """Reads a single worker's tensors into the engine's plan for one of the calls below: (elements, generation of the tensors'
+    sizes), or None."""
+    eng = reducer._fused or _engine(reducer)
+    return None if eng.solo_handle() is None else eng.ext.collect(eng.plan, grad_in, grad_out, merge)
+
+
+def solo_topk(reducer, counts, per_tensor, memory, scratch):
+    eng = reducer._fused
+    eng.ext.solo_topk(eng.plan, counts.data_ptr(), int(per_tensor), memory.data_ptr(), scratch.state.data_ptr(), scratch.lists.data_ptr())
+    nat.count_launch(4)
+
+
 def allreduce_mean(reducer, flat, grad_out):
     eng = _engine(reducer)
     return eng.allreduce_mean(reducer, flat, grad_out) if eng else False

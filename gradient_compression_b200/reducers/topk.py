@@ -5,14 +5,15 @@ into segments (one per tensor, or one for everything) and in how K is derived.  
 ``a = g + memory``; per segment the K largest |a| are selected; ``memory = a`` with the selected entries
 zeroed; every worker's (index, value) list reaches every other worker and the mean of the scattered
 contributions becomes the gradient.  On CUDA the selection is the batched radix select of ``ops.topk``
-(7 launches for any number of tensors); with the fused backend the exchange + scatter-add is one kernel
-over peer memory, otherwise two all-gathers and ``index_add_``.
+(4 launches for up to 320 tensors); with the fused backend the exchange + scatter-add is one kernel
+over peer memory, otherwise two all-gathers and ``index_add_``.  A single worker has nothing to exchange: the selection
+kernels write the sparse gradient themselves.
 """
 from __future__ import annotations
 
 import torch
 
-from ..ops.topk import TopKSelector
+from ..ops.topk import TopKScratch, TopKSelector
 from ..parallel import engine as fused
 from .base import Reducer, TensorBuffer
 
@@ -27,6 +28,7 @@ class _TopKBase(Reducer):
         self._memory = None
         self._selector = None
         self._selector_key = None
+        self._solo = None           # single worker: (generation of the tensors' sizes, counts, scratch, total)
 
     def _top_size(self, numel):
         raise NotImplementedError
@@ -40,6 +42,25 @@ class _TopKBase(Reducer):
                 segs = [(0, flat.total, self._top_size(flat.total))]
             self._selector, self._selector_key = TopKSelector(segs, flat.buffer.device), key
         return self._selector
+
+    def _solo_reduce(self, grad_in, grad_out):
+        found = fused.solo_collect(self, grad_in, grad_out, not self.layerwise)
+        if found is None:
+            return None
+        n, generation = found
+        if self._memory is None:
+            self._memory = torch.zeros(n, device=self._device)
+        if self._memory.numel() != n or not self._memory.is_contiguous():
+            return None
+        if self._solo is None or self._solo[0] != generation:
+            lengths = [t.numel() for t in grad_in if t.numel()] if self.layerwise else [n]
+            counts = torch.tensor([min(self._top_size(m), m) for m in lengths], dtype=torch.int64)
+            self._solo = (generation, counts, TopKScratch(lengths, self._device), int(counts.sum()))
+        _, counts, scratch, total = self._solo
+        with self._timer("reduce.topk", verbosity=2):
+            fused.solo_topk(self, counts, self.layerwise, self._memory, scratch)
+        self.last_wire_bits = total * 64
+        return total * (32 + self.position_bits)
 
     def reduce(self, grad_in, grad_out):
         with self._timer("reduce.flat_pack"):
@@ -114,6 +135,9 @@ class GlobalTopKReducer(_TopKBase):
 
     def _top_size(self, numel):
         return min(numel, self._K)
+
+    def _solo_reduce(self, grad_in, grad_out):
+        return None if self._compat else super()._solo_reduce(grad_in, grad_out)
 
     def reduce(self, grad_in, grad_out):
         if not self._compat:

@@ -74,3 +74,67 @@ def test_overlapping_tensors_take_the_general_path():
     gpu.reduce(send, outs)
     for w, g in zip(want, outs):
         assert torch.equal(w, g.cpu())
+
+
+def _topk_values(kind, sizes):
+    host = _values(sizes, 5)
+    if kind == "zeros":             # more entries asked for than differ from zero
+        return [torch.where(torch.arange(t.numel()) % 211 == 3, t, torch.zeros(())) for t in host]
+    if kind == "constant":          # one bin holds everything: no room on the candidate lists
+        return [torch.full_like(t, 0.25) for t in host]
+    if kind == "tiny":              # subnormals: the lowest bin, with larger entries above it
+        return [torch.where(torch.arange(t.numel()) % 301 == 7, t, t * 1e-39) for t in host]
+    if kind == "close":             # one bin, all different
+        return [1.0 + t * 1e-4 for t in host]
+    return host
+
+
+@pytest.mark.parametrize("layout", ["flat", "separate", "shifted"])
+@pytest.mark.parametrize("sizes", ["one", "tile+1", "two-blocks", "kept", "many", "odd starts", "most", "too many"])
+@pytest.mark.parametrize("kind", ["normal", "zeros", "constant", "tiny", "close"])
+@pytest.mark.parametrize("name,config", [("TopKReducerRatio", {"compression": 0.01}), ("TopKReducer", {"K": 60}), ("GlobalTopKReducer", {"K": 500})])
+def test_topk(name, config, kind, sizes, layout):
+    host = _topk_values(kind, SIZES[sizes])
+    red = make_reducer(name, "cuda", None, config)
+    groups = host if name != "GlobalTopKReducer" else [torch.cat(host)]
+    mem = [torch.zeros_like(t) for t in groups]
+    for step in range(2):
+        send = _on_gpu([t * (1 + step) for t in host], layout)
+        outs = send if step else _on_gpu([torch.full_like(t, 9.0) for t in host], layout)
+        assert red.reduce(send, outs) == sum(red._top_size(t.numel()) for t in groups) * (32 + red.position_bits)
+        flat_out = torch.cat([t.cpu() for t in outs])
+        got = flat_out.split([t.numel() for t in groups])
+        now = red.state_dict()["memory"].cpu().split([t.numel() for t in groups])
+        for t, o, e, e_before in zip(groups, got, now, mem):
+            a = t * (1 + step) + e_before
+            k = red._top_size(t.numel())
+            assert torch.equal(o + e, a) and not ((o != 0) & (e != 0)).any()
+            threshold = torch.topk(a.abs(), k)[0][-1]
+            assert (o != 0).sum() == min(k, int((a != 0).sum()))
+            assert (o[o != 0].abs() >= threshold).all() and (e.abs() <= threshold).all()
+        mem = now
+
+
+@pytest.mark.parametrize("kind", ["normal", "zeros", "constant", "tiny"])
+@pytest.mark.parametrize("memory", [False, True])
+def test_topk_lists(kind, memory):
+    from gradient_compression_b200.ops.topk import TopKSelector
+
+    host = _topk_values(kind, SIZES["many"] + [200003])
+    a, segs, off = torch.cat(host), [], 0
+    for t in host:
+        segs.append((off, t.numel(), max(1, t.numel() // 50)))
+        off += t.numel()
+    sel = TopKSelector(segs, "cuda")
+    for _ in range(2):
+        e = torch.zeros(off, device="cuda") if memory else None
+        idx, val = (t.cpu() for t in sel.select(a.cuda(), e))
+        assert torch.equal(val, a[idx.long()]) and idx.unique().numel() == idx.numel()
+        for (s, n, k), o in zip(sel.segments, sel.offsets):
+            mine = idx[o: o + k].long()
+            assert ((mine >= s) & (mine < s + n)).all()
+            assert (a[mine].abs() >= torch.topk(a[s: s + n].abs(), k)[0][-1]).all()
+        if memory:
+            want = a.clone()
+            want[idx.long()] = 0
+            assert torch.equal(e.cpu(), want)
