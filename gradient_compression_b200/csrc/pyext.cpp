@@ -33,6 +33,8 @@ struct Api {
   int (*solo_maxnorm)(void*, const void*, int, int64_t, int, int, uint64_t, uint32_t, int, int, void*);
   int (*solo_copy)(void*, const void*, int, int64_t, void*);
   int (*topk_run)(const void*, int, int64_t, const int64_t*, int, float*, void*, void*, int32_t*, float*, void*);
+  int (*psgd_solo)(int, const void*, int, float*, const int64_t*, int, int64_t, int64_t, int, const int64_t*, int, float*, float*, float*, int64_t, uint64_t,
+                   uint32_t, uint32_t*, void*);
 } api;
 int max_segs = 0;
 
@@ -42,15 +44,16 @@ const Entry entries[] = {
     {"gc_solo_maxnorm", (void**)&api.solo_maxnorm},
     {"gc_solo_copy", (void**)&api.solo_copy},
     {"gc_cuda_topk_run", (void**)&api.topk_run},
+    {"gc_cuda_psgd_solo", (void**)&api.psgd_solo},
 };
 
 // What one reducer saw last: its segment table, and the fact that its inputs and outputs do not overlap in an unsafe way
 // (checked once per set of addresses).
 struct Plan {
   std::vector<SegDesc> segs, checked;
-  std::vector<int64_t> starts;     // the sizes behind `generation`
+  std::vector<int64_t> shape, shape_seen;     // dimensions, first extent and elements of every tensor
   int64_t n = 0;
-  int64_t generation = 0;          // counts changes of the tensors' sizes
+  int64_t generation = 0;          // counts changes of the tensors' shapes
   int device = -1;
 };
 
@@ -109,6 +112,7 @@ bool collect(Plan& p, PyObject* ins, PyObject* outs, bool merge = true) {
   const Py_ssize_t k = PySequence_Fast_GET_SIZE(fa);
   bool ok = k > 0 && PySequence_Fast_GET_SIZE(fb) == k;
   p.segs.clear();
+  p.shape.clear();
   p.n = 0;
   p.device = -1;
   for (Py_ssize_t i = 0; ok && i < k; ++i) {
@@ -119,6 +123,14 @@ bool collect(Plan& p, PyObject* ins, PyObject* outs, bool merge = true) {
     float* b = a;
     if (pa == pb) { nb = na; db = da; ob = oa; }
     else b = dense_ptr(pb, &nb, &db, &ob);
+    if (a != nullptr || na == 0) {
+      if (THPVariable_Check(pa)) {
+        const at::Tensor& t = THPVariable_Unpack(pa);
+        p.shape.push_back(t.dim());
+        p.shape.push_back(t.dim() > 0 ? t.size(0) : 1);
+        p.shape.push_back(na);
+      }
+    }
     if (na == 0 && nb == 0 && THPVariable_Check(pa) && THPVariable_Check(pb)) continue;
     if (a == nullptr || b == nullptr || na != nb || da != db || oa != ob || (p.device >= 0 && da != p.device)) { ok = false; break; }
     if (oa == 1 && pa != pb && THPVariable_Unpack(pa).sizes() != THPVariable_Unpack(pb).sizes()) { ok = false; break; }
@@ -196,21 +208,38 @@ PyObject* solo_copy(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   return PyLong_FromLongLong(p->n);
 }
 
-// collect(plan, grad_in, grad_out, merge) -> (elements, generation of the tensors' sizes), or None
+// collect(plan, grad_in, grad_out, merge) -> (elements, generation of the tensors' shapes, segments), or None.
+// merge: 1 neighbours become one segment, 0 a segment per tensor, 2 one segment if all of them are neighbours, else one per tensor
 PyObject* collect_py(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   if (!want(nargs, 4, "collect")) return nullptr;
   Plan* p = plan_of(a[0]);
   if (!p) return nullptr;
-  if (!collect(*p, a[1], a[2], PyObject_IsTrue(a[3]) == 1)) { if (PyErr_Occurred()) return nullptr; Py_RETURN_NONE; }
-  bool same = p->starts.size() == p->segs.size() + 1 && p->starts.back() == p->n;
-  for (size_t i = 0; same && i < p->segs.size(); ++i) same = p->starts[i] == p->segs[i].start;
-  if (!same) {
-    p->starts.clear();
-    for (const SegDesc& s : p->segs) p->starts.push_back(s.start);
-    p->starts.push_back(p->n);
+  const int merge = (int)as_int(a[3]);
+  bool ok = collect(*p, a[1], a[2], merge != 0);
+  if (ok && merge == 2 && p->segs.size() > 1) ok = collect(*p, a[1], a[2], false);
+  if (!ok) { if (PyErr_Occurred()) return nullptr; Py_RETURN_NONE; }
+  if (p->shape != p->shape_seen) {
+    p->shape_seen = p->shape;
     ++p->generation;
   }
-  return Py_BuildValue("LL", (long long)p->n, (long long)p->generation);
+  return Py_BuildValue("LLn", (long long)p->n, (long long)p->generation, (Py_ssize_t)p->segs.size());
+}
+
+// solo_psgd(plan, rank, memory, tab, n_mats, rows, tiles, max_rows, vtab, n_vecs, q, p, q_parts, q_total, seed, stream, step or 0)
+PyObject* solo_psgd(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
+  if (!want(nargs, 17, "solo_psgd")) return nullptr;
+  Plan* p = plan_of(a[0]);
+  if (!p) return nullptr;
+  const int rank = (int)as_int(a[1]);
+  uint64_t v[16] = {};
+  for (int i = 1; i < 16; ++i) v[i] = i == 13 ? PyLong_AsUnsignedLongLongMask(a[i + 1]) : PyLong_AsUnsignedLongLong(a[i + 1]);
+  if (PyErr_Occurred()) return nullptr;
+  c10::cuda::OptionalCUDAGuard guard(c10::Device(c10::kCUDA, (c10::DeviceIndex)p->device));
+  const int err = api.psgd_solo(rank, p->segs.data(), (int)p->segs.size(), (float*)v[1], (const int64_t*)v[2], (int)v[3], (int64_t)v[4], (int64_t)v[5], (int)v[6],
+                                (const int64_t*)v[7], (int)v[8], (float*)v[9], (float*)v[10], (float*)v[11], (int64_t)v[12], v[13], (uint32_t)v[14],
+                                (uint32_t*)v[15], stream_on(p->device));
+  if (err) return cuda_error("solo_psgd", err);
+  Py_RETURN_NONE;
 }
 
 // solo_topk(plan, counts (address of int64 per group), per_tensor, memory, state, lists: addresses): on what collect() found
@@ -257,6 +286,7 @@ PyMethodDef methods[] = {
     {"solo_maxnorm", (PyCFunction)(void (*)(void))solo_maxnorm, METH_FASTCALL, "QSGD-MaxNorm reduce of a single worker"},
     {"solo_copy", (PyCFunction)(void (*)(void))solo_copy, METH_FASTCALL, "plain mean of a single worker"},
     {"collect", (PyCFunction)(void (*)(void))collect_py, METH_FASTCALL, "reads two lists of tensors into a plan"},
+    {"solo_psgd", (PyCFunction)(void (*)(void))solo_psgd, METH_FASTCALL, "PowerSGD step of a single worker"},
     {"solo_topk", (PyCFunction)(void (*)(void))solo_topk, METH_FASTCALL, "top-k with error feedback of a single worker"},
     {nullptr, nullptr, 0, nullptr}};
 

@@ -143,12 +143,14 @@ def cuda():
         _declare(lib, "gc_cuda_head_forward", c_int, [P, c_int, c_int, c_int, P, P, c_int, P, P, P, P, P, P, P])
         _declare(lib, "gc_cuda_head_backward", c_int, [P, P, P, P, c_int, c_int, c_int, c_int, P, P, P, P])
         _declare(lib, "gc_cuda_psgd_max_rank", c_int, [])
-        _declare(lib, "gc_cuda_psgd_p", c_int, [P, P, P, c_int, c_i64, P, P, P, c_int, c_i64, P])
+        _declare(lib, "gc_cuda_psgd_p", c_int, [c_int, P, P, P, c_int, c_i64, P, P, P, c_int, c_i64, P])
         _declare(lib, "gc_cuda_psgd_gs", c_int, [P, P, c_int, c_float, P])
         _declare(lib, "gc_cuda_psgd_q_chunks", c_int, [c_int])
         _declare(lib, "gc_cuda_psgd_q_blocks", c_i64, [c_int, c_int])
-        _declare(lib, "gc_cuda_psgd_q", c_int, [P, P, c_int, c_i64, P, P, c_i64, c_int, P])
-        _declare(lib, "gc_cuda_psgd_out", c_int, [P, P, P, c_int, c_i64, P, P, P, c_int, P, c_float, P])
+        _declare(lib, "gc_cuda_psgd_q", c_int, [c_int, P, P, c_int, c_i64, P, P, c_i64, c_int, P])
+        _declare(lib, "gc_cuda_psgd_out", c_int, [c_int, P, P, P, c_int, c_i64, P, P, P, c_int, P, c_float, P])
+        _declare(lib, "gc_cuda_psgd_row_blocks", c_i64, [c_int, c_int])
+        _declare(lib, "gc_cuda_psgd_solo", c_int, [c_int, P, c_int, P, P, c_int, c_i64, c_i64, c_int, P, c_int, P, P, P, c_i64, c_u64, c_u32, P, P])
         _declare(lib, "gc_cuda_topk_max_segs", c_int, [])
         _declare(lib, "gc_cuda_topk_state_bytes", c_i64, [c_int])
         _declare(lib, "gc_cuda_topk_list_bytes", c_i64, [c_i64])

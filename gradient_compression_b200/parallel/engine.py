@@ -292,19 +292,19 @@ class FusedEngine:
             return cache
         rows, tiles, mats = 0, 0, []
         for (i, n, m, r, po, qo) in plan["hi"]:
-            mats.append([flat._start_idx[i], n, m, r, po, qo, rows, tiles])
-            rows += n
+            mats.append([flat._start_idx[i], n, m, r, po, qo, rows, tiles, 0])
+            rows += int(nat.cuda().gc_cuda_psgd_row_blocks(n, m))
             tiles += int(nat.cuda().gc_cuda_psgd_q_blocks(n, m))        # 128-column tiles x row chunks of this matrix
         vecs, voff = [], 0
         for i in plan["lo"]:
             ln = flat._end_idx[i] - flat._start_idx[i]
-            vecs.append([flat._start_idx[i], ln, voff])
+            vecs.append([flat._start_idx[i], ln, voff, 0])
             voff += ln
         dev = flat.buffer.device
         cache = {"key": plan["key"], "rows": rows, "tiles": tiles, "n_mats": len(mats), "n_vecs": len(vecs),
                  "v_total": voff,
-                 "tab": torch.tensor(mats or [[0] * 8], dtype=torch.int64, device=dev),
-                 "vtab": torch.tensor(vecs or [[0] * 3], dtype=torch.int64, device=dev),
+                 "tab": torch.tensor(mats or [[0] * 9], dtype=torch.int64, device=dev),
+                 "vtab": torch.tensor(vecs or [[0] * 4], dtype=torch.int64, device=dev),
                  "stage": torch.zeros(plan["p_total"] + voff, device=dev),       # zeroed: the alignment gaps are never written
                  "reduced": torch.zeros(plan["p_total"] + voff, device=dev),
                  "max_rows": max([n for (_, n, _, _, _, _) in plan["hi"]] or [1]),
@@ -335,7 +335,7 @@ class FusedEngine:
         st = nat.stream_ptr
         with torch.cuda.device(g.device):
             with reducer._timer("reduce.compute.p", verbosity=2):
-                nat.check(lib.gc_cuda_psgd_p(g.data_ptr(), e.data_ptr(), c["tab"].data_ptr(), c["n_mats"], c["rows"],
+                nat.check(lib.gc_cuda_psgd_p(reducer.rank_r, g.data_ptr(), e.data_ptr(), c["tab"].data_ptr(), c["n_mats"], c["rows"],
                                              reducer.q_memory.data_ptr(), c["stage"].data_ptr(), c["vtab"].data_ptr(),
                                              c["n_vecs"], p_total, st()), "psgd_p")
             with reducer._timer("reduce.p", verbosity=2):
@@ -344,14 +344,14 @@ class FusedEngine:
                 nat.check(lib.gc_cuda_psgd_gs(c["reduced"].data_ptr(), c["tab"].data_ptr(), c["n_mats"], 1e-8, st()),
                           "psgd_gs")
             with reducer._timer("reduce.compute.q", verbosity=2):
-                nat.check(lib.gc_cuda_psgd_q(e.data_ptr(), c["tab"].data_ptr(), c["n_mats"], c["tiles"],
+                nat.check(lib.gc_cuda_psgd_q(reducer.rank_r, e.data_ptr(), c["tab"].data_ptr(), c["n_mats"], c["tiles"],
                                              c["reduced"].data_ptr(), c["q_local"].data_ptr(), q_total, c["max_rows"],
                                              st()), "psgd_q")
             with reducer._timer("reduce.q", verbosity=2):
                 ops.small_sum(c["q_local"][:max(q_total, 1)], reducer.q_memory[:max(q_total, 1)] if q_total else c["q_local"],
                               alpha=1.0 / reducer.n_workers)
             with reducer._timer("reduce.outerprod", verbosity=2):
-                nat.check(lib.gc_cuda_psgd_out(dest.data_ptr(), e.data_ptr(), c["tab"].data_ptr(), c["n_mats"], c["rows"],
+                nat.check(lib.gc_cuda_psgd_out(reducer.rank_r, dest.data_ptr(), e.data_ptr(), c["tab"].data_ptr(), c["n_mats"], c["rows"],
                                                c["reduced"].data_ptr(), reducer.q_memory.data_ptr(),
                                                c["vtab"].data_ptr(), c["n_vecs"],
                                                c["reduced"][p_total:].data_ptr() if c["v_total"] else None,
@@ -403,7 +403,8 @@ def solo_copy(reducer, grad_in, grad_out):
 
 def solo_collect(reducer, grad_in, grad_out, merge):
     """Reads a single worker's tensors into the engine's plan for one of the calls below: (elements, generation of the tensors'
-    sizes), or None."""
+    shapes, segments), or None.  ``merge``: 1 neighbours in memory become one segment, 0 a segment per tensor, 2 one segment if
+    all of them are neighbours, else one per tensor."""
     eng = reducer._fused or _engine(reducer)
     return None if eng.solo_handle() is None else eng.ext.collect(eng.plan, grad_in, grad_out, merge)
 
@@ -412,6 +413,43 @@ def solo_topk(reducer, counts, per_tensor, memory, scratch):
     eng = reducer._fused
     eng.ext.solo_topk(eng.plan, counts.data_ptr(), int(per_tensor), memory.data_ptr(), scratch.state.data_ptr(), scratch.lists.data_ptr())
     nat.count_launch(4)
+
+
+_psgd_rank = None
+
+
+def max_psgd_rank():
+    global _psgd_rank
+    if _psgd_rank is None:
+        _psgd_rank = int(nat.cuda().gc_cuda_psgd_max_rank())
+    return _psgd_rank
+
+
+def solo_psgd_tables(plan, starts, tensor_of, device):
+    """Device tables and partial sums of a single worker's PowerSGD step (``csrc/gc_powersgd.cu``): ``starts[i]`` is the first
+    flat element of tensor i, ``tensor_of[i]`` its place among the tensors that are not empty."""
+    rows, tiles, mats = 0, 0, []
+    for (i, n, m, r, po, qo) in plan["hi"]:
+        mats.append([starts[i], n, m, r, po, qo, rows, tiles, tensor_of[i]])
+        rows += int(nat.cuda().gc_cuda_psgd_row_blocks(n, m))
+        tiles += int(nat.cuda().gc_cuda_psgd_q_blocks(n, m))
+    vecs = [[starts[i], starts[i + 1] - starts[i], 0, tensor_of[i]] for i in plan["lo"]]
+    max_rows = max([n for (_, n, _, _, _, _) in plan["hi"]] or [1])
+    chunks = nat.cuda().gc_cuda_psgd_q_chunks(max_rows)
+    return {"rows": rows, "tiles": tiles, "n_mats": len(mats), "n_vecs": len(vecs), "max_rows": max_rows, "v_total": sum(v[1] for v in vecs),
+            "tab": torch.tensor(mats or [[0] * 9], dtype=torch.int64).to(device), "vtab": torch.tensor(vecs or [[0] * 4], dtype=torch.int64).to(device),
+            # chunks of rows that a matrix does not have are never written: zeroed once
+            "q_parts": torch.zeros(max(plan["q_total"], 1) * (chunks if chunks > 1 else 0), device=device)}
+
+
+def solo_psgd(reducer, c, q_total, draw):
+    from ..ops import philox
+
+    eng = reducer._fused
+    eng.ext.solo_psgd(eng.plan, reducer.rank_r, reducer._memory.data_ptr(), c["tab"].data_ptr(), c["n_mats"], c["rows"], c["tiles"], c["max_rows"], c["vtab"].data_ptr(),
+                      c["n_vecs"], reducer.q_memory.data_ptr(), reducer.p_memory.data_ptr(), c["q_parts"].data_ptr(), q_total, reducer._seed,
+                      philox.stream_id(0, philox.PURPOSE_QINIT), reducer._device_step().data_ptr() if draw else 0)
+    nat.count_launch((4 + draw + (c["q_parts"].numel() > 0) if c["n_mats"] else 0) or 1)
 
 
 def allreduce_mean(reducer, flat, grad_out):

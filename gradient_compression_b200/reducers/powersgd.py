@@ -17,7 +17,7 @@ import torch
 from .. import ops
 from ..ops import philox
 from ..parallel import engine as fused
-from .base import Reducer, TensorBuffer, n_bits
+from .base import Reducer, TensorBuffer, n_bits, physical
 
 
 class RankKReducer(Reducer):
@@ -34,6 +34,7 @@ class RankKReducer(Reducer):
         self._step = 0
         self._step_dev = None     # device copy of the step counter of the query stream (fused path)
         self._layout = None
+        self._solo = None         # single worker: (generation of the tensors' shapes, one flat segment?, plan, device tables)
 
     def _device_step(self):
         if self._step_dev is None:
@@ -68,6 +69,37 @@ class RankKReducer(Reducer):
         self._layout = {"key": key, "hi": hi, "lo": lo, "p_total": p_off, "q_total": q_off, "p_elems": p_elems,
                         "q_elems": q_elems}
         return self._layout
+
+    def _solo_reduce(self, grad_in, grad_out):
+        if self.rank_r > fused.max_psgd_rank():
+            return None
+        found = fused.solo_collect(self, grad_in, grad_out, 2)
+        if found is None:
+            return None
+        n, generation, segments = found
+        if self._solo is None or self._solo[:2] != (generation, segments == 1):
+            plan = self._plan([physical(t) for t in grad_in])
+            starts, tensor_of, off, seen = [0], [], 0, 0
+            for t in grad_in:
+                off += t.numel()
+                starts.append(off)
+                tensor_of.append(seen if segments > 1 else 0)
+                seen += t.numel() > 0
+            self._solo = (generation, segments == 1, plan, fused.solo_psgd_tables(plan, starts, tensor_of, self._device))
+        plan, tables = self._solo[2:]
+        fresh = self.p_memory is None
+        if fresh:
+            self.p_memory = torch.zeros(plan["p_total"], device=self._device)
+            self.q_memory = torch.zeros(plan["q_total"], device=self._device)
+        if self._memory is None:
+            self._memory = torch.zeros(n, device=self._device)
+        if self._memory.numel() != n or self.p_memory.numel() != plan["p_total"] or self.q_memory.numel() != plan["q_total"]:
+            return None
+        with self._timer("reduce.fused", verbosity=2):
+            fused.solo_psgd(self, tables, plan["q_total"], not (self.reuse_query and not fresh))
+        self._step += 1
+        self.last_wire_bits = 32 * (plan["p_elems"] + plan["q_elems"] + tables["v_total"])
+        return self.last_wire_bits
 
     def reduce(self, grad_in, grad_out):
         flat = TensorBuffer(grad_in)

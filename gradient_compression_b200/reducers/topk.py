@@ -44,10 +44,10 @@ class _TopKBase(Reducer):
         return self._selector
 
     def _solo_reduce(self, grad_in, grad_out):
-        found = fused.solo_collect(self, grad_in, grad_out, not self.layerwise)
+        found = fused.solo_collect(self, grad_in, grad_out, 0 if self.layerwise else 1)
         if found is None:
             return None
-        n, generation = found
+        n, generation, _ = found
         if self._memory is None:
             self._memory = torch.zeros(n, device=self._device)
         if self._memory.numel() != n or not self._memory.is_contiguous():

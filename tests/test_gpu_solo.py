@@ -138,3 +138,25 @@ def test_topk_lists(kind, memory):
             want = a.clone()
             want[idx.long()] = 0
             assert torch.equal(e.cpu(), want)
+
+
+@pytest.mark.parametrize("layout", ["flat", "separate", "shifted"])
+@pytest.mark.parametrize("rank", [1, 2, 3, 4])
+@pytest.mark.parametrize("reuse", [False, True])
+def test_powersgd(rank, reuse, layout):
+    from gradient_compression_b200.reducers import RankKReducer
+
+    # ragged rows, fewer rows or columns than the rank, more rows than one chunk, vectors in between
+    shapes = [(64, 3, 3, 3), (64,), (1, 7), (130, 65), (2, 4096), (257, 128), (10,), (3, 1), (65, 64, 1, 1)]
+    host = [t.view(s) for t, s in zip(_values([int(torch.Size(s).numel()) for s in shapes], 4), shapes)]
+    cpu, gpu = (RankKReducer(d, None, rank=rank, seed=5, reuse_query=reuse) for d in ("cpu", "cuda"))
+    for step in range(3):
+        now = [t * (1 + 0.1 * step) for t in host]
+        want = [torch.empty_like(t) for t in now]
+        send = [t.view(s) for t, s in zip(_on_gpu([t.reshape(-1) for t in now], layout), shapes)]
+        outs = send if step == 1 else [torch.empty_like(t) for t in send]
+        assert gpu.reduce(send, outs) == cpu.reduce([t.clone() for t in now], want)
+        for w, g in zip(want, outs):
+            torch.testing.assert_close(g.cpu(), w, rtol=2e-4, atol=2e-4 * float(w.abs().max()))
+        torch.testing.assert_close(gpu.state_dict()["_memory"].cpu(), cpu.state_dict()["_memory"], rtol=1e-3, atol=2e-4)
+    assert reuse or gpu.state_dict()["step"] == cpu.state_dict()["step"] == 3
