@@ -94,6 +94,12 @@ struct SegCursor {
     const int64_t ahead = DIR > 0 ? (b - (e0 + 4 * SEG_TILE)) / (4 * SEG_TILE) : (e0 - (a + 3) / 4 * 4) / (4 * SEG_TILE);
     run = whole && ahead > 0 ? (int)ahead : 0;
   }
+  // any other tile
+  __device__ __forceinline__ void jump(const SegTable<CAP>& t, uint32_t to) {
+    tile = to;
+    s = seg_of_tile(t, tile);
+    enter(t);
+  }
   // N further tiles at once, all of them whole (N <= run)
   template <int N>
   __device__ __forceinline__ void skip() {

@@ -2,6 +2,7 @@
 // straight from the gradient tensors into the gradient tensors.
 //
 //   solo_maxnorm_kernel  QSGD-MaxNorm and its two-scale variant: one persistent block of 1024 threads per SM.
+//   solo_randk_kernel    GlobalRandK-MaxNorm and its two-scale variant.
 //   solo_copy_kernel     AllReduce-SGD: the mean over one worker.
 //
 // What bounds solo_maxnorm.  The vector has to be read before its norm is known and is needed again after, so DRAM moves
@@ -16,6 +17,7 @@
 #include <stdint.h>
 
 #include "gc_comm.cuh"
+#include "gc_perm.h"
 #include "gc_segs.cuh"
 #include "gc_solo.h"
 
@@ -81,36 +83,43 @@ __device__ __forceinline__ void copy16_async(float4* dst, const float* src) {
 __device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void copy_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+// The counters of the grid barrier as a launch finds them (read by thread 0 of each block before its first arrival).
+struct SoloSync {
+  uint32_t passed, turn;
+  __device__ __forceinline__ explicit SoloSync(const ArenaHeader* h)
+      : passed(*((volatile const uint32_t*)&h->solo_passed)), turn(*((volatile const uint32_t*)&h->solo_turn)) {}
+};
+
 // Maximum over all threads of all blocks; valid in every thread.  Thread 0 of each block folds its block's maximum into one of
-// the header's two slots (the other one is cleared for the next launch) and arrives; the arrival count only ever grows, so nothing has to be reset between launches.
-__device__ __forceinline__ float solo_grid_max(Waiter& w, float v, uint32_t epoch, int nblocks, float* smem) {
+// the header's two slots (the other one is cleared for the next launch) and arrives; the arrival count only ever grows, so
+// nothing has to be reset between launches.  A further barrier of the same launch (v = 0) does not carry a maximum.
+__device__ __forceinline__ float solo_grid_max(Waiter& w, SoloSync& sync, float v, int nblocks, float* smem) {
   float m = block_max(v, smem);
   if (nblocks > 1) {
     if (threadIdx.x == 0) {
       ArenaHeader* h = w.hdr;
-      const uint32_t target = *((volatile uint32_t*)&h->solo_passed) + (uint32_t)nblocks;
-      const uint32_t turn = *((volatile uint32_t*)&h->solo_turn);
-      atomicMax(&h->solo_max[turn & 1], __float_as_uint(m));     // bit patterns of non-negative floats order like the floats
+      sync.passed += (uint32_t)nblocks;
+      atomicMax(&h->solo_max[sync.turn & 1], __float_as_uint(m));     // bit patterns of non-negative floats order like the floats
       __threadfence();
       atomicAdd(&h->solo_arrived, 1u);
       int it = 0;
-      while ((int32_t)(ld_acquire_gpu(&h->solo_arrived) - target) < 0) {
+      while ((int32_t)(ld_acquire_gpu(&h->solo_arrived) - sync.passed) < 0) {
         if ((++it & 63) == 0) {
           if (w.aborted()) break;
           if (global_ns() > w.deadline) { w.fail(0x90, 0xfffe); break; }
         }
       }
-      smem[0] = __uint_as_float(*((volatile uint32_t*)&h->solo_max[turn & 1]));
-      if (blockIdx.x == 0) {               // every block has read the counters of this launch: advance them
-        h->solo_passed = target;
-        h->solo_turn = turn + 1u;
-        h->solo_max[(turn & 1) ^ 1] = 0u;
+      smem[0] = __uint_as_float(*((volatile uint32_t*)&h->solo_max[sync.turn & 1]));
+      ++sync.turn;
+      if (blockIdx.x == 0) {               // for the next launch: every block has read the counters of this one
+        h->solo_passed = sync.passed;
+        h->solo_turn = sync.turn;
+        h->solo_max[sync.turn & 1] = 0u;
       }
     }
     __syncthreads();
     m = smem[0];
   }
-  commit_epoch(w.hdr, epoch, blockIdx.x);
   return m;
 }
 
@@ -120,6 +129,7 @@ __global__ void __launch_bounds__(THREADS, 1) solo_maxnorm_kernel(const __grid_c
   extern __shared__ float4 slots[];        // [SLOTS][THREADS]; a thread only ever touches its own column
   __shared__ float smem[32];
   Waiter waiter{p.hdr, global_ns() + p.timeout_ns};
+  SoloSync sync(p.hdr);
   const uint32_t epoch = next_epoch(p.hdr);
   const uint32_t step = p.step + (p.step_from_device ? launch_calls(p.hdr) : 0u);
   const uint32_t tiles = t.tile0[t.n], nb = gridDim.x;
@@ -169,7 +179,8 @@ __global__ void __launch_bounds__(THREADS, 1) solo_maxnorm_kernel(const __grid_c
     }
     copy_wait<0>();
   }
-  const float norm = solo_grid_max(waiter, abs_for_max(m), epoch, (int)nb, smem);
+  const float norm = solo_grid_max(waiter, sync, abs_for_max(m), (int)nb, smem);
+  commit_epoch(p.hdr, epoch, blockIdx.x);
   const float s_lo = (float)p.s_lo, s_hi = (float)p.s_hi;
   const float sc_lo = norm > 0.0f ? s_lo / norm : 0.0f, dq_lo = dequant_scale(norm, p.s_lo, 1);
   const float sc_hi = TWO && norm > 0.0f ? s_hi / norm : 0.0f, dq_hi = TWO ? dequant_scale(norm, p.s_hi, 1) : 0.0f;
@@ -229,14 +240,112 @@ __global__ void __launch_bounds__(THREADS, 1) solo_maxnorm_kernel(const __grid_c
     if (!c.empty(t)) c.store(t, value(slot(it), c.quad));
 }
 
+// This block's share of out = in (or out = 0): four whole tiles in flight.
 template <int CAP>
-__global__ void __launch_bounds__(THREADS) solo_copy_kernel(const __grid_constant__ SegTable<CAP> t) {
+__device__ __forceinline__ void copy_tiles(const SegTable<CAP>& t, bool zero) {
   const uint32_t tiles = t.tile0[t.n], per = (tiles + gridDim.x - 1) / gridDim.x, first = blockIdx.x * per;
   if (first >= tiles) return;
-  const uint32_t last = tiles - first < per ? tiles : first + per;
+  uint32_t left = tiles - first < per ? tiles - first : per;
+  const float4 nothing = make_float4(0.f, 0.f, 0.f, 0.f);
   SegCursor<CAP, 1> c(t, first);
-  for (uint32_t tile = first; tile < last; ++tile, c.step(t))
-    if (!c.empty(t)) c.store(t, c.load(t));
+  while (left > 0) {
+    if (!zero && c.in == c.out) {            // this tensor stays what it is
+      const uint32_t rest = t.tile0[c.s + 1] - c.tile;
+      if (rest >= left) return;
+      left -= rest;
+      c.jump(t, c.tile + rest);
+      continue;
+    }
+    if (left >= 4 && c.run >= 3 && c.fast_out && (zero || c.fast_in)) {
+      float4 x[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) x[u] = zero ? nothing : __ldcs(reinterpret_cast<const float4*>(c.in) + u * SEG_TILE);
+#pragma unroll
+      for (int u = 0; u < 4; ++u) __stcs(reinterpret_cast<float4*>(c.out) + u * SEG_TILE, x[u]);
+      left -= 4;
+      c.template skip<3>();
+    } else {
+      if (!c.empty(t)) c.store(t, zero ? nothing : c.load(t));
+      --left;
+    }
+    if (left > 0) c.step(t);
+  }
+}
+
+template <int CAP>
+__global__ void __launch_bounds__(THREADS) solo_copy_kernel(const __grid_constant__ SegTable<CAP> t) {
+  copy_tiles(t, false);
+}
+
+// Rand-K: the selected coordinates are gathered into registers, everything else becomes what it becomes (in or 0), and behind
+// the grid barrier that the norm needs anyway the quantised values are put in their places.  Where zeros would overwrite
+// coordinates that another block has still to gather (in place), the zeros wait for that barrier and a second one follows.
+constexpr int RANDK_PER_THREAD = 4;
+
+struct SoloRandk {
+  PermKey perm;
+  int64_t start, k;        // the window [start, start + k) of the permutation, cut off at n
+  int64_t* window;         // device-resident start (advanced here); NULL: `start`
+  int zero, in_place;
+};
+
+template <int CAP>
+__global__ void __launch_bounds__(THREADS) solo_randk_kernel(const __grid_constant__ SegTable<CAP> t, const __grid_constant__ SoloParams p,
+                                                             const __grid_constant__ SoloRandk r) {
+  __shared__ float smem[32];
+  Waiter waiter{p.hdr, global_ns() + p.timeout_ns};
+  SoloSync sync(p.hdr);
+  const uint32_t epoch = next_epoch(p.hdr);
+  const uint32_t step = p.step + (p.step_from_device ? launch_calls(p.hdr) : 0u);
+  const int64_t n = t.start[t.n];
+  const int64_t start = r.window != nullptr ? *((volatile const int64_t*)r.window) : r.start;
+  const int64_t k = r.k < n - start ? r.k : n - start;
+  float x[RANDK_PER_THREAD];
+  float* to[RANDK_PER_THREAD];
+  float m = 0.0f;
+#pragma unroll
+  for (int u = 0; u < RANDK_PER_THREAD; ++u) {
+    const int64_t i = ((int64_t)u * THREADS + threadIdx.x) * gridDim.x + blockIdx.x;
+    to[u] = nullptr;
+    x[u] = 0.0f;
+    if (i < k) {
+      const uint64_t at = perm_eval(r.perm, (uint64_t)(start + i));
+      if (GC_INDEX_OK(waiter, at, n)) {
+        const int s = seg_of_elem(t, (int64_t)at);
+        x[u] = t.in[s][(int64_t)at - t.start[s]];
+        to[u] = t.out[s] + ((int64_t)at - t.start[s]);
+      }
+    }
+    m = fmaxf(m, abs_for_max(x[u]));
+  }
+  const bool late = r.zero && r.in_place;
+  if (!late) copy_tiles(t, r.zero != 0);
+  const float norm = solo_grid_max(waiter, sync, m, (int)gridDim.x, smem);
+  commit_epoch(p.hdr, epoch, blockIdx.x);
+  if (r.window != nullptr && blockIdx.x == 0 && threadIdx.x == 0) *r.window = start + k >= n ? 0 : start + k;      // (every block has read it)
+  if (late) {
+    copy_tiles(t, true);
+    __syncthreads();
+    solo_grid_max(waiter, sync, 0.0f, (int)gridDim.x, smem);
+    __syncthreads();
+  }
+  const bool two = p.s_hi > 0;
+  const float s_lo = (float)p.s_lo, s_hi = (float)p.s_hi;
+  const float sc_lo = norm > 0.0f ? s_lo / norm : 0.0f, dq_lo = dequant_scale(norm, p.s_lo, 1);
+  const float sc_hi = two && norm > 0.0f ? s_hi / norm : 0.0f, dq_hi = two ? dequant_scale(norm, p.s_hi, 1) : 0.0f;
+  auto word = [](const U4& v, int j) { return j == 0 ? v.x : j == 1 ? v.y : j == 2 ? v.z : v.w; };
+#pragma unroll
+  for (int u = 0; u < RANDK_PER_THREAD; ++u) {
+    if (to[u] == nullptr) continue;
+    const int64_t i = ((int64_t)u * THREADS + threadIdx.x) * gridDim.x + blockIdx.x;
+    if (two) {
+      const U4 h = solo_philox(p, (uint64_t)(i >> 2), step, PURPOSE_ROUND_HI);
+      const float lev = round_level(x[u], sc_hi, s_hi, word(h, (int)(i & 3)));
+      if (lev <= s_lo) { *to[u] = signed_value(x[u], lev, dq_hi); continue; }
+    }
+    const U4 l = solo_philox(p, (uint64_t)(i >> 2), step, PURPOSE_ROUND);
+    *to[u] = signed_value(x[u], round_level(x[u], sc_lo, s_lo, word(l, (int)(i & 3))), dq_lo);
+  }
 }
 
 template <bool TWO, int CAP>
@@ -277,6 +386,45 @@ int copy_segs(const SegDesc* segs, int n_seg, int64_t n, int sm_count, cudaStrea
   return (int)cudaGetLastError();
 }
 
+SoloParams make_params(CommCtx* c, int bits_lo, int bits_hi, uint64_t seed, uint32_t step, int timeout_ms) {
+  SoloParams p;
+  p.hdr = (ArenaHeader*)c->local;
+  p.step_from_device = c->step_from_device;
+  p.timeout_ns = (unsigned long long)(timeout_ms > 0 ? timeout_ms : 30000) * 1000000ull;
+  for (int r = 0; r < 10; ++r) {
+    p.rk0[r] = (uint32_t)seed + (uint32_t)r * 0x9E3779B9u;
+    p.rk1[r] = (uint32_t)(seed >> 32) + (uint32_t)r * 0xBB67AE85u;
+  }
+  p.step = step;
+  p.stream = (uint32_t)c->rank << 8;
+  p.s_lo = (1 << bits_lo) - 1;
+  p.s_hi = bits_hi > 0 ? (1 << bits_hi) - 1 : 0;
+  return p;
+}
+
+template <int CAP>
+int randk_segs(CommCtx* c, const SegDesc* segs, int n_seg, int64_t n, const SoloParams& p, SoloRandk r, int max_blocks, cudaStream_t st) {
+  SegTable<CAP> t;
+  if (!seg_table(t, segs, n_seg, n)) return (int)cudaErrorInvalidValue;
+  r.in_place = 0;
+  bool dense = r.zero != 0;
+  for (int i = 0; i < n_seg; ++i) {
+    if (segs[i].in == segs[i].out) r.in_place = 1;
+    else dense = true;
+  }
+  // 128 gathers a block keep every one of them in flight at once; a dense pass wants every SM
+  int64_t blocks = (r.k + 127) / 128;
+  if (dense && blocks < t.tile0[n_seg]) blocks = t.tile0[n_seg];
+  if (blocks > c->sm_count) blocks = c->sm_count;
+  if (max_blocks > 0 && blocks > max_blocks) blocks = max_blocks;
+  if (blocks < 1) blocks = 1;
+  if (r.k > blocks * THREADS * RANDK_PER_THREAD) return (int)cudaErrorInvalidValue;
+  void* args[3] = {(void*)&t, (void*)&p, (void*)&r};
+  const void* kernel = (const void*)solo_randk_kernel<CAP>;
+  if (blocks == 1) return (int)cudaLaunchKernel(kernel, dim3(1), dim3(THREADS), args, 0, st);
+  return (int)cudaLaunchCooperativeKernel(kernel, dim3((unsigned)blocks), dim3(THREADS), args, 0, st);
+}
+
 }  // namespace
 
 extern "C" {
@@ -290,18 +438,7 @@ int gc_solo_maxnorm(void* ctx, const void* segs, int n_seg, int64_t n, int bits_
   CommCtx* c = (CommCtx*)ctx;
   if (c->world != 1 || bits_lo < 1 || bits_lo > 16 || bits_hi < 0 || bits_hi > 16) return (int)cudaErrorInvalidValue;
   if (n <= 0) return 0;
-  SoloParams p;
-  p.hdr = (ArenaHeader*)c->local;
-  p.step_from_device = c->step_from_device;
-  p.timeout_ns = (unsigned long long)(timeout_ms > 0 ? timeout_ms : 30000) * 1000000ull;
-  for (int r = 0; r < 10; ++r) {
-    p.rk0[r] = (uint32_t)seed + (uint32_t)r * 0x9E3779B9u;
-    p.rk1[r] = (uint32_t)(seed >> 32) + (uint32_t)r * 0xBB67AE85u;
-  }
-  p.step = step;
-  p.stream = (uint32_t)c->rank << 8;
-  p.s_lo = (1 << bits_lo) - 1;
-  p.s_hi = bits_hi > 0 ? (1 << bits_hi) - 1 : 0;
+  const SoloParams p = make_params(c, bits_lo, bits_hi, seed, step, timeout_ms);
   const SegDesc* d = (const SegDesc*)segs;
   cudaStream_t st = (cudaStream_t)cs;
   if (n_seg == 1) return maxnorm_segs<1>(c, d, n_seg, n, bits_lo, bits_hi, p, max_blocks, st);
@@ -315,6 +452,31 @@ int gc_solo_copy(void* ctx, const void* segs, int n_seg, int64_t n, void* cs) {
   const SegDesc* d = (const SegDesc*)segs;
   if (n_seg == 1) return copy_segs<1>(d, n_seg, n, c->sm_count, (cudaStream_t)cs);
   return copy_segs<SEG_CAP_MANY>(d, n_seg, n, c->sm_count, (cudaStream_t)cs);
+}
+
+// Most coordinates a single worker's Rand-K takes (they are kept in registers); max_blocks as in the call.
+int64_t gc_solo_randk_limit(void* ctx, int max_blocks) {
+  const int sms = ((CommCtx*)ctx)->sm_count;
+  return (int64_t)(max_blocks > 0 && max_blocks < sms ? max_blocks : sms) * THREADS * RANDK_PER_THREAD;
+}
+
+// One Rand-K reduce of a single worker (bits_hi > 0: two scales) on the window [start, start + k) of the keyed permutation of
+// [0, n); window (device, may be NULL): the start is read from it and the next one stored.
+int gc_solo_randk(void* ctx, const void* segs, int n_seg, int64_t n, uint64_t index_seed, uint32_t npass, int64_t start, int64_t k, int64_t* window,
+                  int bits_lo, int bits_hi, int zero, uint32_t step, int timeout_ms, int max_blocks, void* cs) {
+  CommCtx* c = (CommCtx*)ctx;
+  if (c->world != 1 || bits_lo < 1 || bits_lo > 16 || bits_hi < 0 || bits_hi > 16) return (int)cudaErrorInvalidValue;
+  if (n <= 0) return 0;
+  const SoloParams p = make_params(c, bits_lo, bits_hi, index_seed, step, timeout_ms);
+  SoloRandk r;
+  r.perm = make_perm_key((uint64_t)n, index_seed, npass);
+  r.start = start;
+  r.k = k < n ? k : n;
+  r.window = window;
+  r.zero = zero;
+  const SegDesc* d = (const SegDesc*)segs;
+  if (n_seg == 1) return randk_segs<1>(c, d, n_seg, n, p, r, max_blocks, (cudaStream_t)cs);
+  return randk_segs<SEG_CAP_MANY>(c, d, n_seg, n, p, r, max_blocks, (cudaStream_t)cs);
 }
 
 }  // extern "C"

@@ -32,6 +32,8 @@ struct Api {
   int (*solo_max_segs)();
   int (*solo_maxnorm)(void*, const void*, int, int64_t, int, int, uint64_t, uint32_t, int, int, void*);
   int (*solo_copy)(void*, const void*, int, int64_t, void*);
+  int64_t (*solo_randk_limit)(void*, int);
+  int (*solo_randk)(void*, const void*, int, int64_t, uint64_t, uint32_t, int64_t, int64_t, int64_t*, int, int, int, uint32_t, int, int, void*);
   int (*topk_run)(const void*, int, int64_t, const int64_t*, int, float*, void*, void*, int32_t*, float*, void*);
   int (*psgd_solo)(int, const void*, int, float*, const int64_t*, int, int64_t, int64_t, int, const int64_t*, int, float*, float*, float*, int64_t, uint64_t,
                    uint32_t, uint32_t*, void*);
@@ -43,6 +45,8 @@ const Entry entries[] = {
     {"gc_solo_max_segs", (void**)&api.solo_max_segs},
     {"gc_solo_maxnorm", (void**)&api.solo_maxnorm},
     {"gc_solo_copy", (void**)&api.solo_copy},
+    {"gc_solo_randk_limit", (void**)&api.solo_randk_limit},
+    {"gc_solo_randk", (void**)&api.solo_randk},
     {"gc_cuda_topk_run", (void**)&api.topk_run},
     {"gc_cuda_psgd_solo", (void**)&api.psgd_solo},
 };
@@ -225,6 +229,34 @@ PyObject* collect_py(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   return Py_BuildValue("LLn", (long long)p->n, (long long)p->generation, (Py_ssize_t)p->segs.size());
 }
 
+// solo_randk(plan, ctx, seed, npass, start, k, window or 0, bits_lo, bits_hi, zero, step, timeout_ms, max_blocks): on what collect() found
+PyObject* solo_randk(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
+  if (!want(nargs, 13, "solo_randk")) return nullptr;
+  Plan* p = plan_of(a[0]);
+  if (!p) return nullptr;
+  void* ctx = (void*)PyLong_AsUnsignedLongLong(a[1]);
+  const uint64_t seed = PyLong_AsUnsignedLongLongMask(a[2]);
+  const uint32_t npass = (uint32_t)PyLong_AsUnsignedLongLongMask(a[3]), step = (uint32_t)PyLong_AsUnsignedLongLongMask(a[10]);
+  const int64_t start = as_int(a[4]), k = as_int(a[5]);
+  int64_t* window = (int64_t*)PyLong_AsUnsignedLongLong(a[6]);
+  const int lo = (int)as_int(a[7]), hi = (int)as_int(a[8]), zero = (int)as_int(a[9]), timeout = (int)as_int(a[11]), blocks = (int)as_int(a[12]);
+  if (PyErr_Occurred()) return nullptr;
+  c10::cuda::OptionalCUDAGuard guard(c10::Device(c10::kCUDA, (c10::DeviceIndex)p->device));
+  const int err = api.solo_randk(ctx, p->segs.data(), (int)p->segs.size(), p->n, seed, npass, start, k, window, lo, hi, zero, step, timeout, blocks,
+                                 stream_on(p->device));
+  if (err) return cuda_error("solo_randk", err);
+  Py_RETURN_NONE;
+}
+
+// solo_randk_limit(ctx, max_blocks) -> most coordinates solo_randk takes
+PyObject* solo_randk_limit(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
+  if (!want(nargs, 2, "solo_randk_limit")) return nullptr;
+  void* ctx = (void*)PyLong_AsUnsignedLongLong(a[0]);
+  const int blocks = (int)as_int(a[1]);
+  if (PyErr_Occurred()) return nullptr;
+  return PyLong_FromLongLong(api.solo_randk_limit(ctx, blocks));
+}
+
 // solo_psgd(plan, rank, memory, tab, n_mats, rows, tiles, max_rows, vtab, n_vecs, q, p, q_parts, q_total, seed, stream, step or 0)
 PyObject* solo_psgd(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   if (!want(nargs, 17, "solo_psgd")) return nullptr;
@@ -286,6 +318,8 @@ PyMethodDef methods[] = {
     {"solo_maxnorm", (PyCFunction)(void (*)(void))solo_maxnorm, METH_FASTCALL, "QSGD-MaxNorm reduce of a single worker"},
     {"solo_copy", (PyCFunction)(void (*)(void))solo_copy, METH_FASTCALL, "plain mean of a single worker"},
     {"collect", (PyCFunction)(void (*)(void))collect_py, METH_FASTCALL, "reads two lists of tensors into a plan"},
+    {"solo_randk", (PyCFunction)(void (*)(void))solo_randk, METH_FASTCALL, "Rand-K reduce of a single worker"},
+    {"solo_randk_limit", (PyCFunction)(void (*)(void))solo_randk_limit, METH_FASTCALL, "most coordinates solo_randk takes"},
     {"solo_psgd", (PyCFunction)(void (*)(void))solo_psgd, METH_FASTCALL, "PowerSGD step of a single worker"},
     {"solo_topk", (PyCFunction)(void (*)(void))solo_topk, METH_FASTCALL, "top-k with error feedback of a single worker"},
     {nullptr, nullptr, 0, nullptr}};

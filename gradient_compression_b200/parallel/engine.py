@@ -409,6 +409,22 @@ def solo_collect(reducer, grad_in, grad_out, merge):
     return None if eng.solo_handle() is None else eng.ext.collect(eng.plan, grad_in, grad_out, merge)
 
 
+def solo_randk_takes(reducer, k):
+    """Whether a single worker's Rand-K kernel holds ``k`` coordinates."""
+    eng = reducer._fused
+    return k <= eng.ext.solo_randk_limit(eng.solo_handle(), eng.max_blocks())
+
+
+def solo_randk(reducer, start, k, npass, bits_lo, bits_hi):
+    eng, noise = reducer._fused, reducer._noise
+    window = reducer._device_window(start)
+    eng.ext.solo_randk(eng.plan, eng.solo_handle(), reducer._queue.seed, npass, start, reducer._K if window is not None else k,
+                       window.data_ptr() if window is not None else 0, bits_lo, bits_hi, reducer._unselected == "zero", noise.step, eng.ops.timeout_ms,
+                       eng.max_blocks())
+    noise.step += 1
+    nat.count_launch()
+
+
 def solo_topk(reducer, counts, per_tensor, memory, scratch):
     eng = reducer._fused
     eng.ext.solo_topk(eng.plan, counts.data_ptr(), int(per_tensor), memory.data_ptr(), scratch.state.data_ptr(), scratch.lists.data_ptr())

@@ -69,6 +69,16 @@ class GlobalRandKMaxNormReducer(Reducer):
             out = self._compressor.decompress(max_norm, levels, self.n_workers)
         return out, bits
 
+    def _solo_reduce(self, grad_in, grad_out):
+        found = fused.solo_collect(self, grad_in, grad_out, 1)
+        if found is None or not fused.solo_randk_takes(self, min(self._K, found[0])):
+            return None
+        start, k, npass = self._queue.next_window(found[0])
+        lo, hi = self._quantization_level, getattr(self, "_higher_quantization_level", 0)
+        with self._timer("reduce.fused", verbosity=2):
+            fused.solo_randk(self, start, k, npass, lo, hi)
+        return 32 + (8 if lo < 8 else 32) * k + (8 * k if hi else 0)
+
     def reduce(self, grad_in, grad_out):
         with self._timer("reduce.flat_pack"):
             flat = TensorBuffer(grad_in)

@@ -160,3 +160,26 @@ def test_powersgd(rank, reuse, layout):
             torch.testing.assert_close(g.cpu(), w, rtol=2e-4, atol=2e-4 * float(w.abs().max()))
         torch.testing.assert_close(gpu.state_dict()["_memory"].cpu(), cpu.state_dict()["_memory"], rtol=1e-3, atol=2e-4)
     assert reuse or gpu.state_dict()["step"] == cpu.state_dict()["step"] == 3
+
+
+@pytest.mark.parametrize("layout", ["flat", "separate", "shifted"])
+@pytest.mark.parametrize("sizes", ["one", "tile+1", "two-blocks", "kept", "many", "most", "too many"])
+@pytest.mark.parametrize("unselected", ["local", "zero"])
+@pytest.mark.parametrize("name,K,bits", [("GlobalRandKMaxNormReducer", 300, (8,)), ("GlobalRandKMaxNormReducer", 200000, (4,)),
+                                         ("GlobalRandKMaxNormTwoScaleReducer", 1000, (2, 6))])
+def test_randk(name, K, bits, unselected, sizes, layout):
+    from gradient_compression_b200 import reducers as R
+
+    host = _values(SIZES[sizes], 6)
+    kw = dict(seed=7, K=K, unselected=unselected)
+    kw.update(quantization_level=bits[0]) if len(bits) == 1 else kw.update(lower_quantization_level=bits[0], higher_quantization_level=bits[1])
+    cpu, gpu = (getattr(R, name)(d, None, **kw) for d in ("cpu", "cuda"))
+    for step in range(3):                   # windows run through the permutation and wrap around
+        want = [torch.empty_like(t) for t in host]
+        bits_cpu = cpu.reduce([t.clone() for t in host], want)
+        send = _on_gpu(host, layout)
+        outs = send if step == 1 else _on_gpu([torch.full_like(t, 9.0) for t in host], layout)
+        assert gpu.reduce(send, outs) == bits_cpu
+        for w, g in zip(want, outs):
+            assert torch.equal(w, g.cpu())
+    assert gpu.state_dict()["queue"]["position"] % sum(SIZES[sizes]) == cpu.state_dict()["queue"]["position"] % sum(SIZES[sizes])
