@@ -55,6 +55,14 @@ def _levels(s):
     return (1 << s) - 1
 
 
+def _scaled(norm, levels):
+    """``norm * levels`` in fp32, by the native dequantiser where it takes the container."""
+    if torch.is_tensor(norm) and norm.numel() == 1 and norm.dtype == torch.float32 and levels.dtype in ops.quant._LEVEL_BYTES and levels.dim() == 1 \
+            and levels.device == norm.device:
+        return ops.dequantize_levels(levels, norm, 1)
+    return norm * levels
+
+
 class _Codec:
     def __init__(self, device, noise=None):
         self._device = device
@@ -104,12 +112,12 @@ class QSGDWECCompressor(_Codec):
         self._quantization_level = quantization_level
         self._dtype = _container(quantization_level)
 
-    def _q(self, tensor):
+    def _q(self, tensor, dtype=torch.int32):
         s = _levels(self._quantization_level)
-        flat = tensor.contiguous().view(-1)
+        flat = tensor.contiguous()
         norm = ops.absmax(flat)
         q = ops.quantize_levels(flat, norm, s, self._noise.seed, self._noise.stream(philox.PURPOSE_ROUND),
-                                self._noise.next_step())
+                                self._noise.next_step(), dtype=dtype)
         return norm.reshape(()) / s, q
 
     def compress(self, tensor):
@@ -124,18 +132,17 @@ class QSGDWECModCompressor(QSGDWECCompressor):
     """Same with sign * xi fused into one array (compressors.py:192-230)."""
 
     def compress(self, tensor):
-        norm, q = self._q(tensor)
-        return norm, q.to(self._dtype)
+        return self._q(tensor, self._dtype)
 
     def decompress(self, norm, sign_xi_array):
-        return norm * sign_xi_array
+        return _scaled(norm, sign_xi_array)
 
 
 class TernGradCompressor(_Codec):
     """TernGrad: scaler = max |g|, b ~ Bernoulli(|g| / scaler) (compressors.py:233-254)."""
 
     def _q(self, tensor):
-        flat = tensor.contiguous().view(-1)
+        flat = tensor.contiguous()
         scaler = ops.absmax(flat)
         q = ops.quantize_levels(flat, scaler, 1, self._noise.seed, self._noise.stream(philox.PURPOSE_ROUND),
                                 self._noise.next_step(), dtype=torch.int8)
@@ -156,7 +163,7 @@ class TernGradModCompressor(TernGradCompressor):
         return self._q(tensor)
 
     def decompress(self, scaler, sign_b_array):
-        return scaler * sign_b_array
+        return _scaled(scaler, sign_b_array)
 
 
 class QSGDMaxNormCompressor(_Codec):
@@ -173,7 +180,7 @@ class QSGDMaxNormCompressor(_Codec):
         return _levels(self._quantization_level)
 
     def compress(self, norm, tensor):
-        flat = tensor.contiguous().view(-1)
+        flat = tensor.contiguous()
         return ops.quantize_levels(flat, norm, self._s(), self._noise.seed, self._noise.stream(philox.PURPOSE_ROUND),
                                    self._noise.next_step(), mode=self._mode, dtype=self._dtype)
 
@@ -227,7 +234,7 @@ class NUQSGDModCompressor(_Codec):
         return norm / s, q
 
     def decompress(self, norm, sign_h_array):
-        return norm * sign_h_array
+        return _scaled(norm, sign_h_array)
 
 
 class QSGDMaxNormTwoScaleCompressor(_Codec):
@@ -259,18 +266,12 @@ class QSGDMaxNormTwoScaleCompressor(_Codec):
     def compress_higher(self, norm, tensor):
         step = self._step if self._step is not None else self._noise.next_step()
         s_lo = _levels(self._lower_quantization_level)
-        q = ops.quantize_levels(tensor.contiguous().view(-1), norm, _levels(self._higher_quantization_level),
-                                self._noise.seed, self._noise.stream(philox.PURPOSE_ROUND_HI), step,
-                                dtype=torch.int32)
-        mask = (q.abs() <= s_lo).to(torch.int8)
-        return q.to(self._dtype), mask
+        return ops.quantize_fit(tensor.contiguous().view(-1), norm, _levels(self._higher_quantization_level), s_lo,
+                                self._noise.seed, self._noise.stream(philox.PURPOSE_ROUND_HI), step, dtype=self._dtype)
 
     def decompress(self, norm, sign_xi_array, higher_resolution_mask, world=1):
         s_lo, s_hi = _levels(self._lower_quantization_level), _levels(self._higher_quantization_level)
-        # both candidates come from the native dequantiser so CPU, GPU and the fused kernel agree bit for bit
-        fine = ops.dequantize_levels(sign_xi_array, norm, s_hi, world)
-        coarse = ops.dequantize_levels(sign_xi_array, norm, s_lo, world)
-        return torch.where(higher_resolution_mask.bool(), fine, coarse)
+        return ops.dequantize_two(sign_xi_array, higher_resolution_mask, norm, s_hi, s_lo, world)
 
 
 class GlobalRandKMaxNormTwoScaleCompressor(QSGDMaxNormTwoScaleCompressor):

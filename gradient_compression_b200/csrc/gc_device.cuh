@@ -67,6 +67,29 @@ __device__ __forceinline__ void store_quad(float* __restrict__ x, int64_t e0, in
   if (e0 + 3 < n) x[e0 + 3] = v.w;
 }
 
+// running maximum of |x| that keeps a NaN (which becomes +inf in the norm)
+__device__ __forceinline__ float max_nan(float m, float x) {
+  float r;
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(m), "f"(fabsf(x)));
+  return r;
+}
+
+// Level of |g| as a float, the same value that quantize_level (gc_common.h) returns as an integer:
+//   floor(l): adding 2^23 rounding down leaves floor(l) in the last mantissa bits (l < s <= 2^16), subtracting it is exact;
+//   u01(rnd) < p with u01 = (rnd >> 8) / 2^24: as integers, (rnd >> 8) < ceil(p * 2^24).  p * 2^-125 rounded up is that
+//   ceiling times 2^-149, the unit of the subnormals, so its bit pattern IS the ceiling.
+__device__ __forceinline__ float round_level(float g, float scale, float s, uint32_t rnd) {
+  const float l = __fmul_rn(fabsf(g), scale);
+  const float fl = __fsub_rn(__fadd_rd(l, 8388608.0f), 8388608.0f);
+  const uint32_t ceil_p = __float_as_uint(__fmul_ru(__fsub_rn(l, fl), __uint_as_float(0x01000000u)));
+  const float lev = (rnd >> 8) < ceil_p ? __fadd_rn(fl, 1.0f) : fl;
+  return fminf(lev, s);                    // l >= s, inf and nan inputs: s
+}
+// dq * (+-level); the FMA with +0 turns the -0 of a negative element of level zero into the +0 an integer level gives
+__device__ __forceinline__ float signed_value(float g, float level, float dq) {
+  return __fmaf_rn(dq, g < 0.0f ? -level : level, 0.0f);
+}
+
 // ---- row codec ------------------------------------------------------------------------------
 // A warp owns row `row` (elements row*128 .. row*128+127); lane owns the quad at 4*lane.
 // Magnitudes are stored in natural element order at MW bits each; bit planes as ballot words.

@@ -100,17 +100,19 @@ __global__ void __launch_bounds__(512) absmax_kernel(const float* __restrict__ x
   int64_t nq = (n + 3) / 4;
   int64_t stride = (int64_t)gridDim.x * blockDim.x;
   int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  // two independent quads per iteration keep more loads in flight
-  for (; q + stride < nq; q += 2 * stride) {
-    float4 a = load_quad(x, q * 4, n, aligned);
-    float4 b = load_quad(x, (q + stride) * 4, n, aligned);
-    m = fmaxf(m, fmaxf(fmaxf(abs_for_max(a.x), abs_for_max(a.y)), fmaxf(abs_for_max(a.z), abs_for_max(a.w))));
-    m = fmaxf(m, fmaxf(fmaxf(abs_for_max(b.x), abs_for_max(b.y)), fmaxf(abs_for_max(b.z), abs_for_max(b.w))));
+  // four independent quads per iteration: 128 KB in flight per SM (with two, 30 M elements took 34 us)
+  for (; q + 3 * stride < nq; q += 4 * stride) {
+    float4 a[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) a[u] = load_quad(x, (q + u * stride) * 4, n, aligned);
+#pragma unroll
+    for (int u = 0; u < 4; ++u) m = max_nan(max_nan(max_nan(max_nan(m, a[u].x), a[u].y), a[u].z), a[u].w);
   }
-  if (q < nq) {
-    float4 a = load_quad(x, q * 4, n, aligned);
-    m = fmaxf(m, fmaxf(fmaxf(abs_for_max(a.x), abs_for_max(a.y)), fmaxf(abs_for_max(a.z), abs_for_max(a.w))));
+  for (; q < nq; q += stride) {
+    const float4 a = load_quad(x, q * 4, n, aligned);
+    m = max_nan(max_nan(max_nan(max_nan(m, a.x), a.y), a.z), a.w);
   }
+  m = abs_for_max(m);
   m = block_max(m, smem);
   if (threadIdx.x == 0) {
     scratch->partial[blockIdx.x] = m;
@@ -132,43 +134,90 @@ __global__ void __launch_bounds__(512) absmax_kernel(const float* __restrict__ x
 }
 
 // --------------------------------------------------------------------------- quantise to level containers
-template <typename OUT>
-__global__ void quantize_levels_kernel(const float* __restrict__ x, int64_t n, bool aligned,
-                                       const float* __restrict__ norm_ptr, int s, int mode, RngKey key,
-                                       OUT* __restrict__ out) {
-  float norm = *norm_ptr;
-  float scale = (norm > 0.0f) ? (float)s / norm : 0.0f;
-  int64_t nq = (n + 3) / 4;
-  int64_t stride = (int64_t)gridDim.x * blockDim.x;
+// Four level containers as one 4-, 8- or 16-byte access.
+template <typename T> struct Quad;
+template <> struct Quad<int8_t> { typedef char4 type; };
+template <> struct Quad<int16_t> { typedef short4 type; };
+template <> struct Quad<int32_t> { typedef int4 type; };
+
+template <typename T>
+__device__ __forceinline__ void store_levels(T* out, int64_t e0, int64_t n, bool aligned, const int (&q)[4]) {
+  if (aligned && e0 + 3 < n) {
+    typename Quad<T>::type v;
+    v.x = (T)q[0]; v.y = (T)q[1]; v.z = (T)q[2]; v.w = (T)q[3];
+    *reinterpret_cast<typename Quad<T>::type*>(out + e0) = v;
+    return;
+  }
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+    if (e0 + j < n) out[e0 + j] = (T)q[j];
+}
+template <typename T>
+__device__ __forceinline__ void load_levels(const T* in, int64_t e0, int64_t n, bool aligned, int (&q)[4]) {
+  if (aligned && e0 + 3 < n) {
+    const typename Quad<T>::type v = *reinterpret_cast<const typename Quad<T>::type*>(in + e0);
+    q[0] = v.x; q[1] = v.y; q[2] = v.z; q[3] = v.w;
+    return;
+  }
+#pragma unroll
+  for (int j = 0; j < 4; ++j) q[j] = e0 + j < n ? (int)in[e0 + j] : 0;
+}
+
+// Stochastic level as an integer, for s < 2^22 (round_level's float is then exact in the low mantissa bits).
+__device__ __forceinline__ int quantize_fast(float g, float scale, float s, uint32_t rnd) {
+  const float lev = round_level(g, scale, s, rnd);
+  const int q = (int)(__float_as_uint(__fadd_rn(lev, 8388608.0f)) & 0x7fffffu);
+  return g < 0.0f ? -q : q;
+}
+
+constexpr int MODE_FAST = 4;       // mode 0 with s < 2^22
+
+// One quad per thread and iteration.  The mode is a template parameter, levels leave as one access per quad (they left byte by
+// byte), and the stochastic mode rounds without int <-> float conversions.  FIT: also mask[i] = |level| <= fit.
+template <typename OUT, int MODE, bool FIT>
+__global__ void __launch_bounds__(256) quantize_levels_kernel(const float* __restrict__ x, int64_t n, bool al_in, bool al_out,
+                                                              const float* __restrict__ norm_ptr, int s, RngKey key, OUT* __restrict__ out, int fit,
+                                                              int8_t* __restrict__ mask) {
+  const float norm = *norm_ptr, sf = (float)s;
+  const float scale = (norm > 0.0f) ? sf / norm : 0.0f;
+  const int64_t nq = (n + 3) / 4, stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t qd = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; qd < nq; qd += stride) {
-    int64_t e0 = qd * 4;
-    float4 v = load_quad(x, e0, n, aligned);
-    U4 r = (mode == 0 || mode == 2) ? philox_block(key, (uint64_t)qd) : U4{0, 0, 0, 0};
-    float g[4] = {v.x, v.y, v.z, v.w};
-    uint32_t rr[4] = {r.x, r.y, r.z, r.w};
+    const int64_t e0 = qd * 4;
+    const float4 v = load_quad(x, e0, n, al_in);
+    const U4 r = (MODE == 0 || MODE == 2 || MODE == MODE_FAST) ? philox_block(key, (uint64_t)qd) : U4{0, 0, 0, 0};
+    const float g[4] = {v.x, v.y, v.z, v.w};
+    const uint32_t rr[4] = {r.x, r.y, r.z, r.w};
     int q[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      switch (mode) {
-        case 0: q[j] = quantize_level(g[j], scale, s, rr[j]); break;
-        case 1: q[j] = quantize_level_biased(g[j], scale, s); break;
-        case 2: q[j] = quantize_level_nu(g[j], scale, s, rr[j], false); break;
-        default: q[j] = quantize_level_nu(g[j], scale, s, rr[j], true); break;
-      }
+      if (MODE == MODE_FAST) q[j] = quantize_fast(g[j], scale, sf, rr[j]);
+      else if (MODE == 0) q[j] = quantize_level(g[j], scale, s, rr[j]);
+      else if (MODE == 1) q[j] = quantize_level_biased(g[j], scale, s);
+      else q[j] = quantize_level_nu(g[j], scale, s, rr[j], MODE == 3);
     }
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-      if (e0 + j < n) out[e0 + j] = (OUT)q[j];
+    store_levels(out, e0, n, al_out, q);
+    if (FIT) {
+      const int f[4] = {abs(q[0]) <= fit, abs(q[1]) <= fit, abs(q[2]) <= fit, abs(q[3]) <= fit};
+      store_levels(mask, e0, n, al_out, f);
+    }
   }
 }
 
-template <typename IN>
-__global__ void dequantize_levels_kernel(const IN* __restrict__ q, int64_t n, const float* __restrict__ norm_ptr,
-                                         int s, int world, float* __restrict__ out) {
-  float sc = dequant_scale(*norm_ptr, s, world);
-  int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride)
-    out[i] = mul_rn(sc, (float)q[i]);
+// TWO: the scale of an element is `s` where mask is set, `s_other` elsewhere.
+template <typename IN, bool TWO>
+__global__ void __launch_bounds__(256) dequantize_levels_kernel(const IN* __restrict__ q, int64_t n, bool al_in, bool al_out,
+                                                                const float* __restrict__ norm_ptr, int s, int world, float* __restrict__ out,
+                                                                const int8_t* __restrict__ mask, int s_other) {
+  const float sc = dequant_scale(*norm_ptr, s, world), other = TWO ? dequant_scale(*norm_ptr, s_other, world) : 0.0f;
+  const int64_t nq = (n + 3) / 4, stride = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t qd = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; qd < nq; qd += stride) {
+    const int64_t e0 = qd * 4;
+    int v[4], f[4] = {1, 1, 1, 1};
+    load_levels(q, e0, n, al_in, v);
+    if (TWO) load_levels(mask, e0, n, al_in, f);
+    store_quad(out, e0, n, al_out, make_float4(mul_rn(f[0] ? sc : other, (float)v[0]), mul_rn(f[1] ? sc : other, (float)v[1]),
+                                               mul_rn(f[2] ? sc : other, (float)v[2]), mul_rn(f[3] ? sc : other, (float)v[3])));
+  }
 }
 
 // --------------------------------------------------------------------------- quantise + pack (wire layout)
@@ -390,29 +439,63 @@ int gc_cuda_absmax(const float* x, int64_t n, void* scratch, float* out, void* c
   return GC_LAUNCH_CHECK();
 }
 
+#define GC_DISPATCH_LEVELS(size, CALL)           \
+  switch (size) {                                \
+    case 1: { typedef int8_t T; CALL; } break;   \
+    case 2: { typedef int16_t T; CALL; } break;  \
+    case 4: { typedef int32_t T; CALL; } break;  \
+    default: return (int)cudaErrorInvalidValue;  \
+  }
+
 int gc_cuda_quantize_levels(const float* x, int64_t n, const float* norm_ptr, int s, int mode, uint64_t seed,
                             uint32_t stream_id, uint32_t step, void* out, int out_elem_size, void* cs) {
   if (n <= 0) return 0;
-  RngKey key = make_key(seed, stream_id, step);
-  int threads = 256, grid = grid_for((n + 3) / 4, threads, 8);
+  const RngKey key = make_key(seed, stream_id, step);
+  const int threads = 256, grid = grid_for((n + 3) / 4, threads, 8);
   cudaStream_t st = (cudaStream_t)cs;
-  bool al = aligned16(x);
-  if (out_elem_size == 1) quantize_levels_kernel<int8_t><<<grid, threads, 0, st>>>(x, n, al, norm_ptr, s, mode, key, (int8_t*)out);
-  else if (out_elem_size == 2) quantize_levels_kernel<int16_t><<<grid, threads, 0, st>>>(x, n, al, norm_ptr, s, mode, key, (int16_t*)out);
-  else if (out_elem_size == 4) quantize_levels_kernel<int32_t><<<grid, threads, 0, st>>>(x, n, al, norm_ptr, s, mode, key, (int32_t*)out);
-  else return (int)cudaErrorInvalidValue;
+  const bool al = aligned16(x), alo = aligned16(out);
+  if (mode == 0 && s < (1 << 22)) mode = MODE_FAST;
+#define GC_MODE(M) GC_DISPATCH_LEVELS(out_elem_size, (quantize_levels_kernel<T, M, false><<<grid, threads, 0, st>>>(x, n, al, alo, norm_ptr, s, key, (T*)out, 0, nullptr)))
+  if (mode == MODE_FAST) GC_MODE(MODE_FAST)
+  else if (mode == 0) GC_MODE(0)
+  else if (mode == 1) GC_MODE(1)
+  else if (mode == 2) GC_MODE(2)
+  else GC_MODE(3)
+#undef GC_MODE
+  return GC_LAUNCH_CHECK();
+}
+
+// Levels of the higher scale together with mask[i] = 1 where the level fits s_fit (s < 2^22).
+int gc_cuda_quantize_fit(const float* x, int64_t n, const float* norm_ptr, int s, int s_fit, uint64_t seed, uint32_t stream_id, uint32_t step, void* out,
+                         int out_elem_size, int8_t* mask, void* cs) {
+  if (n <= 0) return 0;
+  if (s >= (1 << 22)) return (int)cudaErrorInvalidValue;
+  const RngKey key = make_key(seed, stream_id, step);
+  const int threads = 256, grid = grid_for((n + 3) / 4, threads, 8);
+  const bool al = aligned16(x), alo = aligned16(out) && aligned16(mask);
+  GC_DISPATCH_LEVELS(out_elem_size,
+                     (quantize_levels_kernel<T, MODE_FAST, true><<<grid, threads, 0, (cudaStream_t)cs>>>(x, n, al, alo, norm_ptr, s, key, (T*)out, s_fit, mask)))
   return GC_LAUNCH_CHECK();
 }
 
 int gc_cuda_dequantize_levels(const void* q, int elem_size, int64_t n, const float* norm_ptr, int s, int world,
                               float* out, void* cs) {
   if (n <= 0) return 0;
-  int threads = 256, grid = grid_for(n, threads, 8);
-  cudaStream_t st = (cudaStream_t)cs;
-  if (elem_size == 1) dequantize_levels_kernel<int8_t><<<grid, threads, 0, st>>>((const int8_t*)q, n, norm_ptr, s, world, out);
-  else if (elem_size == 2) dequantize_levels_kernel<int16_t><<<grid, threads, 0, st>>>((const int16_t*)q, n, norm_ptr, s, world, out);
-  else if (elem_size == 4) dequantize_levels_kernel<int32_t><<<grid, threads, 0, st>>>((const int32_t*)q, n, norm_ptr, s, world, out);
-  else return (int)cudaErrorInvalidValue;
+  const int threads = 256, grid = grid_for((n + 3) / 4, threads, 8);
+  const bool al = aligned16(q), alo = aligned16(out);
+  GC_DISPATCH_LEVELS(elem_size,
+                     (dequantize_levels_kernel<T, false><<<grid, threads, 0, (cudaStream_t)cs>>>((const T*)q, n, al, alo, norm_ptr, s, world, out, nullptr, 0)))
+  return GC_LAUNCH_CHECK();
+}
+
+// Levels of two scales: s_hi where mask is set, s_lo elsewhere.
+int gc_cuda_dequantize_two(const void* q, int elem_size, const int8_t* mask, int64_t n, const float* norm_ptr, int s_hi, int s_lo, int world, float* out,
+                           void* cs) {
+  if (n <= 0) return 0;
+  const int threads = 256, grid = grid_for((n + 3) / 4, threads, 8);
+  const bool al = aligned16(q) && aligned16(mask), alo = aligned16(out);
+  GC_DISPATCH_LEVELS(elem_size,
+                     (dequantize_levels_kernel<T, true><<<grid, threads, 0, (cudaStream_t)cs>>>((const T*)q, n, al, alo, norm_ptr, s_hi, world, out, mask, s_lo)))
   return GC_LAUNCH_CHECK();
 }
 

@@ -37,6 +37,12 @@ struct Api {
   int (*topk_run)(const void*, int, int64_t, const int64_t*, int, float*, void*, void*, int32_t*, float*, void*);
   int (*psgd_solo)(int, const void*, int, float*, const int64_t*, int, int64_t, int64_t, int, const int64_t*, int, float*, float*, float*, int64_t, uint64_t,
                    uint32_t, uint32_t*, void*);
+  int64_t (*absmax_scratch_bytes)();
+  int (*absmax)(const float*, int64_t, void*, float*, void*);
+  int (*quantize)(const float*, int64_t, const float*, int, int, uint64_t, uint32_t, uint32_t, void*, int, void*);
+  int (*quantize_fit)(const float*, int64_t, const float*, int, int, uint64_t, uint32_t, uint32_t, void*, int, int8_t*, void*);
+  int (*dequantize)(const void*, int, int64_t, const float*, int, int, float*, void*);
+  int (*dequantize_two)(const void*, int, const int8_t*, int64_t, const float*, int, int, int, float*, void*);
 } api;
 int max_segs = 0;
 
@@ -49,6 +55,12 @@ const Entry entries[] = {
     {"gc_solo_randk", (void**)&api.solo_randk},
     {"gc_cuda_topk_run", (void**)&api.topk_run},
     {"gc_cuda_psgd_solo", (void**)&api.psgd_solo},
+    {"gc_cuda_absmax_scratch_bytes", (void**)&api.absmax_scratch_bytes},
+    {"gc_cuda_absmax", (void**)&api.absmax},
+    {"gc_cuda_quantize_levels", (void**)&api.quantize},
+    {"gc_cuda_quantize_fit", (void**)&api.quantize_fit},
+    {"gc_cuda_dequantize_levels", (void**)&api.dequantize},
+    {"gc_cuda_dequantize_two", (void**)&api.dequantize_two},
 };
 
 // What one reducer saw last: its segment table, and the fact that its inputs and outputs do not overlap in an unsafe way
@@ -289,6 +301,97 @@ PyObject* solo_topk(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   Py_RETURN_NONE;
 }
 
+// ---- codecs ------------------------------------------------------------------------------------------------------
+// Each returns None where a tensor is not the kernel's case (the caller then takes its general path).
+
+const at::Tensor* tensor_of(PyObject* o) { return THPVariable_Check(o) ? &THPVariable_Unpack(o) : nullptr; }
+
+const at::Tensor* plain(PyObject* o, at::ScalarType type) {
+  const at::Tensor* t = tensor_of(o);
+  return t && t->is_cuda() && t->scalar_type() == type && t->layout() == at::kStrided && t->is_contiguous() ? t : nullptr;
+}
+
+int level_size(at::ScalarType t) { return t == at::kChar ? 1 : t == at::kShort ? 2 : t == at::kInt ? 4 : 0; }
+at::ScalarType level_type(int64_t size) { return size == 1 ? at::kChar : size == 2 ? at::kShort : at::kInt; }
+
+// absmax(x, out or None) -> one-element tensor
+PyObject* absmax(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
+  if (!want(nargs, 2, "absmax")) return nullptr;
+  const at::Tensor* x = plain(a[0], at::kFloat);
+  const at::Tensor* given = a[1] == Py_None ? nullptr : plain(a[1], at::kFloat);
+  if (!x || x->numel() == 0 || (a[1] != Py_None && !given)) Py_RETURN_NONE;
+  const int dev = x->device().index();
+  if (dev >= 64 || (given && given->device() != x->device())) Py_RETURN_NONE;
+  c10::cuda::OptionalCUDAGuard guard(x->device());
+  static at::Tensor scratch[64];           // zeroed once; the kernel leaves it ready for the next call
+  if (!scratch[dev].defined()) scratch[dev] = at::zeros({api.absmax_scratch_bytes()}, x->options().dtype(at::kByte));
+  at::Tensor out = given ? *given : at::empty({1}, x->options());
+  const int err = api.absmax((const float*)x->data_ptr(), x->numel(), scratch[dev].data_ptr(), (float*)out.data_ptr(), stream_on(dev));
+  if (err) return cuda_error("absmax", err);
+  return THPVariable_Wrap(out);
+}
+
+// quantize(x, norm, s, mode, seed, stream, step, size, out or None) -> levels
+PyObject* quantize(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
+  if (!want(nargs, 9, "quantize")) return nullptr;
+  const at::Tensor *x = plain(a[0], at::kFloat), *norm = plain(a[1], at::kFloat), *given = a[8] == Py_None ? nullptr : tensor_of(a[8]);
+  if (!x || !norm || norm->numel() != 1 || norm->device() != x->device() || x->numel() == 0) Py_RETURN_NONE;
+  const int64_t s = as_int(a[2]), mode = as_int(a[3]), size = as_int(a[7]);
+  const uint64_t seed = PyLong_AsUnsignedLongLongMask(a[4]);
+  const uint32_t stream = (uint32_t)PyLong_AsUnsignedLongLongMask(a[5]), step = (uint32_t)PyLong_AsUnsignedLongLongMask(a[6]);
+  if (PyErr_Occurred()) return nullptr;
+  if (given && (!given->is_cuda() || !given->is_contiguous() || given->device() != x->device() || level_size(given->scalar_type()) != size)) Py_RETURN_NONE;
+  c10::cuda::OptionalCUDAGuard guard(x->device());
+  at::Tensor out = given ? *given : at::empty({x->numel()}, x->options().dtype(level_type(size)));
+  const int err = api.quantize((const float*)x->data_ptr(), x->numel(), (const float*)norm->data_ptr(), (int)s, (int)mode, seed, stream, step, out.data_ptr(),
+                               (int)size, stream_on(x->device().index()));
+  if (err) return cuda_error("quantize_levels", err);
+  return THPVariable_Wrap(out);
+}
+
+// quantize_fit(x, norm, s, s_fit, seed, stream, step, size) -> (levels, int8 mask of those that fit s_fit)
+PyObject* quantize_fit(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
+  if (!want(nargs, 8, "quantize_fit")) return nullptr;
+  const at::Tensor *x = plain(a[0], at::kFloat), *norm = plain(a[1], at::kFloat);
+  const int64_t s = as_int(a[2]), fit = as_int(a[3]), size = as_int(a[7]);
+  const uint64_t seed = PyLong_AsUnsignedLongLongMask(a[4]);
+  const uint32_t stream = (uint32_t)PyLong_AsUnsignedLongLongMask(a[5]), step = (uint32_t)PyLong_AsUnsignedLongLongMask(a[6]);
+  if (PyErr_Occurred()) return nullptr;
+  if (!x || !norm || norm->numel() != 1 || norm->device() != x->device() || x->numel() == 0 || s >= (1 << 22)) Py_RETURN_NONE;
+  c10::cuda::OptionalCUDAGuard guard(x->device());
+  at::Tensor out = at::empty({x->numel()}, x->options().dtype(level_type(size))), mask = at::empty({x->numel()}, x->options().dtype(at::kChar));
+  const int err = api.quantize_fit((const float*)x->data_ptr(), x->numel(), (const float*)norm->data_ptr(), (int)s, (int)fit, seed, stream, step,
+                                   out.data_ptr(), (int)size, (int8_t*)mask.data_ptr(), stream_on(x->device().index()));
+  if (err) return cuda_error("quantize_fit", err);
+  PyObject *po = THPVariable_Wrap(out), *pm = THPVariable_Wrap(mask);
+  PyObject* r = PyTuple_Pack(2, po, pm);
+  Py_XDECREF(po);
+  Py_XDECREF(pm);
+  return r;
+}
+
+// dequantize(q, mask or None, norm, s, s_other, world, out or None) -> values
+PyObject* dequantize(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
+  if (!want(nargs, 7, "dequantize")) return nullptr;
+  const at::Tensor *q = tensor_of(a[0]), *mask = a[1] == Py_None ? nullptr : plain(a[1], at::kChar), *norm = plain(a[2], at::kFloat);
+  const at::Tensor* given = a[6] == Py_None ? nullptr : plain(a[6], at::kFloat);
+  const int64_t s = as_int(a[3]), other = as_int(a[4]), world = as_int(a[5]);
+  if (PyErr_Occurred()) return nullptr;
+  if (!q || !q->is_cuda() || !q->is_contiguous() || q->numel() == 0 || !level_size(q->scalar_type()) || !norm || norm->numel() != 1 ||
+      norm->device() != q->device() || (a[1] != Py_None && (!mask || mask->numel() != q->numel() || mask->device() != q->device())) ||
+      (a[6] != Py_None && (!given || given->numel() != q->numel() || given->device() != q->device())))
+    Py_RETURN_NONE;
+  c10::cuda::OptionalCUDAGuard guard(q->device());
+  at::Tensor out = given ? *given : at::empty({q->numel()}, norm->options());
+  const int size = level_size(q->scalar_type());
+  void* st = stream_on(q->device().index());
+  const int err = mask ? api.dequantize_two(q->data_ptr(), size, (const int8_t*)mask->data_ptr(), q->numel(), (const float*)norm->data_ptr(), (int)s, (int)other,
+                                            (int)world, (float*)out.data_ptr(), st)
+                       : api.dequantize(q->data_ptr(), size, q->numel(), (const float*)norm->data_ptr(), (int)s, (int)world, (float*)out.data_ptr(), st);
+  if (err) return cuda_error("dequantize_levels", err);
+  return THPVariable_Wrap(out);
+}
+
 // bind({name: address}): the kernel library's entry points
 PyObject* bind(PyObject*, PyObject* table) {
   for (const Entry& e : entries) {
@@ -322,6 +425,10 @@ PyMethodDef methods[] = {
     {"solo_randk_limit", (PyCFunction)(void (*)(void))solo_randk_limit, METH_FASTCALL, "most coordinates solo_randk takes"},
     {"solo_psgd", (PyCFunction)(void (*)(void))solo_psgd, METH_FASTCALL, "PowerSGD step of a single worker"},
     {"solo_topk", (PyCFunction)(void (*)(void))solo_topk, METH_FASTCALL, "top-k with error feedback of a single worker"},
+    {"absmax", (PyCFunction)(void (*)(void))absmax, METH_FASTCALL, "largest magnitude"},
+    {"quantize", (PyCFunction)(void (*)(void))quantize, METH_FASTCALL, "levels of a vector"},
+    {"quantize_fit", (PyCFunction)(void (*)(void))quantize_fit, METH_FASTCALL, "levels of the higher scale and where they fit the lower one"},
+    {"dequantize", (PyCFunction)(void (*)(void))dequantize, METH_FASTCALL, "values of levels of one or two scales"},
     {nullptr, nullptr, 0, nullptr}};
 
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "gcb200_ext", "native front end of the reducers", -1, methods};

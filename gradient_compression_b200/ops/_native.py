@@ -115,6 +115,8 @@ def cuda():
         _declare(lib, "gc_cuda_absmax", c_int, [P, c_i64, P, P, P])
         _declare(lib, "gc_cuda_quantize_levels", c_int, [P, c_i64, P, c_int, c_int, c_u64, c_u32, c_u32, P, c_int, P])
         _declare(lib, "gc_cuda_dequantize_levels", c_int, [P, c_int, c_i64, P, c_int, c_int, P, P])
+        _declare(lib, "gc_cuda_quantize_fit", c_int, [P, c_i64, P, c_int, c_int, c_u64, c_u32, c_u32, P, c_int, P, P])
+        _declare(lib, "gc_cuda_dequantize_two", c_int, [P, c_int, P, c_i64, P, c_int, c_int, c_int, P, P])
         _declare(lib, "gc_cuda_qsgd_pack", c_int, [P, c_i64, P, c_int, c_u64, c_u32, c_u32, P, P, P])
         _declare(lib, "gc_cuda_qsgd_unpack_dequant", c_int, [P, P, c_i64, P, c_int, c_int, P, P])
         _declare(lib, "gc_cuda_pack_levels", c_int, [P, c_i64, c_int, P, P, P])

@@ -7,6 +7,7 @@ import torch
 from . import _native as nat
 
 MODE_STOCHASTIC, MODE_BIASED, MODE_NU, MODE_NU_BIASED = 0, 1, 2, 3
+_LEVEL_BYTES = {torch.int8: 1, torch.int16: 2, torch.int32: 4}
 _scratch = {}
 
 
@@ -44,6 +45,11 @@ def absmax(x, out=None):
 
     Reference: ``flat_grad.buffer.abs().max()`` (reducer.py:516) -- two kernels and a temporary there.
     """
+    if x.is_cuda:
+        r = nat.ext().absmax(x, out)
+        if r is not None:
+            nat.count_launch()
+            return r
     x = _flat32(x)
     if out is None:
         out = torch.zeros(1, dtype=torch.float32, device=x.device)
@@ -71,6 +77,11 @@ def quantize_levels(x, norm, s, seed=0, stream=0, step=0, mode=MODE_STOCHASTIC, 
     ``mode`` 0/1: uniform levels (compressors.py:299-316 / :562-568), 2/3: power-of-two levels with
     s = 2**b (compressors.py:520-541 / :593-603).  ``dtype`` is the container (int8/int16/int32).
     """
+    if x.is_cuda and torch.is_tensor(norm):
+        r = nat.ext().quantize(x, norm, s, mode, seed, stream, step, _LEVEL_BYTES.get(dtype if out is None else out.dtype, 0), out)
+        if r is not None:
+            nat.count_launch()
+            return r
     x = _flat32(x)
     n = x.numel()
     if out is None:
@@ -94,6 +105,11 @@ def quantize_levels(x, norm, s, seed=0, stream=0, step=0, mode=MODE_STOCHASTIC, 
 
 def dequantize_levels(q, norm, s, world=1, out=None):
     """fp32 ``norm / (s * world) * q`` (compressors.py:318-321 with the 1/W average folded in)."""
+    if q.is_cuda and torch.is_tensor(norm):
+        r = nat.ext().dequantize(q, None, norm, s, 0, world, out)
+        if r is not None:
+            nat.count_launch()
+            return r
     q = q.contiguous().view(-1)
     n = q.numel()
     if out is None:
@@ -110,6 +126,29 @@ def dequantize_levels(q, norm, s, world=1, out=None):
         q32 = q if q.dtype == torch.int32 else q.to(torch.int32)
         nat.host().gc_host_dequantize_levels(q32.data_ptr(), n, float(norm), int(s), int(world), out.data_ptr())
     return out
+
+
+def quantize_fit(x, norm, s, s_fit, seed=0, stream=0, step=0, dtype=torch.int32):
+    """``(levels, mask)``: stochastic levels of scale ``s`` in ``dtype``, and an int8 mask of those within ``[-s_fit, s_fit]``
+    (the two-scale codec's higher scale, compressors.py:640-661)."""
+    if x.is_cuda and torch.is_tensor(norm):
+        r = nat.ext().quantize_fit(x, norm, s, s_fit, seed, stream, step, _LEVEL_BYTES[dtype])
+        if r is not None:
+            nat.count_launch()
+            return r
+    q = quantize_levels(x, norm, s, seed, stream, step, dtype=torch.int32)
+    return q.to(dtype), (q.abs() <= s_fit).to(torch.int8)
+
+
+def dequantize_two(q, mask, norm, s_hi, s_lo, world=1):
+    """``dequantize_levels`` with scale ``s_hi`` where ``mask`` is set and ``s_lo`` elsewhere."""
+    if q.is_cuda and torch.is_tensor(norm):
+        r = nat.ext().dequantize(q, mask, norm, s_hi, s_lo, world, None)
+        if r is not None:
+            nat.count_launch()
+            return r
+    # both candidates come from the native dequantiser so CPU, GPU and the fused kernel agree bit for bit
+    return torch.where(mask.bool(), dequantize_levels(q, norm, s_hi, world), dequantize_levels(q, norm, s_lo, world))
 
 
 def packed_sizes(n, bits):

@@ -183,3 +183,25 @@ def test_randk(name, K, bits, unselected, sizes, layout):
         for w, g in zip(want, outs):
             assert torch.equal(w, g.cpu())
     assert gpu.state_dict()["queue"]["position"] % sum(SIZES[sizes]) == cpu.state_dict()["queue"]["position"] % sum(SIZES[sizes])
+
+
+@pytest.mark.parametrize("n", [1, 3, 4, 5, 1023, 4096, 148 * 8 * 1024 + 1])
+@pytest.mark.parametrize("shift", [0, 1])
+@pytest.mark.parametrize("s", [1, 3, 127, 255, 65535, (1 << 22) - 1, 1 << 22])
+def test_level_kernels(n, shift, s):
+    from gradient_compression_b200 import ops
+
+    host = _values([n + shift], 8)[0][shift:].contiguous()
+    dev = torch.cat([torch.zeros(1), host]).cuda()[1:] if shift else host.cuda()
+    norm = ops.absmax(host) * 0.75           # some values beyond the largest level
+    for dtype in (torch.int8, torch.int16, torch.int32):
+        want = ops.quantize_levels(host, norm, s, 5, 9, 2, dtype=torch.int32)
+        got = ops.quantize_levels(dev, norm.cuda(), s, 5, 9, 2, dtype=dtype)
+        assert torch.equal(got.cpu(), want.to(dtype))
+        assert torch.equal(ops.dequantize_levels(got, norm.cuda(), s, 3).cpu(), ops.dequantize_levels(want.to(dtype).to(torch.int32), norm, s, 3))
+        q, mask = ops.quantize_fit(dev, norm.cuda(), s, s // 4, 5, 9, 2, dtype=dtype)
+        assert torch.equal(q.cpu(), want.to(dtype)) and torch.equal(mask.cpu(), (want.abs() <= s // 4).to(torch.int8))
+        two = ops.dequantize_two(q, mask, norm.cuda(), s, s // 4 + 1, 2).cpu()
+        fine, coarse = (ops.dequantize_levels(q.cpu().to(torch.int32), norm, l, 2) for l in (s, s // 4 + 1))
+        assert torch.equal(two, torch.where(mask.cpu().bool(), fine, coarse))
+    assert torch.equal(ops.absmax(dev).cpu(), ops.absmax(host))
