@@ -22,7 +22,7 @@ LIBDIR = os.path.join(HERE, "_lib")
 
 HOST_SOURCES = ["host_oracle.cpp"]
 EXT_SOURCES = ["pyext.cpp"]
-CUDA_SOURCES = ["gc_kernels.cu", "gc_fused.cu", "gc_solo.cu", "gc_noalloc.cu", "gc_bn.cu", "gc_head.cu", "gc_powersgd.cu", "gc_topk.cu", "gc_gemm_tc.cu", "gc_conv_tc.cu", "gc_varpack.cu", "gc_augment.cu"]
+CUDA_SOURCES = ["gc_kernels.cu", "gc_fused.cu", "gc_solo.cu", "gc_noalloc.cu", "gc_bn.cu", "gc_bn_fused.cu", "gc_head.cu", "gc_powersgd.cu", "gc_topk.cu", "gc_gemm_tc.cu", "gc_conv_tc.cu", "gc_varpack.cu", "gc_augment.cu"]
 NVCC_ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
 

@@ -136,10 +136,11 @@ int gc_cuda_conv_fwd_supported(int N, int H, int W, int Cin, int Cout, int R, in
 }
 
 // y[N*Ho*Wo, Cout] (=, += when accumulate) conv(x[N, H, W, Cin], w[Cout, R*R*Cin]) (+ bias[Cout]); x, w, y 16-byte aligned.
-// col_partials (may be NULL): [ceil(N*Ho*Wo / 128)][2][Cout] per-tile column sums and sums of squares of y.
+// col_partials (may be NULL): [ceil(N*Ho*Wo / 128)][2][Cout] per-tile column sums and sums of squares of y; with cta_sums
+// [gc_cuda_conv_stat_rows()][2][Cout], one row per CTA of a column tile.
 // bn_fin (may be NULL): a BnFinHost; the kernel then finishes the batch-norm statistics of y itself.
 int gc_cuda_conv_fwd(const float* x, const float* w, float* y, const float* bias, int N, int H, int W, int Cin, int Cout, int R,
-                     int stride, int pad, int accumulate, float* col_partials, int* error_flag, void* cs, const void* bn_fin) {
+                     int stride, int pad, int accumulate, float* col_partials, int* error_flag, void* cs, const void* bn_fin, int cta_sums) {
   Shape s;
   if (!make_shape(N, H, W, Cin, Cout, R, stride, pad, &s) || !fwd_ok(s)) return (int)cudaErrorInvalidValue;
   if ((reinterpret_cast<uintptr_t>(x) & 15u) || (reinterpret_cast<uintptr_t>(w) & 15u) || (reinterpret_cast<uintptr_t>(y) & 15u))
@@ -164,11 +165,17 @@ int gc_cuda_conv_fwd(const float* x, const float* w, float* y, const float* bias
   }
   const int acc = (accumulate || splits > 1) ? 1 : 0;
   switch (tile) {
-    case 64: return launch_persistent_maps<64>(ma, mb, mc, ca, bias, M, Cout, K, acc, col_partials, error_flag, st, fin, nullptr, splits);
-    case 128: return launch_persistent_maps<128>(ma, mb, mc, ca, bias, M, Cout, K, acc, col_partials, error_flag, st, fin, nullptr, splits);
-    case 256: return launch_persistent_maps<256>(ma, mb, mc, ca, bias, M, Cout, K, acc, col_partials, error_flag, st, fin, nullptr, splits);
+    case 64: return launch_persistent_maps<64>(ma, mb, mc, ca, bias, M, Cout, K, acc, col_partials, error_flag, st, fin, nullptr, splits, cta_sums);
+    case 128: return launch_persistent_maps<128>(ma, mb, mc, ca, bias, M, Cout, K, acc, col_partials, error_flag, st, fin, nullptr, splits, cta_sums);
+    case 256: return launch_persistent_maps<256>(ma, mb, mc, ca, bias, M, Cout, K, acc, col_partials, error_flag, st, fin, nullptr, splits, cta_sums);
     default: return (int)cudaErrorInvalidValue;
   }
+}
+
+// Rows of col_partials that gc_cuda_conv_fwd (and, for R = 1 with stride 1, gc_cuda_gemm_tf32) writes with cta_sums; 0: not available.
+int gc_cuda_conv_stat_rows(int M, int Cout, int K) {
+  if (Cout <= 16) return 0;
+  return cta_sum_rows(M, Cout, gctc::tile_choice ? gctc::tile_choice : pick_bn_persistent(M, Cout, K));
 }
 
 // Contraction splits gc_cuda_conv_fwd would use for this shape if the caller gave up the in-kernel column statistics and

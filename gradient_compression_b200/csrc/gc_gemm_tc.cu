@@ -267,7 +267,7 @@ int launch(const float* A, const float* B, float* C, const float* bias, int M, i
 
 template <int BN>
 int launch_persistent(const float* A, const float* B, float* C, const float* bias, int M, int N, int K, int64_t lda,
-                      int64_t ldb, int64_t ldc, int accumulate, float* col_partials, int* error_flag, cudaStream_t st,
+                      int64_t ldb, int64_t ldc, int accumulate, float* col_partials, int* error_flag, cudaStream_t st, int cta_sums,
                       const BnFin* fin, int splits) {
   CUtensorMap ma, mb, mc;
   if (make_map(&ma, A, M, K, lda, BM) != 0 || make_map(&mb, B, N, K, ldb, BN) != 0 || make_map(&mc, C, M, N, ldc, BM) != 0)
@@ -277,7 +277,7 @@ int launch_persistent(const float* A, const float* B, float* C, const float* bia
     if (e != cudaSuccess) return (int)e;
   }
   return launch_persistent_maps<BN>(ma, mb, mc, ConvA{}, bias, M, N, K, (accumulate || splits > 1) ? 1 : 0, col_partials, error_flag,
-                                    st, fin, nullptr, splits);
+                                    st, fin, nullptr, splits, cta_sums);
 }
 
 template <int BN>
@@ -346,21 +346,21 @@ void gc_cuda_gemm_tf32_config(int kernel, int tile_n) {
 // 1 / sqrt(var + eps) into stats[2N], running statistics updated) instead of emitting col_partials.  Persistent kernel only.
 int gc_cuda_gemm_tf32(const float* A, const float* B, float* C, const float* bias, int M, int N, int K, int64_t lda,
                       int64_t ldb, int64_t ldc, int accumulate, float* col_partials, int* error_flag, void* cs,
-                      const void* bn_fin) {
+                      const void* bn_fin, int cta_sums) {
   if (!gc_cuda_gemm_tf32_supported(A, B, M, N, K, lda, ldb)) return (int)cudaErrorInvalidValue;
   cudaStream_t st = (cudaStream_t)cs;
   const BnFin fin_dev = bn_fin_from_host(bn_fin);
   const BnFin* fin = fin_dev.acc != nullptr ? &fin_dev : nullptr;
   bool persistent = (g_kernel_choice != 1 || accumulate || fin != nullptr) && N > 16 && tma_store_ok(C, ldc);
-  if ((accumulate || fin != nullptr) && !persistent) return (int)cudaErrorInvalidValue;
+  if ((accumulate || fin != nullptr || cta_sums) && !persistent) return (int)cudaErrorInvalidValue;
   if (persistent) {
     int bn = gctc::tile_choice ? gctc::tile_choice : pick_bn_persistent(M, N, K), splits = 1;
     if (col_partials == nullptr && fin == nullptr)
       plan_persistent(M, N, K, accumulate ? 0.0 : zero_cycles((int64_t)M * N), &bn, &splits);
     switch (bn) {
-      case 64: return launch_persistent<64>(A, B, C, bias, M, N, K, lda, ldb, ldc, accumulate, col_partials, error_flag, st, fin, splits);
-      case 128: return launch_persistent<128>(A, B, C, bias, M, N, K, lda, ldb, ldc, accumulate, col_partials, error_flag, st, fin, splits);
-      case 256: return launch_persistent<256>(A, B, C, bias, M, N, K, lda, ldb, ldc, accumulate, col_partials, error_flag, st, fin, splits);
+      case 64: return launch_persistent<64>(A, B, C, bias, M, N, K, lda, ldb, ldc, accumulate, col_partials, error_flag, st, cta_sums, fin, splits);
+      case 128: return launch_persistent<128>(A, B, C, bias, M, N, K, lda, ldb, ldc, accumulate, col_partials, error_flag, st, cta_sums, fin, splits);
+      case 256: return launch_persistent<256>(A, B, C, bias, M, N, K, lda, ldb, ldc, accumulate, col_partials, error_flag, st, cta_sums, fin, splits);
       default: return (int)cudaErrorInvalidValue;
     }
   }

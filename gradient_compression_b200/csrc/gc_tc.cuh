@@ -319,7 +319,7 @@ __global__ void __launch_bounds__(PERSISTENT_THREADS, 1)
 gemm_tf32_persistent_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
                             const __grid_constant__ CUtensorMap tma_c, const ConvA ca, const float* __restrict__ bias, int M, int N, int K,
                             int tiles_m, int tiles_n, int splits, int accumulate, float* __restrict__ col_partials,
-                            int* __restrict__ error_flag, int tma_mode, const BnFin fin, const ConvC cc) {
+                            int* __restrict__ error_flag, int tma_mode, const BnFin fin, const ConvC cc, int cta_sums) {
   using S = PSmem<BN>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -469,7 +469,7 @@ gemm_tf32_persistent_kernel(const __grid_constant__ CUtensorMap tma_a, const __g
     uint32_t lt = 0, sc = 0;                                   // tiles drained, slabs staged by this group
     const bool fin_on = fin.acc != nullptr;
     const bool want_sums = col_partials != nullptr || fin_on;
-    float run_a = 0.f, run_b = 0.f;                            // fin_on: this thread's column, summed over the CTA's tiles
+    float run_a = 0.f, run_b = 0.f;                            // fin_on, cta_sums: this thread's column, summed over the CTA's tiles
     bool drained_all = true;
     for (int t = blockIdx.x; t < total_items; t += gridDim.x, ++lt) {
       const int tile = t / splits;
@@ -571,7 +571,7 @@ gemm_tf32_persistent_kernel(const __grid_constant__ CUtensorMap tma_a, const __g
           if (gc < N) {
             float a = (my_colsum[c * 2] + my_colsum[(BN + c) * 2]) + (my_colsum[(2 * BN + c) * 2] + my_colsum[(3 * BN + c) * 2]);
             float b = (my_colsum[c * 2 + 1] + my_colsum[(BN + c) * 2 + 1]) + (my_colsum[(2 * BN + c) * 2 + 1] + my_colsum[(3 * BN + c) * 2 + 1]);
-            if (fin_on) {
+            if (fin_on || cta_sums) {
               run_a += a;
               run_b += b;
             } else {
@@ -580,6 +580,15 @@ gemm_tf32_persistent_kernel(const __grid_constant__ CUtensorMap tma_a, const __g
             }
           }
         }
+      }
+    }
+    if (cta_sums && drained_all && te < (SLABS / EPI_GROUPS) * 32) {
+      // one row of partial sums per CTA that stays on this column tile (instead of one per row tile)
+      const int gc = (int)(blockIdx.x % (unsigned)tiles_n) * BN + (grp + EPI_GROUPS * (te >> 5)) * 32 + (te & 31);
+      const int64_t row = (int64_t)(blockIdx.x / (unsigned)tiles_n) * 2;
+      if (gc < N) {
+        col_partials[row * N + gc] = run_a;
+        col_partials[(row + 1) * N + gc] = run_b;
       }
     }
     if (fin_on && drained_all) {
@@ -909,7 +918,7 @@ int make_map_mn3(CUtensorMap* map, const float* base, int64_t K, int64_t D, int6
 template <int BN>
 int launch_persistent_maps(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mc, const ConvA& ca, const float* bias,
                            int M, int N, int K, int accumulate, float* col_partials, int* error_flag, cudaStream_t st,
-                           const BnFin* fin = nullptr, const ConvC* cc = nullptr, int splits = 1) {
+                           const BnFin* fin = nullptr, const ConvC* cc = nullptr, int splits = 1, int cta_sums = 0) {
   using S = PSmem<BN>;
   static bool configured = false;
   if (!configured) {
@@ -931,10 +940,21 @@ int launch_persistent_maps(const CUtensorMap& ma, const CUtensorMap& mb, const C
     grid = grid / tiles_n * tiles_n;             // every CTA stays on one column tile
     f = *fin;
   }
+  if (cta_sums) {
+    if (col_partials == nullptr || splits > 1 || tiles_n > grid) return (int)cudaErrorInvalidValue;
+    grid = grid / tiles_n * tiles_n;
+  }
   gc::launch_pdl(gemm_tf32_persistent_kernel<BN>, dim3((unsigned)grid), dim3(PERSISTENT_THREADS), (size_t)S::TOTAL, st, ma, mb, mc, ca,
                  bias, M, N, K, tiles_m, tiles_n, splits, accumulate, col_partials, error_flag, gctc::tma_mode, f,
-                 cc != nullptr ? *cc : ConvC{0, 0});
+                 cc != nullptr ? *cc : ConvC{0, 0}, cta_sums);
   return (int)cudaGetLastError();
+}
+
+// Rows of partial sums a launch with cta_sums leaves for tiles of `bn` columns.
+inline int cta_sum_rows(int M, int N, int bn) {
+  const int64_t tiles_n = (N + bn - 1) / bn, total = (int64_t)((M + BM - 1) / BM) * tiles_n;
+  const int64_t grid = total < sm_count() ? total : sm_count();
+  return tiles_n > grid ? 0 : (int)(grid / tiles_n);
 }
 
 // Launch the split-K TN kernel on ready-made tensor maps.  At most tn_ctas_per_sm CTAs per SM over all tiles, at least

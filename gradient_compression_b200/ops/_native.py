@@ -159,7 +159,7 @@ def cuda():
         _declare(lib, "gc_cuda_topk_run", c_int, [P, c_int, c_i64, P, c_int, P, P, P, P, P, P])
         _declare(lib, "gc_cuda_batched_transpose", c_int, [P, c_int, c_i64, P])
         _declare(lib, "gc_cuda_gemm_tf32_supported", c_int, [P, P, c_int, c_int, c_int, c_i64, c_i64])
-        _declare(lib, "gc_cuda_gemm_tf32", c_int, [P, P, P, P, c_int, c_int, c_int, c_i64, c_i64, c_i64, c_int, P, P, P, P])
+        _declare(lib, "gc_cuda_gemm_tf32", c_int, [P, P, P, P, c_int, c_int, c_int, c_i64, c_i64, c_i64, c_int, P, P, P, P, c_int])
         _declare(lib, "gc_cuda_bn_fin_scratch_bytes", c_i64, [c_int])
         _declare(lib, "gc_cuda_gemm_tf32_m_tiles", c_int, [c_int])
         _declare(lib, "gc_cuda_gemm_tn_config", None, [c_int, c_int])
@@ -174,7 +174,12 @@ def cuda():
         _declare(lib, "gc_cuda_conv_dgrad", c_int, [P, P, P, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, P, P])
         _declare(lib, "gc_cuda_gemm_tf32_splits", c_int, [c_int] * 3)
         _declare(lib, "gc_cuda_tc_split_config", None, [c_int])
-        _declare(lib, "gc_cuda_conv_fwd", c_int, [P, P, P, P] + [c_int] * 9 + [P, P, P, P])
+        _declare(lib, "gc_cuda_conv_fwd", c_int, [P, P, P, P] + [c_int] * 9 + [P, P, P, P, c_int])
+        _declare(lib, "gc_cuda_conv_stat_rows", c_int, [c_int] * 3)
+        _declare(lib, "gc_cuda_bn_fused_supported", c_int, [c_i64, c_int])
+        _declare(lib, "gc_cuda_bn_fused_scratch_bytes", c_i64, [])
+        _declare(lib, "gc_cuda_bn_fused_forward", c_int, [P] + [c_int] * 5 + [P, c_int, P, P, P, c_int, P, P, c_float, c_float, P, P, P, P, P])
+        _declare(lib, "gc_cuda_bn_fused_backward", c_int, [P, P, P] + [c_int] * 5 + [P, P, P, c_int, P, P, P, P, P, P])
         _declare(lib, "gc_cuda_conv_dgrad_s2_supported", c_int, [c_int] * 7)
         _declare(lib, "gc_cuda_conv_dgrad_s2", c_int, [P, P, P] + [c_int] * 7 + [P, P])
         _declare(lib, "gc_cuda_conv_wgrad_supported", c_int, [c_int] * 8)

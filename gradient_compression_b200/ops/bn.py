@@ -81,6 +81,9 @@ def take_owned_grad(t):
     return r is not None and r() is t
 
 _scratch = {}
+# One launch per direction (csrc/gc_bn_fused.cu) where the channels come in groups of 32; off: separate reduction, finalize and apply.
+FUSED = os.environ.get("GCB200_BN_FUSED", "1") == "1"
+_fused_scratch = {}
 FUSED_BWD_FINALIZE = os.environ.get("GCB200_BN_FUSED_BWD_FINALIZE", "0") == "1"
 
 
@@ -92,6 +95,39 @@ def _scratch_for(device, channels):
         cur = torch.empty(max(need, nat.cuda().gc_cuda_bn_scratch_bytes(2048)), dtype=torch.uint8, device=device)
         _scratch[key] = cur
     return cur
+
+
+def fused_scratch(device):
+    """Barrier counts and partial sums of the one-launch kernels: zeroed once, every launch leaves them ready for the next."""
+    key = (device.type, device.index)
+    cur = _fused_scratch.get(key)
+    if cur is None:
+        cur = _fused_scratch[key] = torch.zeros(nat.cuda().gc_cuda_bn_fused_scratch_bytes(), dtype=torch.uint8, device=device)
+    return cur
+
+
+def fused_ok(m, c):
+    return FUSED and bool(nat.cuda().gc_cuda_bn_fused_supported(m, c))
+
+
+def fused_forward(x, pool, partials, gamma, beta, residual, relu, running_mean, running_var, momentum, eps, stats, y):
+    """Statistics (from the convolution's partial sums when given), running statistics and apply of ``x`` [N, C, H, W]."""
+    from . import gemm
+
+    n, c, h, w = x.shape
+    nat.check(nat.cuda().gc_cuda_bn_fused_forward(
+        x.data_ptr(), n, h, w, c, int(pool), nat.ptr(partials), partials.shape[0] if partials is not None else 0, gamma.data_ptr(), beta.data_ptr(),
+        nat.ptr(residual), int(relu), nat.ptr(running_mean), nat.ptr(running_var), float(momentum), float(eps), stats.data_ptr(), y.data_ptr(),
+        fused_scratch(x.device).data_ptr(), gemm._error_flag(x.device).data_ptr(), nat.stream_ptr()), "bn_fused_forward")
+
+
+def fused_backward(dy, x, y, pool, stats, gamma, beta, relu, sums, dx, dres):
+    from . import gemm
+
+    n, c, h, w = x.shape
+    nat.check(nat.cuda().gc_cuda_bn_fused_backward(
+        dy.data_ptr(), x.data_ptr(), nat.ptr(y), n, h, w, c, int(pool), stats.data_ptr(), gamma.data_ptr(), beta.data_ptr(), int(relu), sums.data_ptr(),
+        dx.data_ptr(), nat.ptr(dres), fused_scratch(x.device).data_ptr(), gemm._error_flag(x.device).data_ptr(), nat.stream_ptr()), "bn_fused_backward")
 
 
 def _fin_ptr(device, channels):
@@ -123,6 +159,13 @@ class _FusedBNAct(torch.autograd.Function):
         lib, st = nat.cuda(), nat.stream_ptr()
         stats = torch.empty(2 * c, dtype=torch.float32, device=x.device)
         with torch.cuda.device(x.device):
+            if training and fused_ok(m, c):
+                y = torch.empty_like(x)
+                fused_forward(x, False, None, weight, bias, _cl(residual) if residual is not None else None, relu, running_mean, running_var, momentum,
+                              eps, stats, y)
+                ctx.relu, ctx.has_res, ctx.training = bool(relu), residual is not None, True
+                ctx.save_for_backward(x, weight, bias, stats, y if (residual is not None and relu) else None)
+                return y
             if training:
                 nat.check(lib.gc_cuda_bn_stats(x.data_ptr(), m, c, _scratch_for(x.device, c).data_ptr(), stats.data_ptr(),
                                                nat.ptr(running_mean), nat.ptr(running_var), float(momentum), float(eps),
@@ -151,6 +194,12 @@ class _FusedBNAct(torch.autograd.Function):
         sums = torch.empty(2 * c, dtype=torch.float32, device=x.device)
         dx = torch.empty_like(x)
         dres = own_grad(torch.empty_like(x)) if (ctx.has_res and ctx.needs_input_grad[3]) else None
+        if fused_ok(m, c):
+            with torch.cuda.device(x.device):
+                fused_backward(dy, x, y, False, stats, weight, bias, ctx.relu, sums, dx, dres)
+            if ctx.has_res and dres is None and ctx.needs_input_grad[3]:
+                dres = dy
+            return dx, sums[c:], sums[:c], dres, None, None, None, None, None, None
         with torch.cuda.device(x.device):
             nat.check(lib.gc_cuda_bn_bwd_reduce(dy.data_ptr(), x.data_ptr(), nat.ptr(y), m, c, stats.data_ptr(),
                                                 weight.data_ptr(), bias.data_ptr(), int(ctx.relu),

@@ -33,7 +33,7 @@ import torch
 
 from . import _native as nat
 from . import gemm
-from .bn import _cl, _fin_ptr, _scratch_for, bn_act, count_batch, own_grad, take_owned_grad
+from .bn import _cl, _fin_ptr, _scratch_for, bn_act, fused_backward, fused_forward, fused_ok, count_batch, own_grad, take_owned_grad
 
 # GCB200_TC_CONV=0 (or ``ENABLED = False``) keeps every convolution on cuDNN.
 ENABLED = os.environ.get("GCB200_TC_CONV", "1") == "1"
@@ -280,7 +280,7 @@ def _err(device):
     return gemm._error_flag(device).data_ptr()
 
 
-def conv_forward(x, w, bias=None, stride=1, pad=1, col_partials=None, out=None, accumulate=False, bn_fin=None):
+def conv_forward(x, w, bias=None, stride=1, pad=1, col_partials=None, out=None, accumulate=False, bn_fin=None, cta_sums=False):
     """``conv2d(x, w, bias, stride, pad)`` of a channels-last activation on the implicit-GEMM kernel; ``w`` is the
     filter in channels-last memory order ``(Cout, Cin, R, R)`` or already a matrix ``[Cout, R*R*Cin]`` together with
     ``x`` of ``Cin`` channels.  ``col_partials`` ([tiles, 2, Cout]) receives per-tile column sums / sums of squares; ``bn_fin`` (``gemm.bn_fin_args``)
@@ -296,7 +296,7 @@ def conv_forward(x, w, bias=None, stride=1, pad=1, col_partials=None, out=None, 
     with torch.cuda.device(x.device):
         nat.check(nat.cuda().gc_cuda_conv_fwd(x.data_ptr(), w2.data_ptr(), out.data_ptr(), nat.ptr(bias), n, h, wd, cin, cout, r,
                                               stride, pad, int(bool(accumulate)), nat.ptr(col_partials), _err(x.device),
-                                              nat.stream_ptr(), bn_fin[0] if bn_fin is not None else None), "conv_fwd")
+                                              nat.stream_ptr(), bn_fin[0] if bn_fin is not None else None, int(cta_sums)), "conv_fwd")
     return out
 
 
@@ -313,6 +313,7 @@ def conv_wgrad(dy, x, r, stride, pad, out=None):
 
 
 _SPLIT_PLAN = {}
+_STAT_ROWS = {}
 
 
 def _split_forward(lib, mode, n, h, wd, cin, cout, r, stride, pad, m):
@@ -328,6 +329,15 @@ def _split_forward(lib, mode, n, h, wd, cin, cout, r, stride, pad, m):
         else:
             hit = False
         _SPLIT_PLAN[key] = hit
+    return hit
+
+
+def _stat_rows(lib, m, cout, k):
+    """Rows of partial sums the forward kernel leaves when every CTA adds its tiles up (cached per shape)."""
+    key = (m, cout, k)
+    hit = _STAT_ROWS.get(key)
+    if hit is None:
+        hit = _STAT_ROWS[key] = int(lib.gc_cuda_conv_stat_rows(m, cout, k))
     return hit
 
 
@@ -351,22 +361,25 @@ class _ConvBNAct(torch.autograd.Function):
         with torch.cuda.device(x.device):
             # training: the kernel that writes yconv also finishes its batch statistics (mean, rstd, running stats)
             fin = partials = None
+            one_launch = training and not FUSED_FINALIZE and fused_ok(m // 4 if pool else m, cout)
+            cta_sums = False
             if training:
                 if FUSED_FINALIZE and cout <= gemm.FIN_MAX_CHANNELS and cout > 16:
                     fin = gemm.bn_fin_args(x.device, stats, running_mean, running_var, momentum, eps)
                 elif not _split_forward(lib, mode, n, h, wd, cin, cout, r, stride, pad, m):
-                    tiles = gemm.m_tiles(m)
-                    partials = torch.empty(tiles, 2, cout, dtype=torch.float32, device=x.device)
+                    rows = _stat_rows(lib, m, cout, cin if mode == "gemm" else (STEM_K if mode == "stem" else r * r * cin)) if one_launch else 0
+                    cta_sums = rows > 0
+                    partials = torch.empty(rows or gemm.m_tiles(m), 2, cout, dtype=torch.float32, device=x.device)
             if mode == "gemm":
-                gemm.gemm_tf32(_as_2d(x), w.reshape(cout, cin), bias=cbias, out=_as_2d(yconv), col_partials=partials, bn_fin=fin)
+                gemm.gemm_tf32(_as_2d(x), w.reshape(cout, cin), bias=cbias, out=_as_2d(yconv), col_partials=partials, bn_fin=fin, cta_sums=cta_sums)
             elif mode == "conv":
-                conv_forward(x, w, cbias, stride, pad, col_partials=partials, out=yconv, bn_fin=fin)
+                conv_forward(x, w, cbias, stride, pad, col_partials=partials, out=yconv, bn_fin=fin, cta_sums=cta_sums)
             else:
                 gathered = torch.empty(m, STEM_K, dtype=torch.float32, device=x.device)
                 wpad = torch.empty(cout, STEM_K, dtype=torch.float32, device=x.device)
                 nat.check(lib.gc_cuda_im2col_small(x.data_ptr(), gathered.data_ptr(), n, h, wd, cin, r, pad, STEM_K,
                                                    w.data_ptr(), wpad.data_ptr(), cout, st()), "im2col_small")
-                gemm.gemm_tf32(gathered, wpad, bias=cbias, out=_as_2d(yconv), col_partials=partials, bn_fin=fin)
+                gemm.gemm_tf32(gathered, wpad, bias=cbias, out=_as_2d(yconv), col_partials=partials, bn_fin=fin, cta_sums=cta_sums)
             res = _cl(residual) if residual is not None else None
             small = (SMALL_BN and training and fin is None and not pool and m * cout <= SMALL_BN_ELEMENTS
                      and lib.gc_cuda_bn_small_supported(m, cout))
@@ -379,6 +392,10 @@ class _ConvBNAct(torch.autograd.Function):
                                                        beta.data_ptr(), nat.ptr(res), int(relu), nat.ptr(running_mean),
                                                        nat.ptr(running_var), float(momentum), float(eps), stats.data_ptr(),
                                                        out.data_ptr(), st()), "bn_small_forward")
+            elif one_launch:
+                out = torch.empty((n, cout, ho // 2, wo // 2), dtype=torch.float32, device=x.device,
+                                  memory_format=torch.channels_last) if pool else torch.empty_like(yconv)
+                fused_forward(yconv, pool, partials, gamma, beta, res, relu, running_mean, running_var, momentum, eps, stats, out)
             else:
                 if partials is not None:
                     nat.check(lib.gc_cuda_bn_finalize_partials(partials.data_ptr(), partials.shape[0], m, cout, stats.data_ptr(),
@@ -420,8 +437,11 @@ class _ConvBNAct(torch.autograd.Function):
         sums = torch.empty(2 * cout, dtype=torch.float32, device=x.device)
         dconv = torch.empty_like(yconv)
         dres = own_grad(torch.empty_like(yconv)) if (ctx.has_res and ctx.needs_input_grad[5]) else None
+        small = not ctx.pool and SMALL_BN and m * cout <= SMALL_BN_ELEMENTS and lib.gc_cuda_bn_small_supported(m, cout)
         with torch.cuda.device(x.device):
-            if ctx.pool:
+            if not small and fused_ok(m // 4 if ctx.pool else m, cout):
+                fused_backward(dy, yconv, out, ctx.pool, stats, gamma, beta, ctx.relu, sums, dconv, dres)
+            elif ctx.pool:
                 # dy is the gradient of the pooled map: both kernels find each window's winner again from yconv
                 nat.check(lib.gc_cuda_bn_bwd_reduce_pool(dy.data_ptr(), yconv.data_ptr(), n, ho, wo, cout, stats.data_ptr(),
                                                          gamma.data_ptr(), beta.data_ptr(), int(ctx.relu),
@@ -431,7 +451,7 @@ class _ConvBNAct(torch.autograd.Function):
                 nat.check(lib.gc_cuda_bn_bwd_apply_pool(dy.data_ptr(), yconv.data_ptr(), n, ho, wo, cout, stats.data_ptr(),
                                                         gamma.data_ptr(), beta.data_ptr(), sums.data_ptr(), int(ctx.relu),
                                                         dconv.data_ptr(), st()), "bn_bwd_apply_pool")
-            elif SMALL_BN and m * cout <= SMALL_BN_ELEMENTS and lib.gc_cuda_bn_small_supported(m, cout):
+            elif small:
                 # small activation: the two gradient sums and the input gradient in one launch (a block owns its channels)
                 nat.check(lib.gc_cuda_bn_small_backward(dy.data_ptr(), yconv.data_ptr(), nat.ptr(out), m, cout, stats.data_ptr(),
                                                         gamma.data_ptr(), beta.data_ptr(), int(ctx.relu), sums.data_ptr(),

@@ -66,9 +66,10 @@ def bn_fin_args(device, stats, running_mean, running_var, momentum, eps):
     return ctypes.byref(a), a
 
 
-def gemm_tf32(a, b_nk, bias=None, out=None, col_partials=None, accumulate=False, bn_fin=None):
+def gemm_tf32(a, b_nk, bias=None, out=None, col_partials=None, accumulate=False, bn_fin=None, cta_sums=False):
     """``col_partials`` (optional, fp32 [m_tiles, 2, N]): receives per 128-row tile the column sums and sums of
-    squares of the product -- batch-norm statistics of a 1x1 convolution's output for free.
+    squares of the product -- batch-norm statistics of a 1x1 convolution's output for free (``cta_sums``: one row per CTA
+    of a column tile instead, ``gc_cuda_conv_stat_rows`` of them).
     ``accumulate=True``: ``out += a @ b_nk.T`` with the additions done by TMA reduce stores (in L2), so the old
     contents of ``out`` never travel to an SM."""
     assert not accumulate or out is not None, "accumulate needs the tensor to add to"
@@ -94,7 +95,7 @@ def gemm_tf32(a, b_nk, bias=None, out=None, col_partials=None, accumulate=False,
                                                a.stride(0), b_nk.stride(0), out.stride(0), int(bool(accumulate)),
                                                nat.ptr(col_partials),
                                                _error_flag(a.device).data_ptr(), nat.stream_ptr(),
-                                               bn_fin[0] if bn_fin is not None else None), "gemm_tf32")
+                                               bn_fin[0] if bn_fin is not None else None, int(cta_sums)), "gemm_tf32")
     return out
 
 
