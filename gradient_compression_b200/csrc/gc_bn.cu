@@ -213,6 +213,28 @@ __global__ void __launch_bounds__(BN_THREADS) bn_apply_kernel(const float* __res
   }
 }
 
+// Inference: the same with running statistics.  A thread keeps its four channels (the stride is a multiple of a row).  x == y is fine.
+__global__ void __launch_bounds__(BN_THREADS) bn_eval_apply_kernel(const float* x, int64_t nq, int vec, const float* __restrict__ mean,
+                                                                   const float* __restrict__ var, float eps, const float* __restrict__ gamma,
+                                                                   const float* __restrict__ beta, const float* __restrict__ residual, int relu, float* y) {
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x, first = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int c4 = (int)(first % vec) * 4;
+  const float4 mu = ld4(mean + c4), vr = ld4(var + c4), g = ld4(gamma + c4), b = ld4(beta + c4);
+  const float4 rs = make_float4(rsqrtf(vr.x + eps), rsqrtf(vr.y + eps), rsqrtf(vr.z + eps), rsqrtf(vr.w + eps));
+#pragma unroll 2
+  for (int64_t q = first; q < nq; q += stride) {
+    const float4 v = ld4(x + q * 4);
+    float4 o = make_float4(fmaf((v.x - mu.x) * rs.x, g.x, b.x), fmaf((v.y - mu.y) * rs.y, g.y, b.y), fmaf((v.z - mu.z) * rs.z, g.z, b.z),
+                           fmaf((v.w - mu.w) * rs.w, g.w, b.w));
+    if (residual != nullptr) {
+      const float4 r = ld4(residual + q * 4);
+      o.x += r.x; o.y += r.y; o.z += r.z; o.w += r.w;
+    }
+    if (relu) { o.x = fmaxf(o.x, 0.f); o.y = fmaxf(o.y, 0.f); o.z = fmaxf(o.z, 0.f); o.w = fmaxf(o.w, 0.f); }
+    st4(y + q * 4, o);
+  }
+}
+
 // ---------------------------------------------------------------------------------- backward reduce
 // g = dy * mask (mask = act output > 0; from the saved output y when given, else recomputed from x);
 // sums[0:C] = sum g (= dbeta), sums[C:2C] = sum g * xhat (= dgamma).
@@ -715,6 +737,14 @@ int gc_cuda_bn_apply(const float* x, int64_t M, int C, const float* stats, const
   if (!bn_shape_ok(M, C)) return (int)cudaErrorInvalidValue;
   launch_pdl(bn_apply_kernel, dim3(apply_grid(M * (C >> 2))), dim3(BN_THREADS), 0, (cudaStream_t)cs, x, M, C, stats, gamma, beta,
              residual, relu, y);
+  return (int)cudaGetLastError();
+}
+
+int gc_cuda_bn_eval_apply(const float* x, int64_t M, int C, const float* mean, const float* var, float eps, const float* gamma, const float* beta,
+                          const float* residual, int relu, float* y, void* cs) {
+  if (!bn_shape_ok(M, C)) return (int)cudaErrorInvalidValue;
+  const int64_t nq = M * (C >> 2);
+  bn_eval_apply_kernel<<<apply_grid(nq), BN_THREADS, 0, (cudaStream_t)cs>>>(x, nq, C >> 2, mean, var, eps, gamma, beta, residual, relu, y);
   return (int)cudaGetLastError();
 }
 

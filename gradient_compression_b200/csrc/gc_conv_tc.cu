@@ -124,9 +124,106 @@ __global__ void __launch_bounds__(256) im2col_small_kernel(const float* __restri
   }
 }
 
+// out = max over 2 x 2 windows of x[N, H, W, C] (H, W even, C a multiple of 4)
+__global__ void __launch_bounds__(256) max_pool2_kernel(const float* __restrict__ x, int H, int W, int C, int64_t quads, float* __restrict__ y) {
+  const int vec = C >> 2, wp = W >> 1, hp = H >> 1;
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < quads; i += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t p = i / vec;
+    const int c = (int)(i - p * vec) * 4, w = (int)(p % wp);
+    const int64_t nh = p / wp;
+    const int h = (int)(nh % hp);
+    const float* a = x + ((nh / hp * H + 2 * h) * (int64_t)W + 2 * w) * C + c;
+    const float4 v0 = __ldcs(reinterpret_cast<const float4*>(a)), v1 = __ldcs(reinterpret_cast<const float4*>(a + C));
+    const float4 v2 = __ldcs(reinterpret_cast<const float4*>(a + (int64_t)W * C)), v3 = __ldcs(reinterpret_cast<const float4*>(a + (int64_t)W * C + C));
+    *reinterpret_cast<float4*>(y + i * 4) = make_float4(fmaxf(fmaxf(v0.x, v1.x), fmaxf(v2.x, v3.x)), fmaxf(fmaxf(v0.y, v1.y), fmaxf(v2.y, v3.y)),
+                                                        fmaxf(fmaxf(v0.z, v1.z), fmaxf(v2.z, v3.z)), fmaxf(fmaxf(v0.w, v1.w), fmaxf(v2.w, v3.w)));
+  }
+}
+
+// Which path runs a convolution in inference: 0 none, 1 plain GEMM, 2 implicit GEMM, 3 gathered stem.
+int eval_mode(int N, int H, int W, int Cin, int Cout, int R, int stride, int pad, Shape* s) {
+  if (!make_shape(N, H, W, Cin, Cout, R, stride, pad, s) || (Cout & 3) || Cout <= 16 || encode_fn() == nullptr) return 0;
+  if ((int64_t)N * s->Ho * s->Wo > 0x7fffffff) return 0;
+  if (R == 1 && stride == 1 && pad == 0) return (Cin & 3) == 0 ? 1 : 0;
+  if (fwd_ok(*s)) return 2;
+  return R * R * Cin <= 32 && stride == 1 && 2 * pad == R - 1 ? 3 : 0;
+}
+
 }  // namespace
 
 extern "C" {
+
+int gc_cuda_im2col_small(const float* x, float* A, int N, int H, int W, int Cin, int R, int pad, int Kp, const float* w, float* wpad, int Cout, void* cs);
+int gc_cuda_bn_eval_apply(const float* x, int64_t M, int C, const float* mean, const float* var, float eps, const float* gamma, const float* beta,
+                          const float* residual, int relu, float* y, void* cs);
+
+// Floats of scratch gc_cuda_conv_bn_eval needs for a layer (-1: it does not take the layer).
+int64_t gc_cuda_conv_bn_eval_scratch(int N, int H, int W, int Cin, int Cout, int R, int stride, int pad) {
+  Shape s;
+  const int mode = eval_mode(N, H, W, Cin, Cout, R, stride, pad, &s);
+  if (mode == 0) return -1;
+  return mode == 3 ? ((int64_t)N * s.Ho * s.Wo + Cout) * 32 : 0;
+}
+
+// Inference of a layer: y = act(gamma * (conv(x, w) + cbias - mean) / sqrt(var + eps) + beta [+ residual]), the batch norm in the
+// convolution's epilogue -- the activation is written once and not read again (ResNet-50, batch 256: the separate apply passes
+// were 1.4 of 4.2 ms).  A layer with few output tiles and a long contraction is split over the SMs instead, where the
+// kernels' cost model says that this pays for a pass over its small output.
+int gc_cuda_conv_bn_eval(const float* x, const float* w, float* y, const float* cbias, int N, int H, int W, int Cin, int Cout, int R, int stride, int pad,
+                         const float* gamma, const float* beta, const float* mean, const float* var, float eps, const float* residual, int relu,
+                         float* scratch, int* error_flag, void* cs) {
+  Shape s;
+  const int mode = eval_mode(N, H, W, Cin, Cout, R, stride, pad, &s);
+  if (mode == 0) return (int)cudaErrorInvalidValue;
+  cudaStream_t st = (cudaStream_t)cs;
+  const int M = N * s.Ho * s.Wo;
+  int K = R * R * Cin;
+  if (mode == 3) {
+    float* wpad = scratch + (int64_t)M * 32;
+    int err = gc_cuda_im2col_small(x, scratch, N, H, W, Cin, R, pad, 32, w, wpad, Cout, cs);
+    if (err) return err;
+    x = scratch;
+    w = wpad;
+    K = 32;
+  }
+  if (((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(residual)) & 15u))
+    return (int)cudaErrorInvalidValue;
+  int tile, splits;
+  plan_persistent(M, Cout, K, zero_cycles((int64_t)M * Cout) + stats_pass_cycles((int64_t)M * Cout), &tile, &splits);
+  CUtensorMap ma, mb, mc;
+  ConvA ca{};
+  if (mode == 2) {
+    int bw, bh, bn;
+    box_for(BM, s.Ho, s.Wo, &bw, &bh, &bn);
+    if (make_map_nhwc(&ma, x, s, bw, bh, bn, CU_TENSOR_MAP_SWIZZLE_128B) != 0) return (int)cudaErrorInvalidValue;
+    ca = conv_a(s);
+  } else if (make_map(&ma, x, M, K, K, BM) != 0) {
+    return (int)cudaErrorInvalidValue;
+  }
+  if (make_map(&mb, w, Cout, K, K, tile) != 0 || make_map(&mc, y, M, Cout, Cout, BM) != 0) return (int)cudaErrorInvalidValue;
+  const Affine aff{gamma, beta, mean, var, residual, eps, relu};
+  if (splits > 1) {
+    cudaError_t e = cudaMemsetAsync(y, 0, (size_t)M * Cout * 4, st);
+    if (e != cudaSuccess) return (int)e;
+  }
+  const Affine* in_kernel = splits > 1 ? nullptr : &aff;
+  int err;
+  switch (tile) {
+    case 64: err = launch_persistent_maps<64>(ma, mb, mc, ca, cbias, M, Cout, K, splits > 1, nullptr, error_flag, st, nullptr, nullptr, splits, 0, in_kernel); break;
+    case 128: err = launch_persistent_maps<128>(ma, mb, mc, ca, cbias, M, Cout, K, splits > 1, nullptr, error_flag, st, nullptr, nullptr, splits, 0, in_kernel); break;
+    default: err = launch_persistent_maps<256>(ma, mb, mc, ca, cbias, M, Cout, K, splits > 1, nullptr, error_flag, st, nullptr, nullptr, splits, 0, in_kernel); break;
+  }
+  if (err || splits == 1) return err;
+  return gc_cuda_bn_eval_apply(y, M, Cout, mean, var, eps, gamma, beta, residual, relu, y, cs);
+}
+
+// y[N, H/2, W/2, C] = 2 x 2 max-pool of x[N, H, W, C].
+int gc_cuda_max_pool2(const float* x, int N, int H, int W, int C, float* y, void* cs) {
+  if ((H | W) & 1 || C & 3) return (int)cudaErrorInvalidValue;
+  const int64_t quads = (int64_t)N * (H / 2) * (W / 2) * (C / 4), blocks = (quads + 255) / 256, most = (int64_t)sm_count() * 8;
+  max_pool2_kernel<<<(unsigned)(blocks < most ? blocks : most), 256, 0, (cudaStream_t)cs>>>(x, H, W, C, quads, y);
+  return (int)cudaGetLastError();
+}
 
 // 1 when forward (and, on rotated weights, the input gradient) of this convolution can run on the tensor cores:
 // Cin a multiple of 32, Cout a multiple of 4 and >= 32, and 128 consecutive output positions form one box.

@@ -181,6 +181,14 @@ struct BnFin {
   float momentum, eps;
 };
 
+// Batch norm of running statistics folded into the epilogue (inference): out = act((acc + bias) * sc + sh [+ residual]) with
+// sc = gamma / sqrt(var + eps) and sh = beta - mean * sc per column.  mean == NULL: off.  residual: [M, N], row pitch N.
+struct Affine {
+  const float *gamma, *beta, *mean, *var, *residual;
+  float eps;
+  int relu;
+};
+
 // What the host passes to ask for it: `scratch` holds the ticket (first 256 bytes) and the totals (2 * N doubles), is
 // zeroed once when allocated (gc_cuda_bn_fin_scratch_bytes) and is left zeroed by every launch that uses it.
 struct BnFinHost {
@@ -319,7 +327,7 @@ __global__ void __launch_bounds__(PERSISTENT_THREADS, 1)
 gemm_tf32_persistent_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
                             const __grid_constant__ CUtensorMap tma_c, const ConvA ca, const float* __restrict__ bias, int M, int N, int K,
                             int tiles_m, int tiles_n, int splits, int accumulate, float* __restrict__ col_partials,
-                            int* __restrict__ error_flag, int tma_mode, const BnFin fin, const ConvC cc, int cta_sums) {
+                            int* __restrict__ error_flag, int tma_mode, const BnFin fin, const ConvC cc, int cta_sums, const Affine aff) {
   using S = PSmem<BN>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -471,12 +479,24 @@ gemm_tf32_persistent_kernel(const __grid_constant__ CUtensorMap tma_a, const __g
     const bool want_sums = col_partials != nullptr || fin_on;
     float run_a = 0.f, run_b = 0.f;                            // fin_on, cta_sums: this thread's column, summed over the CTA's tiles
     bool drained_all = true;
+    const bool aff_on = aff.mean != nullptr, with_res = aff_on && aff.residual != nullptr;
+    float* col_affine = colsum + ew * 64;                      // aff_on: 32 scales and 32 shifts of the slab, per warp
+    float4 res[8];                                             // with_res: the next slab's residual, 4 rows of 128 bytes per load of a warp
+    auto load_residual = [&](int m0, int col0) {
+      const int c = col0 + (te & 7) * 4;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const int row = m0 + (te >> 3) + 16 * i;
+        res[i] = row < M && c < N ? __ldcs(reinterpret_cast<const float4*>(aff.residual + (int64_t)row * N + c)) : make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+    };
     for (int t = blockIdx.x; t < total_items; t += gridDim.x, ++lt) {
       const int tile = t / splits;
       const bool add_bias = bias != nullptr && t == tile * splits;      // the first split of a tile carries the bias
       const int mi = tile / tiles_n;
       const int m0 = mi * BM, n0 = (tile % tiles_n) * BN;
       const uint32_t buf = lt & 1u, aphase = (lt >> 1) & 1u;
+      if (with_res) load_residual(m0, n0 + grp * 32);
       const bool got = (tma_mode & 4) ? mbar_wait_idle(&acc_full[buf], aphase, &abort_flag, 128u) : mbar_wait(&acc_full[buf], aphase, &abort_flag);
       // one thread decides for the group: the TMEM loads are warp-collective and the named barriers below
       // involve all four warps, so either every one of them drains this tile or none does
@@ -492,6 +512,28 @@ gemm_tf32_persistent_kernel(const __grid_constant__ CUtensorMap tma_a, const __g
         // the store that last read this buffer was committed RING groups ago
         if (issuer) asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(RING - 1) : "memory");
         group_bar(grp);
+        if (aff_on) {
+          const int col = n0 + sl * 32 + lane;
+          float sc = 0.f, sh = 0.f;
+          if (col < N) {
+            sc = aff.gamma[col] * rsqrtf(aff.var[col] + aff.eps);
+            sh = fmaf((bias != nullptr ? bias[col] : 0.f) - aff.mean[col], sc, aff.beta[col]);
+          }
+          __syncwarp();
+          col_affine[lane] = sc;
+          col_affine[32 + lane] = sh;
+          if (with_res) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+              const int row = (te >> 3) + 16 * i;
+              *reinterpret_cast<float4*>(slab + row * 128 + (((te & 7) ^ (row & 7)) << 4)) = res[i];
+            }
+            if (sl + EPI_GROUPS < SLABS) load_residual(m0, n0 + (sl + EPI_GROUPS) * 32);
+            group_bar(grp);
+          } else {
+            __syncwarp();
+          }
+        }
         uint32_t ra[16], rb[16];
         tmem_ld16_nowait(lane_base + (uint32_t)(sl * 32), ra);
         tmem_ld16_nowait(lane_base + (uint32_t)(sl * 32 + 16), rb);
@@ -504,12 +546,21 @@ gemm_tf32_persistent_kernel(const __grid_constant__ CUtensorMap tma_a, const __g
         for (int c = 0; c < 8; ++c) {
           const uint32_t* src = c < 4 ? &ra[c * 4] : &rb[(c - 4) * 4];
           float4 o = make_float4(__uint_as_float(src[0]), __uint_as_float(src[1]), __uint_as_float(src[2]), __uint_as_float(src[3]));
-          if (add_bias) {
+          float4* to = reinterpret_cast<float4*>(slab + r * 128 + ((c ^ (r & 7)) << 4));           // 128-byte swizzle of the store map
+          if (aff_on) {
+            const float4 sc = *reinterpret_cast<const float4*>(col_affine + c * 4), sh = *reinterpret_cast<const float4*>(col_affine + 32 + c * 4);
+            o = make_float4(fmaf(o.x, sc.x, sh.x), fmaf(o.y, sc.y, sh.y), fmaf(o.z, sc.z, sh.z), fmaf(o.w, sc.w, sh.w));
+            if (with_res) {
+              const float4 q = *to;
+              o.x += q.x; o.y += q.y; o.z += q.z; o.w += q.w;
+            }
+            if (aff.relu) { o.x = fmaxf(o.x, 0.f); o.y = fmaxf(o.y, 0.f); o.z = fmaxf(o.z, 0.f); o.w = fmaxf(o.w, 0.f); }
+          } else if (add_bias) {
             int col = n0 + sl * 32 + c * 4;
             o.x += col < N ? bias[col] : 0.f; o.y += col + 1 < N ? bias[col + 1] : 0.f;
             o.z += col + 2 < N ? bias[col + 2] : 0.f; o.w += col + 3 < N ? bias[col + 3] : 0.f;
           }
-          *reinterpret_cast<float4*>(slab + r * 128 + ((c ^ (r & 7)) << 4)) = o;     // 128-byte swizzle of the store map
+          *to = o;
         }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         group_bar(grp);
@@ -918,7 +969,7 @@ int make_map_mn3(CUtensorMap* map, const float* base, int64_t K, int64_t D, int6
 template <int BN>
 int launch_persistent_maps(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mc, const ConvA& ca, const float* bias,
                            int M, int N, int K, int accumulate, float* col_partials, int* error_flag, cudaStream_t st,
-                           const BnFin* fin = nullptr, const ConvC* cc = nullptr, int splits = 1, int cta_sums = 0) {
+                           const BnFin* fin = nullptr, const ConvC* cc = nullptr, int splits = 1, int cta_sums = 0, const Affine* aff = nullptr) {
   using S = PSmem<BN>;
   static bool configured = false;
   if (!configured) {
@@ -940,13 +991,14 @@ int launch_persistent_maps(const CUtensorMap& ma, const CUtensorMap& mb, const C
     grid = grid / tiles_n * tiles_n;             // every CTA stays on one column tile
     f = *fin;
   }
+  if (aff != nullptr && (splits > 1 || accumulate || col_partials != nullptr || fin != nullptr || cc != nullptr)) return (int)cudaErrorInvalidValue;
   if (cta_sums) {
     if (col_partials == nullptr || splits > 1 || tiles_n > grid) return (int)cudaErrorInvalidValue;
     grid = grid / tiles_n * tiles_n;
   }
   gc::launch_pdl(gemm_tf32_persistent_kernel<BN>, dim3((unsigned)grid), dim3(PERSISTENT_THREADS), (size_t)S::TOTAL, st, ma, mb, mc, ca,
                  bias, M, N, K, tiles_m, tiles_n, splits, accumulate, col_partials, error_flag, gctc::tma_mode, f,
-                 cc != nullptr ? *cc : ConvC{0, 0}, cta_sums);
+                 cc != nullptr ? *cc : ConvC{0, 0}, cta_sums, aff != nullptr ? *aff : Affine{});
   return (int)cudaGetLastError();
 }
 

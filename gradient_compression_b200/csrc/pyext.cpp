@@ -42,6 +42,12 @@ struct Api {
   int (*quantize)(const float*, int64_t, const float*, int, int, uint64_t, uint32_t, uint32_t, void*, int, void*);
   int (*quantize_fit)(const float*, int64_t, const float*, int, int, uint64_t, uint32_t, uint32_t, void*, int, int8_t*, void*);
   int (*dequantize)(const void*, int, int64_t, const float*, int, int, float*, void*);
+  int64_t (*conv_bn_eval_scratch)(int, int, int, int, int, int, int, int);
+  int (*conv_bn_eval)(const float*, const float*, float*, const float*, int, int, int, int, int, int, int, int, const float*, const float*, const float*,
+                      const float*, float, const float*, int, float*, int*, void*);
+  int (*max_pool2)(const float*, int, int, int, int, float*, void*);
+  int (*bn_supported)(int64_t, int);
+  int (*bn_eval_apply)(const float*, int64_t, int, const float*, const float*, float, const float*, const float*, const float*, int, float*, void*);
   int (*dequantize_two)(const void*, int, const int8_t*, int64_t, const float*, int, int, int, float*, void*);
 } api;
 int max_segs = 0;
@@ -60,6 +66,11 @@ const Entry entries[] = {
     {"gc_cuda_quantize_levels", (void**)&api.quantize},
     {"gc_cuda_quantize_fit", (void**)&api.quantize_fit},
     {"gc_cuda_dequantize_levels", (void**)&api.dequantize},
+    {"gc_cuda_conv_bn_eval_scratch", (void**)&api.conv_bn_eval_scratch},
+    {"gc_cuda_conv_bn_eval", (void**)&api.conv_bn_eval},
+    {"gc_cuda_max_pool2", (void**)&api.max_pool2},
+    {"gc_cuda_bn_supported", (void**)&api.bn_supported},
+    {"gc_cuda_bn_eval_apply", (void**)&api.bn_eval_apply},
     {"gc_cuda_dequantize_two", (void**)&api.dequantize_two},
 };
 
@@ -392,6 +403,82 @@ PyObject* dequantize(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   return THPVariable_Wrap(out);
 }
 
+// ---- inference ---------------------------------------------------------------------------------------------------
+// A dense fp32 CUDA activation in channels-last memory order, 16-byte aligned.
+const at::Tensor* activation(PyObject* o) {
+  const at::Tensor* t = tensor_of(o);
+  return t && t->is_cuda() && t->scalar_type() == at::kFloat && t->dim() == 4 && t->numel() > 0 && t->is_contiguous(at::MemoryFormat::ChannelsLast) &&
+                 ((uintptr_t)t->data_ptr() & 15u) == 0
+             ? t
+             : nullptr;
+}
+// Per-channel parameters: c floats on x's device.
+const float* channels(PyObject* o, const at::Tensor& x, int64_t c) {
+  const at::Tensor* t = plain(o, at::kFloat);
+  return t && t->numel() == c && t->device() == x.device() && ((uintptr_t)t->data_ptr() & 15u) == 0 ? (const float*)t->data_ptr() : nullptr;
+}
+at::Tensor like_activation(const at::Tensor& x, int64_t n, int64_t c, int64_t h, int64_t w) {
+  return at::empty({n, c, h, w}, x.options(), at::MemoryFormat::ChannelsLast);
+}
+
+// conv_bn_eval(x, w, cbias or None, gamma, beta, mean, var, eps, residual or None, relu, stride, pad, pool, error flag (address)) -> y
+PyObject* conv_bn_eval(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
+  if (!want(nargs, 14, "conv_bn_eval")) return nullptr;
+  const at::Tensor *x = activation(a[0]), *w = tensor_of(a[1]), *res = a[8] == Py_None ? nullptr : activation(a[8]);
+  if (!x || !w || (a[8] != Py_None && !res)) Py_RETURN_NONE;
+  if (!w->is_cuda() || w->scalar_type() != at::kFloat || w->dim() != 4 || w->device() != x->device() || w->size(1) != x->size(1) || w->size(2) != w->size(3))
+    Py_RETURN_NONE;
+  const int64_t n = x->size(0), cin = x->size(1), h = x->size(2), wd = x->size(3), cout = w->size(0), r = w->size(2);
+  if (!(w->is_contiguous(at::MemoryFormat::ChannelsLast) || (r == 1 && w->is_contiguous()))) Py_RETURN_NONE;
+  const double eps = PyFloat_AsDouble(a[7]);
+  const int relu = PyObject_IsTrue(a[9]), stride = (int)as_int(a[10]), pad = (int)as_int(a[11]), pool = PyObject_IsTrue(a[12]);
+  int* flag = (int*)PyLong_AsUnsignedLongLong(a[13]);
+  if (PyErr_Occurred()) return nullptr;
+  const float *cbias = a[2] == Py_None ? nullptr : channels(a[2], *x, cout), *gamma = channels(a[3], *x, cout), *beta = channels(a[4], *x, cout),
+              *mean = channels(a[5], *x, cout), *var = channels(a[6], *x, cout);
+  if ((a[2] != Py_None && !cbias) || !gamma || !beta || !mean || !var || stride < 1 || n > INT32_MAX || n * h * wd > INT32_MAX) Py_RETURN_NONE;
+  const int64_t ho = (h + 2 * pad - r) / stride + 1, wo = (wd + 2 * pad - r) / stride + 1;
+  if (ho < 1 || wo < 1 || h + 2 * pad < r || wd + 2 * pad < r || !api.bn_supported(n * ho * wo, (int)cout)) Py_RETURN_NONE;
+  if (res && (res->device() != x->device() || res->size(0) != n || res->size(1) != cout || res->size(2) != ho || res->size(3) != wo)) Py_RETURN_NONE;
+  if (pool && (res || ((ho | wo) & 1))) Py_RETURN_NONE;
+  const int64_t floats = api.conv_bn_eval_scratch((int)n, (int)h, (int)wd, (int)cin, (int)cout, (int)r, stride, pad);
+  if (floats < 0) Py_RETURN_NONE;
+  c10::cuda::OptionalCUDAGuard guard(x->device());
+  at::Tensor y = like_activation(*x, n, cout, ho, wo), scratch;
+  if (floats) scratch = at::empty({floats}, x->options());
+  void* st = stream_on(x->device().index());
+  int err = api.conv_bn_eval((const float*)x->data_ptr(), (const float*)w->data_ptr(), (float*)y.data_ptr(), cbias, (int)n, (int)h, (int)wd, (int)cin,
+                             (int)cout, (int)r, stride, pad, gamma, beta, mean, var, (float)eps, res ? (const float*)res->data_ptr() : nullptr, relu,
+                             floats ? (float*)scratch.data_ptr() : nullptr, flag, st);
+  if (err) return cuda_error("conv_bn_eval", err);
+  if (pool) {
+    at::Tensor p = like_activation(*x, n, cout, ho / 2, wo / 2);
+    err = api.max_pool2((const float*)y.data_ptr(), (int)n, (int)ho, (int)wo, (int)cout, (float*)p.data_ptr(), st);
+    if (err) return cuda_error("max_pool2", err);
+    y = p;
+  }
+  return THPVariable_Wrap(y);
+}
+
+// bn_eval(x, gamma, beta, mean, var, eps, residual or None, relu) -> y
+PyObject* bn_eval(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
+  if (!want(nargs, 8, "bn_eval")) return nullptr;
+  const at::Tensor *x = activation(a[0]), *res = a[6] == Py_None ? nullptr : activation(a[6]);
+  if (!x || (a[6] != Py_None && (!res || res->sizes() != x->sizes() || res->device() != x->device()))) Py_RETURN_NONE;
+  const int64_t c = x->size(1), m = x->numel() / c;
+  const float *gamma = channels(a[1], *x, c), *beta = channels(a[2], *x, c), *mean = channels(a[3], *x, c), *var = channels(a[4], *x, c);
+  const double eps = PyFloat_AsDouble(a[5]);
+  const int relu = PyObject_IsTrue(a[7]);
+  if (PyErr_Occurred()) return nullptr;
+  if (!gamma || !beta || !mean || !var || !api.bn_supported(m, (int)c)) Py_RETURN_NONE;
+  c10::cuda::OptionalCUDAGuard guard(x->device());
+  at::Tensor y = like_activation(*x, x->size(0), c, x->size(2), x->size(3));
+  const int err = api.bn_eval_apply((const float*)x->data_ptr(), m, (int)c, mean, var, (float)eps, gamma, beta, res ? (const float*)res->data_ptr() : nullptr,
+                                    relu, (float*)y.data_ptr(), stream_on(x->device().index()));
+  if (err) return cuda_error("bn_eval", err);
+  return THPVariable_Wrap(y);
+}
+
 // bind({name: address}): the kernel library's entry points
 PyObject* bind(PyObject*, PyObject* table) {
   for (const Entry& e : entries) {
@@ -425,6 +512,8 @@ PyMethodDef methods[] = {
     {"solo_randk_limit", (PyCFunction)(void (*)(void))solo_randk_limit, METH_FASTCALL, "most coordinates solo_randk takes"},
     {"solo_psgd", (PyCFunction)(void (*)(void))solo_psgd, METH_FASTCALL, "PowerSGD step of a single worker"},
     {"solo_topk", (PyCFunction)(void (*)(void))solo_topk, METH_FASTCALL, "top-k with error feedback of a single worker"},
+    {"conv_bn_eval", (PyCFunction)(void (*)(void))conv_bn_eval, METH_FASTCALL, "convolution, batch norm of running statistics, residual, ReLU, pool"},
+    {"bn_eval", (PyCFunction)(void (*)(void))bn_eval, METH_FASTCALL, "batch norm of running statistics, residual, ReLU"},
     {"absmax", (PyCFunction)(void (*)(void))absmax, METH_FASTCALL, "largest magnitude"},
     {"quantize", (PyCFunction)(void (*)(void))quantize, METH_FASTCALL, "levels of a vector"},
     {"quantize_fit", (PyCFunction)(void (*)(void))quantize_fit, METH_FASTCALL, "levels of the higher scale and where they fit the lower one"},

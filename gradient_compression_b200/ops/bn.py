@@ -217,6 +217,11 @@ class _FusedBNAct(torch.autograd.Function):
 def bn_act(bn, x, residual=None, relu=True):
     """``relu(bn(x) + residual)`` with ``bn`` a ``torch.nn.BatchNorm2d`` (affine, tracking running stats)."""
     training = bn.training or bn.running_mean is None
+    if not training and x.is_cuda and bn.affine and not torch.is_grad_enabled():
+        y = nat.ext().bn_eval(x, bn.weight, bn.bias, bn.running_mean, bn.running_var, bn.eps, residual, relu)
+        if y is not None:
+            nat.count_launch()
+            return y
     use_kernel = kernel_path_ok(x) and bn.affine and not (not training and torch.is_grad_enabled() and x.requires_grad)
     if not use_kernel:
         y = bn(x)

@@ -580,12 +580,30 @@ def _mode(conv, bn, x):
     return mode if mode in PATHS else None
 
 
+def _eval(conv, bn, x, residual, relu, pool):
+    """``conv_bn_act`` in inference: running statistics, nothing kept for a backward.  None: not a case for the kernels."""
+    params, stats = bn._parameters, bn._buffers
+    w, k, s, p = conv._parameters["weight"], conv.kernel_size, conv.stride, conv.padding
+    if (conv.groups != 1 or conv.dilation != (1, 1) or k[0] != k[1] or s[0] != s[1] or isinstance(p, str) or p[0] != p[1] or conv.padding_mode != "zeros"
+            or params["weight"] is None or not torch.backends.cudnn.allow_tf32):
+        return None
+    y = nat.ext().conv_bn_eval(x, w, conv._parameters["bias"], params["weight"], params["bias"], stats["running_mean"], stats["running_var"], bn.eps,
+                               residual, relu, s[0], p[0], pool, _err(x.device))
+    if y is not None:
+        nat.count_launch()
+    return y
+
+
 def conv_bn_act(conv, bn, x, residual=None, relu=True, link=None, donate=None, pool=False):
     """``act(bn(conv(x)) + residual)`` on the tensor-core kernels where the layer qualifies (cuDNN + the fused BN kernels
     otherwise).  ``link``: see ``GradLink``.  ``donate``: the ``GradLink`` of an earlier-created layer that reads the same
     ``x`` (a block's first convolution, when this layer is the projection shortcut): this layer's input gradient is then
     handed to that layer's input-gradient kernel to add onto.  ``pool=True``: a 2x2 / stride-2 max-pool of the result, folded
     into the BN kernels (no residual)."""
+    if ENABLED and not bn.training and x.is_cuda and not torch.is_grad_enabled() and type(conv) is torch.nn.Conv2d and bn._buffers["running_mean"] is not None:
+        y = _eval(conv, bn, x, residual, relu, pool)
+        if y is not None:
+            return y
     mode = _mode(conv, bn, x)
     if mode is not None and pool:
         n, _, h, w = x.shape

@@ -1,0 +1,62 @@
+"""Inference layers (convolution, batch norm of running statistics, residual, ReLU, pool in one go) against PyTorch in fp64."""
+import pytest
+import torch
+import torch.nn as nn
+import torch.nn.functional as F
+
+pytestmark = pytest.mark.gpu
+
+#          n, cin, h, cout, r, stride, pad
+LAYERS = [(3, 3, 32, 64, 3, 1, 1),           # stem
+          (1, 64, 8, 64, 1, 1, 0), (5, 64, 16, 256, 1, 1, 0), (2, 36, 8, 100, 1, 1, 0), (1, 20, 4, 36, 1, 1, 0),
+          (2, 64, 32, 64, 3, 1, 1), (3, 128, 16, 256, 3, 2, 1), (1, 256, 8, 512, 1, 2, 0),
+          (2, 512, 4, 512, 3, 1, 1),         # few tiles, long contraction: split over the SMs
+          (130, 64, 2, 96, 3, 1, 1),
+          (2, 32, 6, 32, 3, 1, 1)]           # a map the tilings exclude
+
+
+@pytest.mark.parametrize("layer", LAYERS)
+@pytest.mark.parametrize("kind", ["relu", "residual", "plain", "bias", "pool"])
+def test_layer(layer, kind):
+    from gradient_compression_b200.ops import conv_bn_act
+
+    n, cin, h, cout, r, stride, pad = layer
+    torch.manual_seed(cout + r)
+    conv = nn.Conv2d(cin, cout, r, stride, pad, bias=kind == "bias").cuda().to(memory_format=torch.channels_last)
+    bn = nn.BatchNorm2d(cout).cuda().eval()
+    with torch.no_grad():
+        for t in (bn.weight, bn.bias, bn.running_mean):
+            t.normal_()
+        bn.running_var.uniform_(0.3, 3.0)
+        x = torch.randn(n, cin, h, h, device="cuda").contiguous(memory_format=torch.channels_last)
+        ho = (h + 2 * pad - r) // stride + 1
+        res = torch.randn(n, cout, ho, ho, device="cuda").contiguous(memory_format=torch.channels_last) if kind == "residual" else None
+        got = conv_bn_act(conv, bn, x, residual=res, relu=kind != "plain", pool=kind == "pool")
+        want = F.conv2d(x.double(), conv.weight.double(), conv.bias.double() if conv.bias is not None else None, stride, pad)
+        want = F.batch_norm(want, bn.running_mean.double(), bn.running_var.double(), bn.weight.double(), bn.bias.double(), False, 0.0, bn.eps)
+        want = want + res.double() if res is not None else want
+        want = F.relu(want) if kind != "plain" else want
+        want = F.max_pool2d(want, 2, 2) if kind == "pool" else want
+        assert got.shape == want.shape and got.is_contiguous(memory_format=torch.channels_last)
+        err = (got.double() - want).abs()
+        assert float(err.max()) < 0.03 * float(want.abs().max()) and float(err.norm() / want.norm()) < 2e-3
+
+
+@pytest.mark.parametrize("name", ["ResNet18", "ResNet50", "VGG11", "MobileNetV2", "densenet_cifar"])
+def test_model_matches_the_layers_one_by_one(name):
+    from gradient_compression_b200 import models
+    from gradient_compression_b200.ops import bn as B, conv as C
+
+    torch.manual_seed(1)
+    model = getattr(models, name)().cuda().to(memory_format=torch.channels_last)
+    x = torch.randn(20, 3, 32, 32, device="cuda").contiguous(memory_format=torch.channels_last)
+    with torch.no_grad():
+        model(x)
+        model.eval()
+        got = model(x)
+        C.ENABLED, kept = False, B.nat.ext
+        try:
+            want = model(x)
+        finally:
+            C.ENABLED = True
+    assert float((got - want).norm() / want.norm()) < 2e-2
