@@ -322,7 +322,8 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
 constexpr int EPI_GROUPS = 2;
 constexpr int PERSISTENT_THREADS = 32 * FIRST_EPI_WARP + 128 * EPI_GROUPS;
 
-template <int BN>
+// AFFINE: the epilogue of inference (a kernel of its own: its residual registers slowed the training epilogue by 3 %).
+template <int BN, bool AFFINE>
 __global__ void __launch_bounds__(PERSISTENT_THREADS, 1)
 gemm_tf32_persistent_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
                             const __grid_constant__ CUtensorMap tma_c, const ConvA ca, const float* __restrict__ bias, int M, int N, int K,
@@ -479,7 +480,8 @@ gemm_tf32_persistent_kernel(const __grid_constant__ CUtensorMap tma_a, const __g
     const bool want_sums = col_partials != nullptr || fin_on;
     float run_a = 0.f, run_b = 0.f;                            // fin_on, cta_sums: this thread's column, summed over the CTA's tiles
     bool drained_all = true;
-    const bool aff_on = aff.mean != nullptr, with_res = aff_on && aff.residual != nullptr;
+    constexpr bool aff_on = AFFINE;
+    const bool with_res = AFFINE && aff.residual != nullptr;
     float* col_affine = colsum + ew * 64;                      // aff_on: 32 scales and 32 shifts of the slab, per warp
     float4 res[8];                                             // with_res: the next slab's residual, 4 rows of 128 bytes per load of a warp
     auto load_residual = [&](int m0, int col0) {
@@ -973,7 +975,8 @@ int launch_persistent_maps(const CUtensorMap& ma, const CUtensorMap& mb, const C
   using S = PSmem<BN>;
   static bool configured = false;
   if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_tf32_persistent_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::TOTAL);
+    cudaError_t e = cudaFuncSetAttribute(gemm_tf32_persistent_kernel<BN, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::TOTAL);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_tf32_persistent_kernel<BN, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::TOTAL);
     if (e != cudaSuccess) return (int)e;
     configured = true;
   }
@@ -996,7 +999,7 @@ int launch_persistent_maps(const CUtensorMap& ma, const CUtensorMap& mb, const C
     if (col_partials == nullptr || splits > 1 || tiles_n > grid) return (int)cudaErrorInvalidValue;
     grid = grid / tiles_n * tiles_n;
   }
-  gc::launch_pdl(gemm_tf32_persistent_kernel<BN>, dim3((unsigned)grid), dim3(PERSISTENT_THREADS), (size_t)S::TOTAL, st, ma, mb, mc, ca,
+  gc::launch_pdl(aff != nullptr ? gemm_tf32_persistent_kernel<BN, true> : gemm_tf32_persistent_kernel<BN, false>, dim3((unsigned)grid), dim3(PERSISTENT_THREADS), (size_t)S::TOTAL, st, ma, mb, mc, ca,
                  bias, M, N, K, tiles_m, tiles_n, splits, accumulate, col_partials, error_flag, gctc::tma_mode, f,
                  cc != nullptr ? *cc : ConvC{0, 0}, cta_sums, aff != nullptr ? *aff : Affine{});
   return (int)cudaGetLastError();
