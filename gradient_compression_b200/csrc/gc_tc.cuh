@@ -84,6 +84,45 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
   return false;
 }
 
+// The same wait for a whole converged warp, with one answer for the warp: what follows stays uniform control flow.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
+  const uint32_t addr = smem_u32(bar);
+  unsigned long long t0 = 0;
+  for (uint32_t it = 0;; ++it) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(addr), "r"(parity)
+        : "memory");
+    if (__all_sync(0xffffffffu, ok)) return true;
+    if ((it & 63u) == 63u) {
+      unsigned long long now;
+      asm volatile("mov.u64 %0, %globaltimer;" : "=l"(now));
+      if (t0 == 0) t0 = now;
+      if (__any_sync(0xffffffffu, *abort_flag != 0 || now - t0 > WAIT_LIMIT_NS)) break;
+    }
+  }
+  *abort_flag = 1;
+  return false;
+}
+
+// One lane of a converged warp, chosen so that the compiler knows it to be one: TMA and MMA instructions under this predicate
+// take their operands from uniform registers.  Under `lane == 0` in a divergent branch each of them first moves its
+// descriptors there one by one: four MMAs and a commit took the issuing thread 340 cycles, a stage's TMA loads 400 (clock64,
+// B200), and a k-block of every width 590 cycles, whatever its tensor time (128 / 256 / 512 cycles at 64 / 128 / 256 columns).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(p));
+  return p != 0;
+}
+
 // The same wait for warps that have nothing to do for a long time (the epilogue warps during a tile's main loop): between
 // polls they sleep, so that their polling does not take issue slots from the single threads that feed the TMA unit and
 // the tensor core on the same SM sub-partitions.
@@ -344,7 +383,7 @@ gemm_tf32_persistent_kernel(const __grid_constant__ CUtensorMap tma_a, const __g
   __shared__ int abort_flag;
   __shared__ int epi_go[EPI_GROUPS];
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   const int num_k = (K + BK - 1) / BK;
   // work item = (output tile, split of the contraction); the splits of one tile are neighbours in the list, so they run
   // at the same time on different SMs and add their partial tiles in L2 (the host passes accumulate = 1 and a zeroed C)
@@ -366,84 +405,80 @@ gemm_tf32_persistent_kernel(const __grid_constant__ CUtensorMap tma_a, const __g
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
   // everything above (barriers, TMEM) overlapped the tail of the previous kernel of the stream; its results are
   // needed from here on
   gc::pdl_wait();
   gc::pdl_launch_dependents();
 
   if (warp < PRODUCER_WARPS) {
-    // producer warp p fills the stages it == p (mod PRODUCER_WARPS) of the ring
-    if (lane == 0) {
-      if (tma_mode & 1) { tma_prefetch_map(&tma_a); tma_prefetch_map(&tma_b); }
-      uint32_t it = 0;                                        // k-blocks issued so far by all producers, over all tiles
-      bool ok = true;
-      for (int t = blockIdx.x; t < total_items && ok; t += gridDim.x) {
-        const int tile = t / splits, sp = t - tile * splits;
-        const int kbeg = sp * kps, kend = min(num_k, kbeg + kps);
-        const int m0 = (tile / tiles_n) * BM, n0 = (tile % tiles_n) * BN;
-        int box[4] = {0, 0, 0, 0};
-        if (ca.taps != 0) conv_box(ca, (int64_t)m0, 0, 0, box);  // pixel of the tile's first position at tap (0, 0)
-        int kk = kbeg;
-        int cb = 0, fr = 0, fs = 0;                             // k-block = (filter tap (fr, fs), 32-channel block cb)
-        if (ca.taps != 0) {
-          const int tap = kk / ca.cblocks;
-          cb = kk - tap * ca.cblocks;
-          fr = tap / ca.fs;
-          fs = tap - fr * ca.fs;
-        }
-        for (int k = kbeg; k < kend; ++k, ++it) {
-          if ((int)(it % PRODUCER_WARPS) == warp) {
-            const int s = (int)(it % S::STAGES);
-            const uint32_t phase = (it / S::STAGES) & 1u;
-            if (!mbar_wait(&empty[s], phase ^ 1u, &abort_flag)) { ok = false; break; }
+    // producer warp p fills the stages of k-blocks it == p (mod PRODUCER_WARPS) of the ring
+    if ((tma_mode & 1) && elect_one()) { tma_prefetch_map(&tma_a); tma_prefetch_map(&tma_b); }
+    uint32_t s = 0, phase = 0;                                // stage and its phase of the next k-block, over all tiles
+    static_assert(PRODUCER_WARPS == 2, "two warps take turns");
+    int turn = 0;                                             // producer warp that fills it
+    bool ok = true;
+    for (int t = blockIdx.x; t < total_items && ok; t += gridDim.x) {
+      const int tile = t / splits, sp = t - tile * splits;
+      const int kbeg = sp * kps, kend = min(num_k, kbeg + kps);
+      const int m0 = (tile / tiles_n) * BM, n0 = (tile % tiles_n) * BN;
+      int box[4] = {0, 0, 0, 0};
+      if (ca.taps != 0) conv_box(ca, (int64_t)m0, 0, 0, box);  // pixel of the tile's first position at tap (0, 0)
+      int cb = 0, fr = 0, fs = 0;                             // k-block = (filter tap (fr, fs), 32-channel block cb)
+      if (ca.taps != 0) {
+        const int tap = kbeg / ca.cblocks;
+        cb = kbeg - tap * ca.cblocks;
+        fr = tap / ca.fs;
+        fs = tap - fr * ca.fs;
+      }
+      for (int k = kbeg; k < kend; ++k) {
+        if (turn == warp) {
+          if (!mbar_wait_warp(&empty[s], phase ^ 1u, &abort_flag)) { ok = false; break; }
+          // b_mn: B is the filter read in place (no transposed copy)
+          const int tapcol = ca.b_mn == 0 || ca.taps == 0 ? 0 : ((ca.b_r0 + ca.b_dr * fr) * ca.b_fs + (ca.b_s0 + ca.b_ds * fs)) * ca.b_ldtap;
+          const int krow = (ca.taps == 0 ? k : cb) * BK;
+          uint8_t *a_dst = a_tiles + s * S::A_BYTES, *b_dst = b_tiles + s * S::B_BYTES;
+          if (elect_one()) {
             mbar_expect_tx(&full[s], (uint32_t)(S::A_BYTES + S::B_BYTES));
-            if (ca.taps == 0)
-              tma_load_2d(a_tiles + s * S::A_BYTES, &tma_a, kk * BK, m0, &full[s]);
-            else
-              tma_load_4d(a_tiles + s * S::A_BYTES, &tma_a, cb * 32, box[1] + fs, box[2] + fr, box[3], &full[s]);
+            if (ca.taps == 0) tma_load_2d(a_dst, &tma_a, k * BK, m0, &full[s]);
+            else tma_load_4d(a_dst, &tma_a, cb * 32, box[1] + fs, box[2] + fr, box[3], &full[s]);
             if (!ca.b_mn) {
-              tma_load_2d(b_tiles + s * S::B_BYTES, &tma_b, kk * BK, n0, &full[s]);
+              tma_load_2d(b_dst, &tma_b, k * BK, n0, &full[s]);
+            } else if (ca.b_mn == 2) {
+              // the matrix seen as {32 floats, K rows, N / 32 chunks}: one box brings all BN / 32 chunks of the stage
+              tma_load_3d(b_dst, &tma_b, 0, krow, (tapcol + n0) >> 5, &full[s]);
             } else {
-              // BN / 32 boxes of 32 N-floats x 32 K-rows: the filter read in place (no transposed copy)
-              const int tapcol = ca.taps == 0 ? 0 : ((ca.b_r0 + ca.b_dr * fr) * ca.b_fs + (ca.b_s0 + ca.b_ds * fs)) * ca.b_ldtap;
-              const int krow = (ca.taps == 0 ? kk : cb) * BK;
-              if (ca.b_mn == 2) {
-                // the matrix seen as {32 floats, K rows, N / 32 chunks}: one box brings all BN / 32 chunks of the stage
-                tma_load_3d(b_tiles + s * S::B_BYTES, &tma_b, 0, krow, (tapcol + n0) >> 5, &full[s]);
-              } else {
+              // BN / 32 boxes of 32 N-floats x 32 K-rows
 #pragma unroll
-                for (int c = 0; c < BN / 32; ++c)
-                  tma_load_2d(b_tiles + s * S::B_BYTES + c * (BK * 128), &tma_b, tapcol + n0 + c * 32, krow, &full[s]);
-              }
+              for (int c = 0; c < BN / 32; ++c) tma_load_2d(b_dst + c * (BK * 128), &tma_b, tapcol + n0 + c * 32, krow, &full[s]);
             }
           }
-          ++kk;
-          if (++cb == ca.cblocks) {                             // (never true for a plain matrix: cblocks == 0)
-            cb = 0;
-            if (++fs == ca.fs) { fs = 0; ++fr; }
-          }
+          __syncwarp();
+        }
+        if (++s == S::STAGES) { s = 0; phase ^= 1u; }
+        turn ^= 1;
+        if (++cb == ca.cblocks) {                             // (never true for a plain matrix: cblocks == 0)
+          cb = 0;
+          if (++fs == ca.fs) { fs = 0; ++fr; }
         }
       }
     }
   } else if (warp == MMA_WARP) {
-    if (lane == 0) {
-      constexpr uint32_t idesc = make_idesc(BN);
-      uint32_t it = 0, lt = 0;                                // k-blocks consumed, tiles started
-      bool ok = true;
-      for (int t = blockIdx.x; t < total_items && ok; t += gridDim.x, ++lt) {
-        const int sp = t % splits;
-        const int nk = min(num_k, (sp + 1) * kps) - sp * kps;
-        const uint32_t buf = lt & 1u, aphase = (lt >> 1) & 1u;
-        if (!mbar_wait(&acc_empty[buf], aphase ^ 1u, &abort_flag)) break;      // first use of a buffer passes at once
+    constexpr uint32_t idesc = make_idesc(BN);
+    uint32_t s = 0, phase = 0, lt = 0;                        // stage of the next k-block and its phase, tiles started
+    bool ok = true;
+    for (int t = blockIdx.x; t < total_items && ok; t += gridDim.x, ++lt) {
+      const int sp = t % splits;
+      const int nk = min(num_k, (sp + 1) * kps) - sp * kps;
+      const uint32_t buf = lt & 1u, aphase = (lt >> 1) & 1u;
+      if (!mbar_wait_warp(&acc_empty[buf], aphase ^ 1u, &abort_flag)) break;      // first use of a buffer passes at once
+      tc_fence_after();
+      const uint32_t tmem_c = tmem_base + buf * (uint32_t)BN;
+      for (int k = 0; k < nk; ++k) {
+        if (!mbar_wait_warp(&full[s], phase, &abort_flag)) { ok = false; break; }
         tc_fence_after();
-        const uint32_t tmem_c = tmem_base + buf * (uint32_t)BN;
-        for (int k = 0; k < nk; ++k, ++it) {
-          const int s = (int)(it % S::STAGES);
-          const uint32_t phase = (it / S::STAGES) & 1u;
-          if (!mbar_wait(&full[s], phase, &abort_flag)) { ok = false; break; }
-          tc_fence_after();
-          const uint64_t adesc = make_smem_desc(a_tiles + s * S::A_BYTES);
+        const uint64_t adesc = make_smem_desc(a_tiles + s * S::A_BYTES);
+        if (elect_one()) {
           if (!ca.b_mn) {
             const uint64_t bdesc = make_smem_desc(b_tiles + s * S::B_BYTES);
 #pragma unroll
@@ -457,8 +492,10 @@ gemm_tf32_persistent_kernel(const __grid_constant__ CUtensorMap tma_a, const __g
               umma_tf32(tmem_c, adesc + (uint64_t)(kk * 2), bdesc + (uint64_t)(kk * 64), idesc | (1u << 16), (k | kk) != 0 ? 1u : 0u);
           }
           umma_commit(&empty[s]);
+          if (k == nk - 1) umma_commit(&acc_full[buf]);
         }
-        if (ok) umma_commit(&acc_full[buf]);
+        __syncwarp();
+        if (++s == S::STAGES) { s = 0; phase ^= 1u; }
       }
     }
   } else {
@@ -740,7 +777,7 @@ gemm_tn_tf32_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_cons
   __shared__ int abort_flag;
   __shared__ int epi_go;
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   const int split = blockIdx.x % splits;
   const int tile = blockIdx.x / splits;
   const int m0 = (tile / tiles_n) * BM, n0 = (tile % tiles_n) * BN;
@@ -764,43 +801,44 @@ gemm_tn_tf32_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_cons
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
 
   if (num_k > 0) {
     if (warp < PRODUCER_WARPS) {
       // a stage is BM / 32 + BN / 32 boxes of 32 floats x TBK rows; producer warp p fills the stages k == p (mod PRODUCER_WARPS)
-      if (lane == 0) {
-        if (tma_mode & 1) { tma_prefetch_map(&tma_a); tma_prefetch_map(&tma_b); }
-        // weight gradient of an R x S convolution: column n of dW[Cout, taps * Cin] belongs to filter tap n / Cin, channel
-        // n % Cin; a tile narrower than Cin stays inside one tap, a wider one (Cin = 64) covers several taps side by side.
-        // Box c of a stage reads the pixels of its tap, shifted by (fr, fs), for the TBK output positions of the k-block.
-        int co[4] = {0, 0, 0, 0};
-        int box_ch[BN / 32], box_fr[BN / 32], box_fs[BN / 32];
-        if (ca.taps != 0) {
-          const int cin = ca.cblocks * 32;
+      if ((tma_mode & 1) && elect_one()) { tma_prefetch_map(&tma_a); tma_prefetch_map(&tma_b); }
+      // weight gradient of an R x S convolution: column n of dW[Cout, taps * Cin] belongs to filter tap n / Cin, channel
+      // n % Cin; a tile narrower than Cin stays inside one tap, a wider one (Cin = 64) covers several taps side by side.
+      // Box c of a stage reads the pixels of its tap, shifted by (fr, fs), for the TBK output positions of the k-block.
+      int co[4] = {0, 0, 0, 0};
+      int box_ch[BN / 32], box_fr[BN / 32], box_fs[BN / 32];
+      if (ca.taps != 0) {
+        const int cin = ca.cblocks * 32;
 #pragma unroll
-          for (int c = 0; c < BN / 32; ++c) {
-            const int n = n0 + c * 32, tap = n / cin;
-            box_ch[c] = n - tap * cin;
-            box_fr[c] = tap / ca.fs;
-            box_fs[c] = tap - box_fr[c] * ca.fs;
-          }
+        for (int c = 0; c < BN / 32; ++c) {
+          const int n = n0 + c * 32, tap = n / cin;
+          box_ch[c] = n - tap * cin;
+          box_fr[c] = tap / ca.fs;
+          box_fs[c] = tap - box_fr[c] * ca.fs;
         }
-        // boxes that lie wholly beyond the matrix (Mo < 128: the 64-channel layers; No < n0 + BN) are not loaded at all: the
-        // rows and columns of the accumulator they feed are never stored
-        int a_boxes = (Mo - m0 + 31) / 32, b_boxes = (No - n0 + 31) / 32;
-        a_boxes = a_boxes < BM / 32 ? a_boxes : BM / 32;
-        b_boxes = b_boxes < BN / 32 ? b_boxes : BN / 32;
-        // box3d bit 0 / 1: the A / B map is the 3-D view {32 floats, rows, chunks} of the matrix and ONE box brings the whole
-        // operand of a stage (chunks beyond the matrix arrive as zeros and count as bytes)
-        const bool a3 = (box3d & 1) != 0, b3 = (box3d & 2) != 0 && ca.taps == 0;
-        const uint32_t stage_tx = (uint32_t)((a3 ? BM / 32 : a_boxes) * S::CHUNK_BYTES + (b3 ? BN / 32 : b_boxes) * S::CHUNK_BYTES);
-        for (int k = warp; k < num_k; k += PRODUCER_WARPS) {
-          const int s = k % S::STAGES;
-          const uint32_t phase = (uint32_t)(k / S::STAGES) & 1u;
-          if (!mbar_wait(&empty[s], phase ^ 1u, &abort_flag)) break;
+      }
+      // boxes that lie wholly beyond the matrix (Mo < 128: the 64-channel layers; No < n0 + BN) are not loaded at all: the
+      // rows and columns of the accumulator they feed are never stored
+      int a_boxes = (Mo - m0 + 31) / 32, b_boxes = (No - n0 + 31) / 32;
+      a_boxes = a_boxes < BM / 32 ? a_boxes : BM / 32;
+      b_boxes = b_boxes < BN / 32 ? b_boxes : BN / 32;
+      // box3d bit 0 / 1: the A / B map is the 3-D view {32 floats, rows, chunks} of the matrix and ONE box brings the whole
+      // operand of a stage (chunks beyond the matrix arrive as zeros and count as bytes)
+      const bool a3 = (box3d & 1) != 0, b3 = (box3d & 2) != 0 && ca.taps == 0;
+      const uint32_t stage_tx = (uint32_t)((a3 ? BM / 32 : a_boxes) * S::CHUNK_BYTES + (b3 ? BN / 32 : b_boxes) * S::CHUNK_BYTES);
+      for (int k = warp; k < num_k; k += PRODUCER_WARPS) {
+        const int s = k % S::STAGES;
+        const uint32_t phase = (uint32_t)(k / S::STAGES) & 1u;
+        if (!mbar_wait_warp(&empty[s], phase ^ 1u, &abort_flag)) break;
+        const int row0 = (k_begin + k) * TBK;
+        if (ca.taps != 0) conv_box(ca, (int64_t)row0, 0, 0, co);           // the k-block's first position at tap (0, 0)
+        if (elect_one()) {
           mbar_expect_tx(&full[s], stage_tx);
-          const int row0 = (k_begin + k) * TBK;
           if (a3) {
             tma_load_3d(a_tiles + s * S::A_BYTES, &tma_a, 0, row0, m0 >> 5, &full[s]);
           } else {
@@ -815,7 +853,6 @@ gemm_tn_tf32_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_cons
             for (int c = 0; c < BN / 32; ++c)
               if (c < b_boxes) tma_load_2d(b_tiles + s * S::B_BYTES + c * S::CHUNK_BYTES, &tma_b, n0 + c * 32, row0, &full[s]);
           } else {
-            conv_box(ca, (int64_t)row0, 0, 0, co);           // the k-block's first position at tap (0, 0)
 #pragma unroll
             for (int c = 0; c < BN / 32; ++c)
               if (c < b_boxes)
@@ -823,24 +860,25 @@ gemm_tn_tf32_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_cons
                             &full[s]);
           }
         }
+        __syncwarp();
       }
     } else if (warp == MMA_WARP) {
-      if (lane == 0) {
-        constexpr uint32_t idesc = make_idesc_mn(BN);
-        bool ok = true;
-        for (int k = 0; k < num_k; ++k) {
-          const int s = k % S::STAGES;
-          const uint32_t phase = (uint32_t)(k / S::STAGES) & 1u;
-          if (!mbar_wait(&full[s], phase, &abort_flag)) { ok = false; break; }
-          tc_fence_after();
-          const uint64_t adesc = make_smem_desc_mn(a_tiles + s * S::A_BYTES);
-          const uint64_t bdesc = make_smem_desc_mn(b_tiles + s * S::B_BYTES);
+      constexpr uint32_t idesc = make_idesc_mn(BN);
+      uint32_t s = 0, phase = 0;
+      for (int k = 0; k < num_k; ++k) {
+        if (!mbar_wait_warp(&full[s], phase, &abort_flag)) break;
+        tc_fence_after();
+        const uint64_t adesc = make_smem_desc_mn(a_tiles + s * S::A_BYTES);
+        const uint64_t bdesc = make_smem_desc_mn(b_tiles + s * S::B_BYTES);
+        if (elect_one()) {
 #pragma unroll
           for (int kk = 0; kk < TBK / UMMA_K; ++kk)    // 8 positions = 8 rows of 128 bytes = 1024 bytes = 64 address units
             umma_tf32(tmem_base, adesc + (uint64_t)(kk * 64), bdesc + (uint64_t)(kk * 64), idesc, (k | kk) != 0 ? 1u : 0u);
           umma_commit(&empty[s]);
+          if (k == num_k - 1) umma_commit(acc_ready);
         }
-        if (ok) umma_commit(acc_ready);
+        __syncwarp();
+        if (++s == S::STAGES) { s = 0; phase ^= 1u; }
       }
     } else {
       const int lg = warp & 3;
