@@ -66,6 +66,12 @@ int make_map_nhwc(CUtensorMap* map, const float* base, const Shape& s, int bw, i
   return r == CUDA_SUCCESS ? 0 : -2;
 }
 
+// Filter taps that read an input pixel.
+double reuse(const Shape& s) {
+  const double taps = (double)(s.R * s.R) / (s.stride * s.stride);
+  return taps > 1.0 ? taps : 1.0;
+}
+
 ConvA conv_a(const Shape& s) { return ConvA{s.R * s.R, s.R, s.Cin / 32, s.Ho * s.Wo, s.Wo, s.stride, s.pad}; }
 
 bool fwd_ok(const Shape& s) {
@@ -188,8 +194,7 @@ int gc_cuda_conv_bn_eval(const float* x, const float* w, float* y, const float* 
   }
   if (((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(residual)) & 15u))
     return (int)cudaErrorInvalidValue;
-  int tile, splits;
-  plan_persistent(M, Cout, K, zero_cycles((int64_t)M * Cout) + stats_pass_cycles((int64_t)M * Cout), &tile, &splits);
+  const Plan pl = plan_persistent(M, Cout, K, zero_ns((int64_t)M * Cout) + stats_pass_ns((int64_t)M * Cout), mode == 2 ? reuse(s) : 1.0);
   CUtensorMap ma, mb, mc;
   ConvA ca{};
   if (mode == 2) {
@@ -200,20 +205,13 @@ int gc_cuda_conv_bn_eval(const float* x, const float* w, float* y, const float* 
   } else if (make_map(&ma, x, M, K, K, BM) != 0) {
     return (int)cudaErrorInvalidValue;
   }
-  if (make_map(&mb, w, Cout, K, K, tile) != 0 || make_map(&mc, y, M, Cout, Cout, BM) != 0) return (int)cudaErrorInvalidValue;
+  if (make_map(&mb, w, Cout, K, K, pl.b_cols()) != 0 || make_map(&mc, y, M, Cout, Cout, BM) != 0) return (int)cudaErrorInvalidValue;
   const Affine aff{gamma, beta, mean, var, residual, eps, relu};
-  if (splits > 1) {
-    cudaError_t e = cudaMemsetAsync(y, 0, (size_t)M * Cout * 4, st);
-    if (e != cudaSuccess) return (int)e;
-  }
-  const Affine* in_kernel = splits > 1 ? nullptr : &aff;
-  int err;
-  switch (tile) {
-    case 64: err = launch_persistent_maps<64>(ma, mb, mc, ca, cbias, M, Cout, K, splits > 1, nullptr, error_flag, st, nullptr, nullptr, splits, 0, in_kernel); break;
-    case 128: err = launch_persistent_maps<128>(ma, mb, mc, ca, cbias, M, Cout, K, splits > 1, nullptr, error_flag, st, nullptr, nullptr, splits, 0, in_kernel); break;
-    default: err = launch_persistent_maps<256>(ma, mb, mc, ca, cbias, M, Cout, K, splits > 1, nullptr, error_flag, st, nullptr, nullptr, splits, 0, in_kernel); break;
-  }
-  if (err || splits == 1) return err;
+  if (pl.splits == 1) return launch_plan<true>(pl, ma, mb, mc, ca, cbias, M, Cout, K, 0, nullptr, error_flag, st, nullptr, nullptr, 0, &aff);
+  cudaError_t e = cudaMemsetAsync(y, 0, (size_t)M * Cout * 4, st);
+  if (e != cudaSuccess) return (int)e;
+  const int err = launch_plan(pl, ma, mb, mc, ca, cbias, M, Cout, K, 1, nullptr, error_flag, st);
+  if (err) return err;
   return gc_cuda_bn_eval_apply(y, M, Cout, mean, var, eps, gamma, beta, residual, relu, y, cs);
 }
 
@@ -248,31 +246,28 @@ int gc_cuda_conv_fwd(const float* x, const float* w, float* y, const float* bias
   cudaStream_t st = (cudaStream_t)cs;
   const BnFin fin_dev = bn_fin_from_host(bn_fin);
   const BnFin* fin = fin_dev.acc != nullptr ? &fin_dev : nullptr;
-  int tile = gctc::tile_choice ? gctc::tile_choice : pick_bn_persistent(M, Cout, K), splits = 1;
-  if (col_partials == nullptr && fin == nullptr)       // few output tiles and a long contraction: split it over the idle SMs
-    plan_persistent(M, Cout, K, accumulate ? 0.0 : zero_cycles((int64_t)M * Cout), &tile, &splits);
+  // few output tiles and a long contraction: split it over the idle SMs, unless the statistics have to come from the kernel
+  const Plan pl = col_partials == nullptr && fin == nullptr ? plan_persistent(M, Cout, K, accumulate ? 0.0 : zero_ns((int64_t)M * Cout), reuse(s))
+                                                            : pick_persistent(M, Cout, K, reuse(s));
   CUtensorMap ma, mb, mc;
-  if (make_map_nhwc(&ma, x, s, bw, bh, bn, CU_TENSOR_MAP_SWIZZLE_128B) != 0 || make_map(&mb, w, Cout, K, K, tile) != 0 ||
+  if (make_map_nhwc(&ma, x, s, bw, bh, bn, CU_TENSOR_MAP_SWIZZLE_128B) != 0 || make_map(&mb, w, Cout, K, K, pl.b_cols()) != 0 ||
       make_map(&mc, y, M, Cout, Cout, BM) != 0)
     return (int)cudaErrorInvalidValue;
-  const ConvA ca = conv_a(s);
-  if (splits > 1 && !accumulate) {
+  if (pl.splits > 1 && !accumulate) {
     cudaError_t e = cudaMemsetAsync(y, 0, (size_t)M * Cout * 4, st);
     if (e != cudaSuccess) return (int)e;
   }
-  const int acc = (accumulate || splits > 1) ? 1 : 0;
-  switch (tile) {
-    case 64: return launch_persistent_maps<64>(ma, mb, mc, ca, bias, M, Cout, K, acc, col_partials, error_flag, st, fin, nullptr, splits, cta_sums);
-    case 128: return launch_persistent_maps<128>(ma, mb, mc, ca, bias, M, Cout, K, acc, col_partials, error_flag, st, fin, nullptr, splits, cta_sums);
-    case 256: return launch_persistent_maps<256>(ma, mb, mc, ca, bias, M, Cout, K, acc, col_partials, error_flag, st, fin, nullptr, splits, cta_sums);
-    default: return (int)cudaErrorInvalidValue;
-  }
+  return launch_plan(pl, ma, mb, mc, conv_a(s), bias, M, Cout, K, accumulate || pl.splits > 1, col_partials, error_flag, st, fin, nullptr, cta_sums);
 }
 
 // Rows of col_partials that gc_cuda_conv_fwd (and, for R = 1 with stride 1, gc_cuda_gemm_tf32) writes with cta_sums; 0: not available.
-int gc_cuda_conv_stat_rows(int M, int Cout, int K) {
+// R, stride: of the convolution where the kernel gathers its taps itself, else 1.
+int gc_cuda_conv_stat_rows(int M, int Cout, int K, int R, int stride) {
   if (Cout <= 16) return 0;
-  return cta_sum_rows(M, Cout, gctc::tile_choice ? gctc::tile_choice : pick_bn_persistent(M, Cout, K));
+  Shape s{};
+  s.R = R;
+  s.stride = stride;
+  return cta_sum_rows(M, Cout, pick_persistent(M, Cout, K, reuse(s)));
 }
 
 // Contraction splits gc_cuda_conv_fwd would use for this shape if the caller gave up the in-kernel column statistics and
@@ -282,21 +277,19 @@ int gc_cuda_conv_fwd_splits(int N, int H, int W, int Cin, int Cout, int R, int s
   Shape s;
   if (!make_shape(N, H, W, Cin, Cout, R, stride, pad, &s) || !fwd_ok(s)) return 1;
   const int M = N * s.Ho * s.Wo;
-  int tile, splits;
-  plan_persistent(M, Cout, R * R * Cin, zero_cycles((int64_t)M * Cout) + stats_pass_cycles((int64_t)M * Cout), &tile, &splits);
-  return splits;
+  return plan_persistent(M, Cout, R * R * Cin, zero_ns((int64_t)M * Cout) + stats_pass_ns((int64_t)M * Cout), reuse(s)).splits;
 }
 
-// Map of the forward filter w[Cout][R*R*Cin] as the MN-major B operand of an input-gradient launch with tiles of `tile`
-// columns: one 3-D box per stage when every tap starts on a 32-float chunk (Cin a multiple of 32), else tile / 32 boxes.
-static int filter_map(CUtensorMap* mb, ConvA* ca, const float* w, int Cout, int R, int Cin, int tile) {
-  const int64_t cols = (int64_t)R * R * Cin;
-  if ((Cin & 31) == 0 && make_map_mn3(mb, w, Cout, cols, cols, BK, tile / 32) == 0) {
+// Map of the forward filter w[Cout][R*R*Cin] as the MN-major B operand of an input-gradient launch whose CTAs load `cols`
+// columns: one 3-D box per stage when every tap starts on a 32-float chunk (Cin a multiple of 32), else cols / 32 boxes.
+static int filter_map(CUtensorMap* mb, ConvA* ca, const float* w, int Cout, int R, int Cin, int cols) {
+  const int64_t all = (int64_t)R * R * Cin;
+  if ((Cin & 31) == 0 && make_map_mn3(mb, w, Cout, all, all, BK, cols / 32) == 0) {
     ca->b_mn = 2;
     return 0;
   }
   ca->b_mn = 1;
-  return make_map_mn(mb, w, Cout, cols, cols, BK);
+  return make_map_mn(mb, w, Cout, all, all, BK);
 }
 
 // 1 when the stride-1 input gradient of conv2d(x[N, H, W, Cin], w[Cout, R, R, Cin], pad) can run on the tensor cores reading
@@ -321,8 +314,7 @@ int gc_cuda_conv_dgrad(const float* dy, const float* w, float* dx, int N, int H,
     return (int)cudaErrorInvalidValue;
   const int M = N * H * W, K = R * R * Cout;
   cudaStream_t st = (cudaStream_t)cs;
-  int tile, splits;
-  plan_persistent(M, Cin, K, accumulate ? 0.0 : zero_cycles((int64_t)M * Cin), &tile, &splits);
+  const Plan pl = plan_persistent(M, Cin, K, accumulate ? 0.0 : zero_ns((int64_t)M * Cin), R * R);
   CUtensorMap ma, mb, mc;
   ConvA ca{};
   if (R == 1 && pad == 0) {
@@ -337,19 +329,13 @@ int gc_cuda_conv_dgrad(const float* dy, const float* w, float* dx, int N, int H,
   }
   ca.b_ldtap = Cin; ca.b_fs = R;
   ca.b_r0 = R - 1; ca.b_dr = -1; ca.b_s0 = R - 1; ca.b_ds = -1;
-  if (filter_map(&mb, &ca, w, Cout, R, Cin, tile) != 0 || make_map(&mc, dx, M, Cin, Cin, BM) != 0)
+  if (filter_map(&mb, &ca, w, Cout, R, Cin, pl.b_cols()) != 0 || make_map(&mc, dx, M, Cin, Cin, BM) != 0)
     return (int)cudaErrorInvalidValue;
-  if (splits > 1 && !accumulate) {
+  if (pl.splits > 1 && !accumulate) {
     cudaError_t e = cudaMemsetAsync(dx, 0, (size_t)M * Cin * 4, st);
     if (e != cudaSuccess) return (int)e;
   }
-  const int acc = (accumulate || splits > 1) ? 1 : 0;
-  switch (tile) {
-    case 64: return launch_persistent_maps<64>(ma, mb, mc, ca, nullptr, M, Cin, K, acc, nullptr, error_flag, st, nullptr, nullptr, splits);
-    case 128: return launch_persistent_maps<128>(ma, mb, mc, ca, nullptr, M, Cin, K, acc, nullptr, error_flag, st, nullptr, nullptr, splits);
-    case 256: return launch_persistent_maps<256>(ma, mb, mc, ca, nullptr, M, Cin, K, acc, nullptr, error_flag, st, nullptr, nullptr, splits);
-    default: return (int)cudaErrorInvalidValue;
-  }
+  return launch_plan(pl, ma, mb, mc, ca, nullptr, M, Cin, K, accumulate || pl.splits > 1, nullptr, error_flag, st);
 }
 
 // For measurements: 1 = weight gradients at Cin = 128 use 256-column tiles that hold two filter taps (measured slower than
@@ -460,12 +446,12 @@ int gc_cuda_conv_dgrad_s2(const float* dy, const float* w, float* dx, int N, int
     const int th = class_taps(ph, pad, R), tw = class_taps(pw, pad, R);
     if (th * tw == 0) continue;
     const int K = th * tw * Cout;
-    const int tile = gctc::tile_choice ? gctc::tile_choice : pick_bn_persistent(M, Cin, K);
+    const Plan pl = pick_persistent(M, Cin, K, th * tw);
     CUtensorMap ma, mb, mc;
     ConvA ca{th * tw, tw, Cout / 32, Ho * Wo, Wo, 1, 0};
     ca.b_ldtap = Cin; ca.b_fs = R;
     ca.b_r0 = ph + pad; ca.b_dr = -2; ca.b_s0 = pw + pad; ca.b_ds = -2;
-    if (make_map_nhwc(&ma, dy, sy, bw, bh, bn, CU_TENSOR_MAP_SWIZZLE_128B) != 0 || filter_map(&mb, &ca, w, Cout, R, Cin, tile) != 0)
+    if (make_map_nhwc(&ma, dy, sy, bw, bh, bn, CU_TENSOR_MAP_SWIZZLE_128B) != 0 || filter_map(&mb, &ca, w, Cout, R, Cin, pl.b_cols()) != 0)
       return (int)cudaErrorInvalidValue;
     {   // pixels (2i + ph, 2j + pw) of dx as the 4-D tensor {Cin, W/2, H/2, N}
       cuuint64_t dims[4] = {(cuuint64_t)Cin, (cuuint64_t)Wo, (cuuint64_t)Ho, (cuuint64_t)N};
@@ -478,13 +464,7 @@ int gc_cuda_conv_dgrad_s2(const float* dy, const float* w, float* dx, int N, int
         return (int)cudaErrorInvalidValue;
     }
     const ConvC cc{Ho * Wo, Wo};
-    int err;
-    switch (tile) {
-      case 64: err = launch_persistent_maps<64>(ma, mb, mc, ca, nullptr, M, Cin, K, 0, nullptr, error_flag, st, nullptr, &cc); break;
-      case 128: err = launch_persistent_maps<128>(ma, mb, mc, ca, nullptr, M, Cin, K, 0, nullptr, error_flag, st, nullptr, &cc); break;
-      case 256: err = launch_persistent_maps<256>(ma, mb, mc, ca, nullptr, M, Cin, K, 0, nullptr, error_flag, st, nullptr, &cc); break;
-      default: err = (int)cudaErrorInvalidValue;
-    }
+    const int err = launch_plan(pl, ma, mb, mc, ca, nullptr, M, Cin, K, 0, nullptr, error_flag, st, nullptr, &cc);
     if (err != 0) return err;
   }
   return 0;

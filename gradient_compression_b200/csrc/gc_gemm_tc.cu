@@ -4,12 +4,13 @@
 //   gemm_tf32_persistent_kernel  C[M, N] (=, +=) A[M, K] * B[N, K]^T (+ bias): both operands K-major.  1x1 convolutions
 //                                on channels-last activations (A = activations [N*H*W, Cin], B = weight [Cout, Cin]) and
 //                                their input gradients; optional per-column sums of C (batch-norm statistics) from the
-//                                epilogue.  One CTA per SM walks the tiles with a double-buffered TMEM accumulator.
+//                                epilogue.  One CTA per SM (or a pair of CTAs per tile) walks the tiles with a double-buffered
+//                                TMEM accumulator.
 //   gemm_tf32_kernel             the same product with one CTA per 128 x BN tile: narrow outputs (N <= 16) and outputs that
 //                                do not meet the TMA store rules (plain-store epilogue).
 //   gemm_tn_tf32_kernel          C[Mo, No] += A[P, Mo]^T * B[P, No]: both operands MN-major, split-K.  Weight gradients.
 //
-// Common structure, no clusters, no multicast (the persistent and the TN kernel are templates in gc_tc.cuh, shared with the
+// Common structure, no TMA multicast (the persistent and the TN kernel are templates in gc_tc.cuh, shared with the
 // convolution entry points of gc_conv_tc.cu; they run two producer warps, the tile kernel in this file one):
 //   producer warps  TMA loads (cp.async.bulk.tensor, 128-byte swizzle) into a ring of shared-memory stages
 //   MMA warp        allocates TMEM, issues tcgen05.mma (one elected thread), commits stages back to the producers
@@ -265,19 +266,17 @@ int launch(const float* A, const float* B, float* C, const float* bias, int M, i
   return (int)cudaGetLastError();
 }
 
-template <int BN>
-int launch_persistent(const float* A, const float* B, float* C, const float* bias, int M, int N, int K, int64_t lda,
+int launch_persistent(const Plan& pl, const float* A, const float* B, float* C, const float* bias, int M, int N, int K, int64_t lda,
                       int64_t ldb, int64_t ldc, int accumulate, float* col_partials, int* error_flag, cudaStream_t st, int cta_sums,
-                      const BnFin* fin, int splits) {
+                      const BnFin* fin) {
   CUtensorMap ma, mb, mc;
-  if (make_map(&ma, A, M, K, lda, BM) != 0 || make_map(&mb, B, N, K, ldb, BN) != 0 || make_map(&mc, C, M, N, ldc, BM) != 0)
+  if (make_map(&ma, A, M, K, lda, BM) != 0 || make_map(&mb, B, N, K, ldb, pl.b_cols()) != 0 || make_map(&mc, C, M, N, ldc, BM) != 0)
     return (int)cudaErrorInvalidValue;
-  if (splits > 1 && !accumulate) {
+  if (pl.splits > 1 && !accumulate) {
     cudaError_t e = cudaMemset2DAsync(C, (size_t)ldc * 4, 0, (size_t)N * 4, (size_t)M, st);
     if (e != cudaSuccess) return (int)e;
   }
-  return launch_persistent_maps<BN>(ma, mb, mc, ConvA{}, bias, M, N, K, (accumulate || splits > 1) ? 1 : 0, col_partials, error_flag,
-                                    st, fin, nullptr, splits, cta_sums);
+  return launch_plan(pl, ma, mb, mc, ConvA{}, bias, M, N, K, accumulate || pl.splits > 1, col_partials, error_flag, st, fin, nullptr, cta_sums);
 }
 
 template <int BN>
@@ -354,15 +353,9 @@ int gc_cuda_gemm_tf32(const float* A, const float* B, float* C, const float* bia
   bool persistent = (g_kernel_choice != 1 || accumulate || fin != nullptr) && N > 16 && tma_store_ok(C, ldc);
   if ((accumulate || fin != nullptr || cta_sums) && !persistent) return (int)cudaErrorInvalidValue;
   if (persistent) {
-    int bn = gctc::tile_choice ? gctc::tile_choice : pick_bn_persistent(M, N, K), splits = 1;
-    if (col_partials == nullptr && fin == nullptr)
-      plan_persistent(M, N, K, accumulate ? 0.0 : zero_cycles((int64_t)M * N), &bn, &splits);
-    switch (bn) {
-      case 64: return launch_persistent<64>(A, B, C, bias, M, N, K, lda, ldb, ldc, accumulate, col_partials, error_flag, st, cta_sums, fin, splits);
-      case 128: return launch_persistent<128>(A, B, C, bias, M, N, K, lda, ldb, ldc, accumulate, col_partials, error_flag, st, cta_sums, fin, splits);
-      case 256: return launch_persistent<256>(A, B, C, bias, M, N, K, lda, ldb, ldc, accumulate, col_partials, error_flag, st, cta_sums, fin, splits);
-      default: return (int)cudaErrorInvalidValue;
-    }
+    const Plan pl = col_partials == nullptr && fin == nullptr ? plan_persistent(M, N, K, accumulate ? 0.0 : zero_ns((int64_t)M * N))
+                                                              : pick_persistent(M, N, K);
+    return launch_persistent(pl, A, B, C, bias, M, N, K, lda, ldb, ldc, accumulate, col_partials, error_flag, st, cta_sums, fin);
   }
   switch (gctc::tile_choice && N > 16 ? gctc::tile_choice : pick_bn(M, N)) {
     case 16: return launch<16>(A, B, C, bias, M, N, K, lda, ldb, ldc, col_partials, error_flag, st);
@@ -376,13 +369,14 @@ int gc_cuda_gemm_tf32(const float* A, const float* B, float* C, const float* bia
 // pass of its own over C instead of asking for col_partials (that pass is charged to the split plan).  1: do not split.
 int gc_cuda_gemm_tf32_splits(int M, int N, int K) {
   if (N <= 16) return 1;
-  int bn, splits;
-  plan_persistent(M, N, K, zero_cycles((int64_t)M * N) + stats_pass_cycles((int64_t)M * N), &bn, &splits);
-  return splits;
+  return plan_persistent(M, N, K, zero_ns((int64_t)M * N) + stats_pass_ns((int64_t)M * N)).splits;
 }
 
 // For measurements: contraction splits of the persistent kernel (0 = modelled, 1 = never, n = n wherever a product allows it).
 void gc_cuda_tc_split_config(int splits) { gctc::split_choice = splits; }
+
+// For measurements: CTA pairs of the persistent kernel (0 = modelled, 1 = never, 2 = wherever there are two row tiles).
+void gc_cuda_tc_pair_config(int pairs) { gctc::pair_choice = pairs; }
 
 // For measurements: how the producer warps issue their TMA loads (bit 0: prefetch the tensor maps; bit 1: spread the
 // loads of a stage over several lanes).

@@ -11,7 +11,7 @@
 //                                a 2-D map or from shifted 4-D boxes of the activation (weight gradient of an R x S
 //                                convolution: one filter tap per output tile).
 //
-// No clusters, no multicast: every CTA loads its own operands.  Every mbarrier wait is bounded; when one runs out
+// No TMA multicast: every CTA loads its own operands (of a CTA pair: its half of them).  Every mbarrier wait is bounded; when one runs out
 // the CTA sets *error_flag, abandons its tile, frees its TMEM and returns.
 #pragma once
 #include <cuda.h>
@@ -25,6 +25,7 @@
 // k-blocks (of 64 rows) a split may get.
 namespace gctc {
 inline int tile_choice = 0;
+inline int pair_choice = 0;    // CTA pairs in the persistent kernel: 0 = modelled, 1 = never, 2 = wherever there are two row tiles
 inline int tn_ctas_per_sm = 1;
 inline int tn_min_kblocks = 4;
 inline int wgrad_two_taps = 0;
@@ -85,18 +86,29 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
 }
 
 // The same wait for a whole converged warp, with one answer for the warp: what follows stays uniform control flow.
+// CLUSTER: arrivals may come from the other CTA of a pair.
+template <bool CLUSTER = false>
 __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
   const uint32_t addr = smem_u32(bar);
   unsigned long long t0 = 0;
   for (uint32_t it = 0;; ++it) {
     uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(addr), "r"(parity)
-        : "memory");
+    if constexpr (CLUSTER)
+      asm volatile(
+          "{\n\t.reg .pred p;\n\t"
+          "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+          "selp.u32 %0, 1, 0, p;\n\t}"
+          : "=r"(ok)
+          : "r"(addr), "r"(parity)
+          : "memory");
+    else
+      asm volatile(
+          "{\n\t.reg .pred p;\n\t"
+          "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+          "selp.u32 %0, 1, 0, p;\n\t}"
+          : "=r"(ok)
+          : "r"(addr), "r"(parity)
+          : "memory");
     if (__all_sync(0xffffffffu, ok)) return true;
     if ((it & 63u) == 63u) {
       unsigned long long now;
@@ -175,6 +187,43 @@ __device__ __forceinline__ void tma_load_4d(void* dst, const CUtensorMap* map, i
       "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];"
       ::"r"(smem_u32(dst)), "l"(map), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
       : "memory");
+}
+
+// The same loads for a CTA of a pair (cta_group::2): the data lands in this CTA's shared memory, the bytes are counted on the
+// barrier of the CTA that issues the MMAs (`bar`: a shared::cluster address).
+__device__ __forceinline__ void tma_load_2d_pair(void* dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes.cta_group::2 [%0], [%1, {%3, %4}], [%2];"
+      ::"r"(smem_u32(dst)), "l"(map), "r"(bar), "r"(x), "r"(y)
+      : "memory");
+}
+__device__ __forceinline__ void tma_load_3d_pair(void* dst, const CUtensorMap* map, int c0, int c1, int c2, uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes.cta_group::2 [%0], [%1, {%3, %4, %5}], [%2];"
+      ::"r"(smem_u32(dst)), "l"(map), "r"(bar), "r"(c0), "r"(c1), "r"(c2)
+      : "memory");
+}
+__device__ __forceinline__ void tma_load_4d_pair(void* dst, const CUtensorMap* map, int c0, int c1, int c2, int c3, uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes.cta_group::2 [%0], [%1, {%3, %4, %5, %6}], [%2];"
+      ::"r"(smem_u32(dst)), "l"(map), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
+      : "memory");
+}
+
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %cluster_ctarank;" : "=r"(r));
+  return r;
+}
+// Address of this CTA's shared variable `p` in the CTA of the cluster with the given rank.
+__device__ __forceinline__ uint32_t cluster_addr(const void* p, uint32_t rank) {
+  uint32_t a;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(rank));
+  return a;
+}
+// Every thread of both CTAs of a pair.
+__device__ __forceinline__ void cluster_sync_all() {
+  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
 }
 
 // Where the rows of an operand come from when it is an NHWC activation [N, H, W, C] read through a 4-D map
@@ -291,13 +340,13 @@ __device__ __forceinline__ uint64_t make_smem_desc_mn_rows(const void* tile, int
 
 __device__ __forceinline__ uint64_t make_smem_desc_mn(const void* tile) { return make_smem_desc_mn_rows(tile, TBK); }
 
-// kind::tf32, fp32 accumulate, both operands K-major, M = 128, N = n.
-__host__ __device__ constexpr uint32_t make_idesc(int n) {
+// kind::tf32, fp32 accumulate, both operands K-major, M = m (128, or 256 rows of a CTA pair), N = n.
+__host__ __device__ constexpr uint32_t make_idesc(int n, int m = BM) {
   return (1u << 4)                 // C format: F32
          | (2u << 7)               // A format: TF32
          | (2u << 10)              // B format: TF32
          | ((uint32_t)(n >> 3) << 17)
-         | ((uint32_t)(BM >> 4) << 24);
+         | ((uint32_t)(m >> 4) << 24);
 }
 
 __device__ __forceinline__ void umma_tf32(uint32_t tmem_c, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
@@ -307,6 +356,21 @@ __device__ __forceinline__ void umma_tf32(uint32_t tmem_c, uint64_t adesc, uint6
       "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}"
       ::"r"(tmem_c), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(0u), "r"(0u), "r"(0u), "r"(0u)
       : "memory");
+}
+// 256 rows in two CTAs: rows 0..127 of A and columns 0..n/2 of B in the first CTA's shared memory, the others at the same
+// offsets in the second's; each CTA's TMEM receives its 128 rows.  Issued by one thread of the first CTA.
+__device__ __forceinline__ void umma_tf32_pair(uint32_t tmem_c, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::tf32 [%0], %1, %2, %3, {%5, %5, %5, %5, %5, %5, %5, %5}, p;\n\t}"
+      ::"r"(tmem_c), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(0u)
+      : "memory");
+}
+// Arrives on the barrier at this offset in both CTAs of the pair.
+__device__ __forceinline__ void umma_commit_pair(uint64_t* bar) {
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
+               ::"r"(smem_u32(bar)), "h"((uint16_t)3) : "memory");
 }
 __device__ __forceinline__ void umma_commit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
@@ -331,11 +395,12 @@ __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.
 // four epilogue warps take alternate 32-column slabs, each group staging them in its own ring of dedicated
 // buffers and waiting for a TMA store only when it needs that store's buffer back.  Tiles are ordered
 // with the column tile fastest: CTAs that run at the same time share the rows of A in L2.
-template <int BN>
+template <int BN, bool PAIR>
 struct PSmem {
-  static constexpr int STAGES = (BN <= 64) ? 5 : ((BN <= 128) ? 4 : 3);
+  static constexpr int STAGES = PAIR ? ((BN <= 64) ? 6 : ((BN <= 128) ? 5 : 4)) : ((BN <= 64) ? 5 : ((BN <= 128) ? 4 : 3));
   static constexpr int A_BYTES = BM * BK * 4;
-  static constexpr int B_BYTES = BN * BK * 4;               // a multiple of 1024 for BN >= 8
+  static constexpr int B_COLS = PAIR ? BN / 2 : BN;         // columns of B in this CTA's shared memory
+  static constexpr int B_BYTES = B_COLS * BK * 4;           // a multiple of 1024
   static constexpr int NSLAB = 4;
   static constexpr int SLAB_BYTES = BM * 128;
   static constexpr int RING_BYTES = STAGES * (A_BYTES + B_BYTES);
@@ -357,18 +422,26 @@ __device__ __forceinline__ void group_bar(int grp) {
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
+__device__ __forceinline__ void mbar_arrive_remote(uint32_t cluster_address) {
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_address) : "memory");
+}
 
 constexpr int EPI_GROUPS = 2;
 constexpr int PERSISTENT_THREADS = 32 * FIRST_EPI_WARP + 128 * EPI_GROUPS;
 
 // AFFINE: the epilogue of inference (a kernel of its own: its residual registers slowed the training epilogue by 3 %).
-template <int BN, bool AFFINE>
+//
+// PAIR: two CTAs of a cluster work on one tile of 256 rows (cta_group::2).  Each loads its 128 rows of A and HALF of the columns
+// of B, so a k-block costs a CTA 128 + BN / 2 rows of shared-memory fill and of operand reads instead of 128 + BN, which is
+// what bounds the single-CTA form.  The first CTA of the pair issues the MMAs and holds the barriers they wait for; commits go
+// to both.  Work items are the pairs' tiles; everything after the accumulator is each CTA's own.
+template <int BN, bool AFFINE, bool PAIR>
 __global__ void __launch_bounds__(PERSISTENT_THREADS, 1)
 gemm_tf32_persistent_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
                             const __grid_constant__ CUtensorMap tma_c, const ConvA ca, const float* __restrict__ bias, int M, int N, int K,
                             int tiles_m, int tiles_n, int splits, int accumulate, float* __restrict__ col_partials,
                             int* __restrict__ error_flag, int tma_mode, const BnFin fin, const ConvC cc, int cta_sums, const Affine aff) {
-  using S = PSmem<BN>;
+  using S = PSmem<BN, PAIR>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   uint8_t* a_tiles = base;
@@ -387,23 +460,31 @@ gemm_tf32_persistent_kernel(const __grid_constant__ CUtensorMap tma_a, const __g
   const int num_k = (K + BK - 1) / BK;
   // work item = (output tile, split of the contraction); the splits of one tile are neighbours in the list, so they run
   // at the same time on different SMs and add their partial tiles in L2 (the host passes accumulate = 1 and a zeroed C)
-  const int total_items = tiles_m * tiles_n * splits;
+  const int total_items = tiles_m * tiles_n * splits;          // tiles_m: of 128 rows, PAIR: of 256
   const int kps = (num_k + splits - 1) / splits;
+  const int rank = PAIR ? (int)cluster_rank() : 0;
+  const int worker = PAIR ? (int)(blockIdx.x >> 1) : (int)blockIdx.x, workers = PAIR ? (int)(gridDim.x >> 1) : (int)gridDim.x;
 
   if (threadIdx.x == 0) {
     abort_flag = 0;
     for (int g = 0; g < EPI_GROUPS; ++g) epi_go[g] = 1;
     for (int s = 0; s < S::STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
-    for (int b = 0; b < 2; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], 128 * EPI_GROUPS); }
+    for (int b = 0; b < 2; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], (PAIR ? 2 : 1) * EPI_GROUPS); }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
   if (warp == MMA_WARP) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"((uint32_t)S::TMEM_COLS) : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    if constexpr (PAIR) {
+      asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"((uint32_t)S::TMEM_COLS) : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    } else {
+      asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"((uint32_t)S::TMEM_COLS) : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
   }
   tc_fence_before();
   __syncthreads();
+  if constexpr (PAIR) cluster_sync_all();      // the other CTA's barriers and TMEM are in place
   tc_fence_after();
   const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
   // everything above (barriers, TMEM) overlapped the tail of the previous kernel of the stream; its results are
@@ -418,10 +499,10 @@ gemm_tf32_persistent_kernel(const __grid_constant__ CUtensorMap tma_a, const __g
     static_assert(PRODUCER_WARPS == 2, "two warps take turns");
     int turn = 0;                                             // producer warp that fills it
     bool ok = true;
-    for (int t = blockIdx.x; t < total_items && ok; t += gridDim.x) {
+    for (int t = worker; t < total_items && ok; t += workers) {
       const int tile = t / splits, sp = t - tile * splits;
       const int kbeg = sp * kps, kend = min(num_k, kbeg + kps);
-      const int m0 = (tile / tiles_n) * BM, n0 = (tile % tiles_n) * BN;
+      const int m0 = (PAIR ? (tile / tiles_n) * 2 + rank : tile / tiles_n) * BM, n0 = (tile % tiles_n) * BN + rank * S::B_COLS;
       int box[4] = {0, 0, 0, 0};
       if (ca.taps != 0) conv_box(ca, (int64_t)m0, 0, 0, box);  // pixel of the tile's first position at tap (0, 0)
       int cb = 0, fr = 0, fs = 0;                             // k-block = (filter tap (fr, fs), 32-channel block cb)
@@ -438,7 +519,22 @@ gemm_tf32_persistent_kernel(const __grid_constant__ CUtensorMap tma_a, const __g
           const int tapcol = ca.b_mn == 0 || ca.taps == 0 ? 0 : ((ca.b_r0 + ca.b_dr * fr) * ca.b_fs + (ca.b_s0 + ca.b_ds * fs)) * ca.b_ldtap;
           const int krow = (ca.taps == 0 ? k : cb) * BK;
           uint8_t *a_dst = a_tiles + s * S::A_BYTES, *b_dst = b_tiles + s * S::B_BYTES;
-          if (elect_one()) {
+          if constexpr (PAIR) {
+            const uint32_t bar = cluster_addr(&full[s], 0);
+            if (elect_one()) {
+              if (rank == 0) mbar_expect_tx(&full[s], (uint32_t)(2 * (S::A_BYTES + S::B_BYTES)));
+              if (ca.taps == 0) tma_load_2d_pair(a_dst, &tma_a, k * BK, m0, bar);
+              else tma_load_4d_pair(a_dst, &tma_a, cb * 32, box[1] + fs, box[2] + fr, box[3], bar);
+              if (!ca.b_mn) {
+                tma_load_2d_pair(b_dst, &tma_b, k * BK, n0, bar);
+              } else if (ca.b_mn == 2) {
+                tma_load_3d_pair(b_dst, &tma_b, 0, krow, (tapcol + n0) >> 5, bar);
+              } else {
+#pragma unroll
+                for (int c = 0; c < S::B_COLS / 32; ++c) tma_load_2d_pair(b_dst + c * (BK * 128), &tma_b, tapcol + n0 + c * 32, krow, bar);
+              }
+            }
+          } else if (elect_one()) {
             mbar_expect_tx(&full[s], (uint32_t)(S::A_BYTES + S::B_BYTES));
             if (ca.taps == 0) tma_load_2d(a_dst, &tma_a, k * BK, m0, &full[s]);
             else tma_load_4d(a_dst, &tma_a, cb * 32, box[1] + fs, box[2] + fr, box[3], &full[s]);
@@ -450,7 +546,7 @@ gemm_tf32_persistent_kernel(const __grid_constant__ CUtensorMap tma_a, const __g
             } else {
               // BN / 32 boxes of 32 N-floats x 32 K-rows
 #pragma unroll
-              for (int c = 0; c < BN / 32; ++c) tma_load_2d(b_dst + c * (BK * 128), &tma_b, tapcol + n0 + c * 32, krow, &full[s]);
+              for (int c = 0; c < S::B_COLS / 32; ++c) tma_load_2d(b_dst + c * (BK * 128), &tma_b, tapcol + n0 + c * 32, krow, &full[s]);
             }
           }
           __syncwarp();
@@ -463,19 +559,35 @@ gemm_tf32_persistent_kernel(const __grid_constant__ CUtensorMap tma_a, const __g
         }
       }
     }
+    if constexpr (PAIR) {
+      // the commits that free the last stages come from the first CTA: see them before this CTA may end.  From the next
+      // k-block's stage on, every stage was last filled in phase `phase ^ 1` (passed at once where it never was).
+      for (int j = 0; j < S::STAGES && ok; ++j) {
+        ok = mbar_wait_warp<true>(&empty[s], phase ^ 1u, &abort_flag);
+        if (++s == S::STAGES) { s = 0; phase ^= 1u; }
+      }
+    }
   } else if (warp == MMA_WARP) {
-    constexpr uint32_t idesc = make_idesc(BN);
+    constexpr uint32_t idesc = make_idesc(BN, PAIR ? 2 * BM : BM);
+    auto mma = [](uint32_t c, uint64_t ad, uint64_t bd, uint32_t id, uint32_t acc) {
+      if constexpr (PAIR) umma_tf32_pair(c, ad, bd, id, acc);
+      else umma_tf32(c, ad, bd, id, acc);
+    };
+    auto commit = [](uint64_t* bar) {
+      if constexpr (PAIR) umma_commit_pair(bar);
+      else umma_commit(bar);
+    };
     uint32_t s = 0, phase = 0, lt = 0;                        // stage of the next k-block and its phase, tiles started
     bool ok = true;
-    for (int t = blockIdx.x; t < total_items && ok; t += gridDim.x, ++lt) {
+    for (int t = worker; rank == 0 && t < total_items && ok; t += workers, ++lt) {
       const int sp = t % splits;
       const int nk = min(num_k, (sp + 1) * kps) - sp * kps;
       const uint32_t buf = lt & 1u, aphase = (lt >> 1) & 1u;
-      if (!mbar_wait_warp(&acc_empty[buf], aphase ^ 1u, &abort_flag)) break;      // first use of a buffer passes at once
+      if (!mbar_wait_warp<PAIR>(&acc_empty[buf], aphase ^ 1u, &abort_flag)) break;      // first use of a buffer passes at once
       tc_fence_after();
       const uint32_t tmem_c = tmem_base + buf * (uint32_t)BN;
       for (int k = 0; k < nk; ++k) {
-        if (!mbar_wait_warp(&full[s], phase, &abort_flag)) { ok = false; break; }
+        if (!mbar_wait_warp<PAIR>(&full[s], phase, &abort_flag)) { ok = false; break; }
         tc_fence_after();
         const uint64_t adesc = make_smem_desc(a_tiles + s * S::A_BYTES);
         if (elect_one()) {
@@ -483,16 +595,16 @@ gemm_tf32_persistent_kernel(const __grid_constant__ CUtensorMap tma_a, const __g
             const uint64_t bdesc = make_smem_desc(b_tiles + s * S::B_BYTES);
 #pragma unroll
             for (int kk = 0; kk < BK / UMMA_K; ++kk)
-              umma_tf32(tmem_c, adesc + (uint64_t)(kk * 2), bdesc + (uint64_t)(kk * 2), idesc, (k | kk) != 0 ? 1u : 0u);
+              mma(tmem_c, adesc + (uint64_t)(kk * 2), bdesc + (uint64_t)(kk * 2), idesc, (k | kk) != 0 ? 1u : 0u);
           } else {
             // B is MN-major: 4 KB chunks of 32 N-floats x 32 K-rows; 8 K-rows = 1024 bytes = 64 address units per MMA
             const uint64_t bdesc = make_smem_desc_mn_rows(b_tiles + s * S::B_BYTES, BK);
 #pragma unroll
             for (int kk = 0; kk < BK / UMMA_K; ++kk)
-              umma_tf32(tmem_c, adesc + (uint64_t)(kk * 2), bdesc + (uint64_t)(kk * 64), idesc | (1u << 16), (k | kk) != 0 ? 1u : 0u);
+              mma(tmem_c, adesc + (uint64_t)(kk * 2), bdesc + (uint64_t)(kk * 64), idesc | (1u << 16), (k | kk) != 0 ? 1u : 0u);
           }
-          umma_commit(&empty[s]);
-          if (k == nk - 1) umma_commit(&acc_full[buf]);
+          commit(&empty[s]);
+          if (k == nk - 1) commit(&acc_full[buf]);
         }
         __syncwarp();
         if (++s == S::STAGES) { s = 0; phase ^= 1u; }
@@ -529,10 +641,10 @@ gemm_tf32_persistent_kernel(const __grid_constant__ CUtensorMap tma_a, const __g
         res[i] = row < M && c < N ? __ldcs(reinterpret_cast<const float4*>(aff.residual + (int64_t)row * N + c)) : make_float4(0.f, 0.f, 0.f, 0.f);
       }
     };
-    for (int t = blockIdx.x; t < total_items; t += gridDim.x, ++lt) {
+    for (int t = worker; t < total_items; t += workers, ++lt) {
       const int tile = t / splits;
       const bool add_bias = bias != nullptr && t == tile * splits;      // the first split of a tile carries the bias
-      const int mi = tile / tiles_n;
+      const int mi = PAIR ? (tile / tiles_n) * 2 + rank : tile / tiles_n;      // row tile of 128; of a pair the second may lie beyond M
       const int m0 = mi * BM, n0 = (tile % tiles_n) * BN;
       const uint32_t buf = lt & 1u, aphase = (lt >> 1) & 1u;
       if (with_res) load_residual(m0, n0 + grp * 32);
@@ -577,10 +689,7 @@ gemm_tf32_persistent_kernel(const __grid_constant__ CUtensorMap tma_a, const __g
         tmem_ld16_nowait(lane_base + (uint32_t)(sl * 32), ra);
         tmem_ld16_nowait(lane_base + (uint32_t)(sl * 32 + 16), rb);
         tmem_ld_wait();
-        if (sl + EPI_GROUPS >= SLABS) {                        // this thread has read its share of the accumulator
-          tc_fence_before();
-          mbar_arrive(&acc_empty[buf]);
-        }
+        tc_fence_before();
 #pragma unroll
         for (int c = 0; c < 8; ++c) {
           const uint32_t* src = c < 4 ? &ra[c * 4] : &rb[(c - 4) * 4];
@@ -604,7 +713,11 @@ gemm_tf32_persistent_kernel(const __grid_constant__ CUtensorMap tma_a, const __g
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         group_bar(grp);
         if (issuer) {
-          if (n0 + sl * 32 < N) {
+          if (sl + EPI_GROUPS >= SLABS) {                      // the group has read its share of the accumulator
+            if constexpr (PAIR) mbar_arrive_remote(cluster_addr(&acc_empty[buf], 0));
+            else mbar_arrive(&acc_empty[buf]);
+          }
+          if (n0 + sl * 32 < N && (!PAIR || m0 < M)) {
             if (cc.hw != 0) {                    // rows = pixels (n, i, j) of a strided sub-grid: 4-D store map
               const int img = m0 / cc.hw, rem = m0 - img * cc.hw;
               const int i0 = rem / cc.w, j0 = rem - i0 * cc.w;
@@ -664,7 +777,7 @@ gemm_tf32_persistent_kernel(const __grid_constant__ CUtensorMap tma_a, const __g
             if (fin_on || cta_sums) {
               run_a += a;
               run_b += b;
-            } else {
+            } else if (!PAIR || m0 < M) {
               col_partials[((int64_t)mi * 2) * N + gc] = a;
               col_partials[((int64_t)mi * 2 + 1) * N + gc] = b;
             }
@@ -674,8 +787,8 @@ gemm_tf32_persistent_kernel(const __grid_constant__ CUtensorMap tma_a, const __g
     }
     if (cta_sums && drained_all && te < (SLABS / EPI_GROUPS) * 32) {
       // one row of partial sums per CTA that stays on this column tile (instead of one per row tile)
-      const int gc = (int)(blockIdx.x % (unsigned)tiles_n) * BN + (grp + EPI_GROUPS * (te >> 5)) * 32 + (te & 31);
-      const int64_t row = (int64_t)(blockIdx.x / (unsigned)tiles_n) * 2;
+      const int gc = (worker % tiles_n) * BN + (grp + EPI_GROUPS * (te >> 5)) * 32 + (te & 31);
+      const int64_t row = (int64_t)(PAIR ? (worker / tiles_n) * 2 + rank : worker / tiles_n) * 2;
       if (gc < N) {
         col_partials[row * N + gc] = run_a;
         col_partials[(row + 1) * N + gc] = run_b;
@@ -686,7 +799,7 @@ gemm_tf32_persistent_kernel(const __grid_constant__ CUtensorMap tma_a, const __g
       // finds every contribution in place and finishes the statistics
       if (te < (SLABS / EPI_GROUPS) * 32) {
         const int c = (grp + EPI_GROUPS * (te >> 5)) * 32 + (te & 31);
-        const int gc = (int)(blockIdx.x % (unsigned)tiles_n) * BN + c;
+        const int gc = (worker % tiles_n) * BN + c;
         if (gc < N) {
           atomicAdd(&fin.acc[gc], (double)run_a);
           atomicAdd(&fin.acc[N + gc], (double)run_b);
@@ -721,9 +834,13 @@ gemm_tf32_persistent_kernel(const __grid_constant__ CUtensorMap tma_a, const __g
   }
   tc_fence_before();
   __syncthreads();
+  if constexpr (PAIR) cluster_sync_all();      // nothing of the other CTA reads or signals this one's shared memory any more
   if (warp == MMA_WARP) {
     tc_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)S::TMEM_COLS) : "memory");
+    if constexpr (PAIR)
+      asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)S::TMEM_COLS) : "memory");
+    else
+      asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)S::TMEM_COLS) : "memory");
   }
   if (threadIdx.x == 0 && abort_flag && error_flag != nullptr) atomicExch(error_flag, 1);
 }
@@ -1005,49 +1122,106 @@ int make_map_mn3(CUtensorMap* map, const float* base, int64_t K, int64_t D, int6
   return r == CUDA_SUCCESS ? 0 : -2;
 }
 
+// How a product runs on the persistent kernel: tile width, splits of the contraction, CTA pairs (256-row tiles) or single CTAs.
+struct Plan {
+  int bn, splits;
+  bool pair;
+  int b_cols() const { return pair ? bn / 2 : bn; }          // columns of B (box rows of its map) one CTA loads
+  int rows() const { return pair ? 2 * BM : BM; }
+};
+
+// CTAs, or CTA pairs, of the persistent kernel that the device runs at once (pairs: half its SMs, unless a GPC has an odd
+// number of them); 0 when the kernel cannot be configured.
+template <int BN, bool AFFINE, bool PAIR>
+int persistent_workers() {
+  using S = PSmem<BN, PAIR>;
+  static int workers = 0;
+  if (workers != 0) return workers;
+  if (cudaFuncSetAttribute(gemm_tf32_persistent_kernel<BN, AFFINE, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::TOTAL) != cudaSuccess) return 0;
+  int n = sm_count();
+  if constexpr (PAIR) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(n / 2 * 2));
+    cfg.blockDim = dim3(PERSISTENT_THREADS);
+    cfg.dynamicSmemBytes = S::TOTAL;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    n /= 2;
+    int fit = 0;
+    if (cudaOccupancyMaxActiveClusters(&fit, gemm_tf32_persistent_kernel<BN, AFFINE, PAIR>, &cfg) == cudaSuccess && fit > 0 && fit < n) n = fit;
+  }
+  return workers = n;
+}
+
 // Launch the persistent kernel on ready-made tensor maps (ca.taps == 0: ma is a 2-D map of A[M, K]).
-template <int BN>
+template <int BN, bool AFFINE, bool PAIR>
 int launch_persistent_maps(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mc, const ConvA& ca, const float* bias,
                            int M, int N, int K, int accumulate, float* col_partials, int* error_flag, cudaStream_t st,
-                           const BnFin* fin = nullptr, const ConvC* cc = nullptr, int splits = 1, int cta_sums = 0, const Affine* aff = nullptr) {
-  using S = PSmem<BN>;
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_tf32_persistent_kernel<BN, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::TOTAL);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_tf32_persistent_kernel<BN, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::TOTAL);
-    if (e != cudaSuccess) return (int)e;
-    configured = true;
-  }
-  int tiles_m = (M + BM - 1) / BM, tiles_n = (N + BN - 1) / BN;
+                           const BnFin* fin, const ConvC* cc, int splits, int cta_sums, const Affine* aff) {
+  using S = PSmem<BN, PAIR>;
+  const int workers_max = persistent_workers<BN, AFFINE, PAIR>();
+  if (workers_max == 0) return (int)cudaGetLastError();
+  constexpr int ROWS = PAIR ? 2 * BM : BM;
+  int tiles_m = (M + ROWS - 1) / ROWS, tiles_n = (N + BN - 1) / BN;
   if (splits < 1 || splits > (K + BK - 1) / BK) return (int)cudaErrorInvalidValue;
   // a split contraction adds partial tiles into C: the caller zeroed C (or wants C += ...), and nothing that needs the
   // finished values (column statistics) or a store map without a reduce form can ride along
   if (splits > 1 && (!accumulate || col_partials != nullptr || (fin != nullptr && fin->acc != nullptr) || cc != nullptr))
     return (int)cudaErrorInvalidValue;
   int64_t total = (int64_t)tiles_m * tiles_n * splits;
-  int64_t grid = total < sm_count() ? total : sm_count();
+  int64_t workers = total < workers_max ? total : workers_max;
   BnFin f{};
   if (fin != nullptr && fin->acc != nullptr) {
-    if (col_partials != nullptr || tiles_n > grid) return (int)cudaErrorInvalidValue;
-    grid = grid / tiles_n * tiles_n;             // every CTA stays on one column tile
+    if (col_partials != nullptr || tiles_n > workers) return (int)cudaErrorInvalidValue;
+    workers = workers / tiles_n * tiles_n;             // every CTA stays on one column tile
     f = *fin;
   }
   if (aff != nullptr && (splits > 1 || accumulate || col_partials != nullptr || fin != nullptr || cc != nullptr)) return (int)cudaErrorInvalidValue;
   if (cta_sums) {
-    if (col_partials == nullptr || splits > 1 || tiles_n > grid) return (int)cudaErrorInvalidValue;
-    grid = grid / tiles_n * tiles_n;
+    if (col_partials == nullptr || splits > 1 || tiles_n > workers) return (int)cudaErrorInvalidValue;
+    workers = workers / tiles_n * tiles_n;
   }
-  gc::launch_pdl(aff != nullptr ? gemm_tf32_persistent_kernel<BN, true> : gemm_tf32_persistent_kernel<BN, false>, dim3((unsigned)grid), dim3(PERSISTENT_THREADS), (size_t)S::TOTAL, st, ma, mb, mc, ca,
-                 bias, M, N, K, tiles_m, tiles_n, splits, accumulate, col_partials, error_flag, gctc::tma_mode, f,
-                 cc != nullptr ? *cc : ConvC{0, 0}, cta_sums, aff != nullptr ? *aff : Affine{});
+  gc::launch_cluster(gemm_tf32_persistent_kernel<BN, AFFINE, PAIR>, PAIR ? 2u : 1u, dim3((unsigned)(PAIR ? 2 * workers : workers)),
+                     dim3(PERSISTENT_THREADS), (size_t)S::TOTAL, st, ma, mb, mc, ca, bias, M, N, K, tiles_m, tiles_n, splits, accumulate,
+                     col_partials, error_flag, gctc::tma_mode, f, cc != nullptr ? *cc : ConvC{0, 0}, cta_sums, aff != nullptr ? *aff : Affine{});
   return (int)cudaGetLastError();
 }
 
-// Rows of partial sums a launch with cta_sums leaves for tiles of `bn` columns.
-inline int cta_sum_rows(int M, int N, int bn) {
-  const int64_t tiles_n = (N + bn - 1) / bn, total = (int64_t)((M + BM - 1) / BM) * tiles_n;
-  const int64_t grid = total < sm_count() ? total : sm_count();
-  return tiles_n > grid ? 0 : (int)(grid / tiles_n);
+template <bool AFFINE = false>
+int launch_plan(const Plan& pl, const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mc, const ConvA& ca, const float* bias,
+                int M, int N, int K, int accumulate, float* col_partials, int* error_flag, cudaStream_t st,
+                const BnFin* fin = nullptr, const ConvC* cc = nullptr, int cta_sums = 0, const Affine* aff = nullptr) {
+  auto run = [&](auto launch) {
+    return launch(ma, mb, mc, ca, bias, M, N, K, accumulate, col_partials, error_flag, st, fin, cc, pl.splits, cta_sums, aff);
+  };
+  switch (pl.bn) {
+    case 64: return pl.pair ? run(launch_persistent_maps<64, AFFINE, true>) : run(launch_persistent_maps<64, AFFINE, false>);
+    case 128: return pl.pair ? run(launch_persistent_maps<128, AFFINE, true>) : run(launch_persistent_maps<128, AFFINE, false>);
+    case 256: return pl.pair ? run(launch_persistent_maps<256, AFFINE, true>) : run(launch_persistent_maps<256, AFFINE, false>);
+    default: return (int)cudaErrorInvalidValue;
+  }
+}
+
+// CTAs or CTA pairs a plan runs at once.
+inline int plan_workers(const Plan& pl) {
+  if (!pl.pair) return sm_count();
+  switch (pl.bn) {
+    case 64: return persistent_workers<64, false, true>();
+    case 128: return persistent_workers<128, false, true>();
+    default: return persistent_workers<256, false, true>();
+  }
+}
+
+// Rows of partial sums a launch with cta_sums leaves.
+inline int cta_sum_rows(int M, int N, const Plan& pl) {
+  const int64_t at_once = plan_workers(pl), tiles_n = (N + pl.bn - 1) / pl.bn, total = (int64_t)((M + pl.rows() - 1) / pl.rows()) * tiles_n;
+  const int64_t workers = total < at_once ? total : at_once;
+  return tiles_n > workers ? 0 : (int)(workers / tiles_n) * (pl.pair ? 2 : 1);
 }
 
 // Launch the split-K TN kernel on ready-made tensor maps.  At most tn_ctas_per_sm CTAs per SM over all tiles, at least
@@ -1078,68 +1252,69 @@ int launch_tn_maps(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorM
   return (int)cudaGetLastError();
 }
 
-// Tile width of the persistent kernel: the candidate with the lowest modelled time.  A tile costs the larger of
-// its DRAM share (C written once, A read once per row of tiles) and its shared-memory fill (A and B per
-// k-block), plus a fixed start-up; CTAs work through ceil(tiles / SMs) tiles one after the other.
-int pick_bn_persistent(int M, int N, int K) {
-  int sms = sm_count();
-  int64_t mt = (M + BM - 1) / BM;
-  const int cand[3] = {256, 128, 64};
-  int best = 64;
-  double best_t = 1e30;
-  for (int i = 0; i < 3; ++i) {
-    int bn = cand[i];
-    if (bn == 256 && N <= 128) continue;
-    if (bn == 128 && N <= 64) continue;
-    int64_t nt = (N + bn - 1) / bn;
-    int64_t waves = (mt * nt + sms - 1) / sms;
-    double dram = (double)BM * bn * 4.0 + (double)BM * K * 4.0 / (double)nt;      // bytes per tile
-    double fill = (double)(BM + bn) * K * 4.0;
-    double t_tile = dram / 40.0;                                                    // ~40 B/ns of DRAM per SM
-    if (fill / 110.0 > t_tile) t_tile = fill / 110.0;                               // ~110 B/ns from L2 into one SM
-    double t = (double)waves * (t_tile + 300.0);
-    if (t < best_t) { best_t = t; best = bn; }
-  }
-  return best;
+// Modelled nanoseconds of a product on the persistent kernel.  A k-block costs a CTA the time its loads and operand reads take
+// in shared memory; measured on a B200 with 3x3 convolutions of 72 and 144 k-blocks per tile (16x16x256, 8x8x512, 4x4x512,
+// batch 128): 235 / 300 / 490 ns at 64 / 128 / 256 columns for single CTAs, 205 / 260 / 400 ns for pairs.  A tile adds about
+// 500 ns of hand-over between the accumulators, a pair's launch about 1500 ns (the two CTAs meet at its start and end).  The product
+// cannot be faster than its operands and its result cross DRAM; the two overlap, not quite perfectly.
+// `reuse`: how often an element of A is read (filter taps per input pixel of a convolution, 1 for a matrix).
+inline double plan_ns(const Plan& p, int M, int N, int K, double reuse) {
+  static constexpr double stage[2][3] = {{235.0, 300.0, 490.0}, {205.0, 260.0, 400.0}};
+  const int num_k = (K + BK - 1) / BK;
+  const int64_t items = (int64_t)((M + p.rows() - 1) / p.rows()) * ((N + p.bn - 1) / p.bn) * p.splits;
+  const int64_t workers = p.pair ? sm_count() / 2 : sm_count(), waves = (items + workers - 1) / workers;
+  const double sm = (double)waves * ((num_k + p.splits - 1) / p.splits * stage[p.pair][p.bn == 64 ? 0 : (p.bn == 128 ? 1 : 2)] + 500.0);
+  const double dram = ((double)M * K / reuse + (double)M * N * (p.splits > 1 ? 2.0 : 1.0) + (double)N * K) * 4.0 / 6500.0;
+  return (sm > dram ? sm + 0.15 * dram : dram + 0.15 * sm) + (p.pair ? 1500.0 : 0.0);
 }
 
-// Modelled cycles of zeroing `elements` floats with a memset node, and of one more pass over them for column statistics.
-inline double zero_cycles(int64_t elements) { return 3000.0 + (double)elements * 4.0 / 3000.0; }
-inline double stats_pass_cycles(int64_t elements) { return 8000.0 + (double)elements * 4.0 / 2000.0; }
-
-// Tile width and number of contraction splits for a product whose output may be built from partial tiles (no column
-// statistics wanted, plain 2-D output).  Modelled cycles of the slowest CTA: a k-block costs the issuing thread about
-// 200 cycles of waiting and committing plus the larger of four MMA issues and their tensor time (420 / 500 / 720 cycles
-// for 64 / 128 / 256 columns, measured with clock64 inside the kernel), a work item about 2500 cycles of fill and
-// drain.  extra_split_cycles: what a caller pays elsewhere when the product is split (zeroing C, a separate pass for the
-// statistics).  Returns splits = 1 with pick_bn_persistent's width when splitting does not pay.
-inline void plan_persistent(int M, int N, int K, double extra_split_cycles, int* bn_out, int* splits_out) {
-  *bn_out = gctc::tile_choice ? gctc::tile_choice : pick_bn_persistent(M, N, K);
-  *splits_out = 1;
-  if (gctc::split_choice == 1) return;
-  const int sms = sm_count();
-  const int num_k = (K + BK - 1) / BK;
-  const int64_t mt = (M + BM - 1) / BM;
-  auto cycles = [&](int bn, int splits) {
-    const double stage = bn == 64 ? 420.0 : (bn == 128 ? 500.0 : 720.0);
-    const int64_t items = mt * ((N + bn - 1) / bn) * splits;
-    const int64_t waves = (items + sms - 1) / sms;
-    return (double)waves * ((double)((num_k + splits - 1) / splits) * stage + 2500.0) + (splits > 1 ? extra_split_cycles : 0.0);
-  };
-  double best = cycles(*bn_out, 1);
+// Candidates of the plan: widths that do not leave half a tile empty, pairs where there are two row tiles.
+template <typename F>
+inline void each_plan(int M, int N, F&& f) {
   const int cand[3] = {256, 128, 64};
   for (int i = 0; i < 3; ++i) {
     const int bn = cand[i];
-    if ((bn == 256 && N <= 128) || (bn == 128 && N <= 64)) continue;
-    if (gctc::tile_choice && bn != gctc::tile_choice) continue;
+    if (gctc::tile_choice ? bn != gctc::tile_choice : ((bn == 256 && N <= 128) || (bn == 128 && N <= 64))) continue;
+    for (int pair = 0; pair < 2; ++pair)
+      if (pair == 0 ? (gctc::pair_choice != 2 || M <= BM) : (gctc::pair_choice != 1 && M > BM)) f(bn, pair != 0);
+  }
+}
+
+// Tile width and pairing of a product that is not split: the candidate with the lowest modelled time.
+inline Plan pick_persistent(int M, int N, int K, double reuse = 1.0) {
+  Plan best{64, 1, false};
+  double best_t = 1e30;
+  each_plan(M, N, [&](int bn, bool pair) {
+    const Plan p{bn, 1, pair};
+    const double t = plan_ns(p, M, N, K, reuse);
+    if (t < best_t) { best_t = t; best = p; }
+  });
+  return best;
+}
+
+// Modelled time of zeroing `elements` floats with a memset node, and of one more pass over them for column statistics.
+inline double zero_ns(int64_t elements) { return 1600.0 + (double)elements * 4.0 / 5700.0; }
+inline double stats_pass_ns(int64_t elements) { return 4200.0 + (double)elements * 4.0 / 3800.0; }
+
+// The same for a product whose output may be built from partial tiles (no column statistics wanted, plain 2-D output): the
+// contraction is also split where that pays.  extra_split_ns: what a caller pays elsewhere when the product is split
+// (zeroing C, a separate pass for the statistics).
+inline Plan plan_persistent(int M, int N, int K, double extra_split_ns, double reuse = 1.0) {
+  Plan pl = pick_persistent(M, N, K, reuse);
+  if (gctc::split_choice == 1) return pl;
+  const int num_k = (K + BK - 1) / BK;
+  double best = plan_ns(pl, M, N, K, reuse);
+  each_plan(M, N, [&](int bn, bool pair) {
     for (int splits = 2; splits <= 16; ++splits) {
       const int per = (num_k + splits - 1) / splits;
       if (per < 6 || (splits - 1) * per >= num_k) continue;      // every split non-empty and long enough to fill the ring
       if (gctc::split_choice > 1 && splits != gctc::split_choice) continue;
-      const double c = cycles(bn, splits);
-      if (c < best * 0.93 || (gctc::split_choice > 1 && *splits_out == 1)) { best = c; *bn_out = bn; *splits_out = splits; }
+      const Plan p{bn, splits, pair};
+      const double t = plan_ns(p, M, N, K, reuse) + extra_split_ns;
+      if (t < best * 0.93 || (gctc::split_choice > 1 && pl.splits == 1)) { best = t; pl = p; }
     }
-  }
+  });
+  return pl;
 }
 
 }  // namespace

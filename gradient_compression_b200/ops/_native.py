@@ -174,12 +174,13 @@ def cuda():
         _declare(lib, "gc_cuda_conv_dgrad", c_int, [P, P, P, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, P, P])
         _declare(lib, "gc_cuda_gemm_tf32_splits", c_int, [c_int] * 3)
         _declare(lib, "gc_cuda_tc_split_config", None, [c_int])
+        _declare(lib, "gc_cuda_tc_pair_config", None, [c_int])
         _declare(lib, "gc_cuda_conv_fwd", c_int, [P, P, P, P] + [c_int] * 9 + [P, P, P, P, c_int])
         _declare(lib, "gc_cuda_conv_bn_eval_scratch", c_i64, [c_int] * 8)
         _declare(lib, "gc_cuda_conv_bn_eval", c_int, [P, P, P, P] + [c_int] * 8 + [P, P, P, P, c_float, P, c_int, P, P, P])
         _declare(lib, "gc_cuda_max_pool2", c_int, [P, c_int, c_int, c_int, c_int, P, P])
         _declare(lib, "gc_cuda_bn_eval_apply", c_int, [P, c_i64, c_int, P, P, c_float, P, P, P, c_int, P, P])
-        _declare(lib, "gc_cuda_conv_stat_rows", c_int, [c_int] * 3)
+        _declare(lib, "gc_cuda_conv_stat_rows", c_int, [c_int] * 5)
         _declare(lib, "gc_cuda_bn_fused_supported", c_int, [c_i64, c_int])
         _declare(lib, "gc_cuda_bn_fused_scratch_bytes", c_i64, [])
         _declare(lib, "gc_cuda_bn_fused_forward", c_int, [P] + [c_int] * 5 + [P, c_int, P, P, P, c_int, P, P, c_float, c_float, P, P, P, P, P])

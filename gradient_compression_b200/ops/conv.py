@@ -332,12 +332,12 @@ def _split_forward(lib, mode, n, h, wd, cin, cout, r, stride, pad, m):
     return hit
 
 
-def _stat_rows(lib, m, cout, k):
+def _stat_rows(lib, m, cout, k, r, stride):
     """Rows of partial sums the forward kernel leaves when every CTA adds its tiles up (cached per shape)."""
-    key = (m, cout, k)
+    key = (m, cout, k, r, stride)
     hit = _STAT_ROWS.get(key)
     if hit is None:
-        hit = _STAT_ROWS[key] = int(lib.gc_cuda_conv_stat_rows(m, cout, k))
+        hit = _STAT_ROWS[key] = int(lib.gc_cuda_conv_stat_rows(*key))
     return hit
 
 
@@ -367,7 +367,10 @@ class _ConvBNAct(torch.autograd.Function):
                 if FUSED_FINALIZE and cout <= gemm.FIN_MAX_CHANNELS and cout > 16:
                     fin = gemm.bn_fin_args(x.device, stats, running_mean, running_var, momentum, eps)
                 elif not _split_forward(lib, mode, n, h, wd, cin, cout, r, stride, pad, m):
-                    rows = _stat_rows(lib, m, cout, cin if mode == "gemm" else (STEM_K if mode == "stem" else r * r * cin)) if one_launch else 0
+                    rows = 0
+                    if one_launch:
+                        rows = _stat_rows(lib, m, cout, r * r * cin, r, stride) if mode == "conv" else \
+                            _stat_rows(lib, m, cout, cin if mode == "gemm" else STEM_K, 1, 1)
                     cta_sums = rows > 0
                     partials = torch.empty(rows or gemm.m_tiles(m), 2, cout, dtype=torch.float32, device=x.device)
             if mode == "gemm":

@@ -142,6 +142,12 @@ def configure_split(splits=0):
     nat.cuda().gc_cuda_tc_split_config(int(splits))
 
 
+def configure_pair(pairs=0):
+    """CTA pairs of the persistent kernel (256-row tiles): 0 = the kernels' cost model decides, 1 = never, 2 = wherever there are
+    two row tiles -- for measurements and tests."""
+    nat.cuda().gc_cuda_tc_pair_config(int(pairs))
+
+
 def configure_tn(ctas_per_sm=1, min_kblocks=4):
     """Split-K policy of ``gemm_tn_tf32`` (for measurements)."""
     nat.cuda().gc_cuda_gemm_tn_config(int(ctas_per_sm), int(min_kblocks))

@@ -1,0 +1,84 @@
+"""CTA pairs of the persistent tensor-core kernel (256-row tiles) against the single-CTA tiles of the same width, whose contraction
+order they share, and against an fp32 reference."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+from gradient_compression_b200.ops import conv, gemm  # noqa: E402
+
+
+@pytest.fixture
+def paired():
+    def use(tile, pairs, splits=1):
+        gemm.configure("auto", tile)
+        gemm.configure_pair(pairs)
+        gemm.configure_split(splits)
+    yield use
+    use(0, 0, 0)
+
+
+def both(paired, tile, call, splits=1):
+    out = []
+    for pairs in (1, 2):
+        paired(tile, pairs, splits)
+        out.append(call().clone())
+    return out
+
+
+def close(a, b, tol=3e-3):
+    assert float((a.double() - b.double()).norm() / b.double().norm()) < tol
+
+
+@pytest.mark.parametrize("tile", [64, 128, 256])
+@pytest.mark.parametrize("m,n,k", [(129, 20, 4), (256, 64, 32), (257, 68, 100), (640, 260, 96), (19000, 256, 64), (40000, 128, 160)])
+def test_gemm(paired, tile, m, n, k):
+    """Second CTA with one row, none of its rows, ragged columns, one and several tiles per pair."""
+    g = torch.Generator(device="cuda").manual_seed(m + n)
+    a, b = torch.randn(m, k, device="cuda", generator=g), torch.randn(n, k, device="cuda", generator=g)
+    bias = torch.randn(n, device="cuda", generator=g)
+    one, two = both(paired, tile, lambda: gemm.gemm_tf32(a, b, bias))
+    assert torch.equal(one, two)
+    close(two, a @ b.t() + bias)
+    base = torch.randn(m, n, device="cuda", generator=g)
+    one, two = both(paired, tile, lambda: gemm.gemm_tf32(a, b, out=base.clone(), accumulate=True))
+    assert torch.equal(one, two)
+
+
+@pytest.mark.parametrize("tile", [64, 128, 256])
+def test_split_and_sums(paired, tile):
+    g = torch.Generator(device="cuda").manual_seed(3)
+    a, b = torch.randn(700, 1024, device="cuda", generator=g), torch.randn(96, 1024, device="cuda", generator=g)
+    one, two = both(paired, tile, lambda: gemm.gemm_tf32(a, b), splits=3)
+    close(two, one, 1e-5)
+    paired(tile, 2)
+    rows = gemm.m_tiles(700)
+    partials = torch.full((rows, 2, 96), float("nan"), device="cuda")
+    y = gemm.gemm_tf32(a, b, col_partials=partials)
+    close(partials[:, 0].double().sum(0), y.double().sum(0), 1e-5)
+    close(partials[:, 1].double().sum(0), (y.double() ** 2).sum(0), 1e-5)
+
+
+@pytest.mark.parametrize("tile", [64, 128, 256])
+@pytest.mark.parametrize("n,h,cin,cout,stride", [(1, 16, 32, 64, 1), (3, 16, 64, 96, 1), (18, 8, 64, 128, 2), (70, 16, 32, 64, 1), (20, 4, 96, 64, 1)])
+def test_conv(paired, tile, n, h, cin, cout, stride):
+    """Forward and input gradient (filter read in place), one image to several tiles per pair; exact on small integers."""
+    lib, st = conv.nat.cuda(), conv.nat.stream_ptr()
+    flag = gemm._error_flag(torch.device("cuda", 0)).data_ptr()
+    g = torch.Generator().manual_seed(n + h)
+    ints = lambda *shape: torch.randint(-3, 4, shape, generator=g).float().cuda().contiguous(memory_format=torch.channels_last)  # noqa: E731
+    x, w, dy = ints(n, cin, h, h), ints(cout, cin, 3, 3), ints(n, cout, h // stride, h // stride)
+    assert lib.gc_cuda_conv_fwd_supported(n, h, h, cin, cout, 3, stride, 1)
+    paired(tile, 2)
+    assert torch.equal(conv.conv_forward(x, w, None, stride, 1), torch.nn.functional.conv2d(x.double(), w.double(), None, stride, 1).float())
+    dx = torch.empty_like(x)
+    if stride == 1:
+        conv.nat.check(lib.gc_cuda_conv_dgrad(dy.data_ptr(), w.data_ptr(), dx.data_ptr(), n, h, h, cin, cout, 3, 1, 0, flag, st), "dgrad")
+    elif lib.gc_cuda_conv_dgrad_s2_supported(n, h, h, cin, cout, 3, 1):
+        conv.nat.check(lib.gc_cuda_conv_dgrad_s2(dy.data_ptr(), w.data_ptr(), dx.data_ptr(), n, h, h, cin, cout, 3, 1, flag, st), "dgrad_s2")
+    else:
+        return
+    ref = torch.ops.aten.convolution_backward(dy.double(), x.double(), w.double(), None, [stride] * 2, [1, 1], [1, 1], False, [0, 0], 1,
+                                              [True, False, False])[0].float()
+    gemm.check()
+    assert torch.equal(dx, ref)
