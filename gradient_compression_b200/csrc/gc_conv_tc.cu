@@ -12,7 +12,7 @@
 //                              kernel on dY with the filter rotated by 180 degrees and its channel axes swapped.
 //                              Batch-norm statistics and bias come from the GEMM epilogue as for the 1x1 case.
 //   weight gradient            dW[Cout, R*S*Cin] += dY[P, Cout]^T * X_shifted[P, Cin] per tap = gemm_tn_tf32_kernel
-//                              whose B operand is a shifted 4-D box of 64 output positions x 32 channels.
+//                              whose B operand is a shifted 4-D box of 32 output positions x 32 channels.
 //   im2col_small_kernel        the 3-channel stem: its rows are 12 bytes apart, which no tensor map can describe,
 //                              so the 27 taps of every position are gathered into rows of 32 floats once and the
 //                              convolution becomes a plain GEMM with K = 32.
@@ -343,7 +343,7 @@ int gc_cuda_conv_dgrad(const float* dy, const float* w, float* dx, int N, int H,
 void gc_cuda_conv_wgrad_two_taps(int on) { gctc::wgrad_two_taps = on ? 1 : 0; }
 
 // 1 when the weight gradient of this convolution can run on the tensor cores: Cin a multiple of 64, Cout of 32, and
-// 64 consecutive output positions form one box.
+// 32 consecutive output positions form one box.
 int gc_cuda_conv_wgrad_supported(int N, int H, int W, int Cin, int Cout, int R, int stride, int pad) {
   Shape s;
   return make_shape(N, H, W, Cin, Cout, R, stride, pad, &s) && wgrad_ok(s) ? 1 : 0;

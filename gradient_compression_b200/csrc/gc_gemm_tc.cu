@@ -385,7 +385,7 @@ void gc_cuda_tc_tma_mode(int mode) { gctc::tma_mode = mode; }
 // For measurements: CTAs per SM the split contraction aims at, and the fewest k-blocks (of 32 rows) a split may get.
 void gc_cuda_gemm_tn_config(int ctas_per_sm, int min_kblocks) {
   gctc::tn_ctas_per_sm = ctas_per_sm > 0 ? ctas_per_sm : 1;
-  gctc::tn_min_kblocks = min_kblocks > 0 ? min_kblocks : 4;
+  gctc::tn_min_kblocks = min_kblocks > 0 ? min_kblocks : 8;
 }
 
 // 1 when C[Mo, No] += A[P, Mo]^T B[P, No] can run on the tensor cores: Mo and No multiples of 32, 16-byte aligned

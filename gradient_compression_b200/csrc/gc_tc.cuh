@@ -22,12 +22,12 @@
 
 // Measurement knobs shared by every translation unit of the library (set through gc_cuda_gemm_tf32_config /
 // gc_cuda_gemm_tn_config): forced tile width (0 = choose), CTAs per SM the split contraction aims at, fewest
-// k-blocks (of 64 rows) a split may get.
+// k-blocks (of TBK rows) a split may get.
 namespace gctc {
 inline int tile_choice = 0;
 inline int pair_choice = 0;    // CTA pairs in the persistent kernel: 0 = modelled, 1 = never, 2 = wherever there are two row tiles
 inline int tn_ctas_per_sm = 1;
-inline int tn_min_kblocks = 4;
+inline int tn_min_kblocks = 8;
 inline int wgrad_two_taps = 0;
 inline int split_choice = 0;   // contraction splits of the persistent kernel: 0 = modelled, 1 = never, n = n where a product allows it
 inline int tma_mode = 1;   // bit 0: prefetch the tensor maps at kernel start; bit 2: epilogue warps sleep between polls while a tile is being accumulated
@@ -38,7 +38,7 @@ namespace {
 constexpr int BM = 128;
 constexpr int BK = 32;                       // 32 fp32 = 128 bytes = one swizzle row
 constexpr int UMMA_K = 8;                    // tf32
-constexpr int TBK = 64;                      // contraction rows per stage of the split-K (MN-major) kernel: 8 KB TMA boxes
+constexpr int TBK = 32;                      // contraction rows per stage of the split-K (MN-major) kernel: 4 KB TMA boxes
 constexpr int GEMM_THREADS = 192;           // one-tile-per-CTA kernel: producer warp, MMA warp, four epilogue warps
 // The persistent and the split-K kernels have TWO producer warps that take alternate stages of the ring.  One thread
 // needs about 500 cycles per stage (a try_wait that succeeds at once ~170, arrive.expect_tx ~55, the first TMA
@@ -858,7 +858,7 @@ gemm_tf32_persistent_kernel(const __grid_constant__ CUtensorMap tma_a, const __g
 // with TMA reduce stores, so C must hold the value to add to (zeros for a plain product).
 template <int BN>
 struct TnSmem {
-  static constexpr int STAGES = (BN <= 64) ? 4 : ((BN <= 128) ? 3 : 2);
+  static constexpr int STAGES = (BN <= 64) ? 8 : ((BN <= 128) ? 6 : 4);
   static constexpr int CHUNK_BYTES = TBK * 128;             // one TMA box: 32 floats of the output dimension x TBK rows
   static constexpr int A_BYTES = BM * TBK * 4;
   static constexpr int B_BYTES = BN * TBK * 4;

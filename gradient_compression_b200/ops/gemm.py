@@ -148,7 +148,7 @@ def configure_pair(pairs=0):
     nat.cuda().gc_cuda_tc_pair_config(int(pairs))
 
 
-def configure_tn(ctas_per_sm=1, min_kblocks=4):
+def configure_tn(ctas_per_sm=1, min_kblocks=8):
     """Split-K policy of ``gemm_tn_tf32`` (for measurements)."""
     nat.cuda().gc_cuda_gemm_tn_config(int(ctas_per_sm), int(min_kblocks))
 
