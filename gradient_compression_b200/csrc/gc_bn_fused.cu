@@ -193,9 +193,11 @@ __global__ void __launch_bounds__(THREADS, 1) bn_fused_fwd_kernel(const Shape s,
     constexpr int P = THREADS / VALUES;
     double t = 0.0;
     int i = part;
-    for (; i + 3 * P < a.nparts; i += 4 * P) {
-      const float v0 = base[(int64_t)i * 2 * C], v1 = base[(int64_t)(i + P) * 2 * C], v2 = base[(int64_t)(i + 2 * P) * 2 * C], v3 = base[(int64_t)(i + 3 * P) * 2 * C];
-      t += ((double)v0 + (double)v1) + ((double)v2 + (double)v3);
+    for (; i + 7 * P < a.nparts; i += 8 * P) {
+      float v[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) v[j] = base[(int64_t)(i + j * P) * 2 * C];
+      t += (((double)v[0] + (double)v[1]) + ((double)v[2] + (double)v[3])) + (((double)v[4] + (double)v[5]) + ((double)v[6] + (double)v[7]));
     }
     for (; i < a.nparts; i += P) t += (double)base[(int64_t)i * 2 * C];
     lane_part[part][value] = t;

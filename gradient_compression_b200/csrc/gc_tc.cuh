@@ -269,8 +269,10 @@ struct BnFin {
   float momentum, eps;
 };
 
-// Batch norm of running statistics folded into the epilogue (inference): out = act((acc + bias) * sc + sh [+ residual]) with
-// sc = gamma / sqrt(var + eps) and sh = beta - mean * sc per column.  mean == NULL: off.  residual: [M, N], row pitch N.
+// Batch norm of running statistics in the epilogue (inference): out = act((acc + bias - mean) * rstd * gamma + beta [+ residual]) per
+// column, rounded as the apply kernels round it: folded into one multiply-add, the rounding alone moved the logits of a
+// ResNet-50 by a per cent (a last bit more or less decides where the next layer's TF32 operands are cut).
+// residual: [M, N], row pitch N.
 struct Affine {
   const float *gamma, *beta, *mean, *var, *residual;
   float eps;
@@ -630,11 +632,20 @@ gemm_tf32_persistent_kernel(const __grid_constant__ CUtensorMap tma_a, const __g
     uint32_t lt = 0, sc = 0;                                   // tiles drained, slabs staged by this group
     const bool fin_on = fin.acc != nullptr;
     const bool want_sums = col_partials != nullptr || fin_on;
-    float run_a = 0.f, run_b = 0.f;                            // fin_on, cta_sums: this thread's column, summed over the CTA's tiles
+    double run_a = 0.0, run_b = 0.0;                           // fin_on, cta_sums: this thread's column, summed over the CTA's tiles
     bool drained_all = true;
     constexpr bool aff_on = AFFINE;
     const bool with_res = AFFINE && aff.residual != nullptr;
-    float* col_affine = colsum + ew * 64;                      // aff_on: 32 scales and 32 shifts of the slab, per warp
+    // aff_on: mean, rstd, gamma, beta and bias of the slab's 32 columns, one array of the first four per warp of the group
+    float* col_affine = reinterpret_cast<float*>(base + S::COLSUM_OFF) + grp * (5 * 32);
+    float cval = 0.f, cbias = 0.f;                             // this thread's of the next slab
+    auto load_columns = [&](int col0) {
+      const int col = col0 + lane, which = ew & 3;
+      const float* from = which == 0 ? aff.mean : which == 1 ? aff.var : which == 2 ? aff.gamma : aff.beta;
+      cval = col < N ? from[col] : 0.f;
+      if (which == 1) cval = rsqrtf(cval + aff.eps);
+      if (which == 0) cbias = col < N && bias != nullptr ? bias[col] : 0.f;
+    };
     float4 res[8];                                             // with_res: the next slab's residual, 4 rows of 128 bytes per load of a warp
     auto load_residual = [&](int m0, int col0) {
       const int c = col0 + (te & 7) * 4;
@@ -650,6 +661,7 @@ gemm_tf32_persistent_kernel(const __grid_constant__ CUtensorMap tma_a, const __g
       const int mi = PAIR ? (tile / tiles_n) * 2 + rank : tile / tiles_n;      // row tile of 128; of a pair the second may lie beyond M
       const int m0 = mi * BM, n0 = (tile % tiles_n) * BN;
       const uint32_t buf = lt & 1u, aphase = (lt >> 1) & 1u;
+      if (aff_on) load_columns(n0 + grp * 32);
       if (with_res) load_residual(m0, n0 + grp * 32);
       const bool got = (tma_mode & 4) ? mbar_wait_idle(&acc_full[buf], aphase, &abort_flag, 128u) : mbar_wait(&acc_full[buf], aphase, &abort_flag);
       // one thread decides for the group: the TMEM loads are warp-collective and the named barriers below
@@ -663,30 +675,22 @@ gemm_tf32_persistent_kernel(const __grid_constant__ CUtensorMap tma_a, const __g
 #pragma unroll 1
       for (int sl = grp; sl < SLABS; sl += EPI_GROUPS, ++sc) {
         uint8_t* slab = my_staging + (sc % RING) * S::SLAB_BYTES;
+        if (aff_on) {                                          // the barrier that ended the last slab lets them be overwritten
+          col_affine[(ew & 3) * 32 + lane] = cval;
+          if ((ew & 3) == 0) col_affine[4 * 32 + lane] = cbias;
+          if (sl + EPI_GROUPS < SLABS) load_columns(n0 + (sl + EPI_GROUPS) * 32);
+        }
         // the store that last read this buffer was committed RING groups ago
         if (issuer) asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(RING - 1) : "memory");
         group_bar(grp);
-        if (aff_on) {
-          const int col = n0 + sl * 32 + lane;
-          float sc = 0.f, sh = 0.f;
-          if (col < N) {
-            sc = aff.gamma[col] * rsqrtf(aff.var[col] + aff.eps);
-            sh = fmaf((bias != nullptr ? bias[col] : 0.f) - aff.mean[col], sc, aff.beta[col]);
-          }
-          __syncwarp();
-          col_affine[lane] = sc;
-          col_affine[32 + lane] = sh;
-          if (with_res) {
+        if (with_res) {
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
-              const int row = (te >> 3) + 16 * i;
-              *reinterpret_cast<float4*>(slab + row * 128 + (((te & 7) ^ (row & 7)) << 4)) = res[i];
-            }
-            if (sl + EPI_GROUPS < SLABS) load_residual(m0, n0 + (sl + EPI_GROUPS) * 32);
-            group_bar(grp);
-          } else {
-            __syncwarp();
+          for (int i = 0; i < 8; ++i) {
+            const int row = (te >> 3) + 16 * i;
+            *reinterpret_cast<float4*>(slab + row * 128 + (((te & 7) ^ (row & 7)) << 4)) = res[i];
           }
+          if (sl + EPI_GROUPS < SLABS) load_residual(m0, n0 + (sl + EPI_GROUPS) * 32);
+          group_bar(grp);
         }
         uint32_t ra[16], rb[16];
         tmem_ld16_nowait(lane_base + (uint32_t)(sl * 32), ra);
@@ -699,8 +703,14 @@ gemm_tf32_persistent_kernel(const __grid_constant__ CUtensorMap tma_a, const __g
           float4 o = make_float4(__uint_as_float(src[0]), __uint_as_float(src[1]), __uint_as_float(src[2]), __uint_as_float(src[3]));
           float4* to = reinterpret_cast<float4*>(slab + r * 128 + ((c ^ (r & 7)) << 4));           // 128-byte swizzle of the store map
           if (aff_on) {
-            const float4 sc = *reinterpret_cast<const float4*>(col_affine + c * 4), sh = *reinterpret_cast<const float4*>(col_affine + 32 + c * 4);
-            o = make_float4(fmaf(o.x, sc.x, sh.x), fmaf(o.y, sc.y, sh.y), fmaf(o.z, sc.z, sh.z), fmaf(o.w, sc.w, sh.w));
+            auto column = [&](int k) { return *reinterpret_cast<const float4*>(col_affine + k * 32 + c * 4); };
+            if (bias != nullptr) {
+              const float4 b = column(4);
+              o.x += b.x; o.y += b.y; o.z += b.z; o.w += b.w;
+            }
+            const float4 mu = column(0), rs = column(1), gm = column(2), bt = column(3);
+            o = make_float4(fmaf((o.x - mu.x) * rs.x, gm.x, bt.x), fmaf((o.y - mu.y) * rs.y, gm.y, bt.y), fmaf((o.z - mu.z) * rs.z, gm.z, bt.z),
+                            fmaf((o.w - mu.w) * rs.w, gm.w, bt.w));
             if (with_res) {
               const float4 q = *to;
               o.x += q.x; o.y += q.y; o.z += q.z; o.w += q.w;
@@ -778,8 +788,8 @@ gemm_tf32_persistent_kernel(const __grid_constant__ CUtensorMap tma_a, const __g
             float a = (my_colsum[c * 2] + my_colsum[(BN + c) * 2]) + (my_colsum[(2 * BN + c) * 2] + my_colsum[(3 * BN + c) * 2]);
             float b = (my_colsum[c * 2 + 1] + my_colsum[(BN + c) * 2 + 1]) + (my_colsum[(2 * BN + c) * 2 + 1] + my_colsum[(3 * BN + c) * 2 + 1]);
             if (fin_on || cta_sums) {
-              run_a += a;
-              run_b += b;
+              run_a += (double)a;
+              run_b += (double)b;
             } else if (!PAIR || m0 < M) {
               col_partials[((int64_t)mi * 2) * N + gc] = a;
               col_partials[((int64_t)mi * 2 + 1) * N + gc] = b;
@@ -789,12 +799,19 @@ gemm_tf32_persistent_kernel(const __grid_constant__ CUtensorMap tma_a, const __g
       }
     }
     if (cta_sums && drained_all && te < (SLABS / EPI_GROUPS) * 32) {
-      // one row of partial sums per CTA that stays on this column tile (instead of one per row tile)
+      // one row of partial sums per CTA that stays on this column tile (instead of one per row tile); where a CTA has several
+      // tiles, a second set of rows carries what the first one's rounding left out
       const int gc = (worker % tiles_n) * BN + (grp + EPI_GROUPS * (te >> 5)) * 32 + (te & 31);
       const int64_t row = (int64_t)(PAIR ? (worker / tiles_n) * 2 + rank : worker / tiles_n) * 2;
       if (gc < N) {
-        col_partials[row * N + gc] = run_a;
-        col_partials[(row + 1) * N + gc] = run_b;
+        const float hi_a = (float)run_a, hi_b = (float)run_b;
+        col_partials[row * N + gc] = hi_a;
+        col_partials[(row + 1) * N + gc] = hi_b;
+        if (total_items > workers) {
+          const int64_t rest = row + (int64_t)(workers / tiles_n) * (PAIR ? 4 : 2);
+          col_partials[rest * N + gc] = (float)(run_a - (double)hi_a);
+          col_partials[(rest + 1) * N + gc] = (float)(run_b - (double)hi_b);
+        }
       }
     }
     if (fin_on && drained_all) {
@@ -804,8 +821,8 @@ gemm_tf32_persistent_kernel(const __grid_constant__ CUtensorMap tma_a, const __g
         const int c = (grp + EPI_GROUPS * (te >> 5)) * 32 + (te & 31);
         const int gc = (worker % tiles_n) * BN + c;
         if (gc < N) {
-          atomicAdd(&fin.acc[gc], (double)run_a);
-          atomicAdd(&fin.acc[N + gc], (double)run_b);
+          atomicAdd(&fin.acc[gc], run_a);
+          atomicAdd(&fin.acc[N + gc], run_b);
         }
       }
       __threadfence();
@@ -1223,8 +1240,8 @@ inline int plan_workers(const Plan& pl) {
 // Rows of partial sums a launch with cta_sums leaves.
 inline int cta_sum_rows(int M, int N, const Plan& pl) {
   const int64_t at_once = plan_workers(pl), tiles_n = (N + pl.bn - 1) / pl.bn, total = (int64_t)((M + pl.rows() - 1) / pl.rows()) * tiles_n;
-  const int64_t workers = total < at_once ? total : at_once;
-  return tiles_n > workers ? 0 : (int)(workers / tiles_n) * (pl.pair ? 2 : 1);
+  const int64_t workers = (total < at_once ? total : at_once) / tiles_n * tiles_n;
+  return (int)(workers / tiles_n) * (pl.pair ? 2 : 1) * (total > workers ? 2 : 1);
 }
 
 // Launch the split-K TN kernel on ready-made tensor maps.  At most tn_ctas_per_sm CTAs per SM over all tiles, at least
