@@ -10,6 +10,9 @@
 //                        (deterministic) into out[0:3] = {mean loss, top-1 rate, top-5 rate}.
 //   head_bwd_dx_kernel   dx[n, p, c] = g * sum_k dlogits[n, k] W[k, c] / positions, the same value at every position
 //   head_bwd_dw_kernel   dW[k, c] = g * sum_n dlogits[n, k] pooled[n, c], db[k] = g * sum_n dlogits[n, k]
+//   head_eval_kernel     inference: pooling and linear layer only (labels come later, with evaluate_predictions)
+//   logit_metrics_kernel cross-entropy, top-1 and top-5 of given logits, one block, one thread per sample: a dozen torch launches
+//                        took 66 of 470 microseconds of a small evaluation batch, and more of its host time
 // g is the gradient that reaches the loss (a device scalar, 1 for a plain loss.backward()).
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -24,17 +27,15 @@ constexpr int HEAD_THREADS = 256;
 constexpr int HEAD_MAX_CLASSES = 32;
 constexpr int HEAD_MAX_CHANNELS = 4096;
 
-__global__ void __launch_bounds__(HEAD_THREADS) head_fwd_kernel(const float* __restrict__ x, int positions, int C,
-                                                                const float* __restrict__ W, const float* __restrict__ bias, int K,
-                                                                const int64_t* __restrict__ labels, int N,
-                                                                float* __restrict__ pooled, float* __restrict__ logits,
-                                                                float* __restrict__ dlogits, float* __restrict__ per_sample,
-                                                                unsigned int* __restrict__ ticket, float* __restrict__ out3) {
-  __shared__ __align__(16) float sp[HEAD_MAX_CHANNELS];
-  __shared__ float slog[HEAD_MAX_CLASSES];
-  __shared__ float spart[HEAD_THREADS / 32][HEAD_MAX_CLASSES];
-  __shared__ int last;
-  const int n = blockIdx.x;
+struct HeadShared {
+  float __align__(16) pooled[HEAD_MAX_CHANNELS];
+  float logit[HEAD_MAX_CLASSES];
+  float part[HEAD_THREADS / 32][HEAD_MAX_CLASSES];
+};
+
+// Pooling and linear layer of sample n, by a whole block: sh.logit[0:K].  pooled (may be NULL), logits: of all samples.
+__device__ __forceinline__ void pooled_logits(HeadShared& sh, const float* __restrict__ x, int n, int positions, int C, const float* __restrict__ W,
+                                              const float* __restrict__ bias, int K, float* __restrict__ pooled, float* __restrict__ logits) {
   const float* xn = x + (int64_t)n * positions * C;
   const float inv_pos = 1.0f / (float)positions;
   for (int q = threadIdx.x; q < (C >> 2); q += HEAD_THREADS) {
@@ -45,49 +46,115 @@ __global__ void __launch_bounds__(HEAD_THREADS) head_fwd_kernel(const float* __r
       acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
     }
     acc.x *= inv_pos; acc.y *= inv_pos; acc.z *= inv_pos; acc.w *= inv_pos;
-    *reinterpret_cast<float4*>(sp + 4 * q) = acc;
-    *reinterpret_cast<float4*>(pooled + (int64_t)n * C + 4 * q) = acc;
+    *reinterpret_cast<float4*>(sh.pooled + 4 * q) = acc;
+    if (pooled != nullptr) *reinterpret_cast<float4*>(pooled + (int64_t)n * C + 4 * q) = acc;
   }
   __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  {
-    // every warp takes 128-channel slices of the pooled vector and all K classes at once (K independent 16-byte loads of
-    // W in flight per lane); the eight warps' partial dot products meet in shared memory in a fixed order
-    float acc[HEAD_MAX_CLASSES];
+  // every warp takes 128-channel slices of the pooled vector and all K classes at once (K independent 16-byte loads of
+  // W in flight per lane); the eight warps' partial dot products meet in shared memory in a fixed order
+  float acc[HEAD_MAX_CLASSES];
 #pragma unroll
-    for (int k = 0; k < HEAD_MAX_CLASSES; ++k) acc[k] = 0.f;
-    for (int c = warp * 128 + lane * 4; c < C; c += (HEAD_THREADS / 32) * 128) {
-      const float4 pv = *reinterpret_cast<const float4*>(sp + c);
-#pragma unroll
-      for (int k = 0; k < HEAD_MAX_CLASSES; ++k)
-        if (k < K) {
-          const float4 wv = *reinterpret_cast<const float4*>(W + (int64_t)k * C + c);
-          acc[k] = fmaf(pv.x, wv.x, fmaf(pv.y, wv.y, fmaf(pv.z, wv.z, fmaf(pv.w, wv.w, acc[k]))));
-        }
-    }
+  for (int k = 0; k < HEAD_MAX_CLASSES; ++k) acc[k] = 0.f;
+  for (int c = warp * 128 + lane * 4; c < C; c += (HEAD_THREADS / 32) * 128) {
+    const float4 pv = *reinterpret_cast<const float4*>(sh.pooled + c);
 #pragma unroll
     for (int k = 0; k < HEAD_MAX_CLASSES; ++k)
       if (k < K) {
-        const float v = warp_sum(acc[k]);
-        if (lane == 0) spart[warp][k] = v;
+        const float4 wv = *reinterpret_cast<const float4*>(W + (int64_t)k * C + c);
+        acc[k] = fmaf(pv.x, wv.x, fmaf(pv.y, wv.y, fmaf(pv.z, wv.z, fmaf(pv.w, wv.w, acc[k]))));
       }
-    __syncthreads();
-    if (threadIdx.x < K) {
-      float v = bias != nullptr ? bias[threadIdx.x] : 0.f;
+  }
 #pragma unroll
-      for (int w = 0; w < HEAD_THREADS / 32; ++w) v += spart[w][threadIdx.x];
-      slog[threadIdx.x] = v;
-      logits[(int64_t)n * K + threadIdx.x] = v;
+  for (int k = 0; k < HEAD_MAX_CLASSES; ++k)
+    if (k < K) {
+      const float v = warp_sum(acc[k]);
+      if (lane == 0) sh.part[warp][k] = v;
     }
+  __syncthreads();
+  if (threadIdx.x < K) {
+    float v = bias != nullptr ? bias[threadIdx.x] : 0.f;
+#pragma unroll
+    for (int w = 0; w < HEAD_THREADS / 32; ++w) v += sh.part[w][threadIdx.x];
+    sh.logit[threadIdx.x] = v;
+    logits[(int64_t)n * K + threadIdx.x] = v;
+  }
+}
+
+__global__ void __launch_bounds__(HEAD_THREADS) head_eval_kernel(const float* __restrict__ x, int positions, int C, const float* __restrict__ W,
+                                                                 const float* __restrict__ bias, int K, float* __restrict__ logits) {
+  __shared__ HeadShared sh;
+  pooled_logits(sh, x, blockIdx.x, positions, C, W, bias, K, nullptr, logits);
+}
+
+// out = {mean cross-entropy, top-1 rate, top-5 rate} of logits[N, K].  Samples labelled -100 do not count in the loss
+// (nn.CrossEntropyLoss's ignore_index); any other label outside the classes makes it NaN.  A NaN ranks above every number and
+// ties go to the lower class.
+constexpr int METRIC_THREADS = 1024, METRIC_MAX_CLASSES = 1024;
+__global__ void __launch_bounds__(METRIC_THREADS) logit_metrics_kernel(const float* __restrict__ logits, const int64_t* __restrict__ labels, int N, int K,
+                                                                       float* __restrict__ out) {
+  __shared__ double part[METRIC_THREADS / 32][4];
+  double loss = 0.0;
+  int counted = 0, top1 = 0, top5 = 0;
+  for (int n = threadIdx.x; n < N; n += METRIC_THREADS) {
+    const float* z = logits + (int64_t)n * K;
+    const int64_t label = labels[n];
+    const bool known = label >= 0 && label < K;
+    const float zl = known ? z[label] : NAN;
+    float zmax = -INFINITY;
+    int ahead = 0;
+#pragma unroll 8
+    for (int k = 0; k < K; ++k) {
+      const float v = z[k];
+      zmax = fmaxf(zmax, v);
+      ahead += v > zl || (isnan(v) && !isnan(zl)) || ((v == zl || (isnan(v) && isnan(zl))) && k < label);
+    }
+    float sum = 0.f;
+#pragma unroll 8
+    for (int k = 0; k < K; ++k) sum += expf(z[k] - zmax);
+    if (label != -100) {
+      loss += (double)(logf(sum) + zmax - zl);
+      ++counted;
+    }
+    top1 += known && ahead == 0;
+    top5 += known && ahead < 5;
+  }
+  double v[4] = {loss, (double)counted, (double)top1, (double)top5};
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    for (int o = 16; o > 0; o >>= 1) v[j] += __shfl_xor_sync(FULL, v[j], o);
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5][j] = v[j];
   }
   __syncthreads();
+  if (threadIdx.x < 4) {
+    double t = 0.0;
+    for (int w = 0; w < (int)blockDim.x / 32; ++w) t += part[w][threadIdx.x];
+    part[0][threadIdx.x] = t;
+  }
+  __syncwarp();
+  if (threadIdx.x == 0) out[0] = (float)(part[0][0] / part[0][1]);
+  if (threadIdx.x == 1 || threadIdx.x == 2) out[threadIdx.x] = (float)part[0][threadIdx.x + 1] * (1.0f / (float)N);     // as a tensor divided by a number
+}
+
+__global__ void __launch_bounds__(HEAD_THREADS) head_fwd_kernel(const float* __restrict__ x, int positions, int C,
+                                                                const float* __restrict__ W, const float* __restrict__ bias, int K,
+                                                                const int64_t* __restrict__ labels, int N,
+                                                                float* __restrict__ pooled, float* __restrict__ logits,
+                                                                float* __restrict__ dlogits, float* __restrict__ per_sample,
+                                                                unsigned int* __restrict__ ticket, float* __restrict__ out3) {
+  __shared__ HeadShared sh;
+  __shared__ int last;
+  const int n = blockIdx.x;
+  pooled_logits(sh, x, n, positions, C, W, bias, K, pooled, logits);
+  __syncthreads();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (warp == 0) {
     const int label = (int)labels[n];
-    const float z = lane < K ? slog[lane] : -INFINITY;
+    const float z = lane < K ? sh.logit[lane] : -INFINITY;
     const float zmax = warp_max(z);
     const float e = lane < K ? __expf(z - zmax) : 0.f;
     const float denom = warp_sum(e);
-    const float zl = (label >= 0 && label < K) ? slog[label] : 0.f;
+    const float zl = (label >= 0 && label < K) ? sh.logit[label] : 0.f;
     // position of the true class in the descending order (ties go to the lower class index, as a stable sort would)
     const int ahead = (lane < K && (z > zl || (z == zl && lane < label))) ? 1 : 0;
     const int rank = __reduce_add_sync(FULL, ahead);
@@ -104,10 +171,11 @@ __global__ void __launch_bounds__(HEAD_THREADS) head_fwd_kernel(const float* __r
   __syncthreads();
   if (!last) return;
   __threadfence();
-  if (threadIdx.x < 3) {
+  if (warp < 3) {                          // one warp per value: a single thread's N loads in a row took 3 us at 128 samples
     float acc = 0.f;
-    for (int i = 0; i < N; ++i) acc += __ldcg(per_sample + 3 * i + threadIdx.x);
-    out3[threadIdx.x] = acc / (float)N;
+    for (int i = lane; i < N; i += 32) acc += __ldcg(per_sample + 3 * i + warp);
+    acc = warp_sum(acc);
+    if (lane == 0) out3[warp] = acc / (float)N;
   }
   if (threadIdx.x == 0) *ticket = 0u;
 }
@@ -183,6 +251,21 @@ extern "C" {
 int gc_cuda_head_supported(int N, int positions, int C, int K) {
   return N >= 1 && positions >= 1 && C >= 4 && (C & 3) == 0 && C <= HEAD_MAX_CHANNELS && K >= 1 && K <= HEAD_MAX_CLASSES &&
          (int64_t)N * K * 4 + (HEAD_THREADS / 32) * K * HEAD_DW_CHANNELS * 4 <= 96 * 1024 ? 1 : 0;
+}
+
+// logits [N, K] of the feature map x [N, positions, C].  C a multiple of 4 up to 4096, at most 32 classes.
+int gc_cuda_head_eval(const float* x, int N, int positions, int C, const float* W, const float* bias, int K, float* logits, void* cs) {
+  if (N < 1 || positions < 1 || C < 4 || (C & 3) || C > HEAD_MAX_CHANNELS || K < 1 || K > HEAD_MAX_CLASSES) return (int)cudaErrorInvalidValue;
+  head_eval_kernel<<<N, HEAD_THREADS, 0, (cudaStream_t)cs>>>(x, positions, C, W, bias, K, logits);
+  return (int)cudaGetLastError();
+}
+
+// out[0:3] of logits [N, K], labels [N].
+int gc_cuda_logit_metrics(const float* logits, const int64_t* labels, int N, int K, float* out, void* cs) {
+  if (N < 1 || K < 1 || K > METRIC_MAX_CLASSES) return (int)cudaErrorInvalidValue;
+  const int threads = N < METRIC_THREADS ? (N + 31) / 32 * 32 : METRIC_THREADS;
+  logit_metrics_kernel<<<1, threads, 0, (cudaStream_t)cs>>>(logits, labels, N, K, out);
+  return (int)cudaGetLastError();
 }
 
 // Bytes of the zero-initialised scratch (ticket + per-sample values) for batches of up to max_batch samples.

@@ -45,6 +45,8 @@ struct Api {
   int64_t (*conv_bn_eval_scratch)(int, int, int, int, int, int, int, int);
   int (*conv_bn_eval)(const float*, const float*, float*, const float*, int, int, int, int, int, int, int, int, const float*, const float*, const float*,
                       const float*, float, const float*, int, float*, int*, void*);
+  int (*head_eval)(const float*, int, int, int, const float*, const float*, int, float*, void*);
+  int (*logit_metrics)(const float*, const int64_t*, int, int, float*, void*);
   int (*max_pool2)(const float*, int, int, int, int, float*, void*);
   int (*bn_supported)(int64_t, int);
   int (*bn_eval_apply)(const float*, int64_t, int, const float*, const float*, float, const float*, const float*, const float*, int, float*, void*);
@@ -68,6 +70,8 @@ const Entry entries[] = {
     {"gc_cuda_dequantize_levels", (void**)&api.dequantize},
     {"gc_cuda_conv_bn_eval_scratch", (void**)&api.conv_bn_eval_scratch},
     {"gc_cuda_conv_bn_eval", (void**)&api.conv_bn_eval},
+    {"gc_cuda_head_eval", (void**)&api.head_eval},
+    {"gc_cuda_logit_metrics", (void**)&api.logit_metrics},
     {"gc_cuda_max_pool2", (void**)&api.max_pool2},
     {"gc_cuda_bn_supported", (void**)&api.bn_supported},
     {"gc_cuda_bn_eval_apply", (void**)&api.bn_eval_apply},
@@ -460,6 +464,45 @@ PyObject* conv_bn_eval(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   return THPVariable_Wrap(y);
 }
 
+// classify(feature map, weight, bias or None) -> logits of the mean over the map, or None
+PyObject* classify(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
+  if (!want(nargs, 3, "classify")) return nullptr;
+  const at::Tensor *x = activation(a[0]), *w = tensor_of(a[1]);
+  if (!x || !w || !w->is_cuda() || w->scalar_type() != at::kFloat || w->dim() != 2 || !w->is_contiguous() || w->device() != x->device() ||
+      w->size(1) != x->size(1) || ((uintptr_t)w->data_ptr() | (uintptr_t)x->data_ptr()) & 15u)
+    Py_RETURN_NONE;
+  const int64_t n = x->size(0), c = x->size(1), positions = x->size(2) * x->size(3), k = w->size(0);
+  const float* bias = a[2] == Py_None ? nullptr : channels(a[2], *x, k);
+  if ((a[2] != Py_None && !bias) || n < 1 || n > INT32_MAX || c < 4 || c & 3 || c > 4096 || positions < 1 || positions > INT32_MAX || k < 1 || k > 32)
+    Py_RETURN_NONE;
+  c10::cuda::OptionalCUDAGuard guard(x->device());
+  at::Tensor logits = at::empty({n, k}, x->options().memory_format(at::MemoryFormat::Contiguous));
+  const int err = api.head_eval((const float*)x->data_ptr(), (int)n, (int)positions, (int)c, (const float*)w->data_ptr(), bias, (int)k,
+                                (float*)logits.data_ptr(), stream_on(x->device().index()));
+  if (err) return cuda_error("classify", err);
+  return THPVariable_Wrap(logits);
+}
+
+// logit_metrics(logits, labels) -> (cross-entropy, top-1 rate, top-5 rate), or None
+PyObject* logit_metrics(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
+  if (!want(nargs, 2, "logit_metrics")) return nullptr;
+  const at::Tensor *z = tensor_of(a[0]), *y = tensor_of(a[1]);
+  if (!z || !y || !z->is_cuda() || z->scalar_type() != at::kFloat || z->dim() != 2 || !z->is_contiguous() || y->scalar_type() != at::kLong ||
+      y->dim() != 1 || !y->is_contiguous() || y->device() != z->device() || y->size(0) != z->size(0))
+    Py_RETURN_NONE;
+  // one block: up to a quarter of a million samples, as many classes as torch.topk(5) needs at least
+  const int64_t n = z->size(0), k = z->size(1);
+  if (n < 1 || n > (1 << 18) || k < 5 || k > 1024 || n * k > (1 << 22)) Py_RETURN_NONE;
+  c10::cuda::OptionalCUDAGuard guard(z->device());
+  at::Tensor out = at::empty({3}, z->options());
+  const int err = api.logit_metrics((const float*)z->data_ptr(), (const int64_t*)y->data_ptr(), (int)n, (int)k, (float*)out.data_ptr(),
+                                    stream_on(z->device().index()));
+  if (err) return cuda_error("logit_metrics", err);
+  PyObject* t = PyTuple_New(3);
+  for (int i = 0; t && i < 3; ++i) PyTuple_SET_ITEM(t, i, THPVariable_Wrap(out.select(0, i)));
+  return t;
+}
+
 // bn_eval(x, gamma, beta, mean, var, eps, residual or None, relu) -> y
 PyObject* bn_eval(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   if (!want(nargs, 8, "bn_eval")) return nullptr;
@@ -515,6 +558,8 @@ PyMethodDef methods[] = {
     {"conv_bn_eval", (PyCFunction)(void (*)(void))conv_bn_eval, METH_FASTCALL, "convolution, batch norm of running statistics, residual, ReLU, pool"},
     {"bn_eval", (PyCFunction)(void (*)(void))bn_eval, METH_FASTCALL, "batch norm of running statistics, residual, ReLU"},
     {"absmax", (PyCFunction)(void (*)(void))absmax, METH_FASTCALL, "largest magnitude"},
+    {"classify", (PyCFunction)(void (*)(void))classify, METH_FASTCALL, "logits of a feature map in inference"},
+    {"logit_metrics", (PyCFunction)(void (*)(void))logit_metrics, METH_FASTCALL, "cross-entropy, top-1 and top-5 of logits"},
     {"quantize", (PyCFunction)(void (*)(void))quantize, METH_FASTCALL, "levels of a vector"},
     {"quantize_fit", (PyCFunction)(void (*)(void))quantize_fit, METH_FASTCALL, "levels of the higher scale and where they fit the lower one"},
     {"dequantize", (PyCFunction)(void (*)(void))dequantize, METH_FASTCALL, "values of levels of one or two scales"},

@@ -10,6 +10,8 @@ from __future__ import annotations
 import torch.nn as nn
 import torch.nn.functional as F
 
+from ..ops.head import classify
+
 
 def conv(cin, cout, k, stride=1, padding=0, groups=1, bias=False):
     return nn.Conv2d(cin, cout, kernel_size=k, stride=stride, padding=padding, groups=groups, bias=bias)
@@ -30,3 +32,9 @@ def head_pool(x, k):
     if x.dim() == 4 and x.shape[2] == k and x.shape[3] == k:
         return x.mean((2, 3))
     return F.avg_pool2d(x, k).flatten(1)
+
+
+def head(x, k, linear):
+    """``linear(head_pool(x, k))``: one kernel in inference when the window covers the whole feature map."""
+    y = classify(x, linear) if x.dim() == 4 and x.shape[2] == k and x.shape[3] == k else None
+    return linear(head_pool(x, k)) if y is None else y

@@ -5,7 +5,7 @@ from __future__ import annotations
 import torch.nn as nn
 
 from ..ops.bn import bn_act, defer_batch_counters
-from .layers import bn, conv, head_pool, linear
+from .layers import bn, conv, head, linear
 
 
 class PreActBlock(nn.Module):
@@ -60,7 +60,7 @@ class PreActResNet(nn.Module):
 
     def forward(self, x):
         x = self.layer4(self.layer3(self.layer2(self.layer1(self.conv1(x)))))
-        return self.linear(head_pool(x, 4))
+        return head(x, 4, self.linear)
 
 
 def PreActResNet18():

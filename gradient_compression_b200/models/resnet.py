@@ -8,7 +8,7 @@ import torch.nn as nn
 from ..ops.bn import defer_batch_counters, flush_batch_counters
 from ..ops.conv import GradLink, conv_bn_act
 from ..ops.head import head_loss
-from .layers import bn, conv, head_pool, linear
+from .layers import bn, conv, head, head_pool, linear
 
 
 def _projection(cin, cout, stride):
@@ -83,7 +83,7 @@ class ResNet(nn.Module):
         return self.layer4(self.layer3(self.layer2(self.layer1(x))))
 
     def forward(self, x):
-        return self.linear(head_pool(self.features(x), 4))
+        return head(self.features(x), 4, self.linear)
 
     def forward_loss(self, x, labels):
         """``(loss, logits, [cross-entropy, top-1, top-5])``: pooling, the linear layer, the loss and the batch metrics in

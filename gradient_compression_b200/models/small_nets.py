@@ -7,7 +7,7 @@ import torch.nn as nn
 import torch.nn.functional as F
 
 from ..ops.bn import bn_act
-from .layers import bn, conv, head_pool, linear
+from .layers import bn, conv, head, linear
 
 
 class LeNet(nn.Module):
@@ -107,7 +107,7 @@ class MobileNet(nn.Module):
 
     def forward(self, x):
         x = self.layers(bn_act(self.bn1, self.conv1(x)))
-        return self.linear(head_pool(x, 2))
+        return head(x, 2, self.linear)
 
 
 class _InvertedResidual(nn.Module):
@@ -151,4 +151,4 @@ class MobileNetV2(nn.Module):
     def forward(self, x):
         x = self.layers(bn_act(self.bn1, self.conv1(x)))
         x = bn_act(self.bn2, self.conv2(x))
-        return self.linear(head_pool(x, 4))
+        return head(x, 4, self.linear)

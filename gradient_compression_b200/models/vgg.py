@@ -8,7 +8,7 @@ import torch.nn as nn
 from ..ops.bn import defer_batch_counters, flush_batch_counters
 from ..ops.conv import conv_bn_act
 from ..ops.head import head_loss
-from .layers import bn, conv, linear
+from .layers import bn, conv, head, linear
 
 CFG = {
     "VGG11": [64, "M", 128, "M", 256, 256, "M", 512, 512, "M", 512, 512, "M"],
@@ -34,7 +34,7 @@ class VGG(nn.Module):
         defer_batch_counters(self)
 
     def forward(self, x):
-        return self.classifier(self._features(x).flatten(1))
+        return head(self._features(x), 1, self.classifier)
 
     def forward_loss(self, x, labels):
         """``(loss, logits, [cross-entropy, top-1, top-5])`` with the linear layer, the loss and the batch metrics in one kernel

@@ -91,3 +91,21 @@ def head_loss(features, linear, labels):
         hit = top5.eq(labels.view(-1, 1))
         metrics = torch.stack([loss.detach(), hit[:, 0].float().mean(), hit.float().sum(1).clamp(max=1).mean()])
     return loss, logits, metrics
+
+
+def classify(features, linear):
+    """Inference: ``linear(mean over H, W of features)`` in one kernel; None where it does not apply."""
+    if not features.is_cuda or torch.is_grad_enabled() or type(linear) is not torch.nn.Linear or torch.is_autocast_enabled():
+        return None
+    y = nat.ext().classify(features, linear.weight, linear.bias)
+    if y is not None:
+        nat.count_launch()
+    return y
+
+
+def logit_metrics(logits, labels):
+    """``(mean cross-entropy, top-1 rate, top-5 rate)`` of a batch of logits in one kernel; None where it does not apply."""
+    out = nat.ext().logit_metrics(logits, labels) if logits.is_cuda else None
+    if out is not None:
+        nat.count_launch()
+    return out

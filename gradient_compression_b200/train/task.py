@@ -13,6 +13,7 @@ import torch
 import torch.distributed as dist
 
 from .. import models
+from ..ops.head import logit_metrics
 from ..parallel.arena import FlatArena
 from ..utils.metrics import AverageMeter
 from ..utils.timer import NullTimer
@@ -161,12 +162,17 @@ class CIFAR:
         """cross-entropy, top-1 and top-5 accuracy of a batch.  The loss computed by the forward pass
         is reused when given (the reference evaluates it a second time, model_dispatcher.py:157)."""
         with torch.no_grad():
-            ce = self._criterion(pred_labels, true_labels) if loss is None else loss
-            top5 = pred_labels.topk(5, 1, True, True)[1]
-            hit = top5.eq(true_labels.view(-1, 1))
-            bs = true_labels.shape[0]
-            top1 = hit[:, 0].float().sum() / bs
-            top5 = hit.float().sum() / bs
+            known = logit_metrics(pred_labels, true_labels)
+            if known is not None:
+                ce, top1, top5 = known
+                ce = ce if loss is None else loss
+            else:
+                ce = self._criterion(pred_labels, true_labels) if loss is None else loss
+                top5 = pred_labels.topk(5, 1, True, True)[1]
+                hit = top5.eq(true_labels.view(-1, 1))
+                bs = true_labels.shape[0]
+                top1 = hit[:, 0].float().sum() / bs
+                top5 = hit.float().sum() / bs
         out = {"cross_entropy_loss": ce, "top1_accuracy": top1, "top5_accuracy": top5}
         if self._sync_metrics:
             out = {k: v.item() for k, v in out.items()}

@@ -1,0 +1,43 @@
+"""Inference head (pooling + linear) and batch metrics of logits against torch."""
+import pytest
+import torch
+import torch.nn.functional as F
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n,c,hw,k,bias", [(1, 4, 1, 1, True), (33, 512, 1, 10, True), (7, 516, 4, 32, False), (300, 2048, 4, 10, True), (5, 4096, 2, 5, True)])
+def test_classify(n, c, hw, k, bias):
+    from gradient_compression_b200.models.layers import head
+    from gradient_compression_b200.ops.head import classify
+
+    g = torch.Generator(device="cuda").manual_seed(n + c)
+    x = torch.randn(n, c, hw, hw, device="cuda", generator=g).contiguous(memory_format=torch.channels_last)
+    linear = torch.nn.Linear(c, k, bias=bias).cuda()
+    assert classify(x, linear) is None                      # a gradient may be wanted
+    with torch.no_grad():
+        y = classify(x, linear)
+        ref = F.linear(x.double().mean((2, 3)), linear.weight.double(), linear.bias.double() if bias else None)
+        assert y.is_contiguous() and torch.allclose(y.double(), ref, rtol=1e-5, atol=1e-5)
+        assert torch.equal(head(x, hw, linear), y)
+        wide = torch.nn.Linear(c, 40).cuda()                # more classes than the kernel takes
+        assert classify(x, wide) is None and head(x, hw, wide).shape == (n, 40)
+
+
+@pytest.mark.parametrize("n,k", [(1, 5), (31, 10), (257, 10), (1500, 100), (70, 1024)])
+def test_logit_metrics(n, k):
+    from gradient_compression_b200.ops.head import logit_metrics
+
+    g = torch.Generator(device="cuda").manual_seed(n + k)
+    z = torch.randn(n, k, device="cuda", generator=g) * 5
+    labels = torch.randint(0, k, (n,), device="cuda", generator=g)
+    for ignore in (0, n // 3):
+        labels[:ignore] = -100
+        ce, top1, top5 = logit_metrics(z, labels)
+        hit = z.topk(5, 1, True, True)[1].eq(labels.view(-1, 1))
+        assert torch.allclose(ce.double(), F.cross_entropy(z.double(), labels), rtol=1e-6)
+        assert float(top1) == float(hit[:, 0].float().sum() / n) and float(top5) == float(hit.float().sum() / n)
+    labels[-1] = 0
+    z[-1, 1] = float("nan")
+    assert torch.isnan(logit_metrics(z, labels)[0])
+    assert logit_metrics(z[:, :4].contiguous(), labels) is None and logit_metrics(z.half(), labels) is None
