@@ -374,13 +374,7 @@ int gc_cuda_conv_wgrad(const float* dy, const float* x, float* dw, int N, int H,
     return (int)cudaErrorInvalidValue;
   const ConvA ca = conv_a(s);
   cudaStream_t st = (cudaStream_t)cs;
-  switch (tile) {
-    case 64: return launch_tn_maps<64>(ma, mb, mc, ca, P, Cout, No, error_flag, st, box3d);
-    case 128: return launch_tn_maps<128>(ma, mb, mc, ca, P, Cout, No, error_flag, st, box3d);
-    case 192: return launch_tn_maps<192>(ma, mb, mc, ca, P, Cout, No, error_flag, st, box3d);
-    case 256: return launch_tn_maps<256>(ma, mb, mc, ca, P, Cout, No, error_flag, st, box3d);
-    default: return (int)cudaErrorInvalidValue;
-  }
+  return launch_tn_plan(tile, tn_pair(P, Cout, No, tile), ma, mb, mc, ca, P, Cout, No, error_flag, st, box3d);
 }
 
 // Taps of a stride-2 convolution that reach input pixels of parity `par` along one axis: r = par + pad - 2 d for d = 0, 1, ...

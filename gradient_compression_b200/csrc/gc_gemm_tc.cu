@@ -279,18 +279,18 @@ int launch_persistent(const Plan& pl, const float* A, const float* B, float* C, 
   return launch_plan(pl, ma, mb, mc, ConvA{}, bias, M, N, K, accumulate || pl.splits > 1, col_partials, error_flag, st, fin, nullptr, cta_sums);
 }
 
-template <int BN>
-int launch_tn(const float* A, const float* B, float* C, int P, int Mo, int No, int64_t lda, int64_t ldb, int64_t ldc,
+int launch_tn(int bn, const float* A, const float* B, float* C, int P, int Mo, int No, int64_t lda, int64_t ldb, int64_t ldc,
               int* error_flag, cudaStream_t st) {
   CUtensorMap ma, mb, mc;
+  const bool pair = tn_pair(P, Mo, No, bn);
   int box3d = 0;        // whole-operand 3-D boxes where the matrix is made of whole 32-float chunks
   if ((Mo & 31) == 0 && make_map_mn3(&ma, A, P, Mo, lda, TBK, BM / 32) == 0) box3d |= 1;
   else if (make_map_mn(&ma, A, P, Mo, lda) != 0) return (int)cudaErrorInvalidValue;
-  if ((No & 31) == 0 && make_map_mn3(&mb, B, P, No, ldb, TBK, BN / 32) == 0) box3d |= 2;
+  if ((No & 31) == 0 && make_map_mn3(&mb, B, P, No, ldb, TBK, (pair ? bn / 2 : bn) / 32) == 0) box3d |= 2;
   else if (make_map_mn(&mb, B, P, No, ldb) != 0) return (int)cudaErrorInvalidValue;
   if (make_map(&mc, C, Mo, No, ldc, BM) != 0)
     return (int)cudaErrorInvalidValue;
-  return launch_tn_maps<BN>(ma, mb, mc, ConvA{}, P, Mo, No, error_flag, st, box3d);
+  return launch_tn_plan(bn, pair, ma, mb, mc, ConvA{}, P, Mo, No, error_flag, st, box3d);
 }
 
 // 0 = choose, 1 = one tile per CTA, 2 = persistent;  tile width 0 = choose
@@ -405,12 +405,7 @@ int gc_cuda_gemm_tn_tf32(const float* A, const float* B, float* C, int P, int Mo
   if (!gc_cuda_gemm_tn_tf32_supported(A, B, C, P, Mo, No, lda, ldb, ldc)) return (int)cudaErrorInvalidValue;
   cudaStream_t st = (cudaStream_t)cs;
   int bn = gctc::tile_choice ? gctc::tile_choice : (No <= 64 ? 64 : (No <= 128 ? 128 : 256));
-  switch (bn) {
-    case 64: return launch_tn<64>(A, B, C, P, Mo, No, lda, ldb, ldc, error_flag, st);
-    case 128: return launch_tn<128>(A, B, C, P, Mo, No, lda, ldb, ldc, error_flag, st);
-    case 256: return launch_tn<256>(A, B, C, P, Mo, No, lda, ldb, ldc, error_flag, st);
-    default: return (int)cudaErrorInvalidValue;
-  }
+  return launch_tn(bn, A, B, C, P, Mo, No, lda, ldb, ldc, error_flag, st);
 }
 
 }  // extern "C"

@@ -876,12 +876,15 @@ gemm_tf32_persistent_kernel(const __grid_constant__ CUtensorMap tma_a, const __g
 // (K = 8 positions) advances the start address by 1024 bytes.
 // Split-K: CTA (tile, split) contracts its slice of positions and adds its 128 x BN partial result onto C
 // with TMA reduce stores, so C must hold the value to add to (zeros for a plain product).
-template <int BN>
+//
+// PAIR: as in the persistent kernel, two CTAs share a tile of 256 x BN, each with its 128 columns of A and half of B's.
+template <int BN, bool PAIR>
 struct TnSmem {
-  static constexpr int STAGES = (BN <= 64) ? 8 : ((BN <= 128) ? 6 : 4);
+  static constexpr int STAGES = PAIR ? ((BN <= 128) ? 8 : 6) : ((BN <= 64) ? 8 : ((BN <= 128) ? 6 : 4));
+  static constexpr int B_COLS = PAIR ? BN / 2 : BN;
   static constexpr int CHUNK_BYTES = TBK * 128;             // one TMA box: 32 floats of the output dimension x TBK rows
   static constexpr int A_BYTES = BM * TBK * 4;
-  static constexpr int B_BYTES = BN * TBK * 4;
+  static constexpr int B_BYTES = B_COLS * TBK * 4;
   static constexpr int RING_BYTES = STAGES * (A_BYTES + B_BYTES);
   static constexpr int NSLAB = 2;
   static constexpr int SLAB_BYTES = BM * 128;
@@ -892,16 +895,16 @@ struct TnSmem {
   static_assert(TOTAL <= 232448, "shared memory of one CTA");
 };
 
-__host__ __device__ constexpr uint32_t make_idesc_mn(int n) {
-  return make_idesc(n) | (1u << 15) | (1u << 16);        // A and B are MN-major
+__host__ __device__ constexpr uint32_t make_idesc_mn(int n, int m = BM) {
+  return make_idesc(n, m) | (1u << 15) | (1u << 16);        // A and B are MN-major
 }
 
-template <int BN>
+template <int BN, bool PAIR>
 __global__ void __launch_bounds__(TN_THREADS, 1)
 gemm_tn_tf32_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
                     const __grid_constant__ CUtensorMap tma_c, const ConvA ca, int P, int Mo, int No, int tiles_n, int splits,
                     int kblocks_per_split, int* __restrict__ error_flag, int tma_mode, int box3d) {
-  using S = TnSmem<BN>;
+  using S = TnSmem<BN, PAIR>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   uint8_t* a_tiles = base;
@@ -915,9 +918,10 @@ gemm_tn_tf32_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_cons
   __shared__ int epi_go;
 
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
-  const int split = blockIdx.x % splits;
-  const int tile = blockIdx.x / splits;
-  const int m0 = (tile / tiles_n) * BM, n0 = (tile % tiles_n) * BN;
+  const int rank = PAIR ? (int)cluster_rank() : 0, worker = PAIR ? (int)(blockIdx.x >> 1) : (int)blockIdx.x;
+  const int split = worker % splits;
+  const int tile = worker / splits;
+  const int m0 = (PAIR ? (tile / tiles_n) * 2 + rank : tile / tiles_n) * BM, n0 = (tile % tiles_n) * BN;
   const int total_k = (P + TBK - 1) / TBK;
   const int k_begin = split * kblocks_per_split;
   const int k_end = k_begin + kblocks_per_split < total_k ? k_begin + kblocks_per_split : total_k;
@@ -932,11 +936,17 @@ gemm_tn_tf32_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_cons
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
   if (warp == MMA_WARP) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"((uint32_t)S::TMEM_COLS) : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    if constexpr (PAIR) {
+      asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"((uint32_t)S::TMEM_COLS) : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    } else {
+      asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"((uint32_t)S::TMEM_COLS) : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
   }
   tc_fence_before();
   __syncthreads();
+  if constexpr (PAIR) cluster_sync_all();
   tc_fence_after();
   const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
 
@@ -948,12 +958,13 @@ gemm_tn_tf32_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_cons
       // n % Cin; a tile narrower than Cin stays inside one tap, a wider one (Cin = 64) covers several taps side by side.
       // Box c of a stage reads the pixels of its tap, shifted by (fr, fs), for the TBK output positions of the k-block.
       int co[4] = {0, 0, 0, 0};
-      int box_ch[BN / 32], box_fr[BN / 32], box_fs[BN / 32];
+      int box_ch[S::B_COLS / 32], box_fr[S::B_COLS / 32], box_fs[S::B_COLS / 32];
+      const int b0 = n0 + rank * S::B_COLS;                 // first column of B this CTA loads
       if (ca.taps != 0) {
         const int cin = ca.cblocks * 32;
 #pragma unroll
-        for (int c = 0; c < BN / 32; ++c) {
-          const int n = n0 + c * 32, tap = n / cin;
+        for (int c = 0; c < S::B_COLS / 32; ++c) {
+          const int n = b0 + c * 32, tap = n / cin;
           box_ch[c] = n - tap * cin;
           box_fr[c] = tap / ca.fs;
           box_fs[c] = tap - box_fr[c] * ca.fs;
@@ -961,58 +972,83 @@ gemm_tn_tf32_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_cons
       }
       // boxes that lie wholly beyond the matrix (Mo < 128: the 64-channel layers; No < n0 + BN) are not loaded at all: the
       // rows and columns of the accumulator they feed are never stored
-      int a_boxes = (Mo - m0 + 31) / 32, b_boxes = (No - n0 + 31) / 32;
-      a_boxes = a_boxes < BM / 32 ? a_boxes : BM / 32;
-      b_boxes = b_boxes < BN / 32 ? b_boxes : BN / 32;
+      auto boxes = [](int left, int most) { return left <= 0 ? 0 : (left + 31) / 32 < most ? (left + 31) / 32 : most; };
+      const int a_boxes = boxes(Mo - m0, BM / 32), b_boxes = boxes(No - b0, S::B_COLS / 32);
       // box3d bit 0 / 1: the A / B map is the 3-D view {32 floats, rows, chunks} of the matrix and ONE box brings the whole
       // operand of a stage (chunks beyond the matrix arrive as zeros and count as bytes)
       const bool a3 = (box3d & 1) != 0, b3 = (box3d & 2) != 0 && ca.taps == 0;
-      const uint32_t stage_tx = (uint32_t)((a3 ? BM / 32 : a_boxes) * S::CHUNK_BYTES + (b3 ? BN / 32 : b_boxes) * S::CHUNK_BYTES);
+      // bytes of a stage, of both CTAs of a pair (the second one's rows and columns follow)
+      int stage_boxes = (a3 ? BM / 32 : a_boxes) + (b3 ? S::B_COLS / 32 : b_boxes);
+      if (PAIR) stage_boxes += (a3 ? BM / 32 : boxes(Mo - m0 - BM, BM / 32)) + (b3 ? S::B_COLS / 32 : boxes(No - b0 - S::B_COLS, S::B_COLS / 32));
+      const uint32_t stage_tx = (uint32_t)(stage_boxes * S::CHUNK_BYTES);
       for (int k = warp; k < num_k; k += PRODUCER_WARPS) {
         const int s = k % S::STAGES;
         const uint32_t phase = (uint32_t)(k / S::STAGES) & 1u;
         if (!mbar_wait_warp(&empty[s], phase ^ 1u, &abort_flag)) break;
         const int row0 = (k_begin + k) * TBK;
         if (ca.taps != 0) conv_box(ca, (int64_t)row0, 0, 0, co);           // the k-block's first position at tap (0, 0)
+        uint8_t *a_dst = a_tiles + s * S::A_BYTES, *b_dst = b_tiles + s * S::B_BYTES;
+        const uint32_t bar = PAIR ? cluster_addr(&full[s], 0) : 0u;
+        auto load_2d = [&](uint8_t* dst, const CUtensorMap* map, int x, int y) {
+          if constexpr (PAIR) tma_load_2d_pair(dst, map, x, y, bar);
+          else tma_load_2d(dst, map, x, y, &full[s]);
+        };
+        auto load_3d = [&](uint8_t* dst, const CUtensorMap* map, int c0, int c1, int c2) {
+          if constexpr (PAIR) tma_load_3d_pair(dst, map, c0, c1, c2, bar);
+          else tma_load_3d(dst, map, c0, c1, c2, &full[s]);
+        };
+        auto load_4d = [&](uint8_t* dst, const CUtensorMap* map, int c0, int c1, int c2, int c3) {
+          if constexpr (PAIR) tma_load_4d_pair(dst, map, c0, c1, c2, c3, bar);
+          else tma_load_4d(dst, map, c0, c1, c2, c3, &full[s]);
+        };
         if (elect_one()) {
-          mbar_expect_tx(&full[s], stage_tx);
+          if (rank == 0) mbar_expect_tx(&full[s], stage_tx);
           if (a3) {
-            tma_load_3d(a_tiles + s * S::A_BYTES, &tma_a, 0, row0, m0 >> 5, &full[s]);
+            load_3d(a_dst, &tma_a, 0, row0, m0 >> 5);
           } else {
 #pragma unroll
             for (int c = 0; c < BM / 32; ++c)
-              if (c < a_boxes) tma_load_2d(a_tiles + s * S::A_BYTES + c * S::CHUNK_BYTES, &tma_a, m0 + c * 32, row0, &full[s]);
+              if (c < a_boxes) load_2d(a_dst + c * S::CHUNK_BYTES, &tma_a, m0 + c * 32, row0);
           }
           if (b3) {
-            tma_load_3d(b_tiles + s * S::B_BYTES, &tma_b, 0, row0, n0 >> 5, &full[s]);
+            load_3d(b_dst, &tma_b, 0, row0, b0 >> 5);
           } else if (ca.taps == 0) {
 #pragma unroll
-            for (int c = 0; c < BN / 32; ++c)
-              if (c < b_boxes) tma_load_2d(b_tiles + s * S::B_BYTES + c * S::CHUNK_BYTES, &tma_b, n0 + c * 32, row0, &full[s]);
+            for (int c = 0; c < S::B_COLS / 32; ++c)
+              if (c < b_boxes) load_2d(b_dst + c * S::CHUNK_BYTES, &tma_b, b0 + c * 32, row0);
           } else {
 #pragma unroll
-            for (int c = 0; c < BN / 32; ++c)
-              if (c < b_boxes)
-                tma_load_4d(b_tiles + s * S::B_BYTES + c * S::CHUNK_BYTES, &tma_b, box_ch[c], co[1] + box_fs[c], co[2] + box_fr[c], co[3],
-                            &full[s]);
+            for (int c = 0; c < S::B_COLS / 32; ++c)
+              if (c < b_boxes) load_4d(b_dst + c * S::CHUNK_BYTES, &tma_b, box_ch[c], co[1] + box_fs[c], co[2] + box_fr[c], co[3]);
           }
         }
         __syncwarp();
       }
+      if constexpr (PAIR)       // see the commits of the last stages before this CTA may end
+        for (int k = (num_k > S::STAGES ? num_k - S::STAGES : 0); k < num_k; ++k)
+          if (!mbar_wait_warp<true>(&empty[k % S::STAGES], (uint32_t)(k / S::STAGES) & 1u, &abort_flag)) break;
     } else if (warp == MMA_WARP) {
-      constexpr uint32_t idesc = make_idesc_mn(BN);
+      constexpr uint32_t idesc = make_idesc_mn(BN, PAIR ? 2 * BM : BM);
       uint32_t s = 0, phase = 0;
-      for (int k = 0; k < num_k; ++k) {
-        if (!mbar_wait_warp(&full[s], phase, &abort_flag)) break;
+      for (int k = 0; rank == 0 && k < num_k; ++k) {
+        if (!mbar_wait_warp<PAIR>(&full[s], phase, &abort_flag)) break;
         tc_fence_after();
         const uint64_t adesc = make_smem_desc_mn(a_tiles + s * S::A_BYTES);
         const uint64_t bdesc = make_smem_desc_mn(b_tiles + s * S::B_BYTES);
         if (elect_one()) {
 #pragma unroll
           for (int kk = 0; kk < TBK / UMMA_K; ++kk)    // 8 positions = 8 rows of 128 bytes = 1024 bytes = 64 address units
-            umma_tf32(tmem_base, adesc + (uint64_t)(kk * 64), bdesc + (uint64_t)(kk * 64), idesc, (k | kk) != 0 ? 1u : 0u);
-          umma_commit(&empty[s]);
-          if (k == num_k - 1) umma_commit(acc_ready);
+          {
+            if constexpr (PAIR) umma_tf32_pair(tmem_base, adesc + (uint64_t)(kk * 64), bdesc + (uint64_t)(kk * 64), idesc, (k | kk) != 0 ? 1u : 0u);
+            else umma_tf32(tmem_base, adesc + (uint64_t)(kk * 64), bdesc + (uint64_t)(kk * 64), idesc, (k | kk) != 0 ? 1u : 0u);
+          }
+          if constexpr (PAIR) {
+            umma_commit_pair(&empty[s]);
+            if (k == num_k - 1) umma_commit_pair(acc_ready);
+          } else {
+            umma_commit(&empty[s]);
+            if (k == num_k - 1) umma_commit(acc_ready);
+          }
         }
         __syncwarp();
         if (++s == S::STAGES) { s = 0; phase ^= 1u; }
@@ -1047,7 +1083,7 @@ gemm_tn_tf32_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_cons
           asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
           asm volatile("bar.sync 1, 128;" ::: "memory");
           if (issuer) {
-            if (n0 + sl * 32 < No)
+            if (n0 + sl * 32 < No && (!PAIR || m0 < Mo))
               asm volatile("cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.tile.bulk_group [%0, {%2, %3}], [%1];"
                            ::"l"(&tma_c), "r"(smem_u32(slab)), "r"(n0 + sl * 32), "r"(m0)
                            : "memory");
@@ -1060,9 +1096,13 @@ gemm_tn_tf32_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_cons
   }
   tc_fence_before();
   __syncthreads();
+  if constexpr (PAIR) cluster_sync_all();
   if (warp == MMA_WARP) {
     tc_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)S::TMEM_COLS) : "memory");
+    if constexpr (PAIR)
+      asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)S::TMEM_COLS) : "memory");
+    else
+      asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)S::TMEM_COLS) : "memory");
   }
   if (threadIdx.x == 0 && abort_flag && error_flag != nullptr) atomicExch(error_flag, 1);
 }
@@ -1150,6 +1190,23 @@ struct Plan {
   int rows() const { return pair ? 2 * BM : BM; }
 };
 
+// CTA pairs of a kernel that the device runs at once.
+inline int pairs_at_once(const void* kernel, int threads, size_t smem) {
+  int n = sm_count() / 2, fit = 0;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(2 * n));
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = smem;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 2;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaOccupancyMaxActiveClusters(&fit, kernel, &cfg) == cudaSuccess && fit > 0 && fit < n ? fit : n;
+}
+
 // CTAs, or CTA pairs, of the persistent kernel that the device runs at once (pairs: half its SMs, unless a GPC has an odd
 // number of them); 0 when the kernel cannot be configured.
 template <int BN, bool AFFINE, bool PAIR>
@@ -1159,22 +1216,7 @@ int persistent_workers() {
   if (workers != 0) return workers;
   if (cudaFuncSetAttribute(gemm_tf32_persistent_kernel<BN, AFFINE, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::TOTAL) != cudaSuccess) return 0;
   int n = sm_count();
-  if constexpr (PAIR) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(n / 2 * 2));
-    cfg.blockDim = dim3(PERSISTENT_THREADS);
-    cfg.dynamicSmemBytes = S::TOTAL;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 2;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    n /= 2;
-    int fit = 0;
-    if (cudaOccupancyMaxActiveClusters(&fit, gemm_tf32_persistent_kernel<BN, AFFINE, PAIR>, &cfg) == cudaSuccess && fit > 0 && fit < n) n = fit;
-  }
+  if constexpr (PAIR) n = pairs_at_once((const void*)gemm_tf32_persistent_kernel<BN, AFFINE, PAIR>, PERSISTENT_THREADS, S::TOTAL);
   return workers = n;
 }
 
@@ -1247,29 +1289,51 @@ inline int cta_sum_rows(int M, int N, const Plan& pl) {
 // Launch the split-K TN kernel on ready-made tensor maps.  At most tn_ctas_per_sm CTAs per SM over all tiles, at least
 // tn_min_kblocks k-blocks each so that the pipeline fills.  One CTA per SM measured 10-25 % faster than two on the
 // 131072- and 32768-position weight gradients of ResNet-50 (fewer partial tiles to add, longer pipelines), equal below.
-template <int BN>
+// CTA pairs for the split contraction: two row tiles, and at least 16 k-blocks for every CTA.  A pair loads 128 + BN / 2 columns a
+// k-block instead of 128 + BN (at BN = 256 about 0.13 us less) and costs about 1.5 us for meeting at both ends: 16x16 256 -> 256 3x3 at batch 128
+// 67.6 -> 53.2 us, 8x8 512 -> 512 64.3 -> 53.2 us; with 8 k-blocks a CTA (8x8 256 -> 1024 1x1 at batch 31) 14.3 -> 16.4 us.
+inline bool tn_pair(int P, int Mo, int No, int bn) {
+  if ((bn != 128 && bn != 256) || Mo <= BM || gctc::pair_choice == 1) return false;
+  const int64_t tiles = (int64_t)((Mo + BM - 1) / BM) * ((No + bn - 1) / bn);
+  return gctc::pair_choice == 2 || tiles * ((P + TBK - 1) / TBK) >= (int64_t)16 * sm_count();
+}
+
+template <int BN, bool PAIR>
 int launch_tn_maps(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mc, const ConvA& ca, int P, int Mo, int No,
-                   int* error_flag, cudaStream_t st, int box3d = 0) {
-  using S = TnSmem<BN>;
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_tn_tf32_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::TOTAL);
+                   int* error_flag, cudaStream_t st, int box3d) {
+  using S = TnSmem<BN, PAIR>;
+  static int at_once = 0;
+  if (at_once == 0) {
+    cudaError_t e = cudaFuncSetAttribute(gemm_tn_tf32_kernel<BN, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::TOTAL);
     if (e != cudaSuccess) return (int)e;
-    configured = true;
+    at_once = PAIR ? pairs_at_once((const void*)gemm_tn_tf32_kernel<BN, PAIR>, TN_THREADS, S::TOTAL) : sm_count();
   }
-  int tiles_m = (Mo + BM - 1) / BM, tiles_n = (No + BN - 1) / BN;
+  constexpr int ROWS = PAIR ? 2 * BM : BM;
+  int tiles_m = (Mo + ROWS - 1) / ROWS, tiles_n = (No + BN - 1) / BN;
   int tiles = tiles_m * tiles_n;
   int total_k = (P + TBK - 1) / TBK;
   // never more CTAs than fit at once (one per SM at this shared-memory size): a second, nearly empty wave would double the
   // kernel's time (measured: 153 CTAs on 148 SMs ran 37 us with the SMs 62 % busy)
-  int splits = gctc::tn_ctas_per_sm * sm_count() / tiles;
+  int splits = gctc::tn_ctas_per_sm * at_once / tiles;
   if (splits > (total_k + gctc::tn_min_kblocks - 1) / gctc::tn_min_kblocks) splits = (total_k + gctc::tn_min_kblocks - 1) / gctc::tn_min_kblocks;
   if (splits < 1) splits = 1;
   int per = (total_k + splits - 1) / splits;
   splits = (total_k + per - 1) / per;
-  gemm_tn_tf32_kernel<BN><<<(unsigned)(tiles * splits), TN_THREADS, S::TOTAL, st>>>(ma, mb, mc, ca, P, Mo, No, tiles_n, splits, per,
-                                                                                     error_flag, gctc::tma_mode, box3d);
-  return (int)cudaGetLastError();
+  const cudaError_t e = gc::launch_cluster(gemm_tn_tf32_kernel<BN, PAIR>, PAIR ? 2u : 1u, dim3((unsigned)((PAIR ? 2 : 1) * tiles * splits)), dim3(TN_THREADS),
+                                           (size_t)S::TOTAL, st, ma, mb, mc, ca, P, Mo, No, tiles_n, splits, per, error_flag, gctc::tma_mode, box3d);
+  return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
+}
+
+inline int launch_tn_plan(int bn, bool pair, const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mc, const ConvA& ca, int P, int Mo, int No,
+                          int* error_flag, cudaStream_t st, int box3d) {
+  auto run = [&](auto launch) { return launch(ma, mb, mc, ca, P, Mo, No, error_flag, st, box3d); };
+  switch (bn) {
+    case 64: return run(launch_tn_maps<64, false>);
+    case 128: return pair ? run(launch_tn_maps<128, true>) : run(launch_tn_maps<128, false>);
+    case 192: return run(launch_tn_maps<192, false>);
+    case 256: return pair ? run(launch_tn_maps<256, true>) : run(launch_tn_maps<256, false>);
+    default: return (int)cudaErrorInvalidValue;
+  }
 }
 
 // Modelled nanoseconds of a product on the persistent kernel.  A k-block costs a CTA the time its loads and operand reads take

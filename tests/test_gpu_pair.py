@@ -82,3 +82,30 @@ def test_conv(paired, tile, n, h, cin, cout, stride):
                                               [True, False, False])[0].float()
     gemm.check()
     assert torch.equal(dx, ref)
+
+
+@pytest.mark.parametrize("tile", [128, 256])
+@pytest.mark.parametrize("p,mo,no", [(1, 160, 32), (33, 256, 96), (1000, 384, 288), (70000, 512, 160), (40, 2048, 512)])
+def test_weight_gradient_matrix(paired, tile, p, mo, no):
+    """Second CTA with 32 rows, all or none of its rows; ragged columns; fewer positions than a stage; exact on small integers."""
+    g = torch.Generator(device="cuda").manual_seed(p + mo)
+    a, b = (torch.randint(-2, 3, (p, d), device="cuda", generator=g).float() for d in (mo, no))
+    paired(tile, 2)
+    out = gemm.gemm_tn_tf32(a, b, out=torch.ones(mo, no, device="cuda"), accumulate=True)
+    gemm.check()
+    assert torch.equal(out, (a.double().t() @ b.double() + 1).float())
+
+
+@pytest.mark.parametrize("n,h,cin,cout,stride", [(2, 8, 128, 160, 1), (5, 8, 256, 256, 2), (3, 16, 256, 384, 1), (40, 4, 512, 512, 1)])
+def test_weight_gradient_conv(paired, n, h, cin, cout, stride):
+    g = torch.Generator().manual_seed(n + h)
+    ints = lambda *shape: torch.randint(-3, 4, shape, generator=g).float().cuda().contiguous(memory_format=torch.channels_last)  # noqa: E731
+    x, dy = ints(n, cin, h, h), ints(n, cout, h // stride, h // stride)
+    paired(0, 2)
+    if not conv.nat.cuda().gc_cuda_conv_wgrad_supported(n, h, h, cin, cout, 3, stride, 1):
+        pytest.skip("not a tensor-core shape")
+    dw = conv.conv_wgrad(dy, x, 3, stride, 1)
+    gemm.check()
+    w = torch.zeros(cout, cin, 3, 3, device="cuda", dtype=torch.float64)
+    ref = torch.ops.aten.convolution_backward(dy.double(), x.double(), w, None, [stride] * 2, [1, 1], [1, 1], False, [0, 0], 1, [False, True, False])[1]
+    assert torch.equal(dw.view(cout, 3, 3, cin), ref.permute(0, 2, 3, 1).float())
