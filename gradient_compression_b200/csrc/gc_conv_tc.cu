@@ -418,8 +418,9 @@ int gc_cuda_conv_dgrad_s2_supported(int N, int H, int W, int Cin, int Cout, int 
 // store map over that strided sub-grid of dx.  w: the forward filter [Cout][R][R][Cin] (channels-last memory order), read in
 // place as the MN-major B operand.  Classes without taps (a 1x1 filter reaches only the even pixels) are zero: dx is cleared
 // first when there is one.
-int gc_cuda_conv_dgrad_s2(const float* dy, const float* w, float* dx, int N, int H, int W, int Cin, int Cout, int R, int pad,
-                          int* error_flag, void* cs) {
+// accumulate: dx += instead, where pixels that no tap reaches are not touched at all.
+int gc_cuda_conv_dgrad_s2_add(const float* dy, const float* w, float* dx, int N, int H, int W, int Cin, int Cout, int R, int pad, int accumulate,
+                              int* error_flag, void* cs) {
   if (!gc_cuda_conv_dgrad_s2_supported(N, H, W, Cin, Cout, R, pad)) return (int)cudaErrorInvalidValue;
   if ((reinterpret_cast<uintptr_t>(dy) & 15u) || (reinterpret_cast<uintptr_t>(w) & 15u) || (reinterpret_cast<uintptr_t>(dx) & 15u))
     return (int)cudaErrorInvalidValue;
@@ -427,7 +428,7 @@ int gc_cuda_conv_dgrad_s2(const float* dy, const float* w, float* dx, int N, int
   const int Ho = H / 2, Wo = W / 2, M = N * Ho * Wo;
   bool any_empty = false;
   for (int c = 0; c < 4; ++c) any_empty |= class_taps(c >> 1, pad, R) * class_taps(c & 1, pad, R) == 0;
-  if (any_empty) {
+  if (any_empty && !accumulate) {
     cudaError_t e = cudaMemsetAsync(dx, 0, (size_t)N * H * W * Cin * 4, st);
     if (e != cudaSuccess) return (int)e;
   }
@@ -458,10 +459,15 @@ int gc_cuda_conv_dgrad_s2(const float* dy, const float* w, float* dx, int N, int
         return (int)cudaErrorInvalidValue;
     }
     const ConvC cc{Ho * Wo, Wo};
-    const int err = launch_plan(pl, ma, mb, mc, ca, nullptr, M, Cin, K, 0, nullptr, error_flag, st, nullptr, &cc);
+    const int err = launch_plan(pl, ma, mb, mc, ca, nullptr, M, Cin, K, accumulate, nullptr, error_flag, st, nullptr, &cc);
     if (err != 0) return err;
   }
   return 0;
+}
+
+int gc_cuda_conv_dgrad_s2(const float* dy, const float* w, float* dx, int N, int H, int W, int Cin, int Cout, int R, int pad,
+                          int* error_flag, void* cs) {
+  return gc_cuda_conv_dgrad_s2_add(dy, w, dx, N, H, W, Cin, Cout, R, pad, 0, error_flag, cs);
 }
 
 // Rows of Kp = 32-float-padded filter taps for a stride-1 convolution with few input channels (the 3-channel stem):

@@ -734,9 +734,14 @@ gemm_tf32_persistent_kernel(const __grid_constant__ CUtensorMap tma_a, const __g
             if (cc.hw != 0) {                    // rows = pixels (n, i, j) of a strided sub-grid: 4-D store map
               const int img = m0 / cc.hw, rem = m0 - img * cc.hw;
               const int i0 = rem / cc.w, j0 = rem - i0 * cc.w;
-              asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.bulk_group [%0, {%2, %3, %4, %5}], [%1];"
-                           ::"l"(&tma_c), "r"(smem_u32(slab)), "r"(n0 + sl * 32), "r"(j0), "r"(i0), "r"(img)
-                           : "memory");
+              if (accumulate)
+                asm volatile("cp.reduce.async.bulk.tensor.4d.global.shared::cta.add.tile.bulk_group [%0, {%2, %3, %4, %5}], [%1];"
+                             ::"l"(&tma_c), "r"(smem_u32(slab)), "r"(n0 + sl * 32), "r"(j0), "r"(i0), "r"(img)
+                             : "memory");
+              else
+                asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.bulk_group [%0, {%2, %3, %4, %5}], [%1];"
+                             ::"l"(&tma_c), "r"(smem_u32(slab)), "r"(n0 + sl * 32), "r"(j0), "r"(i0), "r"(img)
+                             : "memory");
             } else if (accumulate)               // C += tile: the add happens in L2, C is never read by the SM
               asm volatile("cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.tile.bulk_group [%0, {%2, %3}], [%1];"
                            ::"l"(&tma_c), "r"(smem_u32(slab)), "r"(n0 + sl * 32), "r"(m0)

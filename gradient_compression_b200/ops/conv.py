@@ -254,6 +254,7 @@ class GradLink:
         self.armed = False          # the convolution took a tensor-core path and will look for a stashed gradient
         self.conv_done = False      # its backward already ran (without finding one)
         self.stash, self.stash_owned = None, False
+        self.later = None           # a strided shortcut's input gradient, to be added when this convolution's is there
 
     def residual(self, x):
         if not (self.armed and torch.is_grad_enabled() and x.requires_grad):
@@ -468,8 +469,15 @@ class _ConvBNAct(torch.autograd.Function):
                                                    gamma.data_ptr(), beta.data_ptr(), sums.data_ptr(), int(ctx.relu),
                                                    dconv.data_ptr(), nat.ptr(dres), st()), "bn_bwd_apply")
             dx = None
-            link = ctx.link
-            if ctx.needs_input_grad[0]:
+            link, donate = ctx.link, ctx.donate
+            if donate is not None and (donate.conv_done or donate.stash is not None or donate.later is not None):
+                donate = None
+            if (donate is not None and ctx.needs_input_grad[0] and mode == "conv" and r == 1 and stride == 2 and link is None and "dgrad_s2" in PATHS
+                    and _filter_in_place_ok(w) and lib.gc_cuda_conv_dgrad_s2_supported(n, x.shape[2], x.shape[3], cin, cout, r, pad)):
+                # a strided 1x1 projection reaches one input pixel in four: added onto the gradient of the link's convolution once
+                # that is written, nothing is zeroed and only those pixels are read and written again
+                donate.later = (dconv, w, pad)
+            elif ctx.needs_input_grad[0]:
                 acc = None
                 if link is not None and link.stash is not None:
                     acc, link.stash = link.stash, None
@@ -516,8 +524,12 @@ class _ConvBNAct(torch.autograd.Function):
                         dx = dx + acc
             if link is not None:
                 link.conv_done = True
-            donate = ctx.donate
-            if donate is not None and dx is not None and not donate.conv_done and donate.stash is None:
+                if link.later is not None:
+                    (later_dy, later_w, later_pad), link.later = link.later, None
+                    dx = dx.contiguous(memory_format=torch.channels_last)
+                    nat.check(lib.gc_cuda_conv_dgrad_s2_add(later_dy.data_ptr(), later_w.data_ptr(), dx.data_ptr(), n, x.shape[2], x.shape[3], cin,
+                                                            later_dy.shape[1], 1, later_pad, 1, _err(x.device), st()), "conv_dgrad_s2")
+            if donate is not None and dx is not None:
                 # this layer shares its input with the link's convolution, whose backward runs later: hand the gradient
                 # over instead of returning it, so that that kernel adds onto it (autograd would sum the two in a pass)
                 donate.stash, donate.stash_owned, dx = dx, True, None

@@ -109,3 +109,19 @@ def test_weight_gradient_conv(paired, n, h, cin, cout, stride):
     w = torch.zeros(cout, cin, 3, 3, device="cuda", dtype=torch.float64)
     ref = torch.ops.aten.convolution_backward(dy.double(), x.double(), w, None, [stride] * 2, [1, 1], [1, 1], False, [0, 0], 1, [False, True, False])[1]
     assert torch.equal(dw.view(cout, 3, 3, cin), ref.permute(0, 2, 3, 1).float())
+
+
+@pytest.mark.parametrize("pairs", [1, 2])
+@pytest.mark.parametrize("r", [1, 3])
+def test_strided_input_gradient_onto_an_existing_one(paired, r, pairs):
+    n, h, cin, cout = 6, 16, 64, 96
+    g = torch.Generator().manual_seed(r)
+    ints = lambda *shape: torch.randint(-3, 4, shape, generator=g).float().cuda().contiguous(memory_format=torch.channels_last)  # noqa: E731
+    x, w, dy, dx = ints(n, cin, h, h), ints(cout, cin, r, r), ints(n, cout, h // 2, h // 2), ints(n, cin, h, h)
+    ref = torch.ops.aten.convolution_backward(dy.double(), x.double(), w.double(), None, [2, 2], [r // 2] * 2, [1, 1], False, [0, 0], 1,
+                                              [True, False, False])[0].float() + dx
+    paired(0, pairs)
+    lib, flag = conv.nat.cuda(), gemm._error_flag(torch.device("cuda", 0)).data_ptr()
+    conv.nat.check(lib.gc_cuda_conv_dgrad_s2_add(dy.data_ptr(), w.data_ptr(), dx.data_ptr(), n, h, h, cin, cout, r, r // 2, 1, flag, conv.nat.stream_ptr()), "add")
+    gemm.check()
+    assert torch.equal(dx, ref)
