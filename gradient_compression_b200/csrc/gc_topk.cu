@@ -247,13 +247,20 @@ __device__ __forceinline__ void select_small(const TopkParams<CAP>& p, int g, ui
       __syncthreads();
     }
   }
-  if (threadIdx.x == 0) found[0] = 0;                  // entries equal to the threshold taken so far
-  __syncthreads();
+  // of the entries equal to the threshold the first ones are taken
+  const bool some = k > 0 && k < len && hist[prefix & 127u] > (uint32_t)rem;
+  int before = 0;
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
     const int64_t i = threadIdx.x + j * THREADS;
     bool take = i < len && k > 0 && (k >= len || key[j] > prefix);
-    if (i < len && k > 0 && k < len && key[j] == prefix) take = atomicAdd(found, 1) < rem;
+    bool equal = i < len && k > 0 && k < len && key[j] == prefix;
+    if (some) {
+      const int order = before + (int)block_exclusive(equal ? 1u : 0u, warp_sums);
+      before += __syncthreads_count(equal);
+      equal = equal && order < rem;
+    }
+    take |= equal;
     if (LISTS) list_take(p, g, take, lo + i, v[j]);
     else if (i < len) t.out[g][i] = take ? v[j] : 0.0f;
     if (take && p.e != nullptr) p.e[lo + i] = 0.0f;
@@ -412,12 +419,17 @@ __global__ void __launch_bounds__(THREADS, 1) topk_split_kernel(const __grid_con
   if (g >= 0) flush(g);
 }
 
+// Entries equal to the threshold that are ordered by index before some of them are taken, so that the selection does not depend on
+// how blocks run.  A few of a million random floats share a value; beyond these the order of arrival decides.
+constexpr int TIES = 128;
+
 // One cluster of blocks per group; the blocks share the group's candidates and add their counts up in rank 0's shared memory.
 template <int CAP, bool LISTS>
 __global__ void __launch_bounds__(THREADS) topk_refine_kernel(const __grid_constant__ TopkParams<CAP> p) {
   __shared__ uint32_t hist[SUB_BINS], warp_sums[32];
   __shared__ int chosen, need;
   __shared__ uint32_t equal_seen;
+  __shared__ Cand ties[TIES];              // rank 0's: entries equal to the threshold
   cg::cluster_group cluster = cg::this_cluster();
   const unsigned rank = cluster.block_rank(), ranks = cluster.num_blocks();
   const SegTable<CAP>& t = p.t;
@@ -483,17 +495,25 @@ __global__ void __launch_bounds__(THREADS) topk_refine_kernel(const __grid_const
     cluster.sync();
   }
   uint32_t* equal = cluster.map_shared_rank(&equal_seen, 0);
-  auto settle = [&](const Cand& c, bool there) {
-    const bool valid = there && in_it(c), taken = there && !listed && (int)(c.key() >> LOW_BITS) > bin;
-    const uint32_t low = c.key() & ((1u << LOW_BITS) - 1u);
-    bool take = valid && (all || low > prefix);
-    if (valid && !all && low == prefix) take = (int)atomicAdd(equal, 1u) < rem;
+  Cand* waiting = cluster.map_shared_rank(&ties[0], 0);
+  auto place = [&](const Cand& c, bool take, bool taken) {
     if (LISTS) list_take(p, g, take, c.at, c.a);
     if (take && !LISTS) {
       const int s = p.per_tensor ? g : seg_of_elem(t, (int64_t)c.at);
       t.out[s][c.at - t.start[s]] = c.a;
     }
     if ((take || taken) && p.e != nullptr) p.e[c.at] = 0.0f;
+  };
+  auto settle = [&](const Cand& c, bool there) {
+    const bool valid = there && in_it(c), taken = there && !listed && (int)(c.key() >> LOW_BITS) > bin;
+    const uint32_t low = c.key() & ((1u << LOW_BITS) - 1u);
+    bool take = valid && (all || low > prefix);
+    if (valid && !all && low == prefix) {
+      const uint32_t at = atomicAdd(equal, 1u);
+      if (at < (uint32_t)TIES) waiting[at] = c;
+      else take = (int)at < rem;
+    }
+    place(c, take, taken);
   };
   int64_t base = from;
   for (; listed && base + 3 * stride + THREADS <= count; base += 4 * stride) {
@@ -506,6 +526,13 @@ __global__ void __launch_bounds__(THREADS) topk_refine_kernel(const __grid_const
     settle(there ? entry(base + threadIdx.x) : Cand{0.0f, 0}, there);
   }
   cluster.sync();                          // rank 0's shared memory stays until every block is done with it
+  if (rank == 0 && threadIdx.x < TIES) {
+    const int n = equal_seen < (uint32_t)TIES ? (int)equal_seen : TIES;
+    const Cand mine = (int)threadIdx.x < n ? ties[threadIdx.x] : Cand{0.0f, 0};
+    int order = 0;
+    for (int j = 0; j < n; ++j) order += ties[j].at < mine.at;
+    place(mine, (int)threadIdx.x < n && order < rem, false);
+  }
 }
 
 int64_t list_room(int64_t len) { return len / 8 + 1024; }

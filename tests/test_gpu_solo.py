@@ -205,3 +205,16 @@ def test_level_kernels(n, shift, s):
         fine, coarse = (ops.dequantize_levels(q.cpu().to(torch.int32), norm, l, 2) for l in (s, s // 4 + 1))
         assert torch.equal(two, torch.where(mask.cpu().bool(), fine, coarse))
     assert torch.equal(ops.absmax(dev).cpu(), ops.absmax(host))
+
+
+@pytest.mark.parametrize("n,step", [(1000, 4), (4096, 8), (4097, 8), (200003, 400), (3000001, 4000)])
+def test_topk_ties_go_to_the_first(n, step):
+    """Rounded values: a dozen to a hundred entries share the threshold; the same ones are taken every time, by index."""
+    from gradient_compression_b200.ops.topk import TopKSelector
+
+    a = torch.round(torch.randn(n, generator=torch.Generator().manual_seed(n)) * step) / step
+    k = n // 50
+    sel = TopKSelector([(0, n, k)], "cuda")
+    want = torch.sort(a.abs(), descending=True, stable=True)[1][:k].sort()[0]
+    for _ in range(3):
+        assert torch.equal(sel.select(a.cuda(), None)[0].cpu().long().sort()[0], want)
