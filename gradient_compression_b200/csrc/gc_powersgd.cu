@@ -77,18 +77,64 @@ __device__ __forceinline__ int find_mat(const int64_t* __restrict__ tab, int n_m
 }
 
 // ------------------------------------------------------------------------------------------ P = (G + E) Q
-// The four query rows of columns k .. k + 3, [t][j].
+// Four columns of a block of 128 for every lane: neighbours up to rank 2, 32 apart above.  There the query rows are what the L1 is busy
+// with: four neighbouring rows of 16 bytes a lane make one load of the warp touch 16 lines, with columns 32 apart 4 (rank 4: L1 80 % busy,
+// DRAM 30 %; VGG-16 P 51 -> 31 us and output 50 -> 30 us, ResNet-50 78 -> 60 and 80 -> 57 us).  At rank 2 the 16-byte loads of the gradient are worth
+// more (VGG-16: P 25 us against 34 us with columns apart).  A lane's first column is `k`; the others may lie beyond the matrix when apart.
 template <int R>
-__device__ __forceinline__ void load_q4(const float* __restrict__ qk, float (&q)[4][R]) {
-  if (R == 1 || R == 2 || R == 4) {
+constexpr bool APART = R > 2;
+template <int R>
+__device__ __forceinline__ int first_column(int lane) { return APART<R> ? lane : lane * 4; }
+
+template <int R, bool STREAM>
+__device__ __forceinline__ void load4(const float* __restrict__ x, int k, int m, float (&v)[4]) {
+  if constexpr (APART<R>) {
+#pragma unroll
+    for (int t = 0; t < 4; ++t) v[t] = k + 32 * t >= m ? 0.f : STREAM ? __ldcs(x + k + 32 * t) : x[k + 32 * t];
+  } else {
+    const float4 o = STREAM ? __ldcs(reinterpret_cast<const float4*>(x + k)) : *reinterpret_cast<const float4*>(x + k);
+    v[0] = o.x; v[1] = o.y; v[2] = o.z; v[3] = o.w;
+  }
+}
+
+template <int R, bool STREAM>
+__device__ __forceinline__ void store4(float* __restrict__ x, int k, int m, const float (&v)[4]) {
+  if constexpr (APART<R>) {
+#pragma unroll
+    for (int t = 0; t < 4; ++t)
+      if (k + 32 * t < m) {
+        if (STREAM) __stcs(x + k + 32 * t, v[t]);
+        else x[k + 32 * t] = v[t];
+      }
+  } else {
+    const float4 o = make_float4(v[0], v[1], v[2], v[3]);
+    if (STREAM) __stcs(reinterpret_cast<float4*>(x + k), o);
+    else *reinterpret_cast<float4*>(x + k) = o;
+  }
+}
+
+// Their query rows, [t][j] (zero beyond the matrix).
+template <int R>
+__device__ __forceinline__ void load_q4(const float* __restrict__ qm, int k, int m, float (&q)[4][R]) {
+  if constexpr (!APART<R>) {
 #pragma unroll
     for (int i = 0; i < R; ++i) {
-      const float4 v = *reinterpret_cast<const float4*>(qk + 4 * i);
+      const float4 v = *reinterpret_cast<const float4*>(qm + (int64_t)k * R + 4 * i);
       (&q[0][0])[4 * i] = v.x; (&q[0][0])[4 * i + 1] = v.y; (&q[0][0])[4 * i + 2] = v.z; (&q[0][0])[4 * i + 3] = v.w;
     }
   } else {
 #pragma unroll
-    for (int i = 0; i < 4 * R; ++i) (&q[0][0])[i] = qk[i];
+    for (int t = 0; t < 4; ++t) {
+      const bool in = k + 32 * t < m;
+      const float* row = qm + (int64_t)(k + 32 * t) * R;
+      if constexpr (R == 4) {
+        const float4 v = in ? *reinterpret_cast<const float4*>(row) : make_float4(0.f, 0.f, 0.f, 0.f);
+        q[t][0] = v.x; q[t][1] = v.y; q[t][2] = v.z; q[t][3] = v.w;
+      } else {
+#pragma unroll
+        for (int j = 0; j < R; ++j) q[t][j] = in ? row[j] : 0.f;
+      }
+    }
   }
 }
 
@@ -120,24 +166,25 @@ __device__ __forceinline__ void p_long_row(const float* __restrict__ g, float* _
   float acc[R];
 #pragma unroll
   for (int j = 0; j < R; ++j) acc[j] = 0.f;
-  for (int k0 = lane * 4; k0 < m; k0 += 128 * PIECES) {
-    float4 a[PIECES], b[PIECES];
+  for (int k0 = first_column<R>(lane); k0 < m; k0 += 128 * PIECES) {
+    float a[PIECES][4], b[PIECES][4];
 #pragma unroll
-    for (int u = 0; u < PIECES; ++u)
-      if (k0 + 128 * u < m) {
-        a[u] = __ldcs(reinterpret_cast<const float4*>(g + k0 + 128 * u));
-        b[u] = *reinterpret_cast<const float4*>(e + k0 + 128 * u);
-      }
+    for (int u = 0; u < PIECES; ++u) {
+      if (k0 + 128 * u >= m) continue;
+      load4<R, true>(g, k0 + 128 * u, m, a[u]);
+      load4<R, false>(e, k0 + 128 * u, m, b[u]);
+    }
 #pragma unroll
-    for (int u = 0; u < PIECES; ++u)
-      if (k0 + 128 * u < m) {
-        float q[4][R];
-        load_q4<R>(qm + (int64_t)(k0 + 128 * u) * R, q);
-        a[u].x += b[u].x; a[u].y += b[u].y; a[u].z += b[u].z; a[u].w += b[u].w;
-        *reinterpret_cast<float4*>(e + k0 + 128 * u) = a[u];
+    for (int u = 0; u < PIECES; ++u) {
+      if (k0 + 128 * u >= m) continue;
+      float q[4][R];
+      load_q4<R>(qm, k0 + 128 * u, m, q);
 #pragma unroll
-        for (int j = 0; j < R; ++j) acc[j] = fmaf(a[u].x, q[0][j], fmaf(a[u].y, q[1][j], fmaf(a[u].z, q[2][j], fmaf(a[u].w, q[3][j], acc[j]))));
-      }
+      for (int t = 0; t < 4; ++t) a[u][t] += b[u][t];
+      store4<R, false>(e, k0 + 128 * u, m, a[u]);
+#pragma unroll
+      for (int j = 0; j < R; ++j) acc[j] = fmaf(a[u][0], q[0][j], fmaf(a[u][1], q[1][j], fmaf(a[u][2], q[2][j], fmaf(a[u][3], q[3][j], acc[j]))));
+    }
   }
 #pragma unroll
   for (int j = 0; j < R; ++j) {
@@ -154,24 +201,25 @@ __device__ __forceinline__ void p_rows(const float* __restrict__ g, float* __res
   float acc[ROWS * RP];
 #pragma unroll
   for (int i = 0; i < ROWS * RP; ++i) acc[i] = 0.f;
-  for (int k = lane * 4; k < m; k += 128) {
-    float4 a[ROWS], b[ROWS];
+  for (int k = first_column<R>(lane); k < m; k += 128) {
+    float a[ROWS][4], b[ROWS][4];
 #pragma unroll
     for (int u = 0; u < ROWS; ++u)
       if (u < rows) {
-        a[u] = __ldcs(reinterpret_cast<const float4*>(g + (int64_t)u * m + k));
-        b[u] = *reinterpret_cast<const float4*>(e + (int64_t)u * m + k);
+        load4<R, true>(g + (int64_t)u * m, k, m, a[u]);
+        load4<R, false>(e + (int64_t)u * m, k, m, b[u]);
       }
     float q[4][R];
-    load_q4<R>(qm + (int64_t)k * R, q);
+    load_q4<R>(qm, k, m, q);
 #pragma unroll
     for (int u = 0; u < ROWS; ++u)
       if (u < rows) {
-        a[u].x += b[u].x; a[u].y += b[u].y; a[u].z += b[u].z; a[u].w += b[u].w;
-        *reinterpret_cast<float4*>(e + (int64_t)u * m + k) = a[u];
+#pragma unroll
+        for (int t = 0; t < 4; ++t) a[u][t] += b[u][t];
+        store4<R, false>(e + (int64_t)u * m, k, m, a[u]);
 #pragma unroll
         for (int j = 0; j < R; ++j)
-          acc[u * RP + j] = fmaf(a[u].x, q[0][j], fmaf(a[u].y, q[1][j], fmaf(a[u].z, q[2][j], fmaf(a[u].w, q[3][j], acc[u * RP + j]))));
+          acc[u * RP + j] = fmaf(a[u][0], q[0][j], fmaf(a[u][1], q[1][j], fmaf(a[u][2], q[2][j], fmaf(a[u][3], q[3][j], acc[u * RP + j]))));
       }
   }
   const float s = warp_sum_many<ROWS * RP>(acc, lane);
@@ -434,25 +482,26 @@ __device__ __forceinline__ void out_long_row(float* __restrict__ g, float* __res
   float pr[R];
 #pragma unroll
   for (int j = 0; j < R; ++j) pr[j] = p[j];
-  for (int k0 = lane * 4; k0 < m; k0 += 128 * PIECES) {
-    float4 a[PIECES];
+  for (int k0 = first_column<R>(lane); k0 < m; k0 += 128 * PIECES) {
+    float a[PIECES][4];
 #pragma unroll
     for (int u = 0; u < PIECES; ++u)
-      if (k0 + 128 * u < m) a[u] = *reinterpret_cast<const float4*>(e + k0 + 128 * u);
+      if (k0 + 128 * u < m) load4<R, false>(e, k0 + 128 * u, m, a[u]);
 #pragma unroll
-    for (int u = 0; u < PIECES; ++u)
-      if (k0 + 128 * u < m) {
-        float q[4][R], o[4];
-        load_q4<R>(qm + (int64_t)(k0 + 128 * u) * R, q);
+    for (int u = 0; u < PIECES; ++u) {
+      if (k0 + 128 * u >= m) continue;
+      float q[4][R], o[4];
+      load_q4<R>(qm, k0 + 128 * u, m, q);
 #pragma unroll
-        for (int t = 0; t < 4; ++t) {
-          o[t] = pr[0] * q[t][0];
+      for (int t = 0; t < 4; ++t) {
+        o[t] = pr[0] * q[t][0];
 #pragma unroll
-          for (int j = 1; j < R; ++j) o[t] = fmaf(pr[j], q[t][j], o[t]);
-        }
-        __stcs(reinterpret_cast<float4*>(g + k0 + 128 * u), make_float4(o[0], o[1], o[2], o[3]));
-        *reinterpret_cast<float4*>(e + k0 + 128 * u) = make_float4(a[u].x - o[0], a[u].y - o[1], a[u].z - o[2], a[u].w - o[3]);
+        for (int j = 1; j < R; ++j) o[t] = fmaf(pr[j], q[t][j], o[t]);
+        a[u][t] -= o[t];
       }
+      store4<R, true>(g, k0 + 128 * u, m, o);
+      store4<R, false>(e, k0 + 128 * u, m, a[u]);
+    }
   }
 }
 
@@ -464,13 +513,13 @@ __device__ __forceinline__ void out_rows(float* __restrict__ g, float* __restric
   for (int u = 0; u < ROWS; ++u)
 #pragma unroll
     for (int j = 0; j < R; ++j) pr[u][j] = u < rows ? p[u * R + j] : 0.f;
-  for (int k = lane * 4; k < m; k += 128) {
-    float4 a[ROWS];
+  for (int k = first_column<R>(lane); k < m; k += 128) {
+    float a[ROWS][4];
 #pragma unroll
     for (int u = 0; u < ROWS; ++u)
-      if (u < rows) a[u] = *reinterpret_cast<const float4*>(e + (int64_t)u * m + k);
+      if (u < rows) load4<R, false>(e + (int64_t)u * m, k, m, a[u]);
     float q[4][R];
-    load_q4<R>(qm + (int64_t)k * R, q);
+    load_q4<R>(qm, k, m, q);
 #pragma unroll
     for (int u = 0; u < ROWS; ++u)
       if (u < rows) {
@@ -480,9 +529,10 @@ __device__ __forceinline__ void out_rows(float* __restrict__ g, float* __restric
           o[t] = pr[u][0] * q[t][0];
 #pragma unroll
           for (int j = 1; j < R; ++j) o[t] = fmaf(pr[u][j], q[t][j], o[t]);
+          a[u][t] -= o[t];
         }
-        __stcs(reinterpret_cast<float4*>(g + (int64_t)u * m + k), make_float4(o[0], o[1], o[2], o[3]));
-        *reinterpret_cast<float4*>(e + (int64_t)u * m + k) = make_float4(a[u].x - o[0], a[u].y - o[1], a[u].z - o[2], a[u].w - o[3]);
+        store4<R, true>(g + (int64_t)u * m, k, m, o);
+        store4<R, false>(e + (int64_t)u * m, k, m, a[u]);
       }
   }
 }

@@ -218,3 +218,18 @@ def test_topk_ties_go_to_the_first(n, step):
     want = torch.sort(a.abs(), descending=True, stable=True)[1][:k].sort()[0]
     for _ in range(3):
         assert torch.equal(sel.select(a.cuda(), None)[0].cpu().long().sort()[0], want)
+
+
+@pytest.mark.parametrize("rank", [3, 4])
+@pytest.mark.parametrize("n,m", [(40, 4), (33, 36), (64, 132), (70, 1060), (17, 4104)])
+def test_powersgd_rows_that_end_inside_a_block_of_columns(rank, n, m):
+    from gradient_compression_b200.reducers import RankKReducer
+
+    host = _values([n * m], 9)[0].view(n, m)
+    cpu, gpu = (RankKReducer(d, None, rank=rank, seed=5) for d in ("cpu", "cuda"))
+    for step in range(2):
+        want, got = torch.empty_like(host), torch.empty(n, m, device="cuda")
+        cpu.reduce([host.clone()], [want])
+        gpu.reduce([host.cuda()], [got])
+        torch.testing.assert_close(got.cpu(), want, rtol=2e-4, atol=2e-4 * float(want.abs().max()))
+        torch.testing.assert_close(gpu.state_dict()["_memory"].cpu(), cpu.state_dict()["_memory"], rtol=1e-3, atol=2e-4)
