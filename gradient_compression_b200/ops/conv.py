@@ -597,12 +597,14 @@ def _mode(conv, bn, x):
 
 def _eval(conv, bn, x, residual, relu, pool):
     """``conv_bn_act`` in inference: running statistics, nothing kept for a backward.  None: not a case for the kernels."""
-    params, stats = bn._parameters, bn._buffers
-    w, k, s, p = conv._parameters["weight"], conv.kernel_size, conv.stride, conv.padding
+    # Parameters and buffers as the modules registered them (a module's attribute lookup walks through these dictionaries anyway).
+    # One that is computed instead -- pruning, weight or spectral normalisation -- has no such entry: the kernels decline.
+    own, params, stats = conv._parameters, bn._parameters, bn._buffers
+    w, k, s, p = own.get("weight"), conv.kernel_size, conv.stride, conv.padding
     if (conv.groups != 1 or conv.dilation != (1, 1) or k[0] != k[1] or s[0] != s[1] or isinstance(p, str) or p[0] != p[1] or conv.padding_mode != "zeros"
-            or params["weight"] is None or not torch.backends.cudnn.allow_tf32):
+            or "bias" not in own or not torch.backends.cudnn.allow_tf32):
         return None
-    y = nat.ext().conv_bn_eval(x, w, conv._parameters["bias"], params["weight"], params["bias"], stats["running_mean"], stats["running_var"], bn.eps,
+    y = nat.ext().conv_bn_eval(x, w, own["bias"], params.get("weight"), params.get("bias"), stats.get("running_mean"), stats.get("running_var"), bn.eps,
                                residual, relu, s[0], p[0], pool, _err(x.device))
     if y is not None:
         nat.count_launch()
@@ -615,7 +617,7 @@ def conv_bn_act(conv, bn, x, residual=None, relu=True, link=None, donate=None, p
     ``x`` (a block's first convolution, when this layer is the projection shortcut): this layer's input gradient is then
     handed to that layer's input-gradient kernel to add onto.  ``pool=True``: a 2x2 / stride-2 max-pool of the result, folded
     into the BN kernels (no residual)."""
-    if ENABLED and not bn.training and x.is_cuda and not torch.is_grad_enabled() and type(conv) is torch.nn.Conv2d and bn._buffers["running_mean"] is not None:
+    if ENABLED and not bn.training and x.is_cuda and not torch.is_grad_enabled() and type(conv) is torch.nn.Conv2d:
         y = _eval(conv, bn, x, residual, relu, pool)
         if y is not None:
             return y

@@ -60,3 +60,40 @@ def test_model_matches_the_layers_one_by_one(name):
         finally:
             C.ENABLED = True
     assert float((got - want).norm() / want.norm()) < 2e-2
+
+
+def _layer(cin=64, cout=64, r=3):
+    torch.manual_seed(3)
+    conv = nn.Conv2d(cin, cout, r, 1, r // 2).cuda().to(memory_format=torch.channels_last)
+    bn = nn.BatchNorm2d(cout).cuda().eval()
+    with torch.no_grad():
+        bn.weight.normal_()
+        bn.running_var.uniform_(0.3, 3.0)
+    return conv, bn, torch.randn(4, cin, 8, 8, device="cuda").contiguous(memory_format=torch.channels_last)
+
+
+def _want(conv_w, conv_b, bn, bn_w, x):
+    y = F.conv2d(x.double(), conv_w.double(), conv_b.double(), 1, conv_w.shape[2] // 2)
+    return F.relu(F.batch_norm(y, bn.running_mean.double(), bn.running_var.double(), bn_w.double(), bn.bias.double(), False, 0.0, bn.eps))
+
+
+@pytest.mark.filterwarnings("ignore:.*weight_norm.*")
+@pytest.mark.parametrize("r", [1, 3])
+@pytest.mark.parametrize("how", ["conv weight pruned", "conv bias pruned", "bn weight pruned", "weight_norm"])
+def test_computed_parameters(how, r):
+    """Layers whose weight is computed from another parameter: not registered under its own name any more."""
+    import torch.nn.utils as U
+    import torch.nn.utils.prune as prune
+
+    from gradient_compression_b200.ops import conv_bn_act
+
+    conv, bn, x = _layer(r=r)
+    if how == "weight_norm":
+        U.weight_norm(conv)
+    else:
+        module, name = bn if "bn" in how else conv, "bias" if "bias" in how else "weight"
+        prune.custom_from_mask(module, name, (torch.rand_like(getattr(module, name)) < 0.5).float())
+    with torch.no_grad():
+        got = conv_bn_act(conv, bn, x)
+        want = _want(conv.weight, conv.bias, bn, bn.weight, x)
+    assert float((got.double() - want).norm() / want.norm()) < 2e-3
