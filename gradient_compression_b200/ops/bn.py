@@ -15,6 +15,20 @@ import torch.nn.functional as F
 
 from . import _native as nat
 
+# Hooks registered for every module of the process (profilers, module trackers).
+_PRE, _FORWARD, _BACKWARD_PRE, _BACKWARD = (getattr(torch.nn.modules.module, n) for n in (
+    "_global_forward_pre_hooks", "_global_forward_hooks", "_global_backward_pre_hooks", "_global_backward_hooks"))
+
+
+def hooked(a, b=None):
+    """Whether calling the module ``a`` (or ``b``) runs more than its forward.  The kernels take a layer's parameters without calling
+    it, so a layer with hooks is called as the module it is: pruning and the weight normalisations recompute the weight in one."""
+    d, e = a.__dict__, (a if b is None else b).__dict__            # (a third of the time of as many attributes)
+    return bool(d["_forward_pre_hooks"] or d["_forward_hooks"] or d["_backward_hooks"] or d["_backward_pre_hooks"] or
+                e["_forward_pre_hooks"] or e["_forward_hooks"] or e["_backward_hooks"] or e["_backward_pre_hooks"] or
+                _PRE or _FORWARD or _BACKWARD_PRE or _BACKWARD)
+
+
 # Gradient tensors this library allocated itself and handed to autograd for a residual input: nobody else holds
 # them, so a later kernel may accumulate into them in place (``ops.conv.GradLink``).  Keyed by address, checked by
 # object identity through a weak reference, so a freed and re-used address never matches.
@@ -217,12 +231,13 @@ class _FusedBNAct(torch.autograd.Function):
 def bn_act(bn, x, residual=None, relu=True):
     """``relu(bn(x) + residual)`` with ``bn`` a ``torch.nn.BatchNorm2d`` (affine, tracking running stats)."""
     training = bn.training or bn.running_mean is None
-    if not training and x.is_cuda and bn.affine and not torch.is_grad_enabled():
+    plain = bn.affine and not hooked(bn)
+    if not training and x.is_cuda and plain and not torch.is_grad_enabled():
         y = nat.ext().bn_eval(x, bn.weight, bn.bias, bn.running_mean, bn.running_var, bn.eps, residual, relu)
         if y is not None:
             nat.count_launch()
             return y
-    use_kernel = kernel_path_ok(x) and bn.affine and not (not training and torch.is_grad_enabled() and x.requires_grad)
+    use_kernel = plain and kernel_path_ok(x) and not (not training and torch.is_grad_enabled() and x.requires_grad)
     if not use_kernel:
         y = bn(x)
         if residual is not None:

@@ -33,7 +33,7 @@ import torch
 
 from . import _native as nat
 from . import gemm
-from .bn import _cl, _fin_ptr, _scratch_for, bn_act, fused_backward, fused_forward, fused_ok, count_batch, own_grad, take_owned_grad
+from .bn import _cl, _fin_ptr, _scratch_for, bn_act, fused_backward, fused_forward, fused_ok, hooked, count_batch, own_grad, take_owned_grad
 
 # GCB200_TC_CONV=0 (or ``ENABLED = False``) keeps every convolution on cuDNN.
 ENABLED = os.environ.get("GCB200_TC_CONV", "1") == "1"
@@ -563,6 +563,8 @@ def _mode(conv, bn, x):
     """Which tensor-core path runs ``conv`` on ``x`` ("gemm", "conv", "stem") or None for cuDNN."""
     if not (ENABLED and x.is_cuda and x.dtype == torch.float32 and x.dim() == 4 and isinstance(conv, torch.nn.Conv2d)):
         return None
+    if hooked(conv, bn):
+        return None
     if not torch.backends.cudnn.allow_tf32:       # the kernels multiply in TF32: only where TF32 convolutions are allowed
         return None
     k, s, p = conv.kernel_size, conv.stride, conv.padding
@@ -602,7 +604,7 @@ def _eval(conv, bn, x, residual, relu, pool):
     own, params, stats = conv._parameters, bn._parameters, bn._buffers
     w, k, s, p = own.get("weight"), conv.kernel_size, conv.stride, conv.padding
     if (conv.groups != 1 or conv.dilation != (1, 1) or k[0] != k[1] or s[0] != s[1] or isinstance(p, str) or p[0] != p[1] or conv.padding_mode != "zeros"
-            or "bias" not in own or not torch.backends.cudnn.allow_tf32):
+            or "bias" not in own or hooked(conv, bn) or not torch.backends.cudnn.allow_tf32):
         return None
     y = nat.ext().conv_bn_eval(x, w, own["bias"], params.get("weight"), params.get("bias"), stats.get("running_mean"), stats.get("running_var"), bn.eps,
                                residual, relu, s[0], p[0], pool, _err(x.device))

@@ -97,3 +97,62 @@ def test_computed_parameters(how, r):
         got = conv_bn_act(conv, bn, x)
         want = _want(conv.weight, conv.bias, bn, bn.weight, x)
     assert float((got.double() - want).norm() / want.norm()) < 2e-3
+
+
+@pytest.mark.filterwarnings("ignore:.*weight_norm.*")
+@pytest.mark.parametrize("training", [False, True])
+@pytest.mark.parametrize("how", ["conv pruned", "bn pruned", "weight_norm", "spectral_norm"])
+def test_recomputed_weights(how, training):
+    """The weight is recomputed from what it is made of at every call, in inference and in training (two steps)."""
+    import torch.nn.utils as U
+    import torch.nn.utils.prune as prune
+
+    from gradient_compression_b200.ops import conv_bn_act
+
+    conv, bn, x = _layer()
+    if "pruned" in how:
+        prune.custom_from_mask(bn if "bn" in how else conv, "weight", (torch.rand_like((bn if "bn" in how else conv).weight) < 0.5).float())
+    else:
+        getattr(U, how)(conv)
+    conv.train(training), bn.train(training)
+    for _ in range(2):
+        with torch.set_grad_enabled(training):
+            got = conv_bn_act(conv, bn, x)
+        with torch.no_grad():
+            y = F.conv2d(x.double(), conv.weight.double(), conv.bias.double(), 1, 1)        # the weight of that call
+            y = F.batch_norm(y, bn.running_mean.double(), bn.running_var.double(), bn.weight.double(), bn.bias.double(), training, 0.0, bn.eps)
+            want = F.relu(y)
+        assert float((got.detach().double() - want).norm() / want.norm()) < 2e-3
+        changed = [p for n, p in list(conv.named_parameters()) + list(bn.named_parameters()) if n in ("weight_orig", "weight_g")]
+        if training:
+            got.square().sum().backward()
+            assert changed and all(p.grad is not None and float(p.grad.abs().max()) > 0 for p in changed)
+            conv.zero_grad(), bn.zero_grad()
+        with torch.no_grad():
+            for p in changed:
+                p.mul_(1.5)
+
+
+@pytest.mark.parametrize("training", [False, True])
+@pytest.mark.parametrize("kind", ["forward", "pre", "backward", "global"])
+def test_hooks_run(kind, training):
+    from gradient_compression_b200.ops import conv_bn_act
+
+    conv, bn, x = _layer()
+    bn.train(training)
+    seen = []
+    with torch.set_grad_enabled(training):
+        plain = conv_bn_act(conv, bn, x)
+        if kind == "global":
+            handles = [nn.modules.module.register_module_forward_hook(lambda m, i, o: seen.append(m))]
+        else:
+            add = {"forward": "register_forward_hook", "pre": "register_forward_pre_hook", "backward": "register_full_backward_hook"}[kind]
+            handles = [getattr(m, add)(lambda m, *_: seen.append(m)) for m in (conv, bn)]
+        got = conv_bn_act(conv, bn, x)
+        if training:
+            got.sum().backward()
+        for h in handles:
+            h.remove()
+        again = conv_bn_act(conv, bn, x)
+    assert set(seen) == (set() if kind == "backward" and not training else {conv, bn})
+    assert float((got - plain).norm() / plain.norm()) < 2e-3 and torch.equal(again, plain)
