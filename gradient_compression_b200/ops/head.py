@@ -15,6 +15,7 @@ import torch
 import torch.nn.functional as F
 
 from . import _native as nat
+from .bn import hooked
 
 _scratch = {}
 
@@ -82,7 +83,7 @@ class _HeadCE(torch.autograd.Function):
 
 def head_loss(features, linear, labels):
     """``(mean cross-entropy, logits, [cross-entropy, top-1, top-5])`` of ``linear(mean over H, W of features)``."""
-    if supported(features, linear.weight, labels):
+    if not hooked(linear) and supported(features, linear.weight, labels):
         return _HeadCE.apply(features, linear.weight, linear.bias, labels)
     logits = linear(features.mean((2, 3)) if features.dim() == 4 else features)
     loss = F.cross_entropy(logits, labels)
@@ -94,8 +95,9 @@ def head_loss(features, linear, labels):
 
 
 def classify(features, linear):
-    """Inference: ``linear(mean over H, W of features)`` in one kernel; None where it does not apply."""
-    if not features.is_cuda or torch.is_grad_enabled() or type(linear) is not torch.nn.Linear or torch.is_autocast_enabled():
+    """Inference: ``linear(mean over H, W of features)`` in one kernel; None where it does not apply (a layer with hooks among others:
+    it is called as the module it is)."""
+    if not features.is_cuda or torch.is_grad_enabled() or type(linear) is not torch.nn.Linear or torch.is_autocast_enabled() or hooked(linear):
         return None
     y = nat.ext().classify(features, linear.weight, linear.bias)
     if y is not None:

@@ -41,3 +41,33 @@ def test_logit_metrics(n, k):
     z[-1, 1] = float("nan")
     assert torch.isnan(logit_metrics(z, labels)[0])
     assert logit_metrics(z[:, :4].contiguous(), labels) is None and logit_metrics(z.half(), labels) is None
+
+
+@pytest.mark.parametrize("name", ["ResNet18", "VGG11"])
+@pytest.mark.parametrize("what", ["forward hook", "pruned"])
+def test_a_classifier_with_hooks_is_called(name, what):
+    import torch.nn.utils.prune as prune
+
+    from gradient_compression_b200 import models
+
+    torch.manual_seed(2)
+    model = getattr(models, name)().cuda().to(memory_format=torch.channels_last)
+    linear = model.linear if name == "ResNet18" else model.classifier
+    x, labels, seen = torch.randn(6, 3, 32, 32, device="cuda").contiguous(memory_format=torch.channels_last), torch.arange(6, device="cuda"), []
+    with torch.no_grad():
+        model(x)
+        plain = model.eval()(x)
+    if what == "pruned":
+        prune.custom_from_mask(linear, "weight", torch.ones_like(linear.weight))
+        with torch.no_grad():
+            linear.weight_orig.mul_(2.0)
+    else:
+        linear.register_forward_hook(lambda m, i, o: seen.append(m) or 2.0 * o)
+    with torch.no_grad():
+        got = model(x)
+        want = 2.0 * plain - (linear.bias if what == "pruned" else 0.0)
+    assert torch.allclose(got, want, rtol=1e-4, atol=1e-4 * float(want.abs().max()))
+    assert seen == [linear] * (what != "pruned")
+    loss, logits, _ = model.train().forward_loss(x, labels)
+    loss.backward()
+    assert torch.isfinite(loss) and (len(seen) == 2 if what == "forward hook" else float(linear.weight_orig.grad.abs().max()) > 0)
