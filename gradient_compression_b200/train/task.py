@@ -13,6 +13,7 @@ import torch
 import torch.distributed as dist
 
 from .. import models
+from ..ops.bn import hooked
 from ..ops.head import logit_metrics
 from ..parallel.arena import FlatArena
 from ..utils.metrics import AverageMeter
@@ -130,12 +131,18 @@ class CIFAR:
         else:
             self._model.zero_grad()
 
+    def _plain_cross_entropy(self):
+        """Whether the criterion is what the kernels of ``ops.head`` compute: the mean cross-entropy without weights or smoothing."""
+        c = self._criterion
+        return (type(c) is torch.nn.CrossEntropyLoss and c.weight is None and c.ignore_index == -100 and c.reduction == "mean"
+                and c.label_smoothing == 0.0 and not hooked(c))
+
     def forward_loss(self, imgs, labels):
         """``(loss, logits, metrics)`` of a batch, the metrics as device scalars.  Models with a fused head (pooling, linear
-        layer, cross-entropy and top-1 / top-5 in one kernel: ``ops.head``) provide all three at once; for the others the
-        loss comes from the criterion and the metrics from ``evaluate_predictions``."""
+        layer, cross-entropy and top-1 / top-5 in one kernel: ``ops.head``) provide all three at once; for the others, and with
+        another criterion, the loss comes from the criterion and the metrics from ``evaluate_predictions``."""
         fused = getattr(self._model, "forward_loss", None)
-        if fused is not None and labels.dtype == torch.int64:
+        if fused is not None and labels.dtype == torch.int64 and self._plain_cross_entropy():
             loss, prediction, m = fused(imgs, labels)
             metrics = {"cross_entropy_loss": m[0], "top1_accuracy": m[1], "top5_accuracy": m[2]}
             return loss, prediction, metrics
@@ -165,7 +172,8 @@ class CIFAR:
             known = logit_metrics(pred_labels, true_labels)
             if known is not None:
                 ce, top1, top5 = known
-                ce = ce if loss is None else loss
+                if loss is not None or not self._plain_cross_entropy():
+                    ce = self._criterion(pred_labels, true_labels) if loss is None else loss
             else:
                 ce = self._criterion(pred_labels, true_labels) if loss is None else loss
                 top5 = pred_labels.topk(5, 1, True, True)[1]

@@ -218,3 +218,26 @@ def test_noise_source_keeps_the_live_rank_on_restore():
     live = NoiseSource(seed=3, rank=1)
     live.load_state_dict(saved.state_dict())
     assert live.rank == 1 and live.step == 17 and live.stream(1) != saved.stream(1)
+
+
+@pytest.mark.parametrize("device", ["cpu", pytest.param("cuda", marks=pytest.mark.gpu)])
+@pytest.mark.parametrize("options", [{}, {"label_smoothing": 0.2}, {"reduction": "sum"}, {"ignore_index": 3}, {"weight": True}])
+def test_the_tasks_criterion_is_used(device, options):
+    if "weight" in options:
+        options = {"weight": torch.linspace(0.1, 2.0, 10, device=device)}
+    task = CIFAR(device, None, "VGG11", seed=1, data="synthetic", synthetic_train_size=1, synthetic_test_size=1)
+    task._criterion = torch.nn.CrossEntropyLoss(**options)
+    x, y = torch.randn(12, 3, 32, 32, device=device), torch.arange(12, device=device) % 10
+    loss, _, metrics = task.batch_loss_with_gradients((x, y))
+    task.model.eval()
+    with torch.no_grad():
+        logits = task.model(x)
+        got = task.evaluate_predictions(logits, y)
+        want = torch.nn.CrossEntropyLoss(**options)(logits, y)
+        assert float(got["cross_entropy_loss"]) == pytest.approx(float(want), rel=1e-5)
+        task.model.train()
+        want = torch.nn.CrossEntropyLoss(**options)(task.model(x), y)         # batch statistics: the same forward as the step's
+    assert float(loss) == pytest.approx(float(want), rel=1e-4)
+    assert float(metrics["cross_entropy_loss"]) == pytest.approx(float(loss), rel=1e-6)
+    hit = logits.topk(5, 1)[1].eq(y.view(-1, 1))
+    assert float(got["top1_accuracy"]) == pytest.approx(float(hit[:, 0].float().mean())) and float(got["top5_accuracy"]) == pytest.approx(float(hit.any(1).float().mean()))
