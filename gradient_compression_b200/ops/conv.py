@@ -606,6 +606,12 @@ def _eval(conv, bn, x, residual, relu, pool):
     if (conv.groups != 1 or conv.dilation != (1, 1) or k[0] != k[1] or s[0] != s[1] or isinstance(p, str) or p[0] != p[1] or conv.padding_mode != "zeros"
             or "bias" not in own or hooked(conv, bn) or not torch.backends.cudnn.allow_tf32):
         return None
+    mode = "gemm" if k[0] == 1 and s[0] == 1 and p[0] == 0 else \
+        "stem" if conv.in_channels * k[0] * k[0] <= STEM_K and s[0] == 1 and 2 * p[0] == k[0] - 1 and conv.out_channels > 16 else "conv"
+    if mode not in PATHS:
+        return None
+    if MIN_ROWS > 0 and x.dim() == 4 and x.shape[0] * ((x.shape[2] + 2 * p[0] - k[0]) // s[0] + 1) * ((x.shape[3] + 2 * p[0] - k[0]) // s[0] + 1) < MIN_ROWS:
+        return None
     y = nat.ext().conv_bn_eval(x, w, own["bias"], params.get("weight"), params.get("bias"), stats.get("running_mean"), stats.get("running_var"), bn.eps,
                                residual, relu, s[0], p[0], pool, _err(x.device))
     if y is not None:

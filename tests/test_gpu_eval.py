@@ -155,4 +155,30 @@ def test_hooks_run(kind, training):
             h.remove()
         again = conv_bn_act(conv, bn, x)
     assert set(seen) == (set() if kind == "backward" and not training else {conv, bn})
+    got, plain, again = got.detach(), plain.detach(), again.detach()
     assert float((got - plain).norm() / plain.norm()) < 2e-3 and torch.equal(again, plain)
+
+
+@pytest.mark.parametrize("training", [False, True])
+@pytest.mark.parametrize("mode,cin,r,stride", [("gemm", 64, 1, 1), ("conv", 64, 3, 1), ("conv", 64, 1, 2), ("stem", 3, 3, 1)])
+def test_switches_act_in_inference_as_in_training(mode, cin, r, stride, training, monkeypatch):
+    from gradient_compression_b200.ops import conv as C
+
+    torch.manual_seed(4)
+    conv = nn.Conv2d(cin, 64, r, stride, r // 2).cuda().to(memory_format=torch.channels_last).train(training)
+    bn = nn.BatchNorm2d(64).cuda().train(training)
+    x = torch.randn(2, cin, 8, 8, device="cuda").contiguous(memory_format=torch.channels_last)
+    rows, calls, forward = 2 * (8 // stride) ** 2, [], nn.Conv2d.forward
+    monkeypatch.setattr(nn.Conv2d, "forward", lambda m, i: calls.append(1) or forward(m, i))        # only cuDNN calls the module
+
+    def on_cudnn(**switches):
+        with monkeypatch.context() as m, torch.set_grad_enabled(training):
+            for k, v in switches.items():
+                m.setattr(C, k, v)
+            del calls[:]
+            C.conv_bn_act(conv, bn, x)
+        return bool(calls)
+
+    every = {"gemm", "conv", "stem", "dgrad_s2"}
+    assert not on_cudnn() and not on_cudnn(PATHS={mode}) and not on_cudnn(MIN_ROWS=rows)
+    assert on_cudnn(PATHS=every - {mode}) and on_cudnn(MIN_ROWS=rows + 1) and on_cudnn(ENABLED=False)
