@@ -926,6 +926,9 @@ int gc_comm_create(int world, int rank, int64_t bytes, void** out_ctx) {
   return 0;
 }
 
+// Device the arena lives on.
+int gc_comm_device(void* ctx) { return ((CommCtx*)ctx)->device; }
+
 int gc_comm_ipc_handle(void* ctx, void* out64) {
   CommCtx* c = (CommCtx*)ctx;
   cudaIpcMemHandle_t h;

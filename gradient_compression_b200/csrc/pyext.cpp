@@ -30,6 +30,7 @@ struct SegDesc {            // csrc/gc_segs.cuh
 // Entry points of the kernel library.
 struct Api {
   int (*solo_max_segs)();
+  int (*comm_device)(void*);
   int (*solo_maxnorm)(void*, const void*, int, int64_t, int, int, uint64_t, uint32_t, int, int, void*);
   int (*solo_copy)(void*, const void*, int, int64_t, void*);
   int64_t (*solo_randk_limit)(void*, int);
@@ -57,6 +58,7 @@ int max_segs = 0;
 struct Entry { const char* name; void** slot; };
 const Entry entries[] = {
     {"gc_solo_max_segs", (void**)&api.solo_max_segs},
+    {"gc_comm_device", (void**)&api.comm_device},
     {"gc_solo_maxnorm", (void**)&api.solo_maxnorm},
     {"gc_solo_copy", (void**)&api.solo_copy},
     {"gc_solo_randk_limit", (void**)&api.solo_randk_limit},
@@ -134,8 +136,9 @@ bool overlap_free(const std::vector<SegDesc>& segs, int64_t n) {
 }
 
 // Fills the plan from two lists of tensors.  False: not a case for the segment kernels (the caller takes the general path).
-// `merge`: neighbours in memory become one segment (otherwise a segment per non-empty tensor).
-bool collect(Plan& p, PyObject* ins, PyObject* outs, bool merge = true) {
+// `merge`: neighbours in memory become one segment (otherwise a segment per non-empty tensor).  The kernels run where the tensors
+// are and synchronise on words of the arena `ctx`: both have to be on one device.
+bool collect(Plan& p, void* ctx, PyObject* ins, PyObject* outs, bool merge = true) {
   PyObject* fa = PySequence_Fast(ins, "reduce() takes lists of tensors");
   if (!fa) return false;
   PyObject* fb = ins == outs ? (Py_INCREF(fa), fa) : PySequence_Fast(outs, "reduce() takes lists of tensors");
@@ -177,7 +180,7 @@ bool collect(Plan& p, PyObject* ins, PyObject* outs, bool merge = true) {
   Py_DECREF(fa);
   Py_DECREF(fb);
   if (PyErr_Occurred()) return false;
-  if (!ok || p.segs.empty() || (int)p.segs.size() > max_segs) return false;
+  if (!ok || p.segs.empty() || (int)p.segs.size() > max_segs || p.device != api.comm_device(ctx)) return false;
   const bool known = p.checked.size() == p.segs.size() + 1 && p.checked.back().start == p.n &&
                      memcmp(p.checked.data(), p.segs.data(), p.segs.size() * sizeof(SegDesc)) == 0;
   if (!known) {
@@ -209,8 +212,9 @@ PyObject* solo_maxnorm(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   if (!want(nargs, 10, "solo_maxnorm")) return nullptr;
   Plan* p = plan_of(a[0]);
   if (!p) return nullptr;
-  if (!collect(*p, a[2], a[3])) { if (PyErr_Occurred()) return nullptr; Py_RETURN_NONE; }
   void* ctx = (void*)PyLong_AsUnsignedLongLong(a[1]);
+  if (PyErr_Occurred()) return nullptr;
+  if (!collect(*p, ctx, a[2], a[3])) { if (PyErr_Occurred()) return nullptr; Py_RETURN_NONE; }
   const int lo = (int)as_int(a[4]), hi = (int)as_int(a[5]), timeout = (int)as_int(a[8]), blocks = (int)as_int(a[9]);
   const uint64_t seed = PyLong_AsUnsignedLongLongMask(a[6]);
   const uint32_t step = (uint32_t)PyLong_AsUnsignedLongLongMask(a[7]);
@@ -226,9 +230,9 @@ PyObject* solo_copy(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   if (!want(nargs, 4, "solo_copy")) return nullptr;
   Plan* p = plan_of(a[0]);
   if (!p) return nullptr;
-  if (!collect(*p, a[2], a[3])) { if (PyErr_Occurred()) return nullptr; Py_RETURN_NONE; }
   void* ctx = (void*)PyLong_AsUnsignedLongLong(a[1]);
   if (PyErr_Occurred()) return nullptr;
+  if (!collect(*p, ctx, a[2], a[3])) { if (PyErr_Occurred()) return nullptr; Py_RETURN_NONE; }
   bool moves = false;
   for (const SegDesc& s : p->segs) moves = moves || s.in != s.out;
   if (moves) {
@@ -239,15 +243,17 @@ PyObject* solo_copy(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   return PyLong_FromLongLong(p->n);
 }
 
-// collect(plan, grad_in, grad_out, merge) -> (elements, generation of the tensors' shapes, segments), or None.
+// collect(plan, ctx, grad_in, grad_out, merge) -> (elements, generation of the tensors' shapes, segments), or None.
 // merge: 1 neighbours become one segment, 0 a segment per tensor, 2 one segment if all of them are neighbours, else one per tensor
 PyObject* collect_py(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
-  if (!want(nargs, 4, "collect")) return nullptr;
+  if (!want(nargs, 5, "collect")) return nullptr;
   Plan* p = plan_of(a[0]);
   if (!p) return nullptr;
-  const int merge = (int)as_int(a[3]);
-  bool ok = collect(*p, a[1], a[2], merge != 0);
-  if (ok && merge == 2 && p->segs.size() > 1) ok = collect(*p, a[1], a[2], false);
+  void* ctx = (void*)PyLong_AsUnsignedLongLong(a[1]);
+  const int merge = (int)as_int(a[4]);
+  if (PyErr_Occurred()) return nullptr;
+  bool ok = collect(*p, ctx, a[2], a[3], merge != 0);
+  if (ok && merge == 2 && p->segs.size() > 1) ok = collect(*p, ctx, a[2], a[3], false);
   if (!ok) { if (PyErr_Occurred()) return nullptr; Py_RETURN_NONE; }
   if (p->shape != p->shape_seen) {
     p->shape_seen = p->shape;

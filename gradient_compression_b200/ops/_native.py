@@ -209,6 +209,7 @@ def cuda():
         _declare(lib, "gc_comm_required_bytes", c_i64, [c_i64])
         _declare(lib, "gc_comm_oneshot_bytes", c_i64, [c_i64])
         _declare(lib, "gc_comm_create", c_int, [c_int, c_int, c_i64, PP])
+        _declare(lib, "gc_comm_device", c_int, [P])
         _declare(lib, "gc_comm_ipc_handle", c_int, [P, P])
         _declare(lib, "gc_comm_open_peers", c_int, [P, P])
         _declare(lib, "gc_comm_set_peer", c_int, [P, c_int, P])

@@ -50,6 +50,8 @@ class TopKSelector:
         if out_val is None:
             out_val = torch.empty(self.total, dtype=torch.float32, device=g.device)
         if g.is_cuda:
+            if e is not None and e.device != g.device:
+                raise ValueError(f"values on {g.device}, error memory on {e.device}")
             with torch.cuda.device(g.device):
                 for run, scratch, counts in self._runs:
                     table = (nat.SegDesc * len(run))(*[(g.data_ptr() + 4 * self.segments[i][0], None, self.segments[i][0]) for i in run])

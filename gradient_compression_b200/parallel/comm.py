@@ -49,6 +49,7 @@ class _Ctx:
         with torch.cuda.device(device):
             _ck(nat.cuda().gc_comm_create(world, rank, self.bytes, ctypes.byref(h)), "comm_create")
         self.handle = h
+        self.device_index = int(nat.cuda().gc_comm_device(h))
 
     def arena_ptr(self):
         return nat.cuda().gc_comm_arena_ptr(self.handle)

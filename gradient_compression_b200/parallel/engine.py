@@ -16,6 +16,13 @@ from ..ops import _native as nat
 from . import comm
 
 
+def _on_device(index, *tensors):
+    """The kernels follow pointers of the arena and of all of these: ``ValueError`` unless every tensor is on that GPU."""
+    for t in tensors:
+        if t is not None and t.is_cuda and t.device.index != index:
+            raise ValueError(f"tensor on {t.device}, but the reducer's arena is on cuda:{index}")
+
+
 class FusedOps:
     def __init__(self, arena, timeout_ms=None, max_blocks=0):
         self.arena = arena
@@ -28,6 +35,7 @@ class FusedOps:
         assert len(ins) == len(outs) == len(self.arena.ctxs)
         for t in ins + outs:
             assert t.is_cuda and t.dtype == torch.float32 and t.is_contiguous()
+        _on_device(self.arena.ctxs[0].device_index, *ins, *outs)
         return ins, outs, self.arena._launch_arrays(ins, outs)
 
     def _run(self, what, err):
@@ -325,9 +333,11 @@ class FusedEngine:
         ops = self._ensure(n, 4 * max(plan["p_total"] + c["v_total"], plan["q_total"], 1))
         dest, tmp = self._out_flat(flat, grad_out)
         g, e = flat.buffer, reducer._memory
+        draw = not (reducer.reuse_query and not fresh)
+        _on_device(ops.arena.ctxs[0].device_index, g, e, dest, reducer.q_memory, reducer._device_step() if draw else None)
         p_total, q_total = plan["p_total"], plan["q_total"]
         with reducer._timer("reduce.prepare.q", verbosity=2):
-            if not (reducer.reuse_query and not fresh):
+            if draw:
                 # the step counter of the query stream lives on the device (a replayed graph draws a new Q every step)
                 philox.normal(q_total, reducer._seed, philox.stream_id(0, philox.PURPOSE_QINIT), 0,
                               device=g.device, out=reducer.q_memory, step_offset=reducer._device_step())
@@ -406,7 +416,8 @@ def solo_collect(reducer, grad_in, grad_out, merge):
     shapes, segments), or None.  ``merge``: 1 neighbours in memory become one segment, 0 a segment per tensor, 2 one segment if
     all of them are neighbours, else one per tensor."""
     eng = reducer._fused or _engine(reducer)
-    return None if eng.solo_handle() is None else eng.ext.collect(eng.plan, grad_in, grad_out, merge)
+    handle = eng.solo_handle()
+    return None if handle is None else eng.ext.collect(eng.plan, handle, grad_in, grad_out, merge)
 
 
 def solo_randk_takes(reducer, k):
@@ -418,6 +429,7 @@ def solo_randk_takes(reducer, k):
 def solo_randk(reducer, start, k, npass, bits_lo, bits_hi):
     eng, noise = reducer._fused, reducer._noise
     window = reducer._device_window(start)
+    _on_device(eng.ops.arena.ctxs[0].device_index, window)
     eng.ext.solo_randk(eng.plan, eng.solo_handle(), reducer._queue.seed, npass, start, reducer._K if window is not None else k,
                        window.data_ptr() if window is not None else 0, bits_lo, bits_hi, reducer._unselected == "zero", noise.step, eng.ops.timeout_ms,
                        eng.max_blocks())
@@ -427,6 +439,7 @@ def solo_randk(reducer, start, k, npass, bits_lo, bits_hi):
 
 def solo_topk(reducer, counts, per_tensor, memory, scratch):
     eng = reducer._fused
+    _on_device(eng.ops.arena.ctxs[0].device_index, memory, scratch.state)
     eng.ext.solo_topk(eng.plan, counts.data_ptr(), int(per_tensor), memory.data_ptr(), scratch.state.data_ptr(), scratch.lists.data_ptr())
     nat.count_launch(4)
 
@@ -462,9 +475,11 @@ def solo_psgd(reducer, c, q_total, draw):
     from ..ops import philox
 
     eng = reducer._fused
+    step = reducer._device_step() if draw else None
+    _on_device(eng.ops.arena.ctxs[0].device_index, reducer._memory, reducer.q_memory, reducer.p_memory, c["tab"], step)
     eng.ext.solo_psgd(eng.plan, reducer.rank_r, reducer._memory.data_ptr(), c["tab"].data_ptr(), c["n_mats"], c["rows"], c["tiles"], c["max_rows"], c["vtab"].data_ptr(),
                       c["n_vecs"], reducer.q_memory.data_ptr(), reducer.p_memory.data_ptr(), c["q_parts"].data_ptr(), q_total, reducer._seed,
-                      philox.stream_id(0, philox.PURPOSE_QINIT), reducer._device_step().data_ptr() if draw else 0)
+                      philox.stream_id(0, philox.PURPOSE_QINIT), step.data_ptr() if draw else 0)
     nat.count_launch((4 + draw + (c["q_parts"].numel() > 0) if c["n_mats"] else 0) or 1)
 
 

@@ -233,3 +233,37 @@ def test_powersgd_rows_that_end_inside_a_block_of_columns(rank, n, m):
         gpu.reduce([host.cuda()], [got])
         torch.testing.assert_close(got.cpu(), want, rtol=2e-4, atol=2e-4 * float(want.abs().max()))
         torch.testing.assert_close(gpu.state_dict()["_memory"].cpu(), cpu.state_dict()["_memory"], rtol=1e-3, atol=2e-4)
+
+
+@pytest.mark.parametrize("name,config", [("QSGDMaxNormReducer", {"quantization_level": 8}), ("NoneAllReducer", {}), ("GlobalRandKMaxNormReducer", {"K": 10}),
+                                         ("QSGDMaxNormTwoScaleReducer", {"quantization_level": 2, "higher_quantization_level": 6}),
+                                         ("TopKReducerRatio", {"compression": 0.1}), ("RankKReducer", {"rank": 2})])
+def test_tensors_of_another_gpu_than_the_arenas_are_refused(name, config):
+    """The arena is made to say that it lives on the next GPU: nothing is launched, the general path reports it."""
+    import ctypes
+
+    from gradient_compression_b200.ops import _native as nat
+
+    red = make_reducer(name, "cuda", None, dict(config, seed=3))
+    x = torch.randn(64, 32, device="cuda")
+    first = torch.empty_like(x)
+    red.reduce([x], [first])
+    ctx = red._fused.ops.arena.ctxs[0]
+    device = ctypes.c_int.from_address(ctx.handle.value + 8)               # CommCtx {world, rank, device, ...}
+    assert nat.cuda().gc_comm_device(ctx.handle) == device.value == ctx.device_index == x.device.index
+    out, before = torch.full_like(x, 5.0), nat.launches()
+    try:
+        device.value += 1
+        ctx.device_index += 1
+        assert red._solo_reduce([x], [out]) is None
+        if name.startswith(("QSGD", "None")):                   # (the others' general path has an arena of its own)
+            with pytest.raises(ValueError, match="arena"):
+                red.reduce([x], [out])
+        assert nat.launches() == before
+    finally:
+        device.value -= 1
+        ctx.device_index -= 1
+    torch.cuda.synchronize()
+    assert bool((out == 5.0).all())
+    red.reduce([x], [out])
+    assert not bool((out == 5.0).any())
