@@ -23,7 +23,7 @@ using namespace gc;
 namespace {
 
 constexpr int THREADS = 1024, CH = 32, QUADS = CH / 4, LANES = THREADS / QUADS;       // 128 rows at once
-constexpr int MAX_GROUPS = 148;
+constexpr int MAX_BLOCKS = 148;          // groups x runs of rows; also the most groups
 constexpr int VALUES = 2 * CH;
 
 __device__ __forceinline__ float4 ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
@@ -45,7 +45,7 @@ __device__ __forceinline__ void pool_rows(const PoolGeom& g, int64_t r, int64_t 
 
 // Arrival counts of the groups' barriers: they only ever grow.  `passed` is what earlier launches account for.
 struct GroupSync {
-  uint32_t arrived[MAX_GROUPS], passed[MAX_GROUPS];
+  uint32_t arrived[MAX_BLOCKS], passed[MAX_BLOCKS];
 };
 
 struct Shape {
@@ -437,17 +437,20 @@ int sm_count() {
   return sms;
 }
 
-// Runs of rows per channel group: as many as SMs allow, two hundred and some rows each at least (two per thread).
-void plan(Shape& s) {
+// Blocks of a launch: one per SM, and no more than the scratch has partial sums for, whatever the chip's size.
+int block_limit(int sms) { return sms < MAX_BLOCKS ? sms : MAX_BLOCKS; }
+
+// Runs of rows per channel group: as many as blocks allow, two hundred and some rows each at least (two per thread).
+void plan(Shape& s, int sms) {
   s.G = s.C / CH;
-  int64_t most = sm_count() / s.G, want = (s.M + 2 * LANES - 1) / (2 * LANES);
+  int64_t most = block_limit(sms) / s.G, want = (s.M + 2 * LANES - 1) / (2 * LANES);
   if (most < 1) most = 1;
   int64_t r = want < most ? want : most;
   s.per = (s.M + r - 1) / r;
   s.R = (int)((s.M + s.per - 1) / s.per);
 }
 
-bool shape_ok(int64_t M, int C) { return M >= 1 && C >= CH && C % CH == 0 && C / CH <= MAX_GROUPS && C / CH <= sm_count(); }
+bool shape_ok(int64_t M, int C, int sms) { return M >= 1 && C >= CH && C % CH == 0 && C / CH <= block_limit(sms); }
 
 template <typename A>
 int launch(const void* kernel, const Shape& s, const A& a, bool barrier, size_t smem, cudaStream_t st) {
@@ -461,10 +464,20 @@ int launch(const void* kernel, const Shape& s, const A& a, bool barrier, size_t 
 
 extern "C" {
 
-int gc_cuda_bn_fused_supported(int64_t M, int C) { return shape_ok(M, C) ? 1 : 0; }
+int gc_cuda_bn_fused_supported(int64_t M, int C) { return shape_ok(M, C, sm_count()) ? 1 : 0; }
+
+// Blocks a launch on M rows of C channels takes on a chip of `sms` SMs, each of which has a row of partial sums (0: not taken).
+int gc_cuda_bn_fused_blocks(int64_t M, int C, int sms) {
+  if (!shape_ok(M, C, sms)) return 0;
+  Shape s{};
+  s.M = M;
+  s.C = C;
+  plan(s, sms);
+  return s.G * s.R;
+}
 
 // Scratch of both directions: barrier counts (zeroed once when allocated; every launch leaves them ready) and partial sums.
-int64_t gc_cuda_bn_fused_scratch_bytes() { return (int64_t)sizeof(GroupSync) + (int64_t)MAX_GROUPS * VALUES * 4; }
+int64_t gc_cuda_bn_fused_scratch_bytes() { return (int64_t)sizeof(GroupSync) + (int64_t)MAX_BLOCKS * VALUES * 4; }
 
 // y = act(gamma * (x - mean) * rstd + beta [+ residual]) of the batch statistics of x, which come from partials[nparts][2][C] when
 // given.  pool (then no residual): x is [N, H, W, C], H and W even, and y the 2x2 max-pool of the activation.  Writes
@@ -475,12 +488,12 @@ int gc_cuda_bn_fused_forward(const float* x, int N, int H, int W, int C, int poo
   Shape s{};
   s.M = (int64_t)N * H * W / (pool ? 4 : 1);
   s.C = C;
-  if (!shape_ok(s.M, C) || (pool && ((H | W) & 1 || residual != nullptr))) return (int)cudaErrorInvalidValue;
+  if (!shape_ok(s.M, C, sm_count()) || (pool && ((H | W) & 1 || residual != nullptr))) return (int)cudaErrorInvalidValue;
   s.pool = PoolGeom{H, W, H / 2, W / 2};
   s.sync = (GroupSync*)scratch;
   s.parts = (float*)((uint8_t*)scratch + sizeof(GroupSync));
   s.error_flag = error_flag;
-  plan(s);
+  plan(s, sm_count());
   const FwdArgs a{x, partials, nparts, gamma, beta, residual, relu, running_mean, running_var, momentum, eps, stats, y};
   const void* k = partials != nullptr ? (pool ? (const void*)bn_fused_fwd_kernel<true, false> : (const void*)bn_fused_fwd_kernel<false, false>)
                                       : (pool ? (const void*)bn_fused_fwd_kernel<true, true> : (const void*)bn_fused_fwd_kernel<false, true>);
@@ -494,12 +507,12 @@ int gc_cuda_bn_fused_backward(const float* dy, const float* x, const float* y, i
   Shape s{};
   s.M = (int64_t)N * H * W / (pool ? 4 : 1);
   s.C = C;
-  if (!shape_ok(s.M, C) || (pool && ((H | W) & 1 || dres != nullptr))) return (int)cudaErrorInvalidValue;
+  if (!shape_ok(s.M, C, sm_count()) || (pool && ((H | W) & 1 || dres != nullptr))) return (int)cudaErrorInvalidValue;
   s.pool = PoolGeom{H, W, H / 2, W / 2};
   s.sync = (GroupSync*)scratch;
   s.parts = (float*)((uint8_t*)scratch + sizeof(GroupSync));
   s.error_flag = error_flag;
-  plan(s);
+  plan(s, sm_count());
   // masks of as many row pairs as shared memory holds (192 KB: 98 K rows of 32 channels a block)
   constexpr int most = 192;
   const int64_t pairs = (s.per + 2 * LANES - 1) / (2 * LANES);
