@@ -11,7 +11,9 @@
 #include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
+#include <torch/csrc/utils/object_ptr.h>
 
 #include <algorithm>
 #include <cstring>
@@ -139,12 +141,12 @@ bool overlap_free(const std::vector<SegDesc>& segs, int64_t n) {
 // `merge`: neighbours in memory become one segment (otherwise a segment per non-empty tensor).  The kernels run where the tensors
 // are and synchronise on words of the arena `ctx`: both have to be on one device.
 bool collect(Plan& p, void* ctx, PyObject* ins, PyObject* outs, bool merge = true) {
-  PyObject* fa = PySequence_Fast(ins, "reduce() takes lists of tensors");
+  const THPObjectPtr fa(PySequence_Fast(ins, "reduce() takes lists of tensors"));
   if (!fa) return false;
-  PyObject* fb = ins == outs ? (Py_INCREF(fa), fa) : PySequence_Fast(outs, "reduce() takes lists of tensors");
-  if (!fb) { Py_DECREF(fa); return false; }
-  const Py_ssize_t k = PySequence_Fast_GET_SIZE(fa);
-  bool ok = k > 0 && PySequence_Fast_GET_SIZE(fb) == k;
+  const THPObjectPtr fb(ins == outs ? Py_NewRef(fa.get()) : PySequence_Fast(outs, "reduce() takes lists of tensors"));
+  if (!fb) return false;
+  const Py_ssize_t k = PySequence_Fast_GET_SIZE(fa.get());
+  bool ok = k > 0 && PySequence_Fast_GET_SIZE(fb.get()) == k;
   p.segs.clear();
   p.shape.clear();
   p.n = 0;
@@ -152,7 +154,7 @@ bool collect(Plan& p, void* ctx, PyObject* ins, PyObject* outs, bool merge = tru
   for (Py_ssize_t i = 0; ok && i < k; ++i) {
     int64_t na = 0, nb = 0;
     int da = 0, db = 0, oa = 0, ob = 0;
-    PyObject *pa = PySequence_Fast_GET_ITEM(fa, i), *pb = PySequence_Fast_GET_ITEM(fb, i);
+    PyObject *pa = PySequence_Fast_GET_ITEM(fa.get(), i), *pb = PySequence_Fast_GET_ITEM(fb.get(), i);
     float* a = dense_ptr(pa, &na, &da, &oa);
     float* b = a;
     if (pa == pb) { nb = na; db = da; ob = oa; }
@@ -177,8 +179,6 @@ bool collect(Plan& p, void* ctx, PyObject* ins, PyObject* outs, bool merge = tru
     p.segs.push_back({a, b, p.n});
     p.n += na;
   }
-  Py_DECREF(fa);
-  Py_DECREF(fb);
   if (PyErr_Occurred()) return false;
   if (!ok || p.segs.empty() || (int)p.segs.size() > max_segs || p.device != api.comm_device(ctx)) return false;
   const bool known = p.checked.size() == p.segs.size() + 1 && p.checked.back().start == p.n &&
@@ -193,6 +193,17 @@ bool collect(Plan& p, void* ctx, PyObject* ins, PyObject* outs, bool merge = tru
 }
 
 void* stream_on(int device) { return (void*)c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)device).stream(); }
+
+// A call's entry from Python: what libtorch throws (out of memory, a tensor without storage) becomes a Python exception instead of
+// leaving through the interpreter's C frames, which ends the process.
+template <PyObject* (*F)(PyObject*, PyObject* const*, Py_ssize_t)>
+PyObject* entry(PyObject* self, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  return F(self, a, n);
+  END_HANDLE_TH_ERRORS
+}
+template <PyObject* (*F)(PyObject*, PyObject* const*, Py_ssize_t)>
+PyCFunction method() { return (PyCFunction)(void (*)(void))entry<F>; }
 
 PyObject* cuda_error(const char* what, int err) {
   PyErr_Format(PyExc_RuntimeError, "%s: CUDA error %d", what, err);
@@ -554,21 +565,21 @@ PyMethodDef methods[] = {
     {"bind", bind, METH_O, "bind(table): addresses of the kernel library's entry points by name"},
     {"names", names, METH_NOARGS, "names() -> the entry points bind() needs"},
     {"plan_new", plan_new, METH_NOARGS, "plan_new() -> a plan, one per reducer"},
-    {"solo_maxnorm", (PyCFunction)(void (*)(void))solo_maxnorm, METH_FASTCALL, "QSGD-MaxNorm reduce of a single worker"},
-    {"solo_copy", (PyCFunction)(void (*)(void))solo_copy, METH_FASTCALL, "plain mean of a single worker"},
-    {"collect", (PyCFunction)(void (*)(void))collect_py, METH_FASTCALL, "reads two lists of tensors into a plan"},
-    {"solo_randk", (PyCFunction)(void (*)(void))solo_randk, METH_FASTCALL, "Rand-K reduce of a single worker"},
-    {"solo_randk_limit", (PyCFunction)(void (*)(void))solo_randk_limit, METH_FASTCALL, "most coordinates solo_randk takes"},
-    {"solo_psgd", (PyCFunction)(void (*)(void))solo_psgd, METH_FASTCALL, "PowerSGD step of a single worker"},
-    {"solo_topk", (PyCFunction)(void (*)(void))solo_topk, METH_FASTCALL, "top-k with error feedback of a single worker"},
-    {"conv_bn_eval", (PyCFunction)(void (*)(void))conv_bn_eval, METH_FASTCALL, "convolution, batch norm of running statistics, residual, ReLU, pool"},
-    {"bn_eval", (PyCFunction)(void (*)(void))bn_eval, METH_FASTCALL, "batch norm of running statistics, residual, ReLU"},
-    {"absmax", (PyCFunction)(void (*)(void))absmax, METH_FASTCALL, "largest magnitude"},
-    {"classify", (PyCFunction)(void (*)(void))classify, METH_FASTCALL, "logits of a feature map in inference"},
-    {"logit_metrics", (PyCFunction)(void (*)(void))logit_metrics, METH_FASTCALL, "cross-entropy, top-1 and top-5 of logits"},
-    {"quantize", (PyCFunction)(void (*)(void))quantize, METH_FASTCALL, "levels of a vector"},
-    {"quantize_fit", (PyCFunction)(void (*)(void))quantize_fit, METH_FASTCALL, "levels of the higher scale and where they fit the lower one"},
-    {"dequantize", (PyCFunction)(void (*)(void))dequantize, METH_FASTCALL, "values of levels of one or two scales"},
+    {"solo_maxnorm", method<solo_maxnorm>(), METH_FASTCALL, "QSGD-MaxNorm reduce of a single worker"},
+    {"solo_copy", method<solo_copy>(), METH_FASTCALL, "plain mean of a single worker"},
+    {"collect", method<collect_py>(), METH_FASTCALL, "reads two lists of tensors into a plan"},
+    {"solo_randk", method<solo_randk>(), METH_FASTCALL, "Rand-K reduce of a single worker"},
+    {"solo_randk_limit", method<solo_randk_limit>(), METH_FASTCALL, "most coordinates solo_randk takes"},
+    {"solo_psgd", method<solo_psgd>(), METH_FASTCALL, "PowerSGD step of a single worker"},
+    {"solo_topk", method<solo_topk>(), METH_FASTCALL, "top-k with error feedback of a single worker"},
+    {"conv_bn_eval", method<conv_bn_eval>(), METH_FASTCALL, "convolution, batch norm of running statistics, residual, ReLU, pool"},
+    {"bn_eval", method<bn_eval>(), METH_FASTCALL, "batch norm of running statistics, residual, ReLU"},
+    {"absmax", method<absmax>(), METH_FASTCALL, "largest magnitude"},
+    {"classify", method<classify>(), METH_FASTCALL, "logits of a feature map in inference"},
+    {"logit_metrics", method<logit_metrics>(), METH_FASTCALL, "cross-entropy, top-1 and top-5 of logits"},
+    {"quantize", method<quantize>(), METH_FASTCALL, "levels of a vector"},
+    {"quantize_fit", method<quantize_fit>(), METH_FASTCALL, "levels of the higher scale and where they fit the lower one"},
+    {"dequantize", method<dequantize>(), METH_FASTCALL, "values of levels of one or two scales"},
     {nullptr, nullptr, 0, nullptr}};
 
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "gcb200_ext", "native front end of the reducers", -1, methods};
