@@ -13,6 +13,7 @@
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
+#include <torch/csrc/jit/frontend/tracer.h>
 #include <torch/csrc/utils/object_ptr.h>
 
 #include <algorithm>
@@ -425,10 +426,17 @@ PyObject* dequantize(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
 }
 
 // ---- inference ---------------------------------------------------------------------------------------------------
+// Whether an operator is expected to leave a trace of itself that these calls do not: a tangent of forward-mode differentiation, a
+// node of a graph being traced, a functorch transform.  The general path says that it has none.
+bool observed(const at::Tensor& t) {
+  constexpr c10::DispatchKeySet wrapped({c10::DispatchKey::FuncTorchBatched, c10::DispatchKey::FuncTorchGradWrapper, c10::DispatchKey::Functionalize});
+  return t._fw_grad(0).defined() || t.key_set().has_any(wrapped) || torch::jit::tracer::isTracing();
+}
+
 // A dense fp32 CUDA activation in channels-last memory order, 16-byte aligned.
 const at::Tensor* activation(PyObject* o) {
   const at::Tensor* t = tensor_of(o);
-  return t && t->is_cuda() && t->scalar_type() == at::kFloat && t->dim() == 4 && t->numel() > 0 && t->is_contiguous(at::MemoryFormat::ChannelsLast) &&
+  return t && !observed(*t) && t->is_cuda() && t->scalar_type() == at::kFloat && t->dim() == 4 && t->numel() > 0 && t->is_contiguous(at::MemoryFormat::ChannelsLast) &&
                  ((uintptr_t)t->data_ptr() & 15u) == 0
              ? t
              : nullptr;
@@ -504,7 +512,7 @@ PyObject* classify(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
 PyObject* logit_metrics(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   if (!want(nargs, 2, "logit_metrics")) return nullptr;
   const at::Tensor *z = tensor_of(a[0]), *y = tensor_of(a[1]);
-  if (!z || !y || !z->is_cuda() || z->scalar_type() != at::kFloat || z->dim() != 2 || !z->is_contiguous() || y->scalar_type() != at::kLong ||
+  if (!z || !y || observed(*z) || !z->is_cuda() || z->scalar_type() != at::kFloat || z->dim() != 2 || !z->is_contiguous() || y->scalar_type() != at::kLong ||
       y->dim() != 1 || !y->is_contiguous() || y->device() != z->device() || y->size(0) != z->size(0))
     Py_RETURN_NONE;
   // one block: up to a quarter of a million samples, as many classes as torch.topk(5) needs at least

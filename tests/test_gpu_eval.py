@@ -182,3 +182,30 @@ def test_switches_act_in_inference_as_in_training(mode, cin, r, stride, training
     every = {"gemm", "conv", "stem", "dgrad_s2"}
     assert not on_cudnn() and not on_cudnn(PATHS={mode}) and not on_cudnn(MIN_ROWS=rows)
     assert on_cudnn(PATHS=every - {mode}) and on_cudnn(MIN_ROWS=rows + 1) and on_cudnn(ENABLED=False)
+
+
+@pytest.mark.parametrize("name", ["ResNet18", "MobileNetV2"])
+@pytest.mark.filterwarnings("ignore")
+@pytest.mark.parametrize("transform", ["forward AD", "vmap", "trace"])
+def test_transforms_the_kernels_know_nothing_of_are_refused(name, transform):
+    """No tangent dropped, no result baked into a graph: the layers' general path refuses these."""
+    import torch.autograd.forward_ad as fwad
+
+    from gradient_compression_b200 import models
+
+    torch.manual_seed(1)
+    model = getattr(models, name)().cuda().to(memory_format=torch.channels_last).eval()
+    x = torch.randn(2, 3, 32, 32, device="cuda").contiguous(memory_format=torch.channels_last)
+    with torch.no_grad(), pytest.raises((RuntimeError, TypeError)):        # (NotImplementedError is a RuntimeError)
+        if transform == "forward AD":
+            with fwad.dual_level():
+                model(fwad.make_dual(x, torch.ones_like(x)))
+        elif transform == "vmap":
+            torch.func.vmap(model)(x[:, None])
+        else:
+            traced = torch.jit.trace(model, x, check_trace=False)
+            other = torch.randn_like(x)
+            assert float((traced(other) - model(other)).norm()) < 1e-3 * float(model(other).norm())
+            raise RuntimeError("traced, and follows its input")
+    with torch.no_grad():
+        assert torch.isfinite(model(x)).all()
