@@ -206,10 +206,35 @@ PyObject* entry(PyObject* self, PyObject* const* a, Py_ssize_t n) {
 template <PyObject* (*F)(PyObject*, PyObject* const*, Py_ssize_t)>
 PyCFunction method() { return (PyCFunction)(void (*)(void))entry<F>; }
 
+// Allocations and launches run without the interpreter lock: either may wait for the GPU (a full launch queue, an allocator that
+// synchronises), and what the GPU waits for may be another thread's next launch.
+struct NoGil {
+  PyThreadState* const state = PyEval_SaveThread();
+  NoGil() = default;
+  NoGil(const NoGil&) = delete;
+  ~NoGil() { PyEval_RestoreThread(state); }
+};
+template <class F>
+auto unlocked(F f) {
+  const NoGil released;
+  return f();
+}
+
 PyObject* cuda_error(const char* what, int err) {
   PyErr_Format(PyExc_RuntimeError, "%s: CUDA error %d", what, err);
   return nullptr;
 }
+
+// A launch's own copy of a plan's tensors: the plan may be filled again while the lock is released.
+struct Tensors {
+  const std::vector<SegDesc> segs;
+  const int64_t n;
+  const int device;
+  explicit Tensors(const Plan& p) : segs(p.segs), n(p.n), device(p.device) {}
+  const void* data() const { return segs.data(); }
+  int count() const { return (int)segs.size(); }
+  void* stream() const { return stream_on(device); }
+};
 
 int64_t as_int(PyObject* o) { return PyLong_AsLongLong(o); }
 
@@ -232,9 +257,10 @@ PyObject* solo_maxnorm(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   const uint32_t step = (uint32_t)PyLong_AsUnsignedLongLongMask(a[7]);
   if (PyErr_Occurred()) return nullptr;
   c10::cuda::OptionalCUDAGuard guard(c10::Device(c10::kCUDA, (c10::DeviceIndex)p->device));
-  const int err = api.solo_maxnorm(ctx, p->segs.data(), (int)p->segs.size(), p->n, lo, hi, seed, step, timeout, blocks, stream_on(p->device));
+  const Tensors t(*p);
+  const int err = unlocked([&] { return api.solo_maxnorm(ctx, t.data(), t.count(), t.n, lo, hi, seed, step, timeout, blocks, t.stream()); });
   if (err) return cuda_error("solo_maxnorm", err);
-  return PyLong_FromLongLong(p->n);
+  return PyLong_FromLongLong(t.n);
 }
 
 // solo_copy(plan, ctx, grad_in, grad_out) -> elements, or None
@@ -249,8 +275,10 @@ PyObject* solo_copy(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   for (const SegDesc& s : p->segs) moves = moves || s.in != s.out;
   if (moves) {
     c10::cuda::OptionalCUDAGuard guard(c10::Device(c10::kCUDA, (c10::DeviceIndex)p->device));
-    const int err = api.solo_copy(ctx, p->segs.data(), (int)p->segs.size(), p->n, stream_on(p->device));
+    const Tensors t(*p);
+    const int err = unlocked([&] { return api.solo_copy(ctx, t.data(), t.count(), t.n, t.stream()); });
     if (err) return cuda_error("solo_copy", err);
+    return PyLong_FromLongLong(t.n);
   }
   return PyLong_FromLongLong(p->n);
 }
@@ -287,8 +315,10 @@ PyObject* solo_randk(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   const int lo = (int)as_int(a[7]), hi = (int)as_int(a[8]), zero = (int)as_int(a[9]), timeout = (int)as_int(a[11]), blocks = (int)as_int(a[12]);
   if (PyErr_Occurred()) return nullptr;
   c10::cuda::OptionalCUDAGuard guard(c10::Device(c10::kCUDA, (c10::DeviceIndex)p->device));
-  const int err = api.solo_randk(ctx, p->segs.data(), (int)p->segs.size(), p->n, seed, npass, start, k, window, lo, hi, zero, step, timeout, blocks,
-                                 stream_on(p->device));
+  const Tensors t(*p);
+  const int err = unlocked([&] {
+    return api.solo_randk(ctx, t.data(), t.count(), t.n, seed, npass, start, k, window, lo, hi, zero, step, timeout, blocks, t.stream());
+  });
   if (err) return cuda_error("solo_randk", err);
   Py_RETURN_NONE;
 }
@@ -312,9 +342,11 @@ PyObject* solo_psgd(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   for (int i = 1; i < 16; ++i) v[i] = i == 13 ? PyLong_AsUnsignedLongLongMask(a[i + 1]) : PyLong_AsUnsignedLongLong(a[i + 1]);
   if (PyErr_Occurred()) return nullptr;
   c10::cuda::OptionalCUDAGuard guard(c10::Device(c10::kCUDA, (c10::DeviceIndex)p->device));
-  const int err = api.psgd_solo(rank, p->segs.data(), (int)p->segs.size(), (float*)v[1], (const int64_t*)v[2], (int)v[3], (int64_t)v[4], (int64_t)v[5], (int)v[6],
-                                (const int64_t*)v[7], (int)v[8], (float*)v[9], (float*)v[10], (float*)v[11], (int64_t)v[12], v[13], (uint32_t)v[14],
-                                (uint32_t*)v[15], stream_on(p->device));
+  const Tensors t(*p);
+  const int err = unlocked([&] {
+    return api.psgd_solo(rank, t.data(), t.count(), (float*)v[1], (const int64_t*)v[2], (int)v[3], (int64_t)v[4], (int64_t)v[5], (int)v[6], (const int64_t*)v[7],
+                         (int)v[8], (float*)v[9], (float*)v[10], (float*)v[11], (int64_t)v[12], v[13], (uint32_t)v[14], (uint32_t*)v[15], t.stream());
+  });
   if (err) return cuda_error("solo_psgd", err);
   Py_RETURN_NONE;
 }
@@ -328,8 +360,10 @@ PyObject* solo_topk(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   for (int i = 1; i < 6; ++i) v[i] = PyLong_AsUnsignedLongLong(a[i]);
   if (PyErr_Occurred()) return nullptr;
   c10::cuda::OptionalCUDAGuard guard(c10::Device(c10::kCUDA, (c10::DeviceIndex)p->device));
-  const int err = api.topk_run(p->segs.data(), (int)p->segs.size(), p->n, (const int64_t*)v[1], (int)v[2], (float*)v[3], (void*)v[4], (void*)v[5], nullptr,
-                               nullptr, stream_on(p->device));
+  const Tensors t(*p);
+  const int err = unlocked([&] {
+    return api.topk_run(t.data(), t.count(), t.n, (const int64_t*)v[1], (int)v[2], (float*)v[3], (void*)v[4], (void*)v[5], nullptr, nullptr, t.stream());
+  });
   if (err) return cuda_error("solo_topk", err);
   Py_RETURN_NONE;
 }
@@ -358,8 +392,12 @@ PyObject* absmax(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   c10::cuda::OptionalCUDAGuard guard(x->device());
   static at::Tensor scratch[64];           // zeroed once; the kernel leaves it ready for the next call
   if (!scratch[dev].defined()) scratch[dev] = at::zeros({api.absmax_scratch_bytes()}, x->options().dtype(at::kByte));
-  at::Tensor out = given ? *given : at::empty({1}, x->options());
-  const int err = api.absmax((const float*)x->data_ptr(), x->numel(), scratch[dev].data_ptr(), (float*)out.data_ptr(), stream_on(dev));
+  void* words = scratch[dev].data_ptr();
+  at::Tensor out;
+  const int err = unlocked([&] {
+    out = given ? *given : at::empty({1}, x->options());
+    return api.absmax((const float*)x->data_ptr(), x->numel(), words, (float*)out.data_ptr(), stream_on(dev));
+  });
   if (err) return cuda_error("absmax", err);
   return THPVariable_Wrap(out);
 }
@@ -375,9 +413,12 @@ PyObject* quantize(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   if (PyErr_Occurred()) return nullptr;
   if (given && (!given->is_cuda() || !given->is_contiguous() || given->device() != x->device() || level_size(given->scalar_type()) != size)) Py_RETURN_NONE;
   c10::cuda::OptionalCUDAGuard guard(x->device());
-  at::Tensor out = given ? *given : at::empty({x->numel()}, x->options().dtype(level_type(size)));
-  const int err = api.quantize((const float*)x->data_ptr(), x->numel(), (const float*)norm->data_ptr(), (int)s, (int)mode, seed, stream, step, out.data_ptr(),
-                               (int)size, stream_on(x->device().index()));
+  at::Tensor out;
+  const int err = unlocked([&] {
+    out = given ? *given : at::empty({x->numel()}, x->options().dtype(level_type(size)));
+    return api.quantize((const float*)x->data_ptr(), x->numel(), (const float*)norm->data_ptr(), (int)s, (int)mode, seed, stream, step, out.data_ptr(), (int)size,
+                        stream_on(x->device().index()));
+  });
   if (err) return cuda_error("quantize_levels", err);
   return THPVariable_Wrap(out);
 }
@@ -392,9 +433,13 @@ PyObject* quantize_fit(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   if (PyErr_Occurred()) return nullptr;
   if (!x || !norm || norm->numel() != 1 || norm->device() != x->device() || x->numel() == 0 || s >= (1 << 22)) Py_RETURN_NONE;
   c10::cuda::OptionalCUDAGuard guard(x->device());
-  at::Tensor out = at::empty({x->numel()}, x->options().dtype(level_type(size))), mask = at::empty({x->numel()}, x->options().dtype(at::kChar));
-  const int err = api.quantize_fit((const float*)x->data_ptr(), x->numel(), (const float*)norm->data_ptr(), (int)s, (int)fit, seed, stream, step,
-                                   out.data_ptr(), (int)size, (int8_t*)mask.data_ptr(), stream_on(x->device().index()));
+  at::Tensor out, mask;
+  const int err = unlocked([&] {
+    out = at::empty({x->numel()}, x->options().dtype(level_type(size)));
+    mask = at::empty({x->numel()}, x->options().dtype(at::kChar));
+    return api.quantize_fit((const float*)x->data_ptr(), x->numel(), (const float*)norm->data_ptr(), (int)s, (int)fit, seed, stream, step, out.data_ptr(),
+                            (int)size, (int8_t*)mask.data_ptr(), stream_on(x->device().index()));
+  });
   if (err) return cuda_error("quantize_fit", err);
   PyObject *po = THPVariable_Wrap(out), *pm = THPVariable_Wrap(mask);
   PyObject* r = PyTuple_Pack(2, po, pm);
@@ -415,12 +460,15 @@ PyObject* dequantize(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
       (a[6] != Py_None && (!given || given->numel() != q->numel() || given->device() != q->device())))
     Py_RETURN_NONE;
   c10::cuda::OptionalCUDAGuard guard(q->device());
-  at::Tensor out = given ? *given : at::empty({q->numel()}, norm->options());
-  const int size = level_size(q->scalar_type());
-  void* st = stream_on(q->device().index());
-  const int err = mask ? api.dequantize_two(q->data_ptr(), size, (const int8_t*)mask->data_ptr(), q->numel(), (const float*)norm->data_ptr(), (int)s, (int)other,
-                                            (int)world, (float*)out.data_ptr(), st)
-                       : api.dequantize(q->data_ptr(), size, q->numel(), (const float*)norm->data_ptr(), (int)s, (int)world, (float*)out.data_ptr(), st);
+  at::Tensor out;
+  const int err = unlocked([&] {
+    out = given ? *given : at::empty({q->numel()}, norm->options());
+    const int size = level_size(q->scalar_type());
+    void* st = stream_on(q->device().index());
+    return mask ? api.dequantize_two(q->data_ptr(), size, (const int8_t*)mask->data_ptr(), q->numel(), (const float*)norm->data_ptr(), (int)s, (int)other, (int)world,
+                                     (float*)out.data_ptr(), st)
+                : api.dequantize(q->data_ptr(), size, q->numel(), (const float*)norm->data_ptr(), (int)s, (int)world, (float*)out.data_ptr(), st);
+  });
   if (err) return cuda_error("dequantize_levels", err);
   return THPVariable_Wrap(out);
 }
@@ -473,20 +521,23 @@ PyObject* conv_bn_eval(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   const int64_t floats = api.conv_bn_eval_scratch((int)n, (int)h, (int)wd, (int)cin, (int)cout, (int)r, stride, pad);
   if (floats < 0) Py_RETURN_NONE;
   c10::cuda::OptionalCUDAGuard guard(x->device());
-  at::Tensor y = like_activation(*x, n, cout, ho, wo), scratch;
-  if (floats) scratch = at::empty({floats}, x->options());
-  void* st = stream_on(x->device().index());
-  int err = api.conv_bn_eval((const float*)x->data_ptr(), (const float*)w->data_ptr(), (float*)y.data_ptr(), cbias, (int)n, (int)h, (int)wd, (int)cin,
-                             (int)cout, (int)r, stride, pad, gamma, beta, mean, var, (float)eps, res ? (const float*)res->data_ptr() : nullptr, relu,
-                             floats ? (float*)scratch.data_ptr() : nullptr, flag, st);
-  if (err) return cuda_error("conv_bn_eval", err);
-  if (pool) {
-    at::Tensor p = like_activation(*x, n, cout, ho / 2, wo / 2);
-    err = api.max_pool2((const float*)y.data_ptr(), (int)n, (int)ho, (int)wo, (int)cout, (float*)p.data_ptr(), st);
-    if (err) return cuda_error("max_pool2", err);
-    y = p;
-  }
-  return THPVariable_Wrap(y);
+  at::Tensor y, pooled;
+  const char* what = "conv_bn_eval";
+  const int err = unlocked([&] {
+    y = like_activation(*x, n, cout, ho, wo);
+    at::Tensor scratch;
+    if (floats) scratch = at::empty({floats}, x->options());
+    void* st = stream_on(x->device().index());
+    const int e = api.conv_bn_eval((const float*)x->data_ptr(), (const float*)w->data_ptr(), (float*)y.data_ptr(), cbias, (int)n, (int)h, (int)wd, (int)cin,
+                                   (int)cout, (int)r, stride, pad, gamma, beta, mean, var, (float)eps, res ? (const float*)res->data_ptr() : nullptr, relu,
+                                   floats ? (float*)scratch.data_ptr() : nullptr, flag, st);
+    if (e || !pool) return e;
+    what = "max_pool2";
+    pooled = like_activation(*x, n, cout, ho / 2, wo / 2);
+    return api.max_pool2((const float*)y.data_ptr(), (int)n, (int)ho, (int)wo, (int)cout, (float*)pooled.data_ptr(), st);
+  });
+  if (err) return cuda_error(what, err);
+  return THPVariable_Wrap(pool ? pooled : y);
 }
 
 // classify(feature map, weight, bias or None) -> logits of the mean over the map, or None
@@ -501,9 +552,12 @@ PyObject* classify(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   if ((a[2] != Py_None && !bias) || n < 1 || n > INT32_MAX || c < 4 || c & 3 || c > 4096 || positions < 1 || positions > INT32_MAX || k < 1 || k > 32)
     Py_RETURN_NONE;
   c10::cuda::OptionalCUDAGuard guard(x->device());
-  at::Tensor logits = at::empty({n, k}, x->options().memory_format(at::MemoryFormat::Contiguous));
-  const int err = api.head_eval((const float*)x->data_ptr(), (int)n, (int)positions, (int)c, (const float*)w->data_ptr(), bias, (int)k,
-                                (float*)logits.data_ptr(), stream_on(x->device().index()));
+  at::Tensor logits;
+  const int err = unlocked([&] {
+    logits = at::empty({n, k}, x->options().memory_format(at::MemoryFormat::Contiguous));
+    return api.head_eval((const float*)x->data_ptr(), (int)n, (int)positions, (int)c, (const float*)w->data_ptr(), bias, (int)k, (float*)logits.data_ptr(),
+                         stream_on(x->device().index()));
+  });
   if (err) return cuda_error("classify", err);
   return THPVariable_Wrap(logits);
 }
@@ -519,9 +573,11 @@ PyObject* logit_metrics(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   const int64_t n = z->size(0), k = z->size(1);
   if (n < 1 || n > (1 << 18) || k < 5 || k > 1024 || n * k > (1 << 22)) Py_RETURN_NONE;
   c10::cuda::OptionalCUDAGuard guard(z->device());
-  at::Tensor out = at::empty({3}, z->options());
-  const int err = api.logit_metrics((const float*)z->data_ptr(), (const int64_t*)y->data_ptr(), (int)n, (int)k, (float*)out.data_ptr(),
-                                    stream_on(z->device().index()));
+  at::Tensor out;
+  const int err = unlocked([&] {
+    out = at::empty({3}, z->options());
+    return api.logit_metrics((const float*)z->data_ptr(), (const int64_t*)y->data_ptr(), (int)n, (int)k, (float*)out.data_ptr(), stream_on(z->device().index()));
+  });
   if (err) return cuda_error("logit_metrics", err);
   PyObject* t = PyTuple_New(3);
   for (int i = 0; t && i < 3; ++i) PyTuple_SET_ITEM(t, i, THPVariable_Wrap(out.select(0, i)));
@@ -540,9 +596,12 @@ PyObject* bn_eval(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   if (PyErr_Occurred()) return nullptr;
   if (!gamma || !beta || !mean || !var || !api.bn_supported(m, (int)c)) Py_RETURN_NONE;
   c10::cuda::OptionalCUDAGuard guard(x->device());
-  at::Tensor y = like_activation(*x, x->size(0), c, x->size(2), x->size(3));
-  const int err = api.bn_eval_apply((const float*)x->data_ptr(), m, (int)c, mean, var, (float)eps, gamma, beta, res ? (const float*)res->data_ptr() : nullptr,
-                                    relu, (float*)y.data_ptr(), stream_on(x->device().index()));
+  at::Tensor y;
+  const int err = unlocked([&] {
+    y = like_activation(*x, x->size(0), c, x->size(2), x->size(3));
+    return api.bn_eval_apply((const float*)x->data_ptr(), m, (int)c, mean, var, (float)eps, gamma, beta, res ? (const float*)res->data_ptr() : nullptr, relu,
+                             (float*)y.data_ptr(), stream_on(x->device().index()));
+  });
   if (err) return cuda_error("bn_eval", err);
   return THPVariable_Wrap(y);
 }

@@ -36,3 +36,38 @@ def test_out_of_memory_is_raised():
     finally:
         torch.cuda.set_per_process_memory_fraction(1.0)
     assert int(ops.quantize_levels(x, norm, 255).abs().max()) == 255
+
+
+@pytest.mark.gpu
+def test_other_threads_run_while_a_launch_waits():
+    """A thousand launches behind a busy stream fill its queue, and the next one waits: not with the interpreter lock held."""
+    import threading
+    import time
+
+    from gradient_compression_b200 import ops
+
+    x, norm = torch.randn(64, device="cuda"), torch.ones(1, device="cuda")
+    out = torch.empty(64, dtype=torch.int8, device="cuda")
+    ops.quantize_levels(x, norm, 7, out=out)
+    torch.cuda.synchronize()
+    longest, stop = [0.0], threading.Event()
+
+    def tick():
+        last = time.perf_counter()
+        while not stop.is_set():
+            time.sleep(0.001)
+            now = time.perf_counter()
+            longest[0], last = max(longest[0], now - last), now
+
+    thread = threading.Thread(target=tick)
+    thread.start()
+    torch.cuda._sleep(1_000_000_000)                # about half a second
+    start = time.perf_counter()
+    for _ in range(4000):
+        ops.quantize_levels(x, norm, 7, out=out)
+    took = time.perf_counter() - start
+    stop.set()
+    thread.join()
+    torch.cuda.synchronize()
+    assert took > 0.2, "the queue never filled up"
+    assert longest[0] < 0.5 * took
