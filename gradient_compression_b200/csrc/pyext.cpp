@@ -236,7 +236,17 @@ struct Tensors {
   void* stream() const { return stream_on(device); }
 };
 
-int64_t as_int(PyObject* o) { return PyLong_AsLongLong(o); }
+// Counts and scales come as any number, as int() takes them.
+int64_t as_int(PyObject* o) {
+  if (PyLong_Check(o)) return PyLong_AsLongLong(o);
+  THPObjectPtr i(PyNumber_Long(o));
+  return i ? PyLong_AsLongLong(i.get()) : -1;
+}
+uint64_t as_bits(PyObject* o) {            // modulo 2^64
+  if (PyLong_Check(o)) return PyLong_AsUnsignedLongLongMask(o);
+  THPObjectPtr i(PyNumber_Long(o));
+  return i ? PyLong_AsUnsignedLongLongMask(i.get()) : 0;
+}
 
 bool want(Py_ssize_t nargs, Py_ssize_t n, const char* name) {
   if (nargs == n) return true;
@@ -408,9 +418,10 @@ PyObject* quantize(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   const at::Tensor *x = plain(a[0], at::kFloat), *norm = plain(a[1], at::kFloat), *given = a[8] == Py_None ? nullptr : tensor_of(a[8]);
   if (!x || !norm || norm->numel() != 1 || norm->device() != x->device() || x->numel() == 0) Py_RETURN_NONE;
   const int64_t s = as_int(a[2]), mode = as_int(a[3]), size = as_int(a[7]);
-  const uint64_t seed = PyLong_AsUnsignedLongLongMask(a[4]);
-  const uint32_t stream = (uint32_t)PyLong_AsUnsignedLongLongMask(a[5]), step = (uint32_t)PyLong_AsUnsignedLongLongMask(a[6]);
+  const uint64_t seed = as_bits(a[4]);
+  const uint32_t stream = (uint32_t)as_bits(a[5]), step = (uint32_t)as_bits(a[6]);
   if (PyErr_Occurred()) return nullptr;
+  if (size != 1 && size != 2 && size != 4) Py_RETURN_NONE;
   if (given && (!given->is_cuda() || !given->is_contiguous() || given->device() != x->device() || level_size(given->scalar_type()) != size)) Py_RETURN_NONE;
   c10::cuda::OptionalCUDAGuard guard(x->device());
   at::Tensor out;
@@ -428,8 +439,8 @@ PyObject* quantize_fit(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   if (!want(nargs, 8, "quantize_fit")) return nullptr;
   const at::Tensor *x = plain(a[0], at::kFloat), *norm = plain(a[1], at::kFloat);
   const int64_t s = as_int(a[2]), fit = as_int(a[3]), size = as_int(a[7]);
-  const uint64_t seed = PyLong_AsUnsignedLongLongMask(a[4]);
-  const uint32_t stream = (uint32_t)PyLong_AsUnsignedLongLongMask(a[5]), step = (uint32_t)PyLong_AsUnsignedLongLongMask(a[6]);
+  const uint64_t seed = as_bits(a[4]);
+  const uint32_t stream = (uint32_t)as_bits(a[5]), step = (uint32_t)as_bits(a[6]);
   if (PyErr_Occurred()) return nullptr;
   if (!x || !norm || norm->numel() != 1 || norm->device() != x->device() || x->numel() == 0 || s >= (1 << 22)) Py_RETURN_NONE;
   c10::cuda::OptionalCUDAGuard guard(x->device());

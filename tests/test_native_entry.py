@@ -71,3 +71,18 @@ def test_other_threads_run_while_a_launch_waits():
     torch.cuda.synchronize()
     assert took > 0.2, "the queue never filled up"
     assert longest[0] < 0.5 * took
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("number", [float, int, __import__("numpy").float64, __import__("numpy").int32, torch.tensor])
+def test_scales_and_seeds_of_any_number_type(number):
+    from gradient_compression_b200 import ops
+
+    x, norm = torch.randn(1000, device="cuda"), torch.full((1,), 3.0, device="cuda")
+    want = ops.quantize_levels(x.cpu(), 3.0, 7, 5, 9, 2)
+    got = ops.quantize_levels(x, norm, number(7), number(5), number(9), number(2), dtype=torch.int8)
+    assert got.dtype == torch.int8 and torch.equal(got.cpu().to(torch.int32), want)
+    assert torch.equal(ops.dequantize_levels(got, norm, number(7), number(2)).cpu(), ops.dequantize_levels(want, 3.0, 7, 2))
+    q, mask = ops.quantize_fit(x, norm, number(7), number(3), number(5), number(9), number(2))
+    assert torch.equal(q.cpu(), want) and torch.equal(mask.cpu(), (want.abs() <= 3).to(torch.int8))
+    assert torch.equal(ops.quantize_levels(x, norm, 7, 5, 9, 2, dtype=torch.uint8).view(torch.int8), got)        # a container of one byte
