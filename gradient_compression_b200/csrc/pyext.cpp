@@ -398,7 +398,7 @@ PyObject* absmax(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   const at::Tensor* given = a[1] == Py_None ? nullptr : plain(a[1], at::kFloat);
   if (!x || x->numel() == 0 || (a[1] != Py_None && !given)) Py_RETURN_NONE;
   const int dev = x->device().index();
-  if (dev >= 64 || (given && given->device() != x->device())) Py_RETURN_NONE;
+  if (dev >= 64 || (given && (given->device() != x->device() || given->numel() < 1))) Py_RETURN_NONE;
   c10::cuda::OptionalCUDAGuard guard(x->device());
   static at::Tensor scratch[64];           // zeroed once; the kernel leaves it ready for the next call
   if (!scratch[dev].defined()) scratch[dev] = at::zeros({api.absmax_scratch_bytes()}, x->options().dtype(at::kByte));
@@ -422,7 +422,9 @@ PyObject* quantize(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   const uint32_t stream = (uint32_t)as_bits(a[5]), step = (uint32_t)as_bits(a[6]);
   if (PyErr_Occurred()) return nullptr;
   if (size != 1 && size != 2 && size != 4) Py_RETURN_NONE;
-  if (given && (!given->is_cuda() || !given->is_contiguous() || given->device() != x->device() || level_size(given->scalar_type()) != size)) Py_RETURN_NONE;
+  if (given && (!given->is_cuda() || !given->is_contiguous() || given->device() != x->device() || level_size(given->scalar_type()) != size ||
+                given->numel() < x->numel()))
+    Py_RETURN_NONE;
   c10::cuda::OptionalCUDAGuard guard(x->device());
   at::Tensor out;
   const int err = unlocked([&] {

@@ -40,6 +40,11 @@ def _absmax_scratch(device):
     return _scratch[key]
 
 
+def _room(out, n):
+    if out.numel() < n:
+        raise ValueError(f"out has {out.numel()} elements, {n} are written")
+
+
 def absmax(x, out=None):
     """max |x| as a 1-element fp32 tensor on x's device (NaN inputs give +inf).
 
@@ -53,6 +58,7 @@ def absmax(x, out=None):
     x = _flat32(x)
     if out is None:
         out = torch.zeros(1, dtype=torch.float32, device=x.device)
+    _room(out, 1)
     if x.numel() == 0:
         out.zero_()
         return out
@@ -86,6 +92,7 @@ def quantize_levels(x, norm, s, seed=0, stream=0, step=0, mode=MODE_STOCHASTIC, 
     n = x.numel()
     if out is None:
         out = torch.empty(n, dtype=dtype, device=x.device)
+    _room(out, n)
     if n == 0:
         return out
     if x.is_cuda:
@@ -114,6 +121,7 @@ def dequantize_levels(q, norm, s, world=1, out=None):
     n = q.numel()
     if out is None:
         out = torch.empty(n, dtype=torch.float32, device=q.device)
+    _room(out, n)
     if n == 0:
         return out
     if q.is_cuda:

@@ -86,3 +86,18 @@ def test_scales_and_seeds_of_any_number_type(number):
     q, mask = ops.quantize_fit(x, norm, number(7), number(3), number(5), number(9), number(2))
     assert torch.equal(q.cpu(), want) and torch.equal(mask.cpu(), (want.abs() <= 3).to(torch.int8))
     assert torch.equal(ops.quantize_levels(x, norm, 7, 5, 9, 2, dtype=torch.uint8).view(torch.int8), got)        # a container of one byte
+
+
+@pytest.mark.parametrize("device", ["cpu", pytest.param("cuda", marks=pytest.mark.gpu)])
+def test_results_that_do_not_fit_are_refused(device):
+    from gradient_compression_b200 import ops
+
+    x, norm = torch.randn(1000, device=device), torch.full((1,), 3.0, device=device)
+    q = ops.quantize_levels(x, norm, 7, out=torch.empty(1001, dtype=torch.int32, device=device))[:1000].contiguous()
+    with pytest.raises(ValueError):
+        ops.quantize_levels(x, norm, 7, out=torch.empty(999, dtype=torch.int32, device=device))
+    with pytest.raises(ValueError):
+        ops.dequantize_levels(q, norm, 7, out=torch.empty(999, device=device))
+    with pytest.raises(ValueError):
+        ops.absmax(x, torch.empty(0, device=device))
+    assert torch.equal(ops.dequantize_levels(q, norm, 7, out=torch.empty(1000, device=device)), ops.dequantize_levels(q, norm, 7))
