@@ -419,15 +419,45 @@ __global__ void __launch_bounds__(THREADS, 1) topk_split_kernel(const __grid_con
   if (g >= 0) flush(g);
 }
 
-// Entries equal to the threshold that are ordered by index before some of them are taken, so that the selection does not depend on
-// how blocks run.  A few of a million random floats share a value; beyond these the order of arrival decides.
+// Of the entries equal to the threshold the first by index are taken, so that the selection does not depend on how blocks run.  Up to
+// this many of them (a few of a million random floats share a value) wait in shared memory and are ordered there; among more of them
+// the index of the last one taken is found as the threshold was, nine bits at a time: two or three more readings of the candidates.
 constexpr int TIES = 128;
 
-// One cluster of blocks per group; the blocks share the group's candidates and add their counts up in rank 0's shared memory.
+// What the blocks of a cluster count together, in rank 0's shared memory.
+struct Tally {
+  uint4 found;                             // the bin, how many of its entries are wanted, how many it has: one read of another block's memory
+  uint32_t hist[SUB_BINS], warp_sums[32];
+};
+
+// The bin of the rem-th entry that the blocks have counted, from the highest bin or from the lowest.  rem: how many entries of that bin
+// are wanted; same: how many it has.
+__device__ __forceinline__ uint32_t settle_bin(Tally& t, bool highest, int& rem, uint32_t& same) {
+  cg::cluster_group cluster = cg::this_cluster();
+  const unsigned rank = cluster.block_rank();
+  cluster.sync();
+  if (rank != 0 && threadIdx.x < SUB_BINS && t.hist[threadIdx.x]) atomicAdd(cluster.map_shared_rank(&t.hist[threadIdx.x], 0), t.hist[threadIdx.x]);
+  cluster.sync();
+  if (rank == 0) {
+    const int at = highest ? SUB_BINS - 1 - (int)threadIdx.x : (int)threadIdx.x;
+    const uint32_t mine = threadIdx.x < SUB_BINS ? t.hist[at] : 0u;
+    const uint32_t before = block_exclusive(mine, t.warp_sums);
+    if (before < (uint32_t)rem && before + mine >= (uint32_t)rem) t.found = make_uint4((uint32_t)at, (uint32_t)rem - before, mine, 0u);
+  }
+  cluster.sync();
+  const uint4 found = *cluster.map_shared_rank(&t.found, 0);
+  cluster.sync();
+  rem = (int)found.y;
+  same = found.z;
+  return found.x;
+}
+
+// One cluster of blocks per group; the blocks share the group's candidates and add their counts up in rank 0's shared memory.  Two blocks
+// an SM where there are many groups (the launch counts on them; ResNet-50's reduce 133.6 -> 129.3 us); a single group has 16 at most,
+// and is faster with the registers (77.4 against 79.6 us at 16 M elements).
 template <int CAP, bool LISTS>
-__global__ void __launch_bounds__(THREADS) topk_refine_kernel(const __grid_constant__ TopkParams<CAP> p) {
-  __shared__ uint32_t hist[SUB_BINS], warp_sums[32];
-  __shared__ int chosen, need;
+__global__ void __launch_bounds__(THREADS, CAP == 1 ? 1 : 2) topk_refine_kernel(const __grid_constant__ TopkParams<CAP> p) {
+  __shared__ Tally tally_of;
   __shared__ uint32_t equal_seen;
   __shared__ Cand ties[TIES];              // rank 0's: entries equal to the threshold
   cg::cluster_group cluster = cg::this_cluster();
@@ -444,7 +474,6 @@ __global__ void __launch_bounds__(THREADS) topk_refine_kernel(const __grid_const
   const int64_t count = listed ? (int64_t)in_bin : p.len(g);
   const int64_t from = (int64_t)rank * THREADS, stride = (int64_t)ranks * THREADS;
   const Cand* list = p.cands + p.room0[g];
-  // entry i of the list; without one, element i of the group
   auto entry = [&](int64_t i) {
     if (listed) return list[i];
     const int64_t at = lo + i;
@@ -453,11 +482,13 @@ __global__ void __launch_bounds__(THREADS) topk_refine_kernel(const __grid_const
     return Cand{t.in[s][at - t.start[s]], (int32_t)at};
   };
   auto in_it = [&](const Cand& c) { return listed || (int)(c.key() >> LOW_BITS) == bin; };
-  uint32_t prefix = 0;
-  int rem = k_rem;
+  uint32_t prefix = 0, same = 0;           // the threshold's low bits; entries equal to it
+  int rem = k_rem;                         // how many of them are taken
+  bool by_index = false;
   const bool all = (uint32_t)k_rem >= in_bin;
   if (threadIdx.x == 0) equal_seen = 0;
   if (!all) {
+    uint32_t* hist = tally_of.hist;
 #pragma unroll
     for (int part = 0; part < 2; ++part) {
       if (threadIdx.x < SUB_BINS) hist[threadIdx.x] = 0;
@@ -477,20 +508,10 @@ __global__ void __launch_bounds__(THREADS) topk_refine_kernel(const __grid_const
         const Cand c = entry(i);
         if (in_it(c)) tally(c);
       }
-      cluster.sync();
-      if (rank != 0 && threadIdx.x < SUB_BINS && hist[threadIdx.x]) atomicAdd(cluster.map_shared_rank(&hist[threadIdx.x], 0), hist[threadIdx.x]);
-      cluster.sync();
-      if (rank == 0) {
-        const uint32_t mine = threadIdx.x < SUB_BINS ? hist[SUB_BINS - 1 - threadIdx.x] : 0u;
-        const uint32_t above = block_exclusive(mine, warp_sums);
-        if (above < (uint32_t)rem && above + mine >= (uint32_t)rem) { chosen = SUB_BINS - 1 - threadIdx.x; need = rem - (int)above; }
-      }
-      cluster.sync();
-      const uint32_t got = (uint32_t)*cluster.map_shared_rank(&chosen, 0);
+      const uint32_t got = settle_bin(tally_of, true, rem, same);
       prefix = part == 0 ? got : (prefix << SUB_BITS) | got;
-      rem = *cluster.map_shared_rank(&need, 0);
-      cluster.sync();
     }
+    by_index = same > (uint32_t)TIES && same > (uint32_t)rem && (bin != 0 || prefix != 0);          // (zeros are all the same)
   } else {
     cluster.sync();
   }
@@ -508,10 +529,10 @@ __global__ void __launch_bounds__(THREADS) topk_refine_kernel(const __grid_const
     const bool valid = there && in_it(c), taken = there && !listed && (int)(c.key() >> LOW_BITS) > bin;
     const uint32_t low = c.key() & ((1u << LOW_BITS) - 1u);
     bool take = valid && (all || low > prefix);
-    if (valid && !all && low == prefix) {
+    if (valid && !all && low == prefix && !by_index) {
       const uint32_t at = atomicAdd(equal, 1u);
       if (at < (uint32_t)TIES) waiting[at] = c;
-      else take = (int)at < rem;
+      else take = (int)at < rem;           // (all of them are, or they are zeros)
     }
     place(c, take, taken);
   };
@@ -532,6 +553,29 @@ __global__ void __launch_bounds__(THREADS) topk_refine_kernel(const __grid_const
     int order = 0;
     for (int j = 0; j < n; ++j) order += ties[j].at < mine.at;
     place(mine, (int)threadIdx.x < n && order < rem, false);
+  }
+  if (!by_index) return;
+  // the index of the rem-th of the equal entries, nine bits at a time, and then all of them up to it
+  const uint32_t key = (uint32_t)bin << LOW_BITS | prefix;
+  uint32_t upper = 0;
+  int shift = 0;
+  while (p.len(g) >> (shift + SUB_BITS)) shift += SUB_BITS;
+#pragma unroll 1
+  for (; shift >= 0; shift -= SUB_BITS) {
+    if (threadIdx.x < SUB_BINS) tally_of.hist[threadIdx.x] = 0;
+    __syncthreads();
+#pragma unroll 1
+    for (int64_t i = from + threadIdx.x; i < count; i += stride) {
+      const Cand c = entry(i);
+      const uint32_t at = (uint32_t)(c.at - lo) >> shift;
+      if (c.key() == key && (at >> SUB_BITS) == upper) atomicAdd(&tally_of.hist[at & (SUB_BINS - 1)], 1u);
+    }
+    upper = (upper << SUB_BITS) | settle_bin(tally_of, false, rem, same);
+  }
+#pragma unroll 1
+  for (base = from; base < count; base += stride) {
+    const Cand c = base + threadIdx.x < count ? entry(base + threadIdx.x) : Cand{0.0f, 0};
+    place(c, base + threadIdx.x < count && c.key() == key && (uint32_t)(c.at - lo) <= upper, false);
   }
 }
 

@@ -267,3 +267,27 @@ def test_tensors_of_another_gpu_than_the_arenas_are_refused(name, config):
     assert bool((out == 5.0).all())
     red.reduce([x], [out])
     assert not bool((out == 5.0).any())
+
+
+@pytest.mark.parametrize("n", [4097, 5000, 200003, 3000001])
+@pytest.mark.parametrize("step", [1, 3, 16, 0])
+@pytest.mark.parametrize("dense", [False, True])
+def test_topk_any_number_of_ties_goes_to_the_first(n, step, dense):
+    """Values rounded to halves, sixths or thirty-seconds, and one value everywhere: from some hundred entries at the threshold to all of
+    them, on the candidate lists and beyond their room."""
+    from gradient_compression_b200.ops.topk import TopKSelector
+
+    gen = torch.Generator().manual_seed(n + step)
+    a = torch.round(torch.randn(n, generator=gen) * 2 * step) / (2 * step) if step else torch.full((n,), -0.375)
+    k = n // 30
+    want = torch.sort(a.abs(), descending=True, stable=True)[1][:k].sort()[0]
+    sel, x = TopKSelector([(0, n, k)], "cuda"), a.cuda()
+    for _ in range(2):
+        if dense:
+            red, out = make_reducer("GlobalTopKReducer", "cuda", None, {"K": k}), torch.empty_like(x)
+            red.reduce([x], [out])
+            got, expected = out.cpu(), torch.zeros(n)
+            expected[want] = a[want]
+            assert torch.equal(got, expected) and torch.equal(red.state_dict()["memory"].cpu(), a - expected)
+        else:
+            assert torch.equal(sel.select(x, None)[0].cpu().long().sort()[0], want)
