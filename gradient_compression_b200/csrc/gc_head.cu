@@ -12,7 +12,8 @@
 //   head_bwd_dw_kernel   dW[k, c] = g * sum_n dlogits[n, k] pooled[n, c], db[k] = g * sum_n dlogits[n, k]
 //   head_eval_kernel     inference: pooling and linear layer only (labels come later, with evaluate_predictions)
 //   logit_metrics_kernel cross-entropy, top-1 and top-5 of given logits, one block, one thread per sample: a dozen torch launches
-//                        took 66 of 470 microseconds of a small evaluation batch, and more of its host time
+//                        took 66 of 470 microseconds of a small evaluation batch, and more of its host time.  Bound by the latency of
+//                        rows read by a thread each, so for small batches or few classes (ops/head.py has the line and its figures)
 // g is the gradient that reaches the loss (a device scalar, 1 for a plain loss.backward()).
 #include <cuda_runtime.h>
 #include <stdint.h>

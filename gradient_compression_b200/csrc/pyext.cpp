@@ -582,7 +582,7 @@ PyObject* logit_metrics(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   if (!z || !y || observed(*z) || !z->is_cuda() || z->scalar_type() != at::kFloat || z->dim() != 2 || !z->is_contiguous() || y->scalar_type() != at::kLong ||
       y->dim() != 1 || !y->is_contiguous() || y->device() != z->device() || y->size(0) != z->size(0))
     Py_RETURN_NONE;
-  // one block: up to a quarter of a million samples, as many classes as torch.topk(5) needs at least
+  // what the kernel computes (top-5 needs five classes, as torch.topk does); where it is the faster way is the caller's rule
   const int64_t n = z->size(0), k = z->size(1);
   if (n < 1 || n > (1 << 18) || k < 5 || k > 1024 || n * k > (1 << 22)) Py_RETURN_NONE;
   c10::cuda::OptionalCUDAGuard guard(z->device());

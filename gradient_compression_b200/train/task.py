@@ -14,7 +14,7 @@ import torch.distributed as dist
 
 from .. import models
 from ..ops.bn import hooked
-from ..ops.head import logit_metrics
+from ..ops.head import logit_metrics, metrics_kernel_pays
 from ..parallel.arena import FlatArena
 from ..utils.metrics import AverageMeter
 from ..utils.timer import NullTimer
@@ -169,7 +169,7 @@ class CIFAR:
         """cross-entropy, top-1 and top-5 accuracy of a batch.  The loss computed by the forward pass
         is reused when given (the reference evaluates it a second time, model_dispatcher.py:157)."""
         with torch.no_grad():
-            known = logit_metrics(pred_labels, true_labels)
+            known = logit_metrics(pred_labels, true_labels) if pred_labels.is_cuda and metrics_kernel_pays(*pred_labels.shape) else None
             if known is not None:
                 ce, top1, top5 = known
                 if loss is not None or not self._plain_cross_entropy():

@@ -71,3 +71,20 @@ def test_a_classifier_with_hooks_is_called(name, what):
     loss, logits, _ = model.train().forward_loss(x, labels)
     loss.backward()
     assert torch.isfinite(loss) and (len(seen) == 2 if what == "forward hook" else float(linear.weight_orig.grad.abs().max()) > 0)
+
+
+@pytest.mark.parametrize("n,k,kernel", [(1, 5, True), (20000, 10, True), (4096, 16, True), (4097, 16, False), (1024, 64, True), (1025, 64, False),
+                                        (256, 256, True), (257, 256, False), (16, 257, False), (30, 1000, False)])
+def test_metrics_of_a_batch_on_both_sides_of_the_line(n, k, kernel):
+    from gradient_compression_b200.ops import _native as nat
+    from gradient_compression_b200.train import CIFAR
+
+    task = CIFAR("cuda", None, "LeNet", data="synthetic", synthetic_train_size=1, synthetic_test_size=1)
+    g = torch.Generator(device="cuda").manual_seed(n + k)
+    z, labels = torch.randn(n, k, device="cuda", generator=g) * 3, torch.randint(0, k, (n,), device="cuda", generator=g)
+    before = nat.launches()
+    got = task.evaluate_predictions(z, labels)
+    assert nat.launches() - before == kernel
+    hit = z.topk(5, 1, True, True)[1].eq(labels.view(-1, 1))
+    assert torch.allclose(got["cross_entropy_loss"].double(), F.cross_entropy(z.double(), labels), rtol=1e-6)
+    assert float(got["top1_accuracy"]) == float(hit[:, 0].float().sum() / n) and float(got["top5_accuracy"]) == float(hit.float().sum() / n)
