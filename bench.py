@@ -288,7 +288,7 @@ def run_ours(args, world, rank, local_rank):
                              "before the clock stops"}
     from gradient_compression_b200.ops import conv as conv_ops
     conv_path = ("own tcgen05 TF32 kernels (paths: %s; >= %d output positions) with BN statistics in the epilogue: forward, "
-                 "input gradient (stride 1) and weight gradient; input gradients of strided convolutions: cuDNN"
+                 "input gradient (stride 1 and 2) and weight gradient"
                  % (",".join(sorted(conv_ops.PATHS)), conv_ops.MIN_ROWS)) if conv_ops.ENABLED \
         else "cuDNN (torch); own tcgen05 paths off (GCB200_TC_CONV=0)"
     first = reducer.reducers[0] if hasattr(reducer, "reducers") else reducer

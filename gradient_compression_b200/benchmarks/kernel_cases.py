@@ -43,7 +43,15 @@ def case_qsgd(n, bits=8):
     red = R.QSGDMaxNormReducer("cuda", quantization_level=bits, seed=1, backend="fused")
     x = torch.randn(n, device="cuda") * 1e-3
     out = [torch.empty_like(x)]
-    return (lambda: red.reduce([x], out)), 4 * n * 3, "qsgd_fused_kernel (W=1): abs-max read + quantise read + dequantised write"
+    return (lambda: red.reduce([x], out)), 4 * n * 3, "solo_maxnorm_kernel: read for the norm, read again, dequantised write (kept tiles and L2 serve part of the second read)"
+
+
+def case_twoscale(n):
+    from .. import reducers as R
+    red = R.QSGDMaxNormTwoScaleReducer("cuda", lower_quantization_level=6, higher_quantization_level=10, seed=1)
+    x = torch.randn(n, device="cuda") * 1e-3
+    out = [torch.empty_like(x)]
+    return (lambda: red.reduce([x], out)), 4 * n * 3, "solo_maxnorm_kernel, two scales: read, read again, write"
 
 
 def case_absmax(n):
@@ -80,9 +88,7 @@ def _bn_tensors(n):
 def case_bn_fwd(n):
     from ..ops.bn import bn_act
     x, bn = _bn_tensors(n)
-    with torch.no_grad():
-        pass
-    return (lambda: bn_act(bn, x)), 4 * x.numel() * 3, "bn_stats + bn_apply (+ReLU): 2 reads, 1 write"
+    return (lambda: bn_act(bn, x)), 4 * x.numel() * 3, "bn_fused_fwd_kernel (statistics + apply + ReLU): 2 reads, 1 write"
 
 
 def case_bn_bwd(n):
@@ -95,15 +101,20 @@ def case_bn_bwd(n):
         y = bn_act(bn, x)
         y.backward(dy)
         x.grad = None
-    return run, 4 * x.numel() * (3 + 5), "bn fwd (3 passes) + bn_bwd_reduce + bn_bwd_apply (4 reads, 1 write)"
+    return run, 4 * x.numel() * (3 + 5), "bn_fused_fwd_kernel (2 reads, 1 write) + bn_fused_bwd_kernel (dy and x twice, 1 write)"
 
 
 def case_topk(n):
-    from ..ops.topk import TopKSelector
-    g = torch.randn(n, device="cuda")
-    e = torch.zeros(n, device="cuda")
-    sel = TopKSelector([(0, n, max(n // 100, 1))], "cuda")
-    return (lambda: sel.select(g, e)), 4 * n * 6, "topk: 3 histogram passes + compaction (pass 0 reads g, e and writes e)"
+    from .. import reducers as R
+    red = R.TopKReducerRatio("cuda", compression=0.01)
+    x = torch.randn(n, device="cuda") * 1e-3
+    out = [torch.empty_like(x)]
+
+    def run():
+        if red._memory is not None:
+            red._memory.zero_()               # the first step's values every time; 4 bytes an element of the time are this
+        red.reduce([x], out)
+    return run, 4 * n * 6, "topk_fold (reads g, e, writes e), topk_pick, topk_split (reads e, writes g), topk_refine; and the memory's reset"
 
 
 def case_psgd(n, rank=2):
@@ -112,12 +123,8 @@ def case_psgd(n, rank=2):
     grads = [torch.randn(s, device="cuda") * 1e-3 for s in shapes]
     red = R.RankKReducer("cuda", rank=rank, seed=1, backend="fused")
     tot = sum(g.numel() for g in grads)
-    flat = torch.cat([g.reshape(-1) for g in grads])
-    views, off = [], 0
-    for g in grads:
-        views.append(flat[off:off + g.numel()].view(g.shape))
-        off += g.numel()
-    return (lambda: red.reduce(views, views)), 4 * tot * 7, "psgd_p (2 reads, 1 write) + psgd_q (1 read) + psgd_out (1 read, 2 writes)"
+    outs = [torch.empty_like(g) for g in grads]
+    return (lambda: red.reduce(grads, outs)), 4 * tot * 7, "psgd_p (2 reads, 1 write) + psgd_gs + psgd_q (1 read) + psgd_out (1 read, 2 writes)"
 
 
 def case_gemm(n):
@@ -161,7 +168,7 @@ def case_gemm_deep(n):
     b = torch.randn(nn, k, device="cuda")
     out = torch.empty(m, nn, device="cuda")
     return (lambda: gemm.gemm_tf32(a, b, out=out)), 4 * (m * k + nn * k + m * nn), \
-        f"gemm_tf32_kernel: {2 * m * nn * k / 1e9:.0f} GFLOP"
+        f"gemm_tf32_persistent_kernel<256>, CTA pairs: {2 * m * nn * k / 1e9:.0f} GFLOP"
 
 
 def _conv_tensors(hw=16, c=128, batch=128):
@@ -191,7 +198,7 @@ def case_conv3x3_wgrad(n):
         f"gemm_tn_tf32_kernel, B from shifted 4-D TMA boxes: {2 * x.shape[0] * 256 * 128 * 1152 / 1e9:.2f} GFLOP"
 
 
-CASES = {"conv3x3": case_conv3x3, "conv3x3_wgrad": case_conv3x3_wgrad, "qsgd": case_qsgd, "absmax": case_absmax, "sgd": case_sgd, "pack": case_pack, "bn_fwd": case_bn_fwd,
+CASES = {"conv3x3": case_conv3x3, "conv3x3_wgrad": case_conv3x3_wgrad, "qsgd": case_qsgd, "twoscale": case_twoscale, "absmax": case_absmax, "sgd": case_sgd, "pack": case_pack, "bn_fwd": case_bn_fwd,
          "bn_bwd": case_bn_bwd, "topk": case_topk, "psgd": case_psgd, "gemm": case_gemm, "gemm_narrow": case_gemm_narrow, "gemm_tn": case_gemm_tn,
          "gemm_deep": case_gemm_deep}
 

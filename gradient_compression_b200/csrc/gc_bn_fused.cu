@@ -513,7 +513,7 @@ int gc_cuda_bn_fused_backward(const float* dy, const float* x, const float* y, i
   s.parts = (float*)((uint8_t*)scratch + sizeof(GroupSync));
   s.error_flag = error_flag;
   plan(s, sm_count());
-  // masks of as many row pairs as shared memory holds (192 KB: 98 K rows of 32 channels a block)
+  // masks of as many row pairs as shared memory holds (192 KB: 49 K rows of 32 channels a block)
   constexpr int most = 192;
   const int64_t pairs = (s.per + 2 * LANES - 1) / (2 * LANES);
   const int masks = y == nullptr || pool ? 0 : (int)(pairs < most ? pairs : most);

@@ -378,8 +378,7 @@ void gc_cuda_tc_split_config(int splits) { gctc::split_choice = splits; }
 // For measurements: CTA pairs of the persistent kernel (0 = modelled, 1 = never, 2 = wherever there are two row tiles).
 void gc_cuda_tc_pair_config(int pairs) { gctc::pair_choice = pairs; }
 
-// For measurements: how the producer warps issue their TMA loads (bit 0: prefetch the tensor maps; bit 1: spread the
-// loads of a stage over several lanes).
+// For measurements: bit 0: prefetch the tensor maps at kernel start; bit 2: epilogue warps sleep between polls of their barrier.
 void gc_cuda_tc_tma_mode(int mode) { gctc::tma_mode = mode; }
 
 // For measurements: CTAs per SM the split contraction aims at, and the fewest k-blocks (of 32 rows) a split may get.

@@ -464,7 +464,7 @@ __global__ void __launch_bounds__(256) psgd_q_kernel(const float* __restrict__ e
   }
 }
 
-// Sum of the row-chunk partials (only launched when some matrix has more than Q_ROWCHUNK rows).
+// Sum of the row-chunk partials (only launched when some matrix has more than MIN_CHUNK rows).
 __global__ void psgd_q_sum_kernel(float* q, const float* parts, int64_t q_total, int chunks) {
   int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < q_total; i += stride) {
