@@ -33,7 +33,7 @@ import torch
 
 from . import _native as nat
 from . import gemm
-from .bn import _cl, _fin_ptr, _scratch_for, bn_act, fused_backward, fused_forward, fused_ok, hooked, count_batch, own_grad, take_owned_grad
+from .bn import _FORWARD, _PRE, _cl, _fin_ptr, _scratch_for, bn_act, fused_backward, fused_forward, fused_ok, hooked, count_batch, own_grad, take_owned_grad
 
 # GCB200_TC_CONV=0 (or ``ENABLED = False``) keeps every convolution on cuDNN.
 ENABLED = os.environ.get("GCB200_TC_CONV", "1") == "1"
@@ -60,6 +60,7 @@ SMALL_BN_ELEMENTS = int(os.environ.get("GCB200_BN_SMALL_ELEMENTS", str(1 << 18))
 # stride-1 input gradients read the forward filter in place (MN-major B operand) instead of a rotated / transposed copy
 DGRAD_IN_PLACE = os.environ.get("GCB200_DGRAD_IN_PLACE", "1") == "1"
 PATHS = set(os.environ.get("GCB200_TC_CONV_PATHS", "gemm,conv,stem,dgrad_s2").split(","))
+_EVERY_MODE = frozenset(("gemm", "conv", "stem"))
 
 
 def _taps(w):
@@ -599,21 +600,24 @@ def _mode(conv, bn, x):
 
 def _eval(conv, bn, x, residual, relu, pool):
     """``conv_bn_act`` in inference: running statistics, nothing kept for a backward.  None: not a case for the kernels."""
-    # Parameters and buffers as the modules registered them (a module's attribute lookup walks through these dictionaries anyway).
-    # One that is computed instead -- pruning, weight or spectral normalisation -- has no such entry: the kernels decline.
-    own, params, stats = conv._parameters, bn._parameters, bn._buffers
-    w, k, s, p = own.get("weight"), conv.kernel_size, conv.stride, conv.padding
-    if (conv.groups != 1 or conv.dilation != (1, 1) or k[0] != k[1] or s[0] != s[1] or isinstance(p, str) or p[0] != p[1] or conv.padding_mode != "zeros"
-            or "bias" not in own or hooked(conv, bn) or not torch.backends.cudnn.allow_tf32):
+    # Everything is read from the modules' own dictionaries: attribute lookups on modules cost a ResNet-50 35 of 765 us of host time.  A parameter
+    # that is computed instead of registered -- pruning, weight or spectral normalisation -- has no entry: the kernels decline.
+    c, b = conv.__dict__, bn.__dict__
+    own, params, stats = c["_parameters"], b["_parameters"], b["_buffers"]
+    (r, r1), (stride, stride1), p, w = c["kernel_size"], c["stride"], c["padding"], own.get("weight")
+    if (c["groups"] != 1 or c["dilation"] != (1, 1) or r != r1 or stride != stride1 or isinstance(p, str) or p[0] != p[1] or c["padding_mode"] != "zeros"
+            or "bias" not in own or not torch.backends.cudnn.allow_tf32):
         return None
-    mode = "gemm" if k[0] == 1 and s[0] == 1 and p[0] == 0 else \
-        "stem" if conv.in_channels * k[0] * k[0] <= STEM_K and s[0] == 1 and 2 * p[0] == k[0] - 1 and conv.out_channels > 16 else "conv"
-    if mode not in PATHS:
+    if c["_forward_pre_hooks"] or c["_forward_hooks"] or b["_forward_pre_hooks"] or b["_forward_hooks"] or _PRE or _FORWARD:       # see ops.bn.hooked
         return None
-    if MIN_ROWS > 0 and x.dim() == 4 and x.shape[0] * ((x.shape[2] + 2 * p[0] - k[0]) // s[0] + 1) * ((x.shape[3] + 2 * p[0] - k[0]) // s[0] + 1) < MIN_ROWS:
-        return None
-    y = nat.ext().conv_bn_eval(x, w, own["bias"], params.get("weight"), params.get("bias"), stats.get("running_mean"), stats.get("running_var"), bn.eps,
-                               residual, relu, s[0], p[0], pool, _err(x.device))
+    if MIN_ROWS > 0 or not _EVERY_MODE <= PATHS:
+        mode = "gemm" if r == 1 and stride == 1 and p[0] == 0 else \
+            "stem" if c["in_channels"] * r * r <= STEM_K and stride == 1 and 2 * p[0] == r - 1 and c["out_channels"] > 16 else "conv"
+        if mode not in PATHS or x.dim() != 4 or \
+                x.shape[0] * ((x.shape[2] + 2 * p[0] - r) // stride + 1) * ((x.shape[3] + 2 * p[0] - r) // stride + 1) < MIN_ROWS:
+            return None
+    y = nat.ext().conv_bn_eval(x, w, own["bias"], params.get("weight"), params.get("bias"), stats.get("running_mean"), stats.get("running_var"), b["eps"],
+                               residual, relu, stride, p[0], pool, _err(x.device))
     if y is not None:
         nat.count_launch()
     return y

@@ -19,10 +19,10 @@ class TensorCoreTimeout(RuntimeError):
 
 
 def _error_flag(device):
-    key = (device.type, device.index)
-    if key not in _err:
-        _err[key] = torch.zeros(1, dtype=torch.int32, device=device)
-    return _err[key]
+    flag = _err.get(device)
+    if flag is None:
+        flag = _err[device] = torch.zeros(1, dtype=torch.int32, device=device)
+    return flag
 
 
 def supported(a, b_nk):
