@@ -25,8 +25,7 @@ def _peak():
 def _time(fn, warmup, iters, flush):
     times = []
     for i in range(warmup + iters):
-        flush.add_(1.0)                   # 256 MB rewrite: L2 holds nothing of the case's tensors
-        torch.cuda.synchronize()
+        flush.add_(1.0)                   # 256 MB rewrite: L2 holds nothing of the case's tensors, and its time hides the launches' latency
         s, e = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
         s.record()
         fn()

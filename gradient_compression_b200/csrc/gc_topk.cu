@@ -5,7 +5,7 @@
 //   topk_fold_kernel     a = g + e -> e, and a histogram of the top 13 bits of |a| per group                 (12 bytes an element)
 //   topk_pick_kernel     per group: the bin that holds the k-th largest (groups of up to 4096 elements: the whole selection)
 //   topk_split_kernel    above that bin: selected.  In it: put on the group's candidate list.  Below: not selected.
-//   topk_refine_kernel   per group: exact selection among the candidates by the remaining 18 bits, in two steps of 9
+//   topk_refine_kernel   per group: exact selection among the candidates by the remaining 18 bits, in two steps of 9, then by index
 //
 // Two outputs.  LISTS (several workers): index and value of the selected entries, for the exchange.  DENSE (a single
 // worker, whose exchange is the identity): the selected entries in an otherwise zero gradient, written by the split
