@@ -70,7 +70,7 @@ def test_other_threads_run_while_a_launch_waits():
     thread.join()
     torch.cuda.synchronize()
     assert took > 0.2, "the queue never filled up"
-    assert longest[0] < 0.5 * took
+    assert longest[0] < 0.8 * took          # (with the lock held: all but the last few milliseconds)
 
 
 @pytest.mark.gpu
