@@ -516,7 +516,8 @@ PyObject* conv_bn_eval(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   if (!want(nargs, 14, "conv_bn_eval")) return nullptr;
   const at::Tensor *x = activation(a[0]), *w = tensor_of(a[1]), *res = a[8] == Py_None ? nullptr : activation(a[8]);
   if (!x || !w || (a[8] != Py_None && !res)) Py_RETURN_NONE;
-  if (!w->is_cuda() || w->scalar_type() != at::kFloat || w->dim() != 4 || w->device() != x->device() || w->size(1) != x->size(1) || w->size(2) != w->size(3))
+  if (!w->is_cuda() || w->scalar_type() != at::kFloat || w->dim() != 4 || w->device() != x->device() || w->size(1) != x->size(1) || w->size(2) != w->size(3) ||
+      ((uintptr_t)w->data_ptr() & 15u))
     Py_RETURN_NONE;
   const int64_t n = x->size(0), cin = x->size(1), h = x->size(2), wd = x->size(3), cout = w->size(0), r = w->size(2);
   if (!(w->is_contiguous(at::MemoryFormat::ChannelsLast) || (r == 1 && w->is_contiguous()))) Py_RETURN_NONE;

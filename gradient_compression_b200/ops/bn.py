@@ -154,7 +154,16 @@ def _fin_ptr(device, channels):
 
 
 def _cl(t):
-    return t if t.is_contiguous(memory_format=torch.channels_last) else t.contiguous(memory_format=torch.channels_last)
+    """``t`` in channels-last memory order, starting on a 16-byte boundary (the kernels read quads of channels)."""
+    if not t.is_contiguous(memory_format=torch.channels_last):
+        return t.contiguous(memory_format=torch.channels_last)
+    return t if t.data_ptr() % 16 == 0 else t.clone(memory_format=torch.channels_last)
+
+
+def on_boundary(p):
+    """The tensor ``p``, or a copy that autograd leads back to it, on a 16-byte boundary.  Parameters of a flat buffer (``FlatArena`` packs
+    them back to back) need not start on one: behind a tensor whose size is no multiple of four none of them do."""
+    return p if p.data_ptr() % 16 == 0 else p.clone(memory_format=torch.preserve_format)
 
 
 def kernel_path_ok(x):
@@ -228,6 +237,17 @@ class _FusedBNAct(torch.autograd.Function):
         return dx, sums[c:], sums[:c], dres, None, None, None, None, None, None
 
 
+def _by_torch(bn, x):
+    """``bn(x)``.  The library's channels-last kernels read quads too (its training batch norm raised a misaligned address on an activation
+    between two boundaries), so it gets copies where ours would."""
+    if x.is_cuda:
+        x = on_boundary(x)
+        moved = {n: on_boundary(p) for n, p in bn._parameters.items() if p is not None and p.data_ptr() % 16}
+        if moved:
+            return torch.func.functional_call(bn, moved, (x,))
+    return bn(x)
+
+
 def bn_act(bn, x, residual=None, relu=True):
     """``relu(bn(x) + residual)`` with ``bn`` a ``torch.nn.BatchNorm2d`` (affine, tracking running stats)."""
     training = bn.training or bn.running_mean is None
@@ -239,7 +259,7 @@ def bn_act(bn, x, residual=None, relu=True):
             return y
     use_kernel = plain and kernel_path_ok(x) and not (not training and torch.is_grad_enabled() and x.requires_grad)
     if not use_kernel:
-        y = bn(x)
+        y = _by_torch(bn, x)
         if residual is not None:
             y = y + residual
         return F.relu(y) if relu else y
@@ -248,4 +268,4 @@ def bn_act(bn, x, residual=None, relu=True):
         count_batch(bn)
     rm = bn.running_mean if bn.track_running_stats else None
     rv = bn.running_var if bn.track_running_stats else None
-    return _FusedBNAct.apply(x, bn.weight, bn.bias, residual, rm, rv, training, momentum, bn.eps, relu)
+    return _FusedBNAct.apply(x, on_boundary(bn.weight), on_boundary(bn.bias), residual, rm, rv, training, momentum, bn.eps, relu)

@@ -33,7 +33,7 @@ import torch
 
 from . import _native as nat
 from . import gemm
-from .bn import _FORWARD, _PRE, _cl, _fin_ptr, _scratch_for, bn_act, fused_backward, fused_forward, fused_ok, hooked, count_batch, own_grad, take_owned_grad
+from .bn import _FORWARD, _PRE, _cl, _fin_ptr, _scratch_for, bn_act, fused_backward, fused_forward, fused_ok, hooked, count_batch, on_boundary, own_grad, take_owned_grad
 
 # GCB200_TC_CONV=0 (or ``ENABLED = False``) keeps every convolution on cuDNN.
 ENABLED = os.environ.get("GCB200_TC_CONV", "1") == "1"
@@ -651,6 +651,6 @@ def conv_bn_act(conv, bn, x, residual=None, relu=True, link=None, donate=None, p
         count_batch(bn)
     rm = bn.running_mean if bn.track_running_stats else None
     rv = bn.running_var if bn.track_running_stats else None
-    return _ConvBNAct.apply(x, conv.weight, conv.bias, bn.weight, bn.bias, residual, rm, rv, training, momentum,
+    return _ConvBNAct.apply(x, on_boundary(conv.weight), conv.bias, on_boundary(bn.weight), on_boundary(bn.bias), residual, rm, rv, training, momentum,
                             bn.eps, relu, link if (link is not None and link.armed) else None, mode, conv.stride[0],
                             conv.padding[0], donate if (donate is not None and donate.armed) else None, bool(pool))

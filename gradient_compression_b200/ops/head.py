@@ -15,7 +15,7 @@ import torch
 import torch.nn.functional as F
 
 from . import _native as nat
-from .bn import hooked
+from .bn import _cl, hooked
 
 _scratch = {}
 
@@ -44,7 +44,7 @@ class _HeadCE(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, weight, bias, labels):
         n, c, h, w = x.shape
-        x = x if x.is_contiguous(memory_format=torch.channels_last) else x.contiguous(memory_format=torch.channels_last)
+        x = _cl(x)
         k = weight.shape[0]
         dev = x.device
         pooled = torch.empty(n, c, dtype=torch.float32, device=dev)

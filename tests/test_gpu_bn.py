@@ -396,3 +396,47 @@ def test_batch_counters_are_batched_but_exact():
     tw = Twice().cuda()
     tw(torch.randn(4, 8, 8, 8, device="cuda").contiguous(memory_format=torch.channels_last))
     assert int(tw.bn.num_batches_tracked) == 2
+
+
+@pytest.mark.parametrize("training", [False, True])
+@pytest.mark.parametrize("odd", [0, 1, 2, 3])
+@pytest.mark.parametrize("r,c", [(0, 64), (1, 64), (3, 64), (0, 60)])          # (60: the library's batch norm)
+def test_parameters_and_activations_off_the_16_byte_boundary(r, c, odd, training):
+    """A flat buffer that starts with a tensor of 1 to 3 elements: the kernels get copies of the parameters behind it, and of activations
+    that start between two boundaries."""
+    import torch.nn.functional as F
+    from gradient_compression_b200.ops import conv_bn_act
+    from gradient_compression_b200.ops.bn import bn_act
+    from gradient_compression_b200.parallel.arena import FlatArena
+
+    def shifted(t):
+        out = torch.empty(t.numel() + odd, device="cuda")[odd:].view(t.shape[0], t.shape[2], t.shape[3], t.shape[1]).permute(0, 3, 1, 2)
+        return out.copy_(t)
+
+    torch.manual_seed(odd + 4 * r)
+    conv = torch.nn.Conv2d(c, c, max(r, 1), 1, r // 2, bias=False).cuda().to(memory_format=torch.channels_last)
+    bn = torch.nn.BatchNorm2d(c).cuda()
+    with torch.no_grad():
+        bn.weight.uniform_(0.5, 1.5)
+        bn.bias.normal_()
+    first = torch.nn.Parameter(torch.zeros(odd, device="cuda"))
+    arena = FlatArena([first, *conv.parameters(), *bn.parameters()])
+    assert (conv.weight.data_ptr() % 16 == 0) == (odd == 0) == (bn.weight.data_ptr() % 16 == 0)
+    conv.train(training), bn.train(training)
+    x, res, dy = (shifted(torch.randn(4, c, 8, 8, device="cuda")) for _ in range(3))
+    x.requires_grad_(training)
+    with torch.set_grad_enabled(training):
+        y = conv_bn_act(conv, bn, x, residual=res) if r else bn_act(bn, x, residual=res)
+    xd, w, g, b = (t.detach().double().requires_grad_(True) for t in (x, conv.weight, bn.weight, bn.bias))
+    z = F.conv2d(xd, w, None, 1, r // 2) if r else xd
+    mean, var = (z.mean((0, 2, 3)), z.var((0, 2, 3), unbiased=False)) if training else (torch.zeros(c, device="cuda").double(), torch.ones(c, device="cuda").double())
+    z = (z - mean[:, None, None]) / (var[:, None, None] + bn.eps).sqrt() * g[:, None, None] + b[:, None, None]
+    want = (z + res.double()).relu()
+    assert float((y.detach().double() - want.detach()).norm() / want.detach().norm()) < 2e-3
+    if training:
+        arena.zero_grad()
+        y.backward(dy)
+        mask = (y > 0).double()                         # a value on the other side of zero is no error of the gradient
+        (z + res.double()).backward(dy.double() * mask)
+        for got, ref in [(x.grad, xd.grad), (bn.weight.grad, g.grad), (bn.bias.grad, b.grad)] + ([(conv.weight.grad, w.grad)] if r else []):
+            assert float((got.double() - ref).norm() / ref.norm()) < 5e-3
