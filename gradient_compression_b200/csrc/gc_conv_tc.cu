@@ -74,6 +74,91 @@ double reuse(const Shape& s) {
 
 ConvA conv_a(const Shape& s) { return ConvA{s.R * s.R, s.R, s.Cin / 32, s.Ho * s.Wo, s.Wo, s.stride, s.pad}; }
 
+// Geometry of the kernel that shares the pixels of a filter column (TapCols) for tiles of BM positions, widths up to 128 columns.  s: the
+// convolution of dY, 3x3 with padding 1, whose tiles are boxes (box_for) of at most 256 pixels, rows above and below included, and whose image rows are
+// whole groups of 8 pixels in shared memory.
+bool tap_cols(const Shape& s, TapCols* t) {
+  int bw, bh, bn;
+  if (s.R != 3 || s.stride != 1 || s.pad != 1 || (s.Cin & 31) || !box_for(BM, s.Ho, s.Wo, &bw, &bh, &bn) || bw != s.Wo) return false;
+  const int row = bw * bn;                   // pixels of one image row of the tile
+  const bool whole = bh == s.Ho;
+  const int pixels = whole ? BM : BM + 2 * row;
+  if ((row & 7) || pixels > 256) return false;
+  *t = TapCols{};
+  t->box_bytes = pixels * 128;
+  t->step = row * 128;
+  t->lead = whole ? t->step : 0;
+  t->first = t->lead;
+  t->pitch = t->box_bytes + t->lead;
+  t->h_off = whole ? 0 : -1;
+  return true;
+}
+
+// Stages of that kernel at the plan's tile; 0: fewer than two.
+int tap_stages(const Plan& pl, TapCols* t) {
+  auto fit = [&](int ring, int filter) {
+    int n = (ring - t->lead) / (t->pitch + filter);
+    if (n > PSmem<64, true, true>::MAX_STAGES) n = PSmem<64, true, true>::MAX_STAGES;
+    t->stages = n;
+    t->b_off = n * t->pitch + t->lead;
+    return n < 2 ? 0 : n;
+  };
+  if (pl.bn == 64) return pl.pair ? fit(PSmem<64, true, true>::RING_BYTES, PSmem<64, true, true>::TAPS_STAGE_B)
+                                  : fit(PSmem<64, false, true>::RING_BYTES, PSmem<64, false, true>::TAPS_STAGE_B);
+  return pl.pair ? fit(PSmem<128, true, true>::RING_BYTES, PSmem<128, true, true>::TAPS_STAGE_B)
+                 : fit(PSmem<128, false, true>::RING_BYTES, PSmem<128, false, true>::TAPS_STAGE_B);
+}
+
+bool taps_ok(const Shape& s) {
+  TapCols t;
+  Plan p{128, 1, false, true};
+  return tap_cols(s, &t) && tap_stages(p, &t) != 0;
+}
+
+// {C, W, N, H} map over an NHWC tensor; box of 32 channels x w x images x h.
+int make_map_wnh(CUtensorMap* map, const float* base, int N, int H, int W, int C, int w, int images, int h) {
+  cuuint64_t dims[4] = {(cuuint64_t)C, (cuuint64_t)W, (cuuint64_t)N, (cuuint64_t)H};
+  cuuint64_t strides[3] = {(cuuint64_t)C * 4, (cuuint64_t)H * W * C * 4, (cuuint64_t)W * C * 4};
+  cuuint32_t box[4] = {32, (cuuint32_t)w, (cuuint32_t)images, (cuuint32_t)h}, estr[4] = {1, 1, 1, 1};
+  return encode_fn()(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, (void*)base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                     CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS ? 0 : -2;
+}
+
+// The filter [Cout][3][3][Cin] of that kernel: one box brings the three taps of a column for 32 rows of the contraction (Cout) and `cols` columns
+// of the input gradient (Cin).
+int make_map_filter_cols(CUtensorMap* map, const float* w, int Cout, int Cin, int cols) {
+  const cuuint64_t tap = (cuuint64_t)Cin * 4;
+  cuuint64_t dims[5] = {32, (cuuint64_t)Cout, (cuuint64_t)Cin / 32, 3, 3}, strides[4] = {9 * tap, 128, tap, 3 * tap};
+  cuuint32_t box[5] = {32, (cuuint32_t)BK, (cuuint32_t)cols / 32, 1, 3}, estr[5] = {1, 1, 1, 1, 1};
+  return encode_fn()(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 5, (void*)w, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B,
+                     CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS ? 0 : -2;
+}
+
+// Everything a launch of a planned R x R convolution needs besides its arguments.
+struct ConvMaps {
+  CUtensorMap a, b, c;
+  ConvA ca;
+  ConvC cc;
+  TapCols tc;
+  const ConvC* store() const { return cc.hw != 0 ? &cc : nullptr; }
+};
+
+// Pixels and output of the convolution s (of dY for an input gradient) under the plan; the filter's map is the caller's.
+int conv_maps(ConvMaps* m, const Plan& pl, const Shape& s, const float* x, float* y) {
+  int bw, bh, bn;
+  box_for(BM, s.Ho, s.Wo, &bw, &bh, &bn);
+  m->ca = ConvA{s.R * s.R, s.R, s.Cin / 32, s.Ho * s.Wo, s.Wo, s.stride, s.pad};
+  m->cc = ConvC{};
+  m->tc = TapCols{};
+  if (!pl.taps)
+    return make_map_nhwc(&m->a, x, s, bw, bh, bn, CU_TENSOR_MAP_SWIZZLE_128B) != 0 || make_map(&m->c, y, (int64_t)s.N * s.Ho * s.Wo, s.Cout, s.Cout, BM) != 0 ? -2 : 0;
+  if (!tap_cols(s, &m->tc) || tap_stages(pl, &m->tc) == 0) return -3;
+  if (make_map_wnh(&m->a, x, s.N, s.H, s.W, s.Cin, bw, bn, bh == s.Ho ? bh : bh + 2) != 0) return -2;
+  if (bn == 1) return make_map(&m->c, y, (int64_t)s.N * s.Ho * s.Wo, s.Cout, s.Cout, BM);
+  m->cc = ConvC{s.Ho * s.Wo, s.Wo, 1};
+  return make_map_wnh(&m->c, y, s.N, s.Ho, s.Wo, s.Cout, bw, bn, bh);
+}
+
 bool fwd_ok(const Shape& s) {
   int bw, bh, bn;
   if ((s.Cin & 31) || (s.Cout & 3) || s.Cout < 32) return false;
@@ -314,28 +399,23 @@ int gc_cuda_conv_dgrad(const float* dy, const float* w, float* dx, int N, int H,
     return (int)cudaErrorInvalidValue;
   const int M = N * H * W, K = R * R * Cout;
   cudaStream_t st = (cudaStream_t)cs;
-  const Plan pl = plan_persistent(M, Cin, K, accumulate ? 0.0 : zero_ns((int64_t)M * Cin), R * R);
-  CUtensorMap ma, mb, mc;
-  ConvA ca{};
-  if (R == 1 && pad == 0) {
-    if (make_map(&ma, dy, M, Cout, Cout, BM) != 0) return (int)cudaErrorInvalidValue;
-  } else {
-    Shape s;
-    make_shape(N, H + 2 * pad - R + 1, W + 2 * pad - R + 1, Cout, Cin, R, 1, R - 1 - pad, &s);
-    int bw, bh, bn;
-    box_for(BM, s.Ho, s.Wo, &bw, &bh, &bn);
-    if (make_map_nhwc(&ma, dy, s, bw, bh, bn, CU_TENSOR_MAP_SWIZZLE_128B) != 0) return (int)cudaErrorInvalidValue;
-    ca = conv_a(s);
-  }
-  ca.b_ldtap = Cin; ca.b_fs = R;
-  ca.b_r0 = R - 1; ca.b_dr = -1; ca.b_s0 = R - 1; ca.b_ds = -1;
-  if (filter_map(&mb, &ca, w, Cout, R, Cin, pl.b_cols()) != 0 || make_map(&mc, dx, M, Cin, Cin, BM) != 0)
+  const bool matrix = R == 1 && pad == 0;
+  Shape s{};
+  if (!matrix) make_shape(N, H + 2 * pad - R + 1, W + 2 * pad - R + 1, Cout, Cin, R, 1, R - 1 - pad, &s);
+  const Plan pl = plan_persistent(M, Cin, K, accumulate ? 0.0 : zero_ns((int64_t)M * Cin), R * R, !matrix && (Cin & 31) == 0 && taps_ok(s));
+  ConvMaps m{};
+  if (matrix ? make_map(&m.a, dy, M, Cout, Cout, BM) != 0 || make_map(&m.c, dx, M, Cin, Cin, BM) != 0 : conv_maps(&m, pl, s, dy, dx) != 0)
+    return (int)cudaErrorInvalidValue;
+  m.ca.b_ldtap = Cin; m.ca.b_fs = R;
+  m.ca.b_r0 = R - 1; m.ca.b_dr = -1; m.ca.b_s0 = R - 1; m.ca.b_ds = -1;
+  if (pl.taps) m.ca.b_mn = 2;
+  if ((pl.taps ? make_map_filter_cols(&m.b, w, Cout, Cin, pl.b_cols()) : filter_map(&m.b, &m.ca, w, Cout, R, Cin, pl.b_cols())) != 0)
     return (int)cudaErrorInvalidValue;
   if (pl.splits > 1 && !accumulate) {
     cudaError_t e = cudaMemsetAsync(dx, 0, (size_t)M * Cin * 4, st);
     if (e != cudaSuccess) return (int)e;
   }
-  return launch_plan(pl, ma, mb, mc, ca, nullptr, M, Cin, K, accumulate || pl.splits > 1, nullptr, error_flag, st);
+  return launch_plan(pl, m.a, m.b, m.c, m.ca, nullptr, M, Cin, K, accumulate || pl.splits > 1, nullptr, error_flag, st, nullptr, m.store(), 0, nullptr, &m.tc);
 }
 
 // For measurements: 1 = weight gradients at Cin = 128 use 256-column tiles that hold two filter taps (measured slower than
@@ -458,7 +538,7 @@ int gc_cuda_conv_dgrad_s2_add(const float* dy, const float* w, float* dx, int N,
              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
         return (int)cudaErrorInvalidValue;
     }
-    const ConvC cc{Ho * Wo, Wo};
+    const ConvC cc{Ho * Wo, Wo, 0};
     const int err = launch_plan(pl, ma, mb, mc, ca, nullptr, M, Cin, K, accumulate, nullptr, error_flag, st, nullptr, &cc);
     if (err != 0) return err;
   }

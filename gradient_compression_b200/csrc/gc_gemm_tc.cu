@@ -378,6 +378,9 @@ void gc_cuda_tc_split_config(int splits) { gctc::split_choice = splits; }
 // For measurements: CTA pairs of the persistent kernel (0 = modelled, 1 = never, 2 = wherever there are two row tiles).
 void gc_cuda_tc_pair_config(int pairs) { gctc::pair_choice = pairs; }
 
+// For measurements: input gradients of 3x3 convolutions with one load of the pixels per filter column (0 = wherever the shape allows it, 1 = never).
+void gc_cuda_tc_taps_config(int taps) { gctc::taps_choice = taps; }
+
 // For measurements: bit 0: prefetch the tensor maps at kernel start; bit 2: epilogue warps sleep between polls of their barrier.
 void gc_cuda_tc_tma_mode(int mode) { gctc::tma_mode = mode; }
 

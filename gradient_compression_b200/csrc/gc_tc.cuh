@@ -30,6 +30,7 @@ inline int tn_ctas_per_sm = 1;
 inline int tn_min_kblocks = 8;
 inline int wgrad_two_taps = 0;
 inline int split_choice = 0;   // contraction splits of the persistent kernel: 0 = modelled, 1 = never, n = n where a product allows it
+inline int taps_choice = 0;    // input gradients of 3x3 convolutions with one load of the pixels per filter column: 0 = wherever the shape allows it, 1 = never
 inline int tma_mode = 1;   // bit 0: prefetch the tensor maps at kernel start; bit 2: epilogue warps sleep between polls while a tile is being accumulated
 }  // namespace gctc
 
@@ -209,6 +210,19 @@ __device__ __forceinline__ void tma_load_4d_pair(void* dst, const CUtensorMap* m
       : "memory");
 }
 
+__device__ __forceinline__ void tma_load_5d(void* dst, const CUtensorMap* map, int c0, int c1, int c2, int c3, int c4, uint64_t* bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.5d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6, %7}], [%2];"
+      ::"r"(smem_u32(dst)), "l"(map), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4)
+      : "memory");
+}
+__device__ __forceinline__ void tma_load_5d_pair(void* dst, const CUtensorMap* map, int c0, int c1, int c2, int c3, int c4, uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.5d.shared::cluster.global.mbarrier::complete_tx::bytes.cta_group::2 [%0], [%1, {%3, %4, %5, %6, %7}], [%2];"
+      ::"r"(smem_u32(dst)), "l"(map), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4)
+      : "memory");
+}
+
 __device__ __forceinline__ uint32_t cluster_rank() {
   uint32_t r;
   asm volatile("mov.u32 %0, %cluster_ctarank;" : "=r"(r));
@@ -246,12 +260,38 @@ struct ConvA {
   int b_mn, b_ldtap, b_fs, b_r0, b_dr, b_s0, b_ds;
 };
 
+// The input gradient of a 3x3, stride-1, padding-1 convolution, where the three taps of a filter COLUMN share one copy of dY's pixels.
+// The map's dimensions are {C, W, N, H}, so a tile of 128 positions lies in shared memory as rows (h, n, w) of 128 bytes and the pixels one
+// image row further down are `step` = W * images * 128 bytes further on: the operand of tap (r, s) is the box of column shift s read
+// from a start address moved by r steps (a multiple of 1024 bytes, so the swizzle pattern stays in place).  A stage holds the box
+// and the filter's three taps of that column and 32-channel block, read in place (ConvA, b_mn = 2); it is good for 3 k-blocks.  A tile of
+// whole images needs no rows from outside: the zeros above and below it are gaps between the stages, written once.  Otherwise the box
+// carries one more image row at each end.
+// Why: with a box per tap a k-block of a CTA pair fills 16 KB of pixels and BN / 2 rows of filter into shared memory, at some 50 bytes a cycle and
+// SM, while its MMAs read the same again; that, not the tensor pipe, took the time.  Pixels are now 5.3 to 8 KB a k-block.  A k-block of a pair at 128
+// columns: 200 -> 144 ns (16x16x128, batch 256 against 128), at 64 columns 205 -> 103.  Input gradients back to back, one B200: 32x32x64 at batch 128
+// 29.9 -> 21.0 us, 16x16x128 20.5 -> 18.5, 2x2x512 12.1 -> 12.2, 16x16x128 at batch 256 34.7 -> 29.1, at batch 31 12.2 -> 10.9.
+// The forward pass keeps a box per tap: this contraction runs through its channel blocks first, and a sum in another order than before moves
+// the last bit of an activation, which moves a ResNet-50's logits by up to 1.2 per cent.
+struct TapCols {
+  int box_bytes;           // pixels of a stage; 0 = off (the kernel variant without it)
+  int pitch;               // bytes between the pixels of neighbouring stages
+  int first;               // offset of the first stage's pixels = the gap in front of them
+  int step;                // one image row further down
+  int lead;                // tap (0, s) starts this many bytes in front of the box (whole images: `step`, else 0)
+  int h_off;               // image row of the box's first pixel, relative to the tile's
+  int stages;
+  int b_off;               // filter taps of the first stage
+};
+
 // Where the rows of the OUTPUT go when it is not a matrix but a strided sub-grid of an NHWC tensor read through a 4-D map
 // {C, W', H', N} (the input gradient of a stride-2 convolution: one launch per parity class of input pixels): row
 // p = (n, i, j) of the result is stored at coordinates (column, j, i, n).  hw == 0: a plain 2-D matrix.
+// nh: the map's dimensions are {C, W', N, H'}, for tiles whose rows run (h, image, w).
 struct ConvC {
   int hw;          // rows per image (H' * W'), 0 = plain matrix
   int w;           // W'
+  int nh;
 };
 
 // Batch-norm statistics finished inside the GEMM that produces the activation: every CTA keeps per-column sums and sums
@@ -396,7 +436,7 @@ __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.
 // four epilogue warps take alternate 32-column slabs, each group staging them in its own ring of dedicated
 // buffers and waiting for a TMA store only when it needs that store's buffer back.  Tiles are ordered
 // with the column tile fastest: CTAs that run at the same time share the rows of A in L2.
-template <int BN, bool PAIR>
+template <int BN, bool PAIR, bool TAPS = false>
 struct PSmem {
   // Up to 128 columns two staging slabs are enough and the ring gets what they leave (28.7 against 29.7 us at 16x16x128 3x3,
   // 65.5 against 74.9 us at 8x8x512 in pairs); at 256 columns the epilogue has as much to store as the ring to load, and
@@ -407,14 +447,19 @@ struct PSmem {
   static constexpr int B_BYTES = B_COLS * BK * 4;           // a multiple of 1024
   static constexpr int NSLAB = BN <= 128 ? 2 : 4;
   static constexpr int SLAB_BYTES = BM * 128;
-  static constexpr int RING_BYTES = STAGES * (A_BYTES + B_BYTES);
+  static constexpr int TAPS_STAGE_B = 3 * B_BYTES;          // TAPS: the filter's three taps of a column
+  static constexpr int MAX_STAGES = 12;
+  static constexpr int LIMIT = 232448;                      // shared memory of one CTA
+  static constexpr int RING_BYTES = TAPS ? (LIMIT - 1024 - 256 - 4 * BN * 2 * 4 - NSLAB * SLAB_BYTES) / 1024 * 1024 : STAGES * (A_BYTES + B_BYTES);
   static constexpr int STAGING_OFF = RING_BYTES;
   static constexpr int BAR_OFF = STAGING_OFF + NSLAB * SLAB_BYTES;
   static constexpr int COLSUM_OFF = BAR_OFF + 256;
   static constexpr int TOTAL = 1024 /* alignment slack */ + COLSUM_OFF + 4 * BN * 2 * 4;
   static constexpr int TMEM_COLS = 2 * BN;
+  static_assert(!TAPS || BN <= 128, "tile widths of the kernel with shared pixels");
+  static_assert((2 * MAX_STAGES + 4) * 8 + 4 <= 256 && STAGES <= MAX_STAGES, "barriers");
   static_assert(BN == 64 || BN == 128 || BN == 256, "tile widths of the persistent kernel");
-  static_assert(TOTAL <= 232448, "shared memory of one CTA");
+  static_assert(TOTAL <= LIMIT, "shared memory of one CTA");
 };
 
 // Named barrier of one epilogue group (ids 1 and 2; 0 is __syncthreads).
@@ -439,21 +484,27 @@ constexpr int PERSISTENT_THREADS = 32 * FIRST_EPI_WARP + 128 * EPI_GROUPS;
 // of B, so a k-block costs a CTA 128 + BN / 2 rows of shared-memory fill and of operand reads instead of 128 + BN, which is
 // what bounds the single-CTA form.  The first CTA of the pair issues the MMAs and holds the barriers they wait for; commits go
 // to both.  Work items are the pairs' tiles; everything after the accumulator is each CTA's own.
-template <int BN, bool AFFINE, bool PAIR>
+//
+// TAPS: the input gradient of a 3x3 convolution whose filter columns share a copy of the pixels (TapCols); a stage is 3 k-blocks.
+template <int BN, bool AFFINE, bool PAIR, bool TAPS>
 __global__ void __launch_bounds__(PERSISTENT_THREADS, 1)
 gemm_tf32_persistent_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
                             const __grid_constant__ CUtensorMap tma_c, const ConvA ca, const float* __restrict__ bias, int M, int N, int K,
                             int tiles_m, int tiles_n, int splits, int accumulate, float* __restrict__ col_partials,
-                            int* __restrict__ error_flag, int tma_mode, const BnFin fin, const ConvC cc, int cta_sums, const Affine aff) {
-  using S = PSmem<BN, PAIR>;
+                            int* __restrict__ error_flag, int tma_mode, const BnFin fin, const ConvC cc, int cta_sums, const Affine aff,
+                            const TapCols tc) {
+  using S = PSmem<BN, PAIR, TAPS>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-  uint8_t* a_tiles = base;
-  uint8_t* b_tiles = base + S::STAGES * S::A_BYTES;
+  const uint32_t stages = TAPS ? (uint32_t)tc.stages : (uint32_t)S::STAGES;
+  const int a_pitch = TAPS ? tc.pitch : S::A_BYTES;
+  constexpr int B_STAGE = TAPS ? S::TAPS_STAGE_B : S::B_BYTES;
+  uint8_t* a_tiles = base + (TAPS ? tc.first : 0);
+  uint8_t* b_tiles = base + (TAPS ? tc.b_off : S::STAGES * S::A_BYTES);
   uint8_t* staging = base + S::STAGING_OFF;
   uint64_t* full = reinterpret_cast<uint64_t*>(base + S::BAR_OFF);
-  uint64_t* empty = full + S::STAGES;
-  uint64_t* acc_full = empty + S::STAGES;      // [2] MMA -> epilogue: accumulator complete
+  uint64_t* empty = full + S::MAX_STAGES;
+  uint64_t* acc_full = empty + S::MAX_STAGES;      // [2] MMA -> epilogue: accumulator complete
   uint64_t* acc_empty = acc_full + 2;          // [2] epilogue -> MMA: accumulator drained
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
   float* colsum = reinterpret_cast<float*>(base + S::COLSUM_OFF);      // [4 row quarters][BN columns][2]
@@ -461,7 +512,7 @@ gemm_tf32_persistent_kernel(const __grid_constant__ CUtensorMap tma_a, const __g
   __shared__ int epi_go[EPI_GROUPS];
 
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
-  const int num_k = (K + BK - 1) / BK;
+  const int num_k = TAPS ? 3 * ca.cblocks : (K + BK - 1) / BK;      // stages of a whole contraction
   // work item = (output tile, split of the contraction); the splits of one tile are neighbours in the list, so they run
   // at the same time on different SMs and add their partial tiles in L2 (the host passes accumulate = 1 and a zeroed C)
   const int total_items = tiles_m * tiles_n * splits;          // tiles_m: of 128 rows, PAIR: of 256
@@ -472,7 +523,7 @@ gemm_tf32_persistent_kernel(const __grid_constant__ CUtensorMap tma_a, const __g
   if (threadIdx.x == 0) {
     abort_flag = 0;
     for (int g = 0; g < EPI_GROUPS; ++g) epi_go[g] = 1;
-    for (int s = 0; s < S::STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
+    for (uint32_t s = 0; s < stages; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
     for (int b = 0; b < 2; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], (PAIR ? 2 : 1) * EPI_GROUPS); }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -485,6 +536,15 @@ gemm_tf32_persistent_kernel(const __grid_constant__ CUtensorMap tma_a, const __g
       asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"((uint32_t)S::TMEM_COLS) : "memory");
       asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
+  }
+  if constexpr (TAPS) {
+    // the zero rows above and below a tile of whole images: the gap in front of every stage's pixels and behind the last one's
+    const int quads = tc.lead >> 4, pitch = tc.pitch;
+    for (int i = threadIdx.x; i < quads * (tc.stages + 1); i += PERSISTENT_THREADS) {
+      const int gap = i / quads;
+      *reinterpret_cast<float4*>(base + gap * pitch + (i - gap * quads) * 16) = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    if (quads != 0) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
   tc_fence_before();
   __syncthreads();
@@ -510,7 +570,10 @@ gemm_tf32_persistent_kernel(const __grid_constant__ CUtensorMap tma_a, const __g
       int box[4] = {0, 0, 0, 0};
       if (ca.taps != 0) conv_box(ca, (int64_t)m0, 0, 0, box);  // pixel of the tile's first position at tap (0, 0)
       int cb = 0, fr = 0, fs = 0;                             // k-block = (filter tap (fr, fs), 32-channel block cb)
-      if (ca.taps != 0) {
+      if constexpr (TAPS) {
+        cb = kbeg / 3;                                        // stage = (32-channel block cb, filter column fs)
+        fs = kbeg - cb * 3;
+      } else if (ca.taps != 0) {
         const int tap = kbeg / ca.cblocks;
         cb = kbeg - tap * ca.cblocks;
         fr = tap / ca.fs;
@@ -519,6 +582,23 @@ gemm_tf32_persistent_kernel(const __grid_constant__ CUtensorMap tma_a, const __g
       for (int k = kbeg; k < kend; ++k) {
         if (turn == warp) {
           if (!mbar_wait_warp(&empty[s], phase ^ 1u, &abort_flag)) { ok = false; break; }
+          if constexpr (TAPS) {
+            uint8_t *a_dst = a_tiles + s * (uint32_t)a_pitch, *b_dst = b_tiles + s * (uint32_t)B_STAGE;
+            const int w0 = fs - 1, h0 = box[2] + ca.pad + tc.h_off;      // pixels {cb * 32, w0, image, h0}: box[2] = row of tap (0, 0)
+            if constexpr (PAIR) {
+              const uint32_t bar = cluster_addr(&full[s], 0);
+              if (elect_one()) {
+                if (rank == 0) mbar_expect_tx(&full[s], (uint32_t)(2 * (tc.box_bytes + B_STAGE)));
+                tma_load_4d_pair(a_dst, &tma_a, cb * 32, w0, box[3], h0, bar);
+                tma_load_5d_pair(b_dst, &tma_b, 0, cb * BK, n0 >> 5, 2 - fs, 0, bar);
+              }
+            } else if (elect_one()) {
+              mbar_expect_tx(&full[s], (uint32_t)(tc.box_bytes + B_STAGE));
+              tma_load_4d(a_dst, &tma_a, cb * 32, w0, box[3], h0, &full[s]);
+              tma_load_5d(b_dst, &tma_b, 0, cb * BK, n0 >> 5, 2 - fs, 0, &full[s]);
+            }
+            __syncwarp();
+          } else {
           // b_mn: B is the filter read in place (no transposed copy)
           const int tapcol = ca.b_mn == 0 || ca.taps == 0 ? 0 : ((ca.b_r0 + ca.b_dr * fr) * ca.b_fs + (ca.b_s0 + ca.b_ds * fs)) * ca.b_ldtap;
           const int krow = (ca.taps == 0 ? k : cb) * BK;
@@ -554,10 +634,13 @@ gemm_tf32_persistent_kernel(const __grid_constant__ CUtensorMap tma_a, const __g
             }
           }
           __syncwarp();
+          }
         }
-        if (++s == S::STAGES) { s = 0; phase ^= 1u; }
+        if (++s == stages) { s = 0; phase ^= 1u; }
         turn ^= 1;
-        if (++cb == ca.cblocks) {                             // (never true for a plain matrix: cblocks == 0)
+        if constexpr (TAPS) {
+          if (++fs == 3) { fs = 0; ++cb; }
+        } else if (++cb == ca.cblocks) {                             // (never true for a plain matrix: cblocks == 0)
           cb = 0;
           if (++fs == ca.fs) { fs = 0; ++fr; }
         }
@@ -566,9 +649,9 @@ gemm_tf32_persistent_kernel(const __grid_constant__ CUtensorMap tma_a, const __g
     if constexpr (PAIR) {
       // the commits that free the last stages come from the first CTA: see them before this CTA may end.  From the next
       // k-block's stage on, every stage was last filled in phase `phase ^ 1` (passed at once where it never was).
-      for (int j = 0; j < S::STAGES && ok; ++j) {
+      for (uint32_t j = 0; j < stages && ok; ++j) {
         ok = mbar_wait_warp<true>(&empty[s], phase ^ 1u, &abort_flag);
-        if (++s == S::STAGES) { s = 0; phase ^= 1u; }
+        if (++s == stages) { s = 0; phase ^= 1u; }
       }
     }
   } else if (warp == MMA_WARP) {
@@ -593,9 +676,19 @@ gemm_tf32_persistent_kernel(const __grid_constant__ CUtensorMap tma_a, const __g
       for (int k = 0; k < nk; ++k) {
         if (!mbar_wait_warp<PAIR>(&full[s], phase, &abort_flag)) { ok = false; break; }
         tc_fence_after();
-        const uint64_t adesc = make_smem_desc(a_tiles + s * S::A_BYTES);
+        const uint64_t adesc = make_smem_desc(a_tiles + s * (uint32_t)a_pitch - (TAPS ? tc.lead : 0));
         if (elect_one()) {
-          if (!ca.b_mn) {
+          if constexpr (TAPS) {
+            // the three taps of the column: pixels `step` bytes further on each, the filter's rows from the last one back
+            const uint64_t down = (uint64_t)(tc.step >> 4);
+            const uint64_t bdesc = make_smem_desc_mn_rows(b_tiles + s * (uint32_t)B_STAGE, BK);
+#pragma unroll
+            for (int r = 0; r < 3; ++r)
+#pragma unroll
+              for (int kk = 0; kk < BK / UMMA_K; ++kk)
+                mma(tmem_c, adesc + (uint64_t)r * down + (uint64_t)(kk * 2), bdesc + (uint64_t)((2 - r) * (S::B_BYTES >> 4) + kk * 64), idesc | (1u << 16),
+                    (k | r | kk) != 0 ? 1u : 0u);
+          } else if (!ca.b_mn) {
             const uint64_t bdesc = make_smem_desc(b_tiles + s * S::B_BYTES);
 #pragma unroll
             for (int kk = 0; kk < BK / UMMA_K; ++kk)
@@ -611,7 +704,7 @@ gemm_tf32_persistent_kernel(const __grid_constant__ CUtensorMap tma_a, const __g
           if (k == nk - 1) commit(&acc_full[buf]);
         }
         __syncwarp();
-        if (++s == S::STAGES) { s = 0; phase ^= 1u; }
+        if (++s == stages) { s = 0; phase ^= 1u; }
       }
     }
   } else {
@@ -733,13 +826,14 @@ gemm_tf32_persistent_kernel(const __grid_constant__ CUtensorMap tma_a, const __g
             if (cc.hw != 0) {                    // rows = pixels (n, i, j) of a strided sub-grid: 4-D store map
               const int img = m0 / cc.hw, rem = m0 - img * cc.hw;
               const int i0 = rem / cc.w, j0 = rem - i0 * cc.w;
+              const int c2 = cc.nh ? img : i0, c3 = cc.nh ? i0 : img;
               if (accumulate)
                 asm volatile("cp.reduce.async.bulk.tensor.4d.global.shared::cta.add.tile.bulk_group [%0, {%2, %3, %4, %5}], [%1];"
-                             ::"l"(&tma_c), "r"(smem_u32(slab)), "r"(n0 + sl * 32), "r"(j0), "r"(i0), "r"(img)
+                             ::"l"(&tma_c), "r"(smem_u32(slab)), "r"(n0 + sl * 32), "r"(j0), "r"(c2), "r"(c3)
                              : "memory");
               else
                 asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.bulk_group [%0, {%2, %3, %4, %5}], [%1];"
-                             ::"l"(&tma_c), "r"(smem_u32(slab)), "r"(n0 + sl * 32), "r"(j0), "r"(i0), "r"(img)
+                             ::"l"(&tma_c), "r"(smem_u32(slab)), "r"(n0 + sl * 32), "r"(j0), "r"(c2), "r"(c3)
                              : "memory");
             } else if (accumulate)               // C += tile: the add happens in L2, C is never read by the SM
               asm volatile("cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.tile.bulk_group [%0, {%2, %3}], [%1];"
@@ -1190,6 +1284,7 @@ int make_map_mn3(CUtensorMap* map, const float* base, int64_t K, int64_t D, int6
 struct Plan {
   int bn, splits;
   bool pair;
+  bool taps;                                                 // 3x3 input gradient with shared pixels (TapCols)
   int b_cols() const { return pair ? bn / 2 : bn; }          // columns of B (box rows of its map) one CTA loads
   int rows() const { return pair ? 2 * BM : BM; }
 };
@@ -1213,31 +1308,32 @@ inline int pairs_at_once(const void* kernel, int threads, size_t smem) {
 
 // CTAs, or CTA pairs, of the persistent kernel that the device runs at once (pairs: half its SMs, unless a GPC has an odd
 // number of them); 0 when the kernel cannot be configured.
-template <int BN, bool AFFINE, bool PAIR>
+template <int BN, bool AFFINE, bool PAIR, bool TAPS>
 int persistent_workers() {
-  using S = PSmem<BN, PAIR>;
+  using S = PSmem<BN, PAIR, TAPS>;
   static int workers = 0;
   if (workers != 0) return workers;
-  if (cudaFuncSetAttribute(gemm_tf32_persistent_kernel<BN, AFFINE, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::TOTAL) != cudaSuccess) return 0;
+  if (cudaFuncSetAttribute(gemm_tf32_persistent_kernel<BN, AFFINE, PAIR, TAPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::TOTAL) != cudaSuccess) return 0;
   int n = sm_count();
-  if constexpr (PAIR) n = pairs_at_once((const void*)gemm_tf32_persistent_kernel<BN, AFFINE, PAIR>, PERSISTENT_THREADS, S::TOTAL);
+  if constexpr (PAIR) n = pairs_at_once((const void*)gemm_tf32_persistent_kernel<BN, AFFINE, PAIR, TAPS>, PERSISTENT_THREADS, S::TOTAL);
   return workers = n;
 }
 
 // Launch the persistent kernel on ready-made tensor maps (ca.taps == 0: ma is a 2-D map of A[M, K]).
-template <int BN, bool AFFINE, bool PAIR>
+template <int BN, bool AFFINE, bool PAIR, bool TAPS>
 int launch_persistent_maps(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mc, const ConvA& ca, const float* bias,
                            int M, int N, int K, int accumulate, float* col_partials, int* error_flag, cudaStream_t st,
-                           const BnFin* fin, const ConvC* cc, int splits, int cta_sums, const Affine* aff) {
-  using S = PSmem<BN, PAIR>;
-  const int workers_max = persistent_workers<BN, AFFINE, PAIR>();
+                           const BnFin* fin, const ConvC* cc, int splits, int cta_sums, const Affine* aff, const TapCols* tc) {
+  using S = PSmem<BN, PAIR, TAPS>;
+  if ((tc != nullptr && tc->box_bytes != 0) != TAPS) return (int)cudaErrorInvalidValue;
+  const int workers_max = persistent_workers<BN, AFFINE, PAIR, TAPS>();
   if (workers_max == 0) return (int)cudaGetLastError();
   constexpr int ROWS = PAIR ? 2 * BM : BM;
   int tiles_m = (M + ROWS - 1) / ROWS, tiles_n = (N + BN - 1) / BN;
-  if (splits < 1 || splits > (K + BK - 1) / BK) return (int)cudaErrorInvalidValue;
+  if (splits < 1 || splits > (TAPS ? 3 * ca.cblocks : (K + BK - 1) / BK)) return (int)cudaErrorInvalidValue;
   // a split contraction adds partial tiles into C: the caller zeroed C (or wants C += ...), and nothing that needs the
-  // finished values (column statistics) or a store map without a reduce form can ride along
-  if (splits > 1 && (!accumulate || col_partials != nullptr || (fin != nullptr && fin->acc != nullptr) || cc != nullptr))
+  // finished values (column statistics) can ride along
+  if (splits > 1 && (!accumulate || col_partials != nullptr || (fin != nullptr && fin->acc != nullptr) || (cc != nullptr && !cc->nh)))
     return (int)cudaErrorInvalidValue;
   int64_t total = (int64_t)tiles_m * tiles_n * splits;
   int64_t workers = total < workers_max ? total : workers_max;
@@ -1252,23 +1348,31 @@ int launch_persistent_maps(const CUtensorMap& ma, const CUtensorMap& mb, const C
     if (col_partials == nullptr || splits > 1 || tiles_n > workers) return (int)cudaErrorInvalidValue;
     workers = workers / tiles_n * tiles_n;
   }
-  gc::launch_cluster(gemm_tf32_persistent_kernel<BN, AFFINE, PAIR>, PAIR ? 2u : 1u, dim3((unsigned)(PAIR ? 2 * workers : workers)),
+  gc::launch_cluster(gemm_tf32_persistent_kernel<BN, AFFINE, PAIR, TAPS>, PAIR ? 2u : 1u, dim3((unsigned)(PAIR ? 2 * workers : workers)),
                      dim3(PERSISTENT_THREADS), (size_t)S::TOTAL, st, ma, mb, mc, ca, bias, M, N, K, tiles_m, tiles_n, splits, accumulate,
-                     col_partials, error_flag, gctc::tma_mode, f, cc != nullptr ? *cc : ConvC{0, 0}, cta_sums, aff != nullptr ? *aff : Affine{});
+                     col_partials, error_flag, gctc::tma_mode, f, cc != nullptr ? *cc : ConvC{}, cta_sums, aff != nullptr ? *aff : Affine{},
+                     tc != nullptr ? *tc : TapCols{});
   return (int)cudaGetLastError();
 }
 
 template <bool AFFINE = false>
 int launch_plan(const Plan& pl, const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mc, const ConvA& ca, const float* bias,
                 int M, int N, int K, int accumulate, float* col_partials, int* error_flag, cudaStream_t st,
-                const BnFin* fin = nullptr, const ConvC* cc = nullptr, int cta_sums = 0, const Affine* aff = nullptr) {
+                const BnFin* fin = nullptr, const ConvC* cc = nullptr, int cta_sums = 0, const Affine* aff = nullptr, const TapCols* tc = nullptr) {
   auto run = [&](auto launch) {
-    return launch(ma, mb, mc, ca, bias, M, N, K, accumulate, col_partials, error_flag, st, fin, cc, pl.splits, cta_sums, aff);
+    return launch(ma, mb, mc, ca, bias, M, N, K, accumulate, col_partials, error_flag, st, fin, cc, pl.splits, cta_sums, aff, tc);
   };
+  if (pl.taps) {
+    if constexpr (!AFFINE) {
+      if (pl.bn == 64) return pl.pair ? run(launch_persistent_maps<64, false, true, true>) : run(launch_persistent_maps<64, false, false, true>);
+      if (pl.bn == 128) return pl.pair ? run(launch_persistent_maps<128, false, true, true>) : run(launch_persistent_maps<128, false, false, true>);
+    }
+    return (int)cudaErrorInvalidValue;
+  }
   switch (pl.bn) {
-    case 64: return pl.pair ? run(launch_persistent_maps<64, AFFINE, true>) : run(launch_persistent_maps<64, AFFINE, false>);
-    case 128: return pl.pair ? run(launch_persistent_maps<128, AFFINE, true>) : run(launch_persistent_maps<128, AFFINE, false>);
-    case 256: return pl.pair ? run(launch_persistent_maps<256, AFFINE, true>) : run(launch_persistent_maps<256, AFFINE, false>);
+    case 64: return pl.pair ? run(launch_persistent_maps<64, AFFINE, true, false>) : run(launch_persistent_maps<64, AFFINE, false, false>);
+    case 128: return pl.pair ? run(launch_persistent_maps<128, AFFINE, true, false>) : run(launch_persistent_maps<128, AFFINE, false, false>);
+    case 256: return pl.pair ? run(launch_persistent_maps<256, AFFINE, true, false>) : run(launch_persistent_maps<256, AFFINE, false, false>);
     default: return (int)cudaErrorInvalidValue;
   }
 }
@@ -1277,9 +1381,9 @@ int launch_plan(const Plan& pl, const CUtensorMap& ma, const CUtensorMap& mb, co
 inline int plan_workers(const Plan& pl) {
   if (!pl.pair) return sm_count();
   switch (pl.bn) {
-    case 64: return persistent_workers<64, false, true>();
-    case 128: return persistent_workers<128, false, true>();
-    default: return persistent_workers<256, false, true>();
+    case 64: return persistent_workers<64, false, true, false>();
+    case 128: return persistent_workers<128, false, true, false>();
+    default: return persistent_workers<256, false, true, false>();
   }
 }
 
@@ -1348,32 +1452,34 @@ inline int launch_tn_plan(int bn, bool pair, const CUtensorMap& ma, const CUtens
 // `reuse`: how often an element of A is read (filter taps per input pixel of a convolution, 1 for a matrix).
 inline double plan_ns(const Plan& p, int M, int N, int K, double reuse) {
   static constexpr double stage[2][3] = {{235.0, 300.0, 490.0}, {205.0, 260.0, 400.0}};
+  static constexpr double taps_stage[2][2] = {{157.0, 200.0}, {103.0, 144.0}};      // 16x16x128, four waves against two
   const int num_k = (K + BK - 1) / BK;
   const int64_t items = (int64_t)((M + p.rows() - 1) / p.rows()) * ((N + p.bn - 1) / p.bn) * p.splits;
   const int64_t workers = p.pair ? sm_count() / 2 : sm_count(), waves = (items + workers - 1) / workers;
-  const double sm = (double)waves * ((num_k + p.splits - 1) / p.splits * stage[p.pair][p.bn == 64 ? 0 : (p.bn == 128 ? 1 : 2)] + 500.0);
+  const double sm = (double)waves * ((num_k + p.splits - 1) / p.splits * (p.taps ? taps_stage[p.pair][p.bn == 64 ? 0 : 1] : stage[p.pair][p.bn == 64 ? 0 : (p.bn == 128 ? 1 : 2)]) + 500.0);
   const double dram = ((double)M * K / reuse + (double)M * N * (p.splits > 1 ? 2.0 : 1.0) + (double)N * K) * 4.0 / 6500.0;
   return (sm > dram ? sm + 0.15 * dram : dram + 0.15 * sm) + (p.pair ? 1500.0 : 0.0);
 }
 
-// Candidates of the plan: widths that do not leave half a tile empty, pairs where there are two row tiles.
+// Candidates of the plan: widths that do not leave half a tile empty, pairs where there are two row tiles; for the input gradient of a 3x3
+// convolution whose filter columns can share their pixels (taps_ok) the kernel that does, which has tiles of up to 128 columns.
 template <typename F>
-inline void each_plan(int M, int N, F&& f) {
+inline void each_plan(int M, int N, bool taps_ok, F&& f) {
   const int cand[3] = {256, 128, 64};
+  const bool taps = taps_ok && gctc::taps_choice != 1;
   for (int i = 0; i < 3; ++i) {
     const int bn = cand[i];
     if (gctc::tile_choice ? bn != gctc::tile_choice : ((bn == 256 && N <= 128) || (bn == 128 && N <= 64))) continue;
     for (int pair = 0; pair < 2; ++pair)
-      if (pair == 0 ? (gctc::pair_choice != 2 || M <= BM) : (gctc::pair_choice != 1 && M > BM)) f(bn, pair != 0);
+      if (pair == 0 ? (gctc::pair_choice != 2 || M <= BM) : (gctc::pair_choice != 1 && M > BM)) f(Plan{bn, 1, pair != 0, taps && bn <= 128});
   }
 }
 
 // Tile width and pairing of a product that is not split: the candidate with the lowest modelled time.
-inline Plan pick_persistent(int M, int N, int K, double reuse = 1.0) {
-  Plan best{64, 1, false};
+inline Plan pick_persistent(int M, int N, int K, double reuse = 1.0, bool taps_ok = false) {
+  Plan best{64, 1, false, false};
   double best_t = 1e30;
-  each_plan(M, N, [&](int bn, bool pair) {
-    const Plan p{bn, 1, pair};
+  each_plan(M, N, taps_ok, [&](const Plan& p) {
     const double t = plan_ns(p, M, N, K, reuse);
     if (t < best_t) { best_t = t; best = p; }
   });
@@ -1387,17 +1493,17 @@ inline double stats_pass_ns(int64_t elements) { return 4200.0 + (double)elements
 // The same for a product whose output may be built from partial tiles (no column statistics wanted, plain 2-D output): the
 // contraction is also split where that pays.  extra_split_ns: what a caller pays elsewhere when the product is split
 // (zeroing C, a separate pass for the statistics).
-inline Plan plan_persistent(int M, int N, int K, double extra_split_ns, double reuse = 1.0) {
-  Plan pl = pick_persistent(M, N, K, reuse);
+inline Plan plan_persistent(int M, int N, int K, double extra_split_ns, double reuse = 1.0, bool taps_ok = false) {
+  Plan pl = pick_persistent(M, N, K, reuse, taps_ok);
   if (gctc::split_choice == 1) return pl;
-  const int num_k = (K + BK - 1) / BK;
   double best = plan_ns(pl, M, N, K, reuse);
-  each_plan(M, N, [&](int bn, bool pair) {
+  each_plan(M, N, taps_ok, [&](Plan p) {
+    const int num = (K + BK - 1) / BK / (p.taps ? 3 : 1);          // stages of the contraction
     for (int splits = 2; splits <= 16; ++splits) {
-      const int per = (num_k + splits - 1) / splits;
-      if (per < 6 || (splits - 1) * per >= num_k) continue;      // every split non-empty and long enough to fill the ring
+      const int per = (num + splits - 1) / splits;
+      if (per < (p.taps ? 2 : 6) || (splits - 1) * per >= num) continue;      // every split non-empty and long enough to fill the ring
       if (gctc::split_choice > 1 && splits != gctc::split_choice) continue;
-      const Plan p{bn, splits, pair};
+      p.splits = splits;
       const double t = plan_ns(p, M, N, K, reuse) + extra_split_ns;
       if (t < best * 0.93 || (gctc::split_choice > 1 && pl.splits == 1)) { best = t; pl = p; }
     }

@@ -183,6 +183,7 @@ def cuda():
         _declare(lib, "gc_cuda_max_pool2", c_int, [P, c_int, c_int, c_int, c_int, P, P])
         _declare(lib, "gc_cuda_bn_eval_apply", c_int, [P, c_i64, c_int, P, P, c_float, P, P, P, c_int, P, P])
         _declare(lib, "gc_cuda_conv_stat_rows", c_int, [c_int] * 5)
+        _declare(lib, "gc_cuda_tc_taps_config", None, [c_int])
         _declare(lib, "gc_cuda_bn_fused_supported", c_int, [c_i64, c_int])
         _declare(lib, "gc_cuda_bn_fused_blocks", c_int, [c_i64, c_int, c_int])
         _declare(lib, "gc_cuda_bn_fused_scratch_bytes", c_i64, [])

@@ -148,6 +148,12 @@ def configure_pair(pairs=0):
     nat.cuda().gc_cuda_tc_pair_config(int(pairs))
 
 
+def configure_taps(taps=0):
+    """Input gradients of 3x3, stride-1 convolutions with one load of the pixels per filter column: 0 = wherever the shape allows it, 1 = never
+    (a load per filter tap) -- for measurements and tests."""
+    nat.cuda().gc_cuda_tc_taps_config(int(taps))
+
+
 def configure_tn(ctas_per_sm=1, min_kblocks=8):
     """Split-K policy of ``gemm_tn_tf32`` (for measurements)."""
     nat.cuda().gc_cuda_gemm_tn_config(int(ctas_per_sm), int(min_kblocks))
