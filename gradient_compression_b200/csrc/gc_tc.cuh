@@ -48,7 +48,6 @@ constexpr int GEMM_THREADS = 192;           // one-tile-per-CTA kernel: producer
 constexpr int PRODUCER_WARPS = 2;
 constexpr int MMA_WARP = PRODUCER_WARPS;     // warp that allocates TMEM and issues tcgen05.mma
 constexpr int FIRST_EPI_WARP = PRODUCER_WARPS + 1;
-constexpr int TN_THREADS = 32 * FIRST_EPI_WARP + 128;
 constexpr unsigned long long WAIT_LIMIT_NS = 2000000000ull;   // a wait gives up after two seconds
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -235,8 +234,11 @@ __device__ __forceinline__ uint32_t cluster_addr(const void* p, uint32_t rank) {
   return a;
 }
 // Every thread of both CTAs of a pair.
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
 __device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+  cluster_arrive();
+  cluster_wait();
 }
 
 // Where the rows of an operand come from when it is an NHWC activation [N, H, W, C] read through a 4-D map
@@ -477,6 +479,7 @@ __device__ __forceinline__ void mbar_arrive_remote(uint32_t cluster_address) {
 
 constexpr int EPI_GROUPS = 2;
 constexpr int PERSISTENT_THREADS = 32 * FIRST_EPI_WARP + 128 * EPI_GROUPS;
+constexpr int TN_THREADS = PERSISTENT_THREADS;
 
 // AFFINE: the epilogue of inference (a kernel of its own: its residual registers slowed the training epilogue by 3 %).
 //
@@ -520,6 +523,7 @@ gemm_tf32_persistent_kernel(const __grid_constant__ CUtensorMap tma_a, const __g
   const int rank = PAIR ? (int)cluster_rank() : 0;
   const int worker = PAIR ? (int)(blockIdx.x >> 1) : (int)blockIdx.x, workers = PAIR ? (int)(gridDim.x >> 1) : (int)gridDim.x;
 
+  if (threadIdx.x == 32 * FIRST_EPI_WARP && (tma_mode & 1)) { tma_prefetch_map(&tma_a); tma_prefetch_map(&tma_b); tma_prefetch_map(&tma_c); }
   if (threadIdx.x == 0) {
     abort_flag = 0;
     for (int g = 0; g < EPI_GROUPS; ++g) epi_go[g] = 1;
@@ -547,8 +551,8 @@ gemm_tf32_persistent_kernel(const __grid_constant__ CUtensorMap tma_a, const __g
     if (quads != 0) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
   tc_fence_before();
-  __syncthreads();
-  if constexpr (PAIR) cluster_sync_all();      // the other CTA's barriers and TMEM are in place
+  if constexpr (PAIR) cluster_sync_all();      // every thread of both CTAs: the other one's barriers and TMEM are in place, too
+  else __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
   // everything above (barriers, TMEM) overlapped the tail of the previous kernel of the stream; its results are
@@ -558,7 +562,6 @@ gemm_tf32_persistent_kernel(const __grid_constant__ CUtensorMap tma_a, const __g
 
   if (warp < PRODUCER_WARPS) {
     // producer warp p fills the stages of k-blocks it == p (mod PRODUCER_WARPS) of the ring
-    if ((tma_mode & 1) && elect_one()) { tma_prefetch_map(&tma_a); tma_prefetch_map(&tma_b); }
     uint32_t s = 0, phase = 0;                                // stage and its phase of the next k-block, over all tiles
     static_assert(PRODUCER_WARPS == 2, "two warps take turns");
     int turn = 0;                                             // producer warp that fills it
@@ -653,6 +656,7 @@ gemm_tf32_persistent_kernel(const __grid_constant__ CUtensorMap tma_a, const __g
         ok = mbar_wait_warp<true>(&empty[s], phase ^ 1u, &abort_flag);
         if (++s == stages) { s = 0; phase ^= 1u; }
       }
+      cluster_arrive();
     }
   } else if (warp == MMA_WARP) {
     constexpr uint32_t idesc = make_idesc(BN, PAIR ? 2 * BM : BM);
@@ -707,6 +711,7 @@ gemm_tf32_persistent_kernel(const __grid_constant__ CUtensorMap tma_a, const __g
         if (++s == stages) { s = 0; phase ^= 1u; }
       }
     }
+    if constexpr (PAIR) cluster_arrive();
   } else {
     // Two epilogue groups of four warps (TMEM lane quarters warp & 3); group g drains the 32-column slabs
     // g, g + 2, ... of every tile through its own half of the staging ring, with its own named barrier and its
@@ -764,17 +769,22 @@ gemm_tf32_persistent_kernel(const __grid_constant__ CUtensorMap tma_a, const __g
       tc_fence_after();
       const uint32_t lane_base = tmem_base + ((uint32_t)(lg * 32) << 16) + buf * (uint32_t)BN;
       const bool full_rows = m0 + BM <= M;
+      // The ring's stages are done with once a CTA's last accumulator is complete: that tile's slabs are staged there, each in a
+      // place of its own, and none waits for a store to have read the one before (the end of a launch, 2.2 us from the last
+      // accumulator to the last store at 128 columns, was mostly that wait).
+      const bool last = t + workers >= total_items;
+      static_assert(SLABS * S::SLAB_BYTES <= S::RING_BYTES, "a tile's slabs in the ring");
 #pragma unroll 1
       for (int sl = grp; sl < SLABS; sl += EPI_GROUPS, ++sc) {
-        uint8_t* slab = my_staging + (sc % RING) * S::SLAB_BYTES;
+        uint8_t* slab = last ? base + sl * S::SLAB_BYTES : my_staging + (sc % RING) * S::SLAB_BYTES;
         if (aff_on) {                                          // the barrier that ended the last slab lets them be overwritten
           col_affine[(ew & 3) * 32 + lane] = cval;
           if ((ew & 3) == 0) col_affine[4 * 32 + lane] = cbias;
           if (sl + EPI_GROUPS < SLABS) load_columns(n0 + (sl + EPI_GROUPS) * 32);
         }
         // the store that last read this buffer was committed RING groups ago
-        if (issuer) asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(RING - 1) : "memory");
-        group_bar(grp);
+        if (issuer && !last) asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(RING - 1) : "memory");
+        if (AFFINE || !last) group_bar(grp);
         if (with_res) {
 #pragma unroll
           for (int i = 0; i < 8; ++i) {
@@ -818,7 +828,9 @@ gemm_tf32_persistent_kernel(const __grid_constant__ CUtensorMap tma_a, const __g
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         group_bar(grp);
         if (issuer) {
-          if (sl + EPI_GROUPS >= SLABS) {                      // the group has read its share of the accumulator
+          // the group has read its share of the accumulator; nobody waits for that where no later tile uses the buffer (and a
+          // signal that nobody waits for could come to a CTA that has ended)
+          if (sl + EPI_GROUPS >= SLABS && t + 2 * workers < total_items) {
             if constexpr (PAIR) mbar_arrive_remote(cluster_addr(&acc_empty[buf], 0));
             else mbar_arrive(&acc_empty[buf]);
           }
@@ -896,6 +908,7 @@ gemm_tf32_persistent_kernel(const __grid_constant__ CUtensorMap tma_a, const __g
         }
       }
     }
+    if constexpr (PAIR) cluster_arrive();
     if (cta_sums && drained_all && te < (SLABS / EPI_GROUPS) * 32) {
       // one row of partial sums per CTA that stays on this column tile (instead of one per row tile); where a CTA has several
       // tiles, a second set of rows carries what the first one's rounding left out
@@ -952,7 +965,9 @@ gemm_tf32_persistent_kernel(const __grid_constant__ CUtensorMap tma_a, const __g
   }
   tc_fence_before();
   __syncthreads();
-  if constexpr (PAIR) cluster_sync_all();      // nothing of the other CTA reads or signals this one's shared memory any more
+  // Every thread of both CTAs has come to the end of its part (cluster_arrive above; the last statistics and the wait for the stores
+  // hide the way there and back): nothing of the other CTA reads or signals this one's shared memory or TMEM any more.
+  if constexpr (PAIR) cluster_wait();
   if (warp == MMA_WARP) {
     tc_fence_after();
     if constexpr (PAIR)
@@ -978,19 +993,18 @@ gemm_tf32_persistent_kernel(const __grid_constant__ CUtensorMap tma_a, const __g
 // PAIR: as in the persistent kernel, two CTAs share a tile of 256 x BN, each with its 128 columns of A and half of B's.
 template <int BN, bool PAIR>
 struct TnSmem {
-  static constexpr int STAGES = PAIR ? ((BN <= 128) ? 8 : 6) : ((BN <= 64) ? 8 : ((BN <= 128) ? 6 : 4));
   static constexpr int B_COLS = PAIR ? BN / 2 : BN;
   static constexpr int CHUNK_BYTES = TBK * 128;             // one TMA box: 32 floats of the output dimension x TBK rows
   static constexpr int A_BYTES = BM * TBK * 4;
   static constexpr int B_BYTES = B_COLS * TBK * 4;
+  static constexpr int STAGES = (232448 - 1024 - 256) / (A_BYTES + B_BYTES);
   static constexpr int RING_BYTES = STAGES * (A_BYTES + B_BYTES);
-  static constexpr int NSLAB = 2;
-  static constexpr int SLAB_BYTES = BM * 128;
-  static constexpr int STAGING_OFF = RING_BYTES;
-  static constexpr int BAR_OFF = STAGING_OFF + NSLAB * SLAB_BYTES;
+  static constexpr int SLAB_BYTES = BM * 128;               // the one tile's slabs are staged in the ring, whose stages are done with by then
+  static constexpr int BAR_OFF = RING_BYTES;
   static constexpr int TOTAL = 1024 + BAR_OFF + 256;
   static constexpr int TMEM_COLS = BN == 192 ? 256 : BN;    // TMEM is allocated in powers of two
-  static_assert(TOTAL <= 232448, "shared memory of one CTA");
+  static_assert(TOTAL <= 232448 && (2 * STAGES + 1) * 8 + 4 <= 256, "shared memory of one CTA");
+  static_assert(BN / 32 * SLAB_BYTES <= RING_BYTES, "a tile's slabs in the ring");
 };
 
 __host__ __device__ constexpr uint32_t make_idesc_mn(int n, int m = BM) {
@@ -1007,13 +1021,12 @@ gemm_tn_tf32_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_cons
   uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   uint8_t* a_tiles = base;
   uint8_t* b_tiles = base + S::STAGES * S::A_BYTES;
-  uint8_t* staging = base + S::STAGING_OFF;
   uint64_t* full = reinterpret_cast<uint64_t*>(base + S::BAR_OFF);
   uint64_t* empty = full + S::STAGES;
   uint64_t* acc_ready = empty + S::STAGES;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_ready + 1);
   __shared__ int abort_flag;
-  __shared__ int epi_go;
+  __shared__ int epi_go[EPI_GROUPS];
 
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   const int rank = PAIR ? (int)cluster_rank() : 0, worker = PAIR ? (int)(blockIdx.x >> 1) : (int)blockIdx.x;
@@ -1025,9 +1038,9 @@ gemm_tn_tf32_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_cons
   const int k_end = k_begin + kblocks_per_split < total_k ? k_begin + kblocks_per_split : total_k;
   const int num_k = k_end > k_begin ? k_end - k_begin : 0;
 
+  if (threadIdx.x == 32 * FIRST_EPI_WARP && (tma_mode & 1)) { tma_prefetch_map(&tma_a); tma_prefetch_map(&tma_b); tma_prefetch_map(&tma_c); }
   if (threadIdx.x == 0) {
     abort_flag = 0;
-    epi_go = 1;
     for (int s = 0; s < S::STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
     mbar_init(acc_ready, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -1043,15 +1056,14 @@ gemm_tn_tf32_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_cons
     }
   }
   tc_fence_before();
-  __syncthreads();
   if constexpr (PAIR) cluster_sync_all();
+  else __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
 
   if (num_k > 0) {
     if (warp < PRODUCER_WARPS) {
       // a stage is BM / 32 + BN / 32 boxes of 32 floats x TBK rows; producer warp p fills the stages k == p (mod PRODUCER_WARPS)
-      if ((tma_mode & 1) && elect_one()) { tma_prefetch_map(&tma_a); tma_prefetch_map(&tma_b); }
       // weight gradient of an R x S convolution: column n of dW[Cout, taps * Cin] belongs to filter tap n / Cin, channel
       // n % Cin; a tile narrower than Cin stays inside one tap, a wider one (Cin = 64) covers several taps side by side.
       // Box c of a stage reads the pixels of its tap, shifted by (fr, fs), for the TBK output positions of the k-block.
@@ -1152,22 +1164,21 @@ gemm_tn_tf32_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_cons
         if (++s == S::STAGES) { s = 0; phase ^= 1u; }
       }
     } else {
+      // two groups of four warps (TMEM lane quarters warp & 3) take alternate slabs
+      const int ew = warp - FIRST_EPI_WARP, grp = ew >> 2;
       const int lg = warp & 3;
       const int r = lg * 32 + lane;
-      const int te = (warp - FIRST_EPI_WARP) * 32 + lane;
-      const bool issuer = te == 0;
+      const bool issuer = (ew & 3) == 0 && lane == 0;
       const bool got = (tma_mode & 4) ? mbar_wait_idle(acc_ready, 0u, &abort_flag, 128u) : mbar_wait(acc_ready, 0u, &abort_flag);
-      if (issuer) epi_go = (got && abort_flag == 0) ? 1 : 0;
-      asm volatile("bar.sync 1, 128;" ::: "memory");
-      if (epi_go) {
+      if (issuer) epi_go[grp] = (got && abort_flag == 0) ? 1 : 0;
+      group_bar(grp);
+      if (epi_go[grp]) {
         tc_fence_after();
         const uint32_t lane_base = tmem_base + ((uint32_t)(lg * 32) << 16);
         constexpr int SLABS = BN / 32;
 #pragma unroll 1
-        for (int sl = 0; sl < SLABS; ++sl) {
-          uint8_t* slab = staging + (sl % S::NSLAB) * S::SLAB_BYTES;
-          if (issuer) asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(S::NSLAB - 1) : "memory");
-          asm volatile("bar.sync 1, 128;" ::: "memory");
+        for (int sl = grp; sl < SLABS; sl += EPI_GROUPS) {
+          uint8_t* slab = base + sl * S::SLAB_BYTES;
           uint32_t ra[16], rb[16];
           tmem_ld16_nowait(lane_base + (uint32_t)(sl * 32), ra);
           tmem_ld16_nowait(lane_base + (uint32_t)(sl * 32 + 16), rb);
@@ -1179,7 +1190,7 @@ gemm_tn_tf32_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_cons
                 make_float4(__uint_as_float(src[0]), __uint_as_float(src[1]), __uint_as_float(src[2]), __uint_as_float(src[3]));
           }
           asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-          asm volatile("bar.sync 1, 128;" ::: "memory");
+          group_bar(grp);
           if (issuer) {
             if (n0 + sl * 32 < No && (!PAIR || m0 < Mo))
               asm volatile("cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.tile.bulk_group [%0, {%2, %3}], [%1];"
@@ -1189,12 +1200,13 @@ gemm_tn_tf32_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_cons
           }
         }
       }
-      if (issuer) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
     }
   }
+  if constexpr (PAIR) cluster_arrive();        // waited for below, behind the stores' reading of shared memory
+  if (num_k > 0 && warp >= FIRST_EPI_WARP && ((warp - FIRST_EPI_WARP) & 3) == 0 && lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
   tc_fence_before();
   __syncthreads();
-  if constexpr (PAIR) cluster_sync_all();
+  if constexpr (PAIR) cluster_wait();
   if (warp == MMA_WARP) {
     tc_fence_after();
     if constexpr (PAIR)
