@@ -430,9 +430,10 @@ int gc_cuda_conv_wgrad_supported(int N, int H, int W, int Cin, int Cout, int R, 
 }
 
 // dw[Cout, R*R*Cin] += dy[N*Ho*Wo, Cout]^T x_shifted: zero dw first for a plain gradient (the split contraction adds its
-// partial tiles with TMA reduce stores, in no fixed order).
+// partial tiles with TMA reduce stores, in no fixed order).  beside: the launch in front on the stream is an input-gradient kernel of this library that
+// writes neither dy, x nor dw: with programmatic launches the two run side by side.
 int gc_cuda_conv_wgrad(const float* dy, const float* x, float* dw, int N, int H, int W, int Cin, int Cout, int R, int stride,
-                       int pad, int* error_flag, void* cs) {
+                       int pad, int* error_flag, void* cs, int beside) {
   Shape s;
   if (!make_shape(N, H, W, Cin, Cout, R, stride, pad, &s) || !wgrad_ok(s)) return (int)cudaErrorInvalidValue;
   if ((reinterpret_cast<uintptr_t>(x) & 15u) || (reinterpret_cast<uintptr_t>(dy) & 15u) || (reinterpret_cast<uintptr_t>(dw) & 15u))
@@ -454,7 +455,7 @@ int gc_cuda_conv_wgrad(const float* dy, const float* x, float* dw, int N, int H,
     return (int)cudaErrorInvalidValue;
   const ConvA ca = conv_a(s);
   cudaStream_t st = (cudaStream_t)cs;
-  return launch_tn_plan(tile, tn_pair(P, Cout, No, tile), ma, mb, mc, ca, P, Cout, No, error_flag, st, box3d);
+  return launch_tn_plan(tile, tn_pair(P, Cout, No, tile), ma, mb, mc, ca, P, Cout, No, error_flag, st, box3d, beside);
 }
 
 // Taps of a stride-2 convolution that reach input pixels of parity `par` along one axis: r = par + pad - 2 d for d = 0, 1, ...

@@ -179,24 +179,19 @@ __device__ __forceinline__ uint32_t ld_acquire_gpu(const uint32_t* p) {
 // draining, which hides its launch latency and prologue.  Such a kernel calls pdl_wait() before it touches
 // memory (the wait returns once the previous kernel has completed and its writes are visible; it returns at once
 // in a kernel launched the ordinary way), and pdl_launch_dependents() to let its own successor be scheduled.
-// Off unless GCB200_PDL=1: inside a replayed CUDA graph, where the training step runs, kernel-to-kernel gaps are
-// already about a microsecond.  Measured on the ResNet-50 step: with an explicit trigger at the top of every kernel 1.8 % slower
-// (successors become resident while their predecessor is in full flight), with the implicit trigger at block exit 0.15 %
-// faster (17 219 / 17 214 against 17 187 / 17 191 img/s); eager (uncaptured) loops are where it can pay.
+// GCB200_PDL=0 turns it off.  Who takes part: the tensor-core kernels (their barriers, TMEM and tensor maps are ready when the previous
+// kernel ends: 1.7 us from launch to launch and 0.5-1.1 us of set-up a launch otherwise), and the small batch-norm kernels.  The fused batch-norm kernels release
+// their successors but are launched the ordinary way (gc_bn_fused.cu says why).  Every kernel releases its successors at its start, behind its own wait: steps of
+// ResNet-50 / VGG-16 / ResNet-18 at batch 31 in us, and an evaluation batch of ResNet-50: 6086 / 1051 / 1056 / 2843 without, 5881 / 1029 / 1012 / 2733 with it;
+// released when the last tile is accumulated instead 5913 / 1030 / 1015 / 2706.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void pdl_launch_dependents() {
-#if defined(GC_PDL_EARLY_TRIGGER)
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");       // at the top of a kernel: successors become resident at once
-#endif
-  // default: no explicit trigger -- the successor is released as this kernel's blocks exit, so only its launch latency and
-  // prologue overlap this kernel's tail, and it never takes SM resources from a kernel that is still in full flight
-}
+__device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 inline bool pdl_enabled() {
   static int on = -1;
   if (on < 0) {
     const char* e = getenv("GCB200_PDL");
-    on = (e != nullptr && e[0] == '1') ? 1 : 0;
+    on = (e != nullptr && e[0] == '0') ? 0 : 1;
   }
   return on == 1;
 }

@@ -280,7 +280,7 @@ int launch_persistent(const Plan& pl, const float* A, const float* B, float* C, 
 }
 
 int launch_tn(int bn, const float* A, const float* B, float* C, int P, int Mo, int No, int64_t lda, int64_t ldb, int64_t ldc,
-              int* error_flag, cudaStream_t st) {
+              int* error_flag, cudaStream_t st, int beside) {
   CUtensorMap ma, mb, mc;
   const bool pair = tn_pair(P, Mo, No, bn);
   int box3d = 0;        // whole-operand 3-D boxes where the matrix is made of whole 32-float chunks
@@ -290,7 +290,7 @@ int launch_tn(int bn, const float* A, const float* B, float* C, int P, int Mo, i
   else if (make_map_mn(&mb, B, P, No, ldb) != 0) return (int)cudaErrorInvalidValue;
   if (make_map(&mc, C, Mo, No, ldc, BM) != 0)
     return (int)cudaErrorInvalidValue;
-  return launch_tn_plan(bn, pair, ma, mb, mc, ConvA{}, P, Mo, No, error_flag, st, box3d);
+  return launch_tn_plan(bn, pair, ma, mb, mc, ConvA{}, P, Mo, No, error_flag, st, box3d, beside);
 }
 
 // 0 = choose, 1 = one tile per CTA, 2 = persistent;  tile width 0 = choose
@@ -401,13 +401,13 @@ int gc_cuda_gemm_tn_tf32_supported(const void* A, const void* B, const void* C, 
 }
 
 // C[Mo, No] += A[P, Mo]^T * B[P, No] (weight gradient of a 1x1 convolution: A = dY, B = X).  The partial products of
-// the split contraction are added onto C by TMA reduce stores: zero C first for a plain product.
+// the split contraction are added onto C by TMA reduce stores: zero C first for a plain product.  beside: as in gc_cuda_conv_wgrad.
 int gc_cuda_gemm_tn_tf32(const float* A, const float* B, float* C, int P, int Mo, int No, int64_t lda, int64_t ldb, int64_t ldc,
-                         int* error_flag, void* cs) {
+                         int* error_flag, void* cs, int beside) {
   if (!gc_cuda_gemm_tn_tf32_supported(A, B, C, P, Mo, No, lda, ldb, ldc)) return (int)cudaErrorInvalidValue;
   cudaStream_t st = (cudaStream_t)cs;
   int bn = gctc::tile_choice ? gctc::tile_choice : (No <= 64 ? 64 : (No <= 128 ? 128 : 256));
-  return launch_tn(bn, A, B, C, P, Mo, No, lda, ldb, ldc, error_flag, st);
+  return launch_tn(bn, A, B, C, P, Mo, No, lda, ldb, ldc, error_flag, st, beside);
 }
 
 }  // extern "C"

@@ -991,6 +991,8 @@ gemm_tf32_persistent_kernel(const __grid_constant__ CUtensorMap tma_a, const __g
 // with TMA reduce stores, so C must hold the value to add to (zeros for a plain product).
 //
 // PAIR: as in the persistent kernel, two CTAs share a tile of 256 x BN, each with its 128 columns of A and half of B's.
+//
+// Two groups of epilogue warps, and no staging buffers beside the ring: with one group and two buffers the ring had one or two stages less.
 template <int BN, bool PAIR>
 struct TnSmem {
   static constexpr int B_COLS = PAIR ? BN / 2 : BN;
@@ -1015,7 +1017,7 @@ template <int BN, bool PAIR>
 __global__ void __launch_bounds__(TN_THREADS, 1)
 gemm_tn_tf32_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
                     const __grid_constant__ CUtensorMap tma_c, const ConvA ca, int P, int Mo, int No, int tiles_n, int splits,
-                    int kblocks_per_split, int* __restrict__ error_flag, int tma_mode, int box3d) {
+                    int kblocks_per_split, int* __restrict__ error_flag, int tma_mode, int box3d, int wait_late) {
   using S = TnSmem<BN, PAIR>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -1060,6 +1062,10 @@ gemm_tn_tf32_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_cons
   else __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+  // wait_late: the kernel in front on the stream is an input-gradient kernel of the same layer, which writes nothing that is read here and let
+  // this one start only when the kernels before it were complete.  The two run side by side; this one ends after the other.
+  if (!wait_late) gc::pdl_wait();
+  gc::pdl_launch_dependents();
 
   if (num_k > 0) {
     if (warp < PRODUCER_WARPS) {
@@ -1204,6 +1210,7 @@ gemm_tn_tf32_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_cons
   }
   if constexpr (PAIR) cluster_arrive();        // waited for below, behind the stores' reading of shared memory
   if (num_k > 0 && warp >= FIRST_EPI_WARP && ((warp - FIRST_EPI_WARP) & 3) == 0 && lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+  if (wait_late) gc::pdl_wait();
   tc_fence_before();
   __syncthreads();
   if constexpr (PAIR) cluster_wait();
@@ -1420,7 +1427,7 @@ inline bool tn_pair(int P, int Mo, int No, int bn) {
 
 template <int BN, bool PAIR>
 int launch_tn_maps(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mc, const ConvA& ca, int P, int Mo, int No,
-                   int* error_flag, cudaStream_t st, int box3d) {
+                   int* error_flag, cudaStream_t st, int box3d, int wait_late) {
   using S = TnSmem<BN, PAIR>;
   static int at_once = 0;
   if (at_once == 0) {
@@ -1440,13 +1447,13 @@ int launch_tn_maps(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorM
   int per = (total_k + splits - 1) / splits;
   splits = (total_k + per - 1) / per;
   const cudaError_t e = gc::launch_cluster(gemm_tn_tf32_kernel<BN, PAIR>, PAIR ? 2u : 1u, dim3((unsigned)((PAIR ? 2 : 1) * tiles * splits)), dim3(TN_THREADS),
-                                           (size_t)S::TOTAL, st, ma, mb, mc, ca, P, Mo, No, tiles_n, splits, per, error_flag, gctc::tma_mode, box3d);
+                                           (size_t)S::TOTAL, st, ma, mb, mc, ca, P, Mo, No, tiles_n, splits, per, error_flag, gctc::tma_mode, box3d, wait_late);
   return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
 }
 
 inline int launch_tn_plan(int bn, bool pair, const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mc, const ConvA& ca, int P, int Mo, int No,
-                          int* error_flag, cudaStream_t st, int box3d) {
-  auto run = [&](auto launch) { return launch(ma, mb, mc, ca, P, Mo, No, error_flag, st, box3d); };
+                          int* error_flag, cudaStream_t st, int box3d, int wait_late) {
+  auto run = [&](auto launch) { return launch(ma, mb, mc, ca, P, Mo, No, error_flag, st, box3d, wait_late); };
   switch (bn) {
     case 64: return run(launch_tn_maps<64, false>);
     case 128: return pair ? run(launch_tn_maps<128, true>) : run(launch_tn_maps<128, false>);

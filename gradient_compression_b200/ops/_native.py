@@ -166,7 +166,7 @@ def cuda():
         _declare(lib, "gc_cuda_gemm_tf32_m_tiles", c_int, [c_int])
         _declare(lib, "gc_cuda_gemm_tn_config", None, [c_int, c_int])
         _declare(lib, "gc_cuda_gemm_tn_tf32_supported", c_int, [P, P, P, c_int, c_int, c_int, c_i64, c_i64, c_i64])
-        _declare(lib, "gc_cuda_gemm_tn_tf32", c_int, [P, P, P, c_int, c_int, c_int, c_i64, c_i64, c_i64, P, P])
+        _declare(lib, "gc_cuda_gemm_tn_tf32", c_int, [P, P, P, c_int, c_int, c_int, c_i64, c_i64, c_i64, P, P, c_int])
         _declare(lib, "gc_cuda_gemm_tf32_config", None, [c_int, c_int])
         _declare(lib, "gc_cuda_tc_tma_mode", None, [c_int])
         _declare(lib, "gc_cuda_conv_fwd_supported", c_int, [c_int] * 8)
@@ -193,7 +193,7 @@ def cuda():
         _declare(lib, "gc_cuda_conv_dgrad_s2", c_int, [P, P, P] + [c_int] * 7 + [P, P])
         _declare(lib, "gc_cuda_conv_dgrad_s2_add", c_int, [P, P, P] + [c_int] * 8 + [P, P])
         _declare(lib, "gc_cuda_conv_wgrad_supported", c_int, [c_int] * 8)
-        _declare(lib, "gc_cuda_conv_wgrad", c_int, [P, P, P] + [c_int] * 8 + [P, P])
+        _declare(lib, "gc_cuda_conv_wgrad", c_int, [P, P, P] + [c_int] * 8 + [P, P] + [c_int])
         _declare(lib, "gc_cuda_im2col_small", c_int, [P, P] + [c_int] * 7 + [P, P, c_int, P])
         _declare(lib, "gc_cuda_bn_finalize_partials", c_int, [P, c_int, c_i64, c_int, P, P, P, c_float, c_float, P])
         _declare(lib, "gc_cuda_varpack_workspace_bytes", c_i64, [c_i64])

@@ -302,7 +302,7 @@ def conv_forward(x, w, bias=None, stride=1, pad=1, col_partials=None, out=None, 
     return out
 
 
-def conv_wgrad(dy, x, r, stride, pad, out=None):
+def conv_wgrad(dy, x, r, stride, pad, out=None, beside=False):
     """Weight gradient ``[Cout, R*R*Cin]`` (channels-last filter order) of ``conv2d(x, w, stride, pad)`` given the
     channels-last output gradient ``dy``; added onto ``out`` when given."""
     n, cin, h, wd = x.shape
@@ -310,7 +310,7 @@ def conv_wgrad(dy, x, r, stride, pad, out=None):
     dw = out if out is not None else torch.zeros(cout, r * r * cin, dtype=torch.float32, device=x.device)
     with torch.cuda.device(x.device):
         nat.check(nat.cuda().gc_cuda_conv_wgrad(dy.data_ptr(), x.data_ptr(), dw.data_ptr(), n, h, wd, cin, cout, r, stride, pad,
-                                                _err(x.device), nat.stream_ptr()), "conv_wgrad")
+                                                _err(x.device), nat.stream_ptr(), int(beside)), "conv_wgrad")
     return dw
 
 
@@ -470,6 +470,7 @@ class _ConvBNAct(torch.autograd.Function):
                                                    gamma.data_ptr(), beta.data_ptr(), sums.data_ptr(), int(ctx.relu),
                                                    dconv.data_ptr(), nat.ptr(dres), st()), "bn_bwd_apply")
             dx = None
+            beside = False          # the last launch is one of the input-gradient kernels
             link, donate = ctx.link, ctx.donate
             if donate is not None and (donate.conv_done or donate.stash is not None or donate.later is not None):
                 donate = None
@@ -496,8 +497,10 @@ class _ConvBNAct(torch.autograd.Function):
                     dx = acc if accumulate else torch.empty_like(x)
                     nat.check(lib.gc_cuda_conv_dgrad(dconv.data_ptr(), w.data_ptr(), dx.data_ptr(), n, h_in, w_in, cin, cout, r, pad,
                                                      int(accumulate), _err(x.device), st()), "conv_dgrad")
+                    beside = True
                     if acc is not None and not accumulate:
                         dx += acc
+                        beside = False
                 elif tc_dgrad:
                     wd_ = _dgrad_weights.get(w)           # [Cin, taps * Cout]: the K-major operand of dX = dY (*) rot(W)
                     accumulate = acc is not None and gemm.can_accumulate(_as_2d(acc))
@@ -516,6 +519,7 @@ class _ConvBNAct(torch.autograd.Function):
                     nat.check(lib.gc_cuda_conv_dgrad_s2(dconv.data_ptr(), w.data_ptr(), dx.data_ptr(), n,
                                                         x.shape[2], x.shape[3], cin, cout, r, pad, _err(x.device), st()),
                               "conv_dgrad_s2")
+                    beside = acc is None
                     if acc is not None:
                         dx += acc
                 else:
@@ -527,6 +531,7 @@ class _ConvBNAct(torch.autograd.Function):
                 link.conv_done = True
                 if link.later is not None:
                     (later_dy, later_w, later_pad), link.later = link.later, None
+                    beside = beside and dx.is_contiguous(memory_format=torch.channels_last)
                     dx = dx.contiguous(memory_format=torch.channels_last)
                     nat.check(lib.gc_cuda_conv_dgrad_s2_add(later_dy.data_ptr(), later_w.data_ptr(), dx.data_ptr(), n, x.shape[2], x.shape[3], cin,
                                                             later_dy.shape[1], 1, later_pad, 1, _err(x.device), st()), "conv_dgrad_s2")
@@ -539,11 +544,11 @@ class _ConvBNAct(torch.autograd.Function):
                 slot = _slot_of(w) if WGRAD_ENABLED else None       # the owner's gradient storage, or None: return a tensor
                 if mode == "gemm" and WGRAD_ENABLED and cout % 32 == 0 and cin % 32 == 0:
                     # dW[Cout, Cin] = dY^T X over all positions: split-K GEMM with MN-major tcgen05 operands
-                    dw2d = gemm.gemm_tn_tf32(_as_2d(dconv), _as_2d(x), out=slot, accumulate=slot is not None)
+                    dw2d = gemm.gemm_tn_tf32(_as_2d(dconv), _as_2d(x), out=slot, accumulate=slot is not None, beside=beside and slot is not None)
                     dw = None if slot is not None else dw2d.view(cout, cin, 1, 1).contiguous(memory_format=torch.channels_last)
                 elif mode == "conv" and WGRAD_ENABLED and lib.gc_cuda_conv_wgrad_supported(n, x.shape[2], x.shape[3], cin, cout, r,
                                                                                            stride, pad):
-                    dw2d = conv_wgrad(dconv, x, r, stride, pad, out=slot)
+                    dw2d = conv_wgrad(dconv, x, r, stride, pad, out=slot, beside=beside and slot is not None)
                     dw = None if slot is not None else dw2d.view(cout, r, r, cin).permute(0, 3, 1, 2)
                 elif mode == "stem" and WGRAD_ENABLED and cout % 32 == 0:
                     dwp = gemm.gemm_tn_tf32(_as_2d(dconv), gathered)                       # [Cout, STEM_K]

@@ -107,11 +107,13 @@ def tn_supported(a_pm, b_pn, out):
                                                           a_pm.shape[1], b_pn.shape[1], a_pm.stride(0), b_pn.stride(0), out.stride(0)))
 
 
-def gemm_tn_tf32(a_pm, b_pn, out=None, accumulate=False):
+def gemm_tn_tf32(a_pm, b_pn, out=None, accumulate=False, beside=False):
     """``out[Mo, No] (+)= a_pm[P, Mo].T @ b_pn[P, No]``: the contraction runs over the rows, which is the weight gradient
     of a 1x1 convolution (``a_pm`` = output gradient, ``b_pn`` = input, rows = positions).  On the tensor-core path both
     operands are MN-major tcgen05 operands and the contraction is split over CTAs whose partial tiles are added onto
-    ``out`` by TMA reduce stores (so the summation order of the partials is not fixed)."""
+    ``out`` by TMA reduce stores (so the summation order of the partials is not fixed).  ``beside``: the launch in front on this
+    stream is the input gradient of the same layer; the two then run side by side (``out`` and the operands must not come
+    from that launch)."""
     if out is None:
         assert not accumulate
         out = torch.zeros(a_pm.shape[1], b_pn.shape[1], dtype=torch.float32, device=a_pm.device)
@@ -123,7 +125,7 @@ def gemm_tn_tf32(a_pm, b_pn, out=None, accumulate=False):
     with torch.cuda.device(a_pm.device):
         nat.check(nat.cuda().gc_cuda_gemm_tn_tf32(a_pm.data_ptr(), b_pn.data_ptr(), out.data_ptr(), a_pm.shape[0], a_pm.shape[1],
                                                   b_pn.shape[1], a_pm.stride(0), b_pn.stride(0), out.stride(0),
-                                                  _error_flag(a_pm.device).data_ptr(), nat.stream_ptr()), "gemm_tn_tf32")
+                                                  _error_flag(a_pm.device).data_ptr(), nat.stream_ptr(), int(beside)), "gemm_tn_tf32")
     return out
 
 
