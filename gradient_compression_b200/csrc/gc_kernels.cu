@@ -45,6 +45,7 @@ inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 
 // --------------------------------------------------------------------------- Philox fills
 template <int KIND>  // 0 uniform float, 1 normal float, 2 raw u32
 __global__ void philox_fill_kernel(RngKey key, const uint32_t* __restrict__ step_offset, int64_t n, void* __restrict__ out_) {
+  pdl_launch_dependents();
   if (step_offset != nullptr) key.step += *step_offset;      // a device-resident step counter: advances under graph replay
   int64_t nblk = (n + 3) / 4;
   int64_t stride = (int64_t)gridDim.x * blockDim.x;

@@ -106,6 +106,7 @@ __global__ void __launch_bounds__(THREADS, 1) topk_fold_kernel(const __grid_cons
   __shared__ uint32_t sh[BINS];
   const SegTable<CAP>& t = p.t;
   for (int i = threadIdx.x; i < BINS; i += THREADS) sh[i] = 0;
+  pdl_launch_dependents();
   __syncthreads();
   const uint32_t tiles = t.tile0[t.n], per = (tiles + gridDim.x - 1) / gridDim.x, first = blockIdx.x * per;
   if (first >= tiles) return;
@@ -275,6 +276,8 @@ __global__ void __launch_bounds__(THREADS) topk_pick_kernel(const __grid_constan
   const int g = blockIdx.x;
   const int64_t k = p.k[g], len = p.len(g);
   GroupState* st = p.state + g;
+  pdl_wait();
+  pdl_launch_dependents();
   if (threadIdx.x == 0) { st->taken = 0; st->listed = 0; }
   __syncthreads();
   if (p.small(g)) { select_small<CAP, LISTS>(p, g, hist, warp_sums, found); return; }
@@ -315,6 +318,8 @@ __global__ void __launch_bounds__(THREADS, 1) topk_split_kernel(const __grid_con
   int* count = held_count + (threadIdx.x >> 5);
   if (lane == 0) *count = 0;
   __syncwarp();
+  pdl_wait();
+  pdl_launch_dependents();
   const uint32_t tiles = t.tile0[t.n], per = (tiles + gridDim.x - 1) / gridDim.x, first = blockIdx.x * per;
   if (first >= tiles) return;
   uint32_t left = tiles - first < per ? tiles - first : per;
@@ -465,6 +470,7 @@ __global__ void __launch_bounds__(THREADS, CAP == 1 ? 1 : 2) topk_refine_kernel(
   const SegTable<CAP>& t = p.t;
   const int g = p.large[blockIdx.x / ranks];
   GroupState* st = p.state + g;
+  pdl_wait();
   const int k_rem = st->k_rem;
   const uint32_t in_bin = st->in_bin;
   if (k_rem <= 0) return;                  // (the whole cluster)
@@ -620,11 +626,11 @@ int run(const SegDesc* segs, int n_seg, int64_t end, const int64_t* k, int per_t
   cudaError_t err = cudaFuncSetAttribute(split, cudaFuncAttributeMaxDynamicSharedMemorySize, held);
   if (err != cudaSuccess) return (int)err;
   topk_fold_kernel<CAP><<<grid, THREADS, 0, st>>>(p);
-  if (lists) topk_pick_kernel<CAP, true><<<p.n_groups, THREADS, 0, st>>>(p);
-  else topk_pick_kernel<CAP, false><<<p.n_groups, THREADS, 0, st>>>(p);
+  // the kernels behind the first one start while their predecessor ends
+  err = lists ? launch_pdl(topk_pick_kernel<CAP, true>, dim3(p.n_groups), dim3(THREADS), 0, st, p) : launch_pdl(topk_pick_kernel<CAP, false>, dim3(p.n_groups), dim3(THREADS), 0, st, p);
+  if (err != cudaSuccess) return (int)err;
   if (p.n_large == 0) return (int)cudaGetLastError();
-  void* args[1] = {&p};
-  err = cudaLaunchKernel(split, dim3(grid), dim3(THREADS), args, held, st);
+  err = lists ? launch_pdl(topk_split_kernel<CAP, true>, dim3(grid), dim3(THREADS), held, st, p) : launch_pdl(topk_split_kernel<CAP, false>, dim3(grid), dim3(THREADS), held, st, p);
   if (err != cudaSuccess) return (int)err;
   // Blocks per group: what the longest group can fill with a few thousand candidates each (with error feedback, values pile up
   // below the threshold and the bin holds some percent of the group), as long as all groups fit on the chip at once, two blocks
@@ -632,22 +638,14 @@ int run(const SegDesc* segs, int n_seg, int64_t end, const int64_t* k, int per_t
   // with eight blocks each, 48 us with sixteen; one group of 64 M elements: 210 us with eight, 84 us with sixteen).
   int ranks = 1;
   while (ranks < (p.n_large <= 4 ? 16 : 8) && longest / 32 > (int64_t)ranks * 4 * THREADS && p.n_large * ranks * 2 <= 2 * sms) ranks *= 2;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(p.n_large * ranks));
-  cfg.blockDim = dim3(THREADS);
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = (unsigned)ranks;
-  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
   if (ranks > 8) {
     const void* refine = lists ? (const void*)topk_refine_kernel<CAP, true> : (const void*)topk_refine_kernel<CAP, false>;
     err = cudaFuncSetAttribute(refine, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     if (err != cudaSuccess) return (int)err;
   }
-  return (int)(lists ? cudaLaunchKernelEx(&cfg, topk_refine_kernel<CAP, true>, p) : cudaLaunchKernelEx(&cfg, topk_refine_kernel<CAP, false>, p));
+  const dim3 blocks((unsigned)(p.n_large * ranks));
+  return (int)(lists ? launch_cluster(topk_refine_kernel<CAP, true>, (unsigned)ranks, blocks, dim3(THREADS), 0, st, p)
+                     : launch_cluster(topk_refine_kernel<CAP, false>, (unsigned)ranks, blocks, dim3(THREADS), 0, st, p));
 }
 
 }  // namespace
