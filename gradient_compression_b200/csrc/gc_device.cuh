@@ -75,19 +75,27 @@ __device__ __forceinline__ float max_nan(float m, float x) {
 }
 
 // Level of |g| as a float, the same value that quantize_level (gc_common.h) returns as an integer:
-//   floor(l): adding 2^23 rounding down leaves floor(l) in the last mantissa bits (l < s <= 2^16), subtracting it is exact;
-//   u01(rnd) < p with u01 = (rnd >> 8) / 2^24: as integers, (rnd >> 8) < ceil(p * 2^24).  p * 2^-125 rounded up is that
-//   ceiling times 2^-149, the unit of the subnormals, so its bit pattern IS the ceiling.
-__device__ __forceinline__ float round_level(float g, float scale, float s, uint32_t rnd) {
+//   floor(l) + (u < l - floor(l)) with u = (rnd >> 8) / 2^24 is ceil(l - u), as 0 <= u < 1.
+//   u: the bit pattern rnd >> 8 is the float (rnd >> 8) * 2^-149 (subnormals and the binade above them are evenly spaced), so one FMA
+//   subtracts it times 2^125.  Rounding that up keeps the ceiling: integers are floats, so no rounding up passes one.
+//   ceil: adding 1.5 * 2^23 rounding up leaves it in the last mantissa bits (-1 < l - u < 2^16 where it matters).
+// Six instructions with the clamp, two of them on the ALU, which Philox keeps busy.  (Flooring, then comparing the fraction with u as
+// integers, takes nine and five: 140 against 81 instructions a quad in the second pass of a single worker's reduce.)
+constexpr float ROUND_BASE = 12582912.0f;
+__device__ __forceinline__ float round_up_base(float g, float scale, uint32_t rnd) {      // ROUND_BASE + level, not clamped
   const float l = __fmul_rn(fabsf(g), scale);
-  const float fl = __fsub_rn(__fadd_rd(l, 8388608.0f), 8388608.0f);
-  const uint32_t ceil_p = __float_as_uint(__fmul_ru(__fsub_rn(l, fl), __uint_as_float(0x01000000u)));
-  const float lev = (rnd >> 8) < ceil_p ? __fadd_rn(fl, 1.0f) : fl;
-  return fminf(lev, s);                    // l >= s, inf and nan inputs: s
+  return __fadd_ru(__fmaf_ru(__uint_as_float(rnd >> 8), -__uint_as_float(0x7e000000u), l), ROUND_BASE);
+}
+__device__ __forceinline__ float round_level(float g, float scale, float s, uint32_t rnd) {
+  return __fsub_rn(fminf(round_up_base(g, scale, rnd), ROUND_BASE + s), ROUND_BASE);      // l >= s, inf and nan inputs: s
 }
 // dq * (+-level); the FMA with +0 turns the -0 of a negative element of level zero into the +0 an integer level gives
 __device__ __forceinline__ float signed_value(float g, float level, float dq) {
   return __fmaf_rn(dq, g < 0.0f ? -level : level, 0.0f);
+}
+// The same where g is no NaN (a negative one would count as negative here): one instruction less.
+__device__ __forceinline__ float signed_value_of_number(float g, float level, float dq) {
+  return __fmaf_rn(dq, __uint_as_float(__float_as_uint(level) | (__float_as_uint(g) & 0x80000000u)), 0.0f);
 }
 
 // ---- row codec ------------------------------------------------------------------------------
