@@ -488,7 +488,7 @@ int gc_cuda_conv_dgrad_s2_supported(int N, int H, int W, int Cin, int Cout, int 
   if ((H & 1) || (W & 1) || !make_shape(N, H, W, Cin, Cout, R, 2, pad, &s) || s.Ho != H / 2 || s.Wo != W / 2) return 0;
   if ((Cout & 31) || (Cin & 3) || Cin < 32) return 0;
   for (int par = 0; par < 2; ++par)
-    if (class_first(par, pad, R) != 0) return 0;
+    if (class_first(par, pad, R) != 0 || par + pad + 2 < R) return 0;      // (a tap in front of offset 0, too)
   int bw, bh, bn;
   return box_for(BM, s.Ho, s.Wo, &bw, &bh, &bn) && encode_fn() != nullptr ? 1 : 0;
 }
