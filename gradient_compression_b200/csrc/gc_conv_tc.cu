@@ -111,7 +111,7 @@ int tap_stages(const Plan& pl, TapCols* t) {
 
 bool taps_ok(const Shape& s) {
   TapCols t;
-  Plan p{128, 1, false, true};
+  Plan p{128, 1, false, true, false};
   return tap_cols(s, &t) && tap_stages(p, &t) != 0;
 }
 
@@ -493,12 +493,13 @@ int gc_cuda_conv_dgrad_s2_supported(int N, int H, int W, int Cin, int Cout, int 
   return box_for(BM, s.Ho, s.Wo, &bw, &bh, &bn) && encode_fn() != nullptr ? 1 : 0;
 }
 
-// dx[N, H, W, Cin] = input gradient of conv2d(x, w, stride 2, pad) given dy[N, H/2, W/2, Cout].  One launch per parity class
+// dx[N, H, W, Cin] = input gradient of conv2d(x, w, stride 2, pad) given dy[N, H/2, W/2, Cout].  One product per parity class
 // (ph, pw) of input pixels: the pixels (2i + ph, 2j + pw) receive a stride-1 convolution of dy with the filter taps
 // r = ph + pad - 2 fr, s = pw + pad - 2 fs (fr, fs = 0, 1, ...: the offsets at which dy is read), and are written through a 4-D
 // store map over that strided sub-grid of dx.  w: the forward filter [Cout][R][R][Cin] (channels-last memory order), read in
 // place as the MN-major B operand.  Classes without taps (a 1x1 filter reaches only the even pixels) are zero: dx is cleared
-// first when there is one.
+// first when there is one.  The four products are one launch (CLASSES) where all have taps and Cin is a multiple of 32 (the store map takes the two
+// pixels of a column pair as one row of 2 Cin floats: a tile of 32 columns must not reach from one into the other), else one launch each.
 // accumulate: dx += instead, where pixels that no tap reaches are not touched at all.
 int gc_cuda_conv_dgrad_s2_add(const float* dy, const float* w, float* dx, int N, int H, int W, int Cin, int Cout, int R, int pad, int accumulate,
                               int* error_flag, void* cs) {
@@ -517,6 +518,26 @@ int gc_cuda_conv_dgrad_s2_add(const float* dy, const float* w, float* dx, int N,
   int bw, bh, bn;
   box_for(BM, Ho, Wo, &bw, &bh, &bn);
   EncodeTiledFn fn = encode_fn();
+  if (!any_empty && (Cin & 31) == 0) {
+    const int t0 = class_taps(0, pad, R), t1 = class_taps(1, pad, R);
+    const Plan pl = pick_classes(M, Cin, Cout, t0, t1);
+    CUtensorMap ma, mb, mc;
+    ConvA ca{t1 * t1, t1, Cout / 32, Ho * Wo, Wo, 1, 0};
+    ca.b_ldtap = Cin; ca.b_fs = R;
+    ca.b_r0 = pad; ca.b_dr = -2; ca.b_s0 = pad; ca.b_ds = -2;
+    ca.class_taps0 = t0; ca.class_taps1 = t1;
+    if (make_map_nhwc(&ma, dy, sy, bw, bh, bn, CU_TENSOR_MAP_SWIZZLE_128B) != 0 || filter_map(&mb, &ca, w, Cout, R, Cin, pl.b_cols()) != 0)
+      return (int)cudaErrorInvalidValue;
+    // dx as {2 Cin (a pixel pair of a row), W/2, 2 (rows), H/2, N}
+    cuuint64_t dims[5] = {(cuuint64_t)2 * Cin, (cuuint64_t)Wo, 2, (cuuint64_t)Ho, (cuuint64_t)N};
+    cuuint64_t strides[4] = {(cuuint64_t)2 * Cin * 4, (cuuint64_t)W * Cin * 4, (cuuint64_t)2 * W * Cin * 4, (cuuint64_t)H * W * Cin * 4};
+    cuuint32_t box[5] = {32, (cuuint32_t)bw, 1, (cuuint32_t)bh, (cuuint32_t)bn}, estr[5] = {1, 1, 1, 1, 1};
+    if (fn(&mc, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 5, (void*)dx, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+           CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+      return (int)cudaErrorInvalidValue;
+    const ConvC cc{Ho * Wo, Wo, 0};
+    return launch_plan(pl, ma, mb, mc, ca, nullptr, M, Cin, t1 * t1 * Cout, accumulate, nullptr, error_flag, st, nullptr, &cc);
+  }
   for (int c = 0; c < 4; ++c) {
     const int ph = c >> 1, pw = c & 1;
     const int th = class_taps(ph, pad, R), tw = class_taps(pw, pad, R);

@@ -260,6 +260,9 @@ struct ConvA {
   // map is the 3-D view {32 floats, K rows, columns / 32} of the same matrix (b_ldtap a multiple of 32) and one box loads
   // a whole stage of B.
   int b_mn, b_ldtap, b_fs, b_r0, b_dr, b_s0, b_ds;
+  // All four parity classes (ph, pw) of a stride-2 input gradient in one launch: taps along an axis of the classes of parity 0 and 1; the
+  // filter tap of class (ph, pw) starts at (b_r0 + ph, b_s0 + pw).  0: not used.
+  int class_taps0, class_taps1;
 };
 
 // The input gradient of a 3x3, stride-1, padding-1 convolution, where the three taps of a filter COLUMN share one copy of dY's pixels.
@@ -488,14 +491,24 @@ constexpr int TN_THREADS = PERSISTENT_THREADS;
 // what bounds the single-CTA form.  The first CTA of the pair issues the MMAs and holds the barriers they wait for; commits go
 // to both.  Work items are the pairs' tiles; everything after the accumulator is each CTA's own.
 //
-// TAPS: the input gradient of a 3x3 convolution whose filter columns share a copy of the pixels (TapCols); a stage is 3 k-blocks.
-template <int BN, bool AFFINE, bool PAIR, bool TAPS>
+// FORM:
+//   PLAIN    one matrix product or convolution
+//   SHARED   the input gradient of a 3x3 convolution whose filter columns share a copy of the pixels (TapCols); a stage is 3 k-blocks
+//   CLASSES  the input gradient of a stride-2 convolution: four products of different depths (one, two, two and four filter taps for 3x3), one per parity
+//            class of input pixels, on the same pixels of dY and the same filter.  Deepest first, and every second round of the workers backwards, so that a
+//            worker gets deep and shallow tiles.  The output is a 5-D map {2 C, W / 2, 2, H / 2, N}.  One launch per class left much of
+//            the chip idle and could not afford wide tiles: 32x32x128 at batch 128 44.5 -> 28.6 us, 16x16x256 40.5 -> 21.1, 8x8x512 48.1 -> 19.1, at
+//            batch 31 32x32x64 -> 128 25.9 -> 8.3, 16x16x128 -> 256 32.9 -> 10.5, 8x8x256 -> 512 45.7 -> 14.2 (back to back).
+constexpr int PLAIN = 0, SHARED = 1, CLASSES = 2;
+
+template <int BN, bool AFFINE, bool PAIR, int FORM>
 __global__ void __launch_bounds__(PERSISTENT_THREADS, 1)
 gemm_tf32_persistent_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
                             const __grid_constant__ CUtensorMap tma_c, const ConvA ca, const float* __restrict__ bias, int M, int N, int K,
                             int tiles_m, int tiles_n, int splits, int accumulate, float* __restrict__ col_partials,
                             int* __restrict__ error_flag, int tma_mode, const BnFin fin, const ConvC cc, int cta_sums, const Affine aff,
                             const TapCols tc) {
+  constexpr bool TAPS = FORM == SHARED;
   using S = PSmem<BN, PAIR, TAPS>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -518,10 +531,15 @@ gemm_tf32_persistent_kernel(const __grid_constant__ CUtensorMap tma_a, const __g
   const int num_k = TAPS ? 3 * ca.cblocks : (K + BK - 1) / BK;      // stages of a whole contraction
   // work item = (output tile, split of the contraction); the splits of one tile are neighbours in the list, so they run
   // at the same time on different SMs and add their partial tiles in L2 (the host passes accumulate = 1 and a zeroed C)
-  const int total_items = tiles_m * tiles_n * splits;          // tiles_m: of 128 rows, PAIR: of 256
+  const int per_class = tiles_m * tiles_n;                     // CLASSES: items of a class (no splits); tiles_m: of 128 rows, PAIR: of 256
+  const int total_items = FORM == CLASSES ? 4 * per_class : per_class * splits;
   const int kps = (num_k + splits - 1) / splits;
   const int rank = PAIR ? (int)cluster_rank() : 0;
   const int worker = PAIR ? (int)(blockIdx.x >> 1) : (int)blockIdx.x, workers = PAIR ? (int)(gridDim.x >> 1) : (int)gridDim.x;
+  // from a worker's item to its next one; CLASSES: the step after that is 2 * workers - step
+  const int first_step = FORM == CLASSES ? 2 * (workers - worker) - 1 : workers;
+  auto turn_step = [&](int step) { return FORM == CLASSES ? 2 * workers - step : step; };
+  auto class_depth = [&](int ph, int pw) { return (ph ? ca.class_taps1 : ca.class_taps0) * (pw ? ca.class_taps1 : ca.class_taps0) * ca.cblocks; };
 
   if (threadIdx.x == 32 * FIRST_EPI_WARP && (tma_mode & 1)) { tma_prefetch_map(&tma_a); tma_prefetch_map(&tma_b); tma_prefetch_map(&tma_c); }
   if (threadIdx.x == 0) {
@@ -566,9 +584,11 @@ gemm_tf32_persistent_kernel(const __grid_constant__ CUtensorMap tma_a, const __g
     static_assert(PRODUCER_WARPS == 2, "two warps take turns");
     int turn = 0;                                             // producer warp that fills it
     bool ok = true;
-    for (int t = worker; t < total_items && ok; t += workers) {
-      const int tile = t / splits, sp = t - tile * splits;
-      const int kbeg = sp * kps, kend = min(num_k, kbeg + kps);
+    for (int t = worker, step = first_step; t < total_items && ok; t += step, step = turn_step(step)) {
+      const int cls = FORM == CLASSES ? 3 - t / per_class : 0, ph = cls >> 1, pw = cls & 1;
+      const int tile = FORM == CLASSES ? t - (3 - cls) * per_class : t / splits, sp = FORM == CLASSES ? 0 : t - tile * splits;
+      const int kbeg = sp * kps, kend = FORM == CLASSES ? class_depth(ph, pw) : min(num_k, kbeg + kps);
+      const int filter_w = FORM == CLASSES ? (pw ? ca.class_taps1 : ca.class_taps0) : ca.fs;
       const int m0 = (PAIR ? (tile / tiles_n) * 2 + rank : tile / tiles_n) * BM, n0 = (tile % tiles_n) * BN + rank * S::B_COLS;
       int box[4] = {0, 0, 0, 0};
       if (ca.taps != 0) conv_box(ca, (int64_t)m0, 0, 0, box);  // pixel of the tile's first position at tap (0, 0)
@@ -576,7 +596,7 @@ gemm_tf32_persistent_kernel(const __grid_constant__ CUtensorMap tma_a, const __g
       if constexpr (TAPS) {
         cb = kbeg / 3;                                        // stage = (32-channel block cb, filter column fs)
         fs = kbeg - cb * 3;
-      } else if (ca.taps != 0) {
+      } else if (FORM == PLAIN && ca.taps != 0) {
         const int tap = kbeg / ca.cblocks;
         cb = kbeg - tap * ca.cblocks;
         fr = tap / ca.fs;
@@ -603,7 +623,7 @@ gemm_tf32_persistent_kernel(const __grid_constant__ CUtensorMap tma_a, const __g
             __syncwarp();
           } else {
           // b_mn: B is the filter read in place (no transposed copy)
-          const int tapcol = ca.b_mn == 0 || ca.taps == 0 ? 0 : ((ca.b_r0 + ca.b_dr * fr) * ca.b_fs + (ca.b_s0 + ca.b_ds * fs)) * ca.b_ldtap;
+          const int tapcol = ca.b_mn == 0 || ca.taps == 0 ? 0 : ((ca.b_r0 + ph + ca.b_dr * fr) * ca.b_fs + (ca.b_s0 + pw + ca.b_ds * fs)) * ca.b_ldtap;
           const int krow = (ca.taps == 0 ? k : cb) * BK;
           uint8_t *a_dst = a_tiles + s * S::A_BYTES, *b_dst = b_tiles + s * S::B_BYTES;
           if constexpr (PAIR) {
@@ -645,7 +665,7 @@ gemm_tf32_persistent_kernel(const __grid_constant__ CUtensorMap tma_a, const __g
           if (++fs == 3) { fs = 0; ++cb; }
         } else if (++cb == ca.cblocks) {                             // (never true for a plain matrix: cblocks == 0)
           cb = 0;
-          if (++fs == ca.fs) { fs = 0; ++fr; }
+          if (++fs == filter_w) { fs = 0; ++fr; }
         }
       }
     }
@@ -670,9 +690,9 @@ gemm_tf32_persistent_kernel(const __grid_constant__ CUtensorMap tma_a, const __g
     };
     uint32_t s = 0, phase = 0, lt = 0;                        // stage of the next k-block and its phase, tiles started
     bool ok = true;
-    for (int t = worker; rank == 0 && t < total_items && ok; t += workers, ++lt) {
-      const int sp = t % splits;
-      const int nk = min(num_k, (sp + 1) * kps) - sp * kps;
+    for (int t = worker, step = first_step; rank == 0 && t < total_items && ok; t += step, step = turn_step(step), ++lt) {
+      const int sp = t % splits, cls = FORM == CLASSES ? 3 - t / per_class : 0;
+      const int nk = FORM == CLASSES ? class_depth(cls >> 1, cls & 1) : min(num_k, (sp + 1) * kps) - sp * kps;
       const uint32_t buf = lt & 1u, aphase = (lt >> 1) & 1u;
       if (!mbar_wait_warp<PAIR>(&acc_empty[buf], aphase ^ 1u, &abort_flag)) break;      // first use of a buffer passes at once
       tc_fence_after();
@@ -752,8 +772,9 @@ gemm_tf32_persistent_kernel(const __grid_constant__ CUtensorMap tma_a, const __g
         res[i] = row < M && c < N ? __ldcs(reinterpret_cast<const float4*>(aff.residual + (int64_t)row * N + c)) : make_float4(0.f, 0.f, 0.f, 0.f);
       }
     };
-    for (int t = worker; t < total_items; t += workers, ++lt) {
-      const int tile = t / splits;
+    for (int t = worker, step = first_step; t < total_items; t += step, step = turn_step(step), ++lt) {
+      const int cls = FORM == CLASSES ? 3 - t / per_class : 0;
+      const int tile = FORM == CLASSES ? t - (3 - cls) * per_class : t / splits;
       const bool add_bias = bias != nullptr && t == tile * splits;      // the first split of a tile carries the bias
       const int mi = PAIR ? (tile / tiles_n) * 2 + rank : tile / tiles_n;      // row tile of 128; of a pair the second may lie beyond M
       const int m0 = mi * BM, n0 = (tile % tiles_n) * BN;
@@ -772,7 +793,7 @@ gemm_tf32_persistent_kernel(const __grid_constant__ CUtensorMap tma_a, const __g
       // The ring's stages are done with once a CTA's last accumulator is complete: that tile's slabs are staged there, each in a
       // place of its own, and none waits for a store to have read the one before (the end of a launch, 2.2 us from the last
       // accumulator to the last store at 128 columns, was mostly that wait).
-      const bool last = t + workers >= total_items;
+      const bool last = t + step >= total_items;
       static_assert(SLABS * S::SLAB_BYTES <= S::RING_BYTES, "a tile's slabs in the ring");
 #pragma unroll 1
       for (int sl = grp; sl < SLABS; sl += EPI_GROUPS, ++sc) {
@@ -835,7 +856,18 @@ gemm_tf32_persistent_kernel(const __grid_constant__ CUtensorMap tma_a, const __g
             else mbar_arrive(&acc_empty[buf]);
           }
           if (n0 + sl * 32 < N && (!PAIR || m0 < M)) {
-            if (cc.hw != 0) {                    // rows = pixels (n, i, j) of a strided sub-grid: 4-D store map
+            if constexpr (FORM == CLASSES) {     // rows = pixels (n, i, j) of class (ph, pw)
+              const int img = m0 / cc.hw, rem = m0 - img * cc.hw;
+              const int i0 = rem / cc.w, j0 = rem - i0 * cc.w;
+              if (accumulate)
+                asm volatile("cp.reduce.async.bulk.tensor.5d.global.shared::cta.add.tile.bulk_group [%0, {%2, %3, %4, %5, %6}], [%1];"
+                             ::"l"(&tma_c), "r"(smem_u32(slab)), "r"((cls & 1) * N + n0 + sl * 32), "r"(j0), "r"(cls >> 1), "r"(i0), "r"(img)
+                             : "memory");
+              else
+                asm volatile("cp.async.bulk.tensor.5d.global.shared::cta.bulk_group [%0, {%2, %3, %4, %5, %6}], [%1];"
+                             ::"l"(&tma_c), "r"(smem_u32(slab)), "r"((cls & 1) * N + n0 + sl * 32), "r"(j0), "r"(cls >> 1), "r"(i0), "r"(img)
+                             : "memory");
+            } else if (cc.hw != 0) {             // rows = pixels (n, i, j) of a strided sub-grid: 4-D store map
               const int img = m0 / cc.hw, rem = m0 - img * cc.hw;
               const int i0 = rem / cc.w, j0 = rem - i0 * cc.w;
               const int c2 = cc.nh ? img : i0, c3 = cc.nh ? i0 : img;
@@ -1304,6 +1336,7 @@ struct Plan {
   int bn, splits;
   bool pair;
   bool taps;                                                 // 3x3 input gradient with shared pixels (TapCols)
+  bool classes;                                              // stride-2 input gradient, all parity classes in one launch
   int b_cols() const { return pair ? bn / 2 : bn; }          // columns of B (box rows of its map) one CTA loads
   int rows() const { return pair ? 2 * BM : BM; }
 };
@@ -1327,25 +1360,26 @@ inline int pairs_at_once(const void* kernel, int threads, size_t smem) {
 
 // CTAs, or CTA pairs, of the persistent kernel that the device runs at once (pairs: half its SMs, unless a GPC has an odd
 // number of them); 0 when the kernel cannot be configured.
-template <int BN, bool AFFINE, bool PAIR, bool TAPS>
+template <int BN, bool AFFINE, bool PAIR, int FORM>
 int persistent_workers() {
-  using S = PSmem<BN, PAIR, TAPS>;
+  using S = PSmem<BN, PAIR, FORM == SHARED>;
   static int workers = 0;
   if (workers != 0) return workers;
-  if (cudaFuncSetAttribute(gemm_tf32_persistent_kernel<BN, AFFINE, PAIR, TAPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::TOTAL) != cudaSuccess) return 0;
+  if (cudaFuncSetAttribute(gemm_tf32_persistent_kernel<BN, AFFINE, PAIR, FORM>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::TOTAL) != cudaSuccess) return 0;
   int n = sm_count();
-  if constexpr (PAIR) n = pairs_at_once((const void*)gemm_tf32_persistent_kernel<BN, AFFINE, PAIR, TAPS>, PERSISTENT_THREADS, S::TOTAL);
+  if constexpr (PAIR) n = pairs_at_once((const void*)gemm_tf32_persistent_kernel<BN, AFFINE, PAIR, FORM>, PERSISTENT_THREADS, S::TOTAL);
   return workers = n;
 }
 
 // Launch the persistent kernel on ready-made tensor maps (ca.taps == 0: ma is a 2-D map of A[M, K]).
-template <int BN, bool AFFINE, bool PAIR, bool TAPS>
+template <int BN, bool AFFINE, bool PAIR, int FORM>
 int launch_persistent_maps(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mc, const ConvA& ca, const float* bias,
                            int M, int N, int K, int accumulate, float* col_partials, int* error_flag, cudaStream_t st,
                            const BnFin* fin, const ConvC* cc, int splits, int cta_sums, const Affine* aff, const TapCols* tc) {
+  constexpr bool TAPS = FORM == SHARED;
   using S = PSmem<BN, PAIR, TAPS>;
-  if ((tc != nullptr && tc->box_bytes != 0) != TAPS) return (int)cudaErrorInvalidValue;
-  const int workers_max = persistent_workers<BN, AFFINE, PAIR, TAPS>();
+  if ((tc != nullptr && tc->box_bytes != 0) != TAPS || (ca.class_taps0 != 0) != (FORM == CLASSES)) return (int)cudaErrorInvalidValue;
+  const int workers_max = persistent_workers<BN, AFFINE, PAIR, FORM>();
   if (workers_max == 0) return (int)cudaGetLastError();
   constexpr int ROWS = PAIR ? 2 * BM : BM;
   int tiles_m = (M + ROWS - 1) / ROWS, tiles_n = (N + BN - 1) / BN;
@@ -1354,7 +1388,8 @@ int launch_persistent_maps(const CUtensorMap& ma, const CUtensorMap& mb, const C
   // finished values (column statistics) can ride along
   if (splits > 1 && (!accumulate || col_partials != nullptr || (fin != nullptr && fin->acc != nullptr) || (cc != nullptr && !cc->nh)))
     return (int)cudaErrorInvalidValue;
-  int64_t total = (int64_t)tiles_m * tiles_n * splits;
+  if (FORM == CLASSES && (splits != 1 || bias != nullptr || col_partials != nullptr || fin != nullptr || cc == nullptr || (N & 31))) return (int)cudaErrorInvalidValue;
+  int64_t total = (int64_t)tiles_m * tiles_n * (FORM == CLASSES ? 4 : splits);
   int64_t workers = total < workers_max ? total : workers_max;
   BnFin f{};
   if (fin != nullptr && fin->acc != nullptr) {
@@ -1367,7 +1402,7 @@ int launch_persistent_maps(const CUtensorMap& ma, const CUtensorMap& mb, const C
     if (col_partials == nullptr || splits > 1 || tiles_n > workers) return (int)cudaErrorInvalidValue;
     workers = workers / tiles_n * tiles_n;
   }
-  gc::launch_cluster(gemm_tf32_persistent_kernel<BN, AFFINE, PAIR, TAPS>, PAIR ? 2u : 1u, dim3((unsigned)(PAIR ? 2 * workers : workers)),
+  gc::launch_cluster(gemm_tf32_persistent_kernel<BN, AFFINE, PAIR, FORM>, PAIR ? 2u : 1u, dim3((unsigned)(PAIR ? 2 * workers : workers)),
                      dim3(PERSISTENT_THREADS), (size_t)S::TOTAL, st, ma, mb, mc, ca, bias, M, N, K, tiles_m, tiles_n, splits, accumulate,
                      col_partials, error_flag, gctc::tma_mode, f, cc != nullptr ? *cc : ConvC{}, cta_sums, aff != nullptr ? *aff : Affine{},
                      tc != nullptr ? *tc : TapCols{});
@@ -1383,15 +1418,23 @@ int launch_plan(const Plan& pl, const CUtensorMap& ma, const CUtensorMap& mb, co
   };
   if (pl.taps) {
     if constexpr (!AFFINE) {
-      if (pl.bn == 64) return pl.pair ? run(launch_persistent_maps<64, false, true, true>) : run(launch_persistent_maps<64, false, false, true>);
-      if (pl.bn == 128) return pl.pair ? run(launch_persistent_maps<128, false, true, true>) : run(launch_persistent_maps<128, false, false, true>);
+      if (pl.bn == 64) return pl.pair ? run(launch_persistent_maps<64, false, true, SHARED>) : run(launch_persistent_maps<64, false, false, SHARED>);
+      if (pl.bn == 128) return pl.pair ? run(launch_persistent_maps<128, false, true, SHARED>) : run(launch_persistent_maps<128, false, false, SHARED>);
+    }
+    return (int)cudaErrorInvalidValue;
+  }
+  if (pl.classes) {
+    if constexpr (!AFFINE) {
+      if (pl.bn == 64) return pl.pair ? run(launch_persistent_maps<64, false, true, CLASSES>) : run(launch_persistent_maps<64, false, false, CLASSES>);
+      if (pl.bn == 128) return pl.pair ? run(launch_persistent_maps<128, false, true, CLASSES>) : run(launch_persistent_maps<128, false, false, CLASSES>);
+      if (pl.bn == 256) return pl.pair ? run(launch_persistent_maps<256, false, true, CLASSES>) : run(launch_persistent_maps<256, false, false, CLASSES>);
     }
     return (int)cudaErrorInvalidValue;
   }
   switch (pl.bn) {
-    case 64: return pl.pair ? run(launch_persistent_maps<64, AFFINE, true, false>) : run(launch_persistent_maps<64, AFFINE, false, false>);
-    case 128: return pl.pair ? run(launch_persistent_maps<128, AFFINE, true, false>) : run(launch_persistent_maps<128, AFFINE, false, false>);
-    case 256: return pl.pair ? run(launch_persistent_maps<256, AFFINE, true, false>) : run(launch_persistent_maps<256, AFFINE, false, false>);
+    case 64: return pl.pair ? run(launch_persistent_maps<64, AFFINE, true, PLAIN>) : run(launch_persistent_maps<64, AFFINE, false, PLAIN>);
+    case 128: return pl.pair ? run(launch_persistent_maps<128, AFFINE, true, PLAIN>) : run(launch_persistent_maps<128, AFFINE, false, PLAIN>);
+    case 256: return pl.pair ? run(launch_persistent_maps<256, AFFINE, true, PLAIN>) : run(launch_persistent_maps<256, AFFINE, false, PLAIN>);
     default: return (int)cudaErrorInvalidValue;
   }
 }
@@ -1400,9 +1443,9 @@ int launch_plan(const Plan& pl, const CUtensorMap& ma, const CUtensorMap& mb, co
 inline int plan_workers(const Plan& pl) {
   if (!pl.pair) return sm_count();
   switch (pl.bn) {
-    case 64: return persistent_workers<64, false, true, false>();
-    case 128: return persistent_workers<128, false, true, false>();
-    default: return persistent_workers<256, false, true, false>();
+    case 64: return persistent_workers<64, false, true, PLAIN>();
+    case 128: return persistent_workers<128, false, true, PLAIN>();
+    default: return persistent_workers<256, false, true, PLAIN>();
   }
 }
 
@@ -1469,13 +1512,15 @@ inline int launch_tn_plan(int bn, bool pair, const CUtensorMap& ma, const CUtens
 // 500 ns of hand-over between the accumulators, a pair's launch about 1500 ns (the two CTAs meet at its start and end).  The product
 // cannot be faster than its operands and its result cross DRAM; the two overlap, not quite perfectly.
 // `reuse`: how often an element of A is read (filter taps per input pixel of a convolution, 1 for a matrix).
+constexpr double stage_ns[2][3] = {{235.0, 300.0, 490.0}, {205.0, 260.0, 400.0}};
+inline double stage_of(const Plan& p) { return stage_ns[p.pair][p.bn == 64 ? 0 : (p.bn == 128 ? 1 : 2)]; }
+
 inline double plan_ns(const Plan& p, int M, int N, int K, double reuse) {
-  static constexpr double stage[2][3] = {{235.0, 300.0, 490.0}, {205.0, 260.0, 400.0}};
   static constexpr double taps_stage[2][2] = {{157.0, 200.0}, {103.0, 144.0}};      // 16x16x128, four waves against two
   const int num_k = (K + BK - 1) / BK;
   const int64_t items = (int64_t)((M + p.rows() - 1) / p.rows()) * ((N + p.bn - 1) / p.bn) * p.splits;
   const int64_t workers = p.pair ? sm_count() / 2 : sm_count(), waves = (items + workers - 1) / workers;
-  const double sm = (double)waves * ((num_k + p.splits - 1) / p.splits * (p.taps ? taps_stage[p.pair][p.bn == 64 ? 0 : 1] : stage[p.pair][p.bn == 64 ? 0 : (p.bn == 128 ? 1 : 2)]) + 500.0);
+  const double sm = (double)waves * ((num_k + p.splits - 1) / p.splits * (p.taps ? taps_stage[p.pair][p.bn == 64 ? 0 : 1] : stage_of(p)) + 500.0);
   const double dram = ((double)M * K / reuse + (double)M * N * (p.splits > 1 ? 2.0 : 1.0) + (double)N * K) * 4.0 / 6500.0;
   return (sm > dram ? sm + 0.15 * dram : dram + 0.15 * sm) + (p.pair ? 1500.0 : 0.0);
 }
@@ -1490,17 +1535,38 @@ inline void each_plan(int M, int N, bool taps_ok, F&& f) {
     const int bn = cand[i];
     if (gctc::tile_choice ? bn != gctc::tile_choice : ((bn == 256 && N <= 128) || (bn == 128 && N <= 64))) continue;
     for (int pair = 0; pair < 2; ++pair)
-      if (pair == 0 ? (gctc::pair_choice != 2 || M <= BM) : (gctc::pair_choice != 1 && M > BM)) f(Plan{bn, 1, pair != 0, taps && bn <= 128});
+      if (pair == 0 ? (gctc::pair_choice != 2 || M <= BM) : (gctc::pair_choice != 1 && M > BM)) f(Plan{bn, 1, pair != 0, taps && bn <= 128, false});
   }
 }
 
 // Tile width and pairing of a product that is not split: the candidate with the lowest modelled time.
 inline Plan pick_persistent(int M, int N, int K, double reuse = 1.0, bool taps_ok = false) {
-  Plan best{64, 1, false, false};
+  Plan best{64, 1, false, false, false};
   double best_t = 1e30;
   each_plan(M, N, taps_ok, [&](const Plan& p) {
     const double t = plan_ns(p, M, N, K, reuse);
     if (t < best_t) { best_t = t; best = p; }
+  });
+  return best;
+}
+
+// The same for the four parity classes of a stride-2 input gradient in one launch: M pixels and K rows of the filter per class, t0 and t1 taps along
+// an axis.  The busiest worker's time, its items dealt out as the kernel does it.
+inline Plan pick_classes(int M, int N, int K, int t0, int t1) {
+  Plan best{64, 1, false, false, true};
+  double best_t = 1e30;
+  each_plan(M, N, false, [&](Plan p) {
+    const int64_t per_class = (int64_t)((M + p.rows() - 1) / p.rows()) * ((N + p.bn - 1) / p.bn), workers = p.pair ? sm_count() / 2 : sm_count();
+    const int64_t first = 4 * per_class < workers ? 4 * per_class : workers;
+    const double taps[4] = {(double)t1 * t1, (double)t1 * t0, (double)t0 * t1, (double)t0 * t0}, stage = stage_of(p) * ((K + BK - 1) / BK);
+    double worst = 0.0;
+    for (int64_t w = 0; w < first; w += 4) {                 // (every fourth worker)
+      double t = 0.0;
+      for (int64_t i = w, step = 2 * (first - w) - 1; i < 4 * per_class; i += step, step = 2 * first - step) t += taps[i / per_class] * stage + 500.0;
+      if (t > worst) worst = t;
+    }
+    const double all = worst + (p.pair ? 1500.0 : 0.0);
+    if (all < best_t) { best_t = all; best = p; best.classes = true; }
   });
   return best;
 }
