@@ -293,9 +293,9 @@ int gc_cuda_conv_bn_eval(const float* x, const float* w, float* y, const float* 
   if (make_map(&mb, w, Cout, K, K, pl.b_cols()) != 0 || make_map(&mc, y, M, Cout, Cout, BM) != 0) return (int)cudaErrorInvalidValue;
   const Affine aff{gamma, beta, mean, var, residual, eps, relu};
   if (pl.splits == 1) return launch_plan<true>(pl, ma, mb, mc, ca, cbias, M, Cout, K, 0, nullptr, error_flag, st, nullptr, nullptr, 0, &aff);
-  cudaError_t e = cudaMemsetAsync(y, 0, (size_t)M * Cout * 4, st);
-  if (e != cudaSuccess) return (int)e;
-  const int err = launch_plan(pl, ma, mb, mc, ca, cbias, M, Cout, K, 1, nullptr, error_flag, st);
+  int err = zero_rows(y, M, Cout, Cout, st);
+  if (err) return err;
+  err = launch_plan(pl, ma, mb, mc, ca, cbias, M, Cout, K, 1, nullptr, error_flag, st);
   if (err) return err;
   return gc_cuda_bn_eval_apply(y, M, Cout, mean, var, eps, gamma, beta, residual, relu, y, cs);
 }
@@ -339,8 +339,8 @@ int gc_cuda_conv_fwd(const float* x, const float* w, float* y, const float* bias
       make_map(&mc, y, M, Cout, Cout, BM) != 0)
     return (int)cudaErrorInvalidValue;
   if (pl.splits > 1 && !accumulate) {
-    cudaError_t e = cudaMemsetAsync(y, 0, (size_t)M * Cout * 4, st);
-    if (e != cudaSuccess) return (int)e;
+    const int err = zero_rows(y, M, Cout, Cout, st);
+    if (err) return err;
   }
   return launch_plan(pl, ma, mb, mc, conv_a(s), bias, M, Cout, K, accumulate || pl.splits > 1, col_partials, error_flag, st, fin, nullptr, cta_sums);
 }
@@ -412,8 +412,8 @@ int gc_cuda_conv_dgrad(const float* dy, const float* w, float* dx, int N, int H,
   if ((pl.taps ? make_map_filter_cols(&m.b, w, Cout, Cin, pl.b_cols()) : filter_map(&m.b, &m.ca, w, Cout, R, Cin, pl.b_cols())) != 0)
     return (int)cudaErrorInvalidValue;
   if (pl.splits > 1 && !accumulate) {
-    cudaError_t e = cudaMemsetAsync(dx, 0, (size_t)M * Cin * 4, st);
-    if (e != cudaSuccess) return (int)e;
+    const int err = zero_rows(dx, M, Cin, Cin, st);
+    if (err) return err;
   }
   return launch_plan(pl, m.a, m.b, m.c, m.ca, nullptr, M, Cin, K, accumulate || pl.splits > 1, nullptr, error_flag, st, nullptr, m.store(), 0, nullptr, &m.tc);
 }
@@ -511,8 +511,8 @@ int gc_cuda_conv_dgrad_s2_add(const float* dy, const float* w, float* dx, int N,
   bool any_empty = false;
   for (int c = 0; c < 4; ++c) any_empty |= class_taps(c >> 1, pad, R) * class_taps(c & 1, pad, R) == 0;
   if (any_empty && !accumulate) {
-    cudaError_t e = cudaMemsetAsync(dx, 0, (size_t)N * H * W * Cin * 4, st);
-    if (e != cudaSuccess) return (int)e;
+    const int err = zero_rows(dx, (int64_t)N * H * W, Cin, Cin, st);
+    if (err) return err;
   }
   Shape sy{N, Ho, Wo, Cout, Cin, 1, 1, 0, Ho, Wo};          // the class problem reads dy at stride 1, no padding
   int bw, bh, bn;

@@ -273,8 +273,8 @@ int launch_persistent(const Plan& pl, const float* A, const float* B, float* C, 
   if (make_map(&ma, A, M, K, lda, BM) != 0 || make_map(&mb, B, N, K, ldb, pl.b_cols()) != 0 || make_map(&mc, C, M, N, ldc, BM) != 0)
     return (int)cudaErrorInvalidValue;
   if (pl.splits > 1 && !accumulate) {
-    cudaError_t e = cudaMemset2DAsync(C, (size_t)ldc * 4, 0, (size_t)N * 4, (size_t)M, st);
-    if (e != cudaSuccess) return (int)e;
+    const int err = zero_rows(C, M, N, ldc, st);
+    if (err) return err;
   }
   return launch_plan(pl, ma, mb, mc, ConvA{}, bias, M, N, K, accumulate || pl.splits > 1, col_partials, error_flag, st, fin, nullptr, cta_sums);
 }
