@@ -162,6 +162,25 @@ __global__ void __launch_bounds__(THREADS, 1) bn_fused_fwd_kernel(const Shape s,
   const int c4 = g * CH + 4 * q, C = s.C;
   const int64_t lo = (int64_t)r * s.per, hi = lo + s.per < s.M ? lo + s.per : s.M;
   pdl_launch_dependents();
+  // The first rows of the apply pass are on their way while the statistics come together (a layer of few rows per thread is latency, not bandwidth).
+  constexpr int U = 4;                       // rows in flight per thread: 64 KB a block (twice that with a residual)
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  int64_t i = hi - 1 - rl;
+  float4 v[U];
+  auto load_rows = [&]() {
+    if (POOL) {
+      int64_t row[4];
+      if (i >= lo) {
+        pool_rows(s.pool, i, row);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) v[j] = ld4(a.x + row[j] * C + c4);
+      }
+    } else {
+#pragma unroll
+      for (int j = 0; j < U; ++j) v[j] = i - j * LANES >= lo ? ld4_last(a.x + (i - j * LANES) * C + c4) : zero;
+    }
+  };
+  if (!SUMS) load_rows();
   if (SUMS) {
     // sums shifted by the channel's value in row 0: no cancellation when |mean| is large against the standard deviation
     const uint32_t passed = threadIdx.x == 0 ? *((volatile uint32_t*)&s.sync->passed[g]) : 0u;
@@ -234,13 +253,9 @@ __global__ void __launch_bounds__(THREADS, 1) bn_fused_fwd_kernel(const Shape s,
   }
   __syncthreads();
   const Channels ch{ld4(mean_s + 4 * q), ld4(rstd_s + 4 * q), ld4(a.gamma + c4), ld4(a.beta + c4)};
+  if (SUMS) load_rows();
   if (POOL) {
-    for (int64_t i = hi - 1 - rl; i >= lo; i -= LANES) {
-      int64_t row[4];
-      pool_rows(s.pool, i, row);
-      float4 v[4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) v[j] = ld4(a.x + row[j] * C + c4);
+    while (i >= lo) {
       float4 o = affine(normalized(v[0], ch), ch);
       if (a.relu) o = relu4(o);
 #pragma unroll
@@ -249,30 +264,26 @@ __global__ void __launch_bounds__(THREADS, 1) bn_fused_fwd_kernel(const Shape s,
         if (a.relu) p = relu4(p);
         o = make_float4(fmaxf(o.x, p.x), fmaxf(o.y, p.y), fmaxf(o.z, p.z), fmaxf(o.w, p.w));
       }
-      st4(a.y + i * C + c4, o);
+      const int64_t at = i * C + c4;
+      i -= LANES;
+      load_rows();
+      st4(a.y + at, o);
     }
     return;
   }
-  constexpr int U = 4;                       // rows in flight per thread: 64 KB a block (twice that with a residual)
-  int64_t i = hi - 1 - rl;
-  auto finish = [&](const float4& v, const float4& res, int64_t at) {
-    float4 o = affine(normalized(v, ch), ch);
-    o.x += res.x; o.y += res.y; o.z += res.z; o.w += res.w;
-    st4(a.y + at, a.relu ? relu4(o) : o);
-  };
-  for (; i - (U - 1) * LANES >= lo; i -= U * LANES) {
-    const int64_t at = i * C + c4;
-    float4 v[U], res[U];
+  while (i >= lo) {
+    float4 res[U];
 #pragma unroll
-    for (int j = 0; j < U; ++j) v[j] = ld4_last(a.x + at - (int64_t)j * LANES * C);
+    for (int j = 0; j < U; ++j) res[j] = a.residual != nullptr && i - j * LANES >= lo ? ld4_last(a.residual + (i - j * LANES) * C + c4) : zero;
 #pragma unroll
-    for (int j = 0; j < U; ++j) res[j] = a.residual != nullptr ? ld4_last(a.residual + at - (int64_t)j * LANES * C) : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-    for (int j = 0; j < U; ++j) finish(v[j], res[j], at - (int64_t)j * LANES * C);
-  }
-  for (; i >= lo; i -= LANES) {
-    const int64_t at = i * C + c4;
-    finish(ld4(a.x + at), a.residual != nullptr ? ld4(a.residual + at) : make_float4(0.f, 0.f, 0.f, 0.f), at);
+    for (int j = 0; j < U; ++j) {
+      if (i - j * LANES < lo) break;
+      float4 o = affine(normalized(v[j], ch), ch);
+      o.x += res[j].x; o.y += res[j].y; o.z += res[j].z; o.w += res[j].w;
+      st4(a.y + (i - j * LANES) * C + c4, a.relu ? relu4(o) : o);
+    }
+    i -= U * LANES;
+    load_rows();
   }
 }
 
@@ -309,7 +320,10 @@ __device__ __forceinline__ float4 keep_bits(const float4& d, uint32_t m) {
 
 // A thread's rows are lo + rl + 128 k; pass 1 takes k upwards in pairs, pass 2 downwards.  Behind a residual the ReLU's mask comes
 // from the saved output; pass 1 leaves it in shared memory, a byte per pair of rows and thread, so that the output is read once.
-template <bool POOL>
+//
+// KEEP: no thread has more than two rows, and what pass 1 read of dy and x stays in registers for pass 2 (8x8x256 at batch 31: 6.4 -> 6.1 us, 4x4x512
+// at 128: 6.5 -> 6.1; four and six rows in shared memory gained nothing: 8x8x256 at batch 128 8.0 -> 8.3).
+template <bool POOL, bool KEEP>
 __global__ void __launch_bounds__(THREADS, 1) bn_fused_bwd_kernel(const Shape s, const BwdArgs a) {
   extern __shared__ uint8_t masks[];       // [a.masks][THREADS]
   __shared__ float warp_part[THREADS / 32][VALUES];
@@ -324,6 +338,7 @@ __global__ void __launch_bounds__(THREADS, 1) bn_fused_bwd_kernel(const Shape s,
   const Channels ch{ld4(a.stats + c4), ld4(a.stats + C + c4), ld4(a.gamma + c4), ld4(a.beta + c4)};
   const bool from_y = a.relu && a.y != nullptr;
   float4 sg = make_float4(0.f, 0.f, 0.f, 0.f), sx = sg;
+  float4 kd0 = sg, kd1 = sg, kv0 = sg, kv1 = sg;       // KEEP: dy behind the ReLU and x normalised of both rows, zeros beyond the last one
 
   if (POOL) {
     for (int64_t i = lo + rl; i < hi; i += LANES) {
@@ -339,6 +354,26 @@ __global__ void __launch_bounds__(THREADS, 1) bn_fused_bwd_kernel(const Shape s,
       if (pool_route(v[0].z, v[1].z, v[2].z, v[3].z, ch.gm.z, ch.bt.z, a.relu, xh) >= 0) { sg.z += d.z; sx.z = fmaf(d.z, xh, sx.z); }
       if (pool_route(v[0].w, v[1].w, v[2].w, v[3].w, ch.gm.w, ch.bt.w, a.relu, xh) >= 0) { sg.w += d.w; sx.w = fmaf(d.w, xh, sx.w); }
     }
+  } else if (KEEP) {
+    const int64_t i = lo + rl, at = i * C + c4, next = at + (int64_t)LANES * C;
+    const bool one = i < hi, two = i + LANES < hi;
+    float4 y0 = sg, y1 = sg;
+    if (one) { kd0 = ld4_last(a.dy + at); kv0 = ld4_last(a.x + at); }
+    if (two) { kd1 = ld4_last(a.dy + next); kv1 = ld4_last(a.x + next); }
+    if (from_y && one) y0 = ld4_last(a.y + at);
+    if (from_y && two) y1 = ld4_last(a.y + next);
+    kv0 = normalized(kv0, ch);
+    kv1 = normalized(kv1, ch);
+    if (a.relu) {
+      kd0 = keep_positive(kd0, from_y ? y0 : affine(kv0, ch));
+      kd1 = keep_positive(kd1, from_y ? y1 : affine(kv1, ch));
+    }
+    auto add = [&](const float4& d, const float4& xh) {
+      sg.x += d.x; sg.y += d.y; sg.z += d.z; sg.w += d.w;
+      sx.x = fmaf(d.x, xh.x, sx.x); sx.y = fmaf(d.y, xh.y, sx.y); sx.z = fmaf(d.z, xh.z, sx.z); sx.w = fmaf(d.w, xh.w, sx.w);
+    };
+    if (one) add(kd0, kv0);
+    if (two) add(kd1, kv1);
   } else {
     auto add = [&](float4 d, const float4& v, uint32_t m) {
       const float4 xh = normalized(v, ch);
@@ -399,6 +434,18 @@ __global__ void __launch_bounds__(THREADS, 1) bn_fused_bwd_kernel(const Shape s,
       for (int j = 0; j < 4; ++j)
         st4(a.dx + row[j] * C + c4,
             input_gradient(make_float4(wx == j ? d.x : 0.f, wy == j ? d.y : 0.f, wz == j ? d.z : 0.f, ww == j ? d.w : 0.f), v[j]));
+    }
+    return;
+  }
+  if (KEEP) {
+    const int64_t i = lo + rl, at = i * C + c4, next = at + (int64_t)LANES * C;
+    if (i < hi) {
+      if (a.dres != nullptr) st4(a.dres + at, kd0);
+      st4(a.dx + at, input_gradient(kd0, kv0));
+    }
+    if (i + LANES < hi) {
+      if (a.dres != nullptr) st4(a.dres + next, kd1);
+      st4(a.dx + next, input_gradient(kd1, kv1));
     }
     return;
   }
@@ -518,12 +565,13 @@ int gc_cuda_bn_fused_backward(const float* dy, const float* x, const float* y, i
   s.parts = (float*)((uint8_t*)scratch + sizeof(GroupSync));
   s.error_flag = error_flag;
   plan(s, sm_count());
+  const int64_t pairs = (s.per + 2 * LANES - 1) / (2 * LANES);
+  const bool keep = !pool && pairs == 1;
   // masks of as many row pairs as shared memory holds (192 KB: 49 K rows of 32 channels a block)
   constexpr int most = 192;
-  const int64_t pairs = (s.per + 2 * LANES - 1) / (2 * LANES);
-  const int masks = y == nullptr || pool ? 0 : (int)(pairs < most ? pairs : most);
+  const int masks = y == nullptr || pool || keep ? 0 : (int)(pairs < most ? pairs : most);
   const BwdArgs a{dy, x, y, stats, gamma, beta, relu, sums, dx, dres, masks};
-  const void* k = pool ? (const void*)bn_fused_bwd_kernel<true> : (const void*)bn_fused_bwd_kernel<false>;
+  const void* k = pool ? (const void*)bn_fused_bwd_kernel<true, false> : keep ? (const void*)bn_fused_bwd_kernel<false, true> : (const void*)bn_fused_bwd_kernel<false, false>;
   if (masks * THREADS > 24 * 1024) {
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, most * THREADS);
     if (e != cudaSuccess) return (int)e;

@@ -60,3 +60,11 @@ def test_one_launch_forward_and_backward(shape, kind, partials):
     assert off(sums[:c], b.grad, 1e-4) <= max(3e-3, 1.0 / c) and off(sums[c:], g.grad, 1e-4) <= max(3e-3, 1.0 / c)
     if dres is not None:
         assert off(dres, rr.grad, 1e-6) < 1e-4
+
+
+@pytest.mark.parametrize("kind", ["relu", "residual", "plain"])
+@pytest.mark.parametrize("rows", [2, 127, 128, 129, 255, 256, 257, 511, 512, 513, 1025])
+def test_rows_of_a_thread(rows, kind):
+    """One, two and three rows per thread of the fullest block, threads without a row: the backward keeps up to two rows, the forward's first four are
+    loaded in front of the statistics."""
+    test_one_launch_forward_and_backward((1, 64, 1, rows), kind, True)
