@@ -142,7 +142,7 @@ __global__ void __launch_bounds__(HEAD_THREADS) head_fwd_kernel(const float* __r
                                                                 const int64_t* __restrict__ labels, int N,
                                                                 float* __restrict__ pooled, float* __restrict__ logits,
                                                                 float* __restrict__ dlogits, float* __restrict__ per_sample,
-                                                                unsigned int* __restrict__ ticket, float* __restrict__ out3) {
+                                                                unsigned int* __restrict__ ticket, float* __restrict__ out3, float* __restrict__ loss) {
   __shared__ HeadShared sh;
   __shared__ int last;
   const int n = blockIdx.x;
@@ -176,7 +176,10 @@ __global__ void __launch_bounds__(HEAD_THREADS) head_fwd_kernel(const float* __r
     float acc = 0.f;
     for (int i = lane; i < N; i += 32) acc += __ldcg(per_sample + 3 * i + warp);
     acc = warp_sum(acc);
-    if (lane == 0) out3[warp] = acc / (float)N;
+    if (lane == 0) {
+      out3[warp] = acc / (float)N;
+      if (warp == 0 && loss != nullptr) *loss = acc / (float)N;
+    }
   }
   if (threadIdx.x == 0) *ticket = 0u;
 }
@@ -273,14 +276,15 @@ int gc_cuda_logit_metrics(const float* logits, const int64_t* labels, int N, int
 int64_t gc_cuda_head_scratch_bytes(int max_batch) { return 256 + (int64_t)max_batch * 3 * 4; }
 
 // x [N, positions, C] (NHWC feature map), W [K, C], bias [K] or NULL, labels [N] int64.  Writes pooled [N, C], logits [N, K],
-// dlogits [N, K] and out3 = {mean cross-entropy, top-1 rate, top-5 rate}.  scratch: gc_cuda_head_scratch_bytes(N), zeroed once.
+// dlogits [N, K], out3 = {mean cross-entropy, top-1 rate, top-5 rate} and, when given, loss = out3[0] (a tensor of its own for autograd).
+// scratch: gc_cuda_head_scratch_bytes(N), zeroed once.
 int gc_cuda_head_forward(const float* x, int N, int positions, int C, const float* W, const float* bias, int K,
-                         const int64_t* labels, float* pooled, float* logits, float* dlogits, void* scratch, float* out3, void* cs) {
+                         const int64_t* labels, float* pooled, float* logits, float* dlogits, void* scratch, float* out3, float* loss, void* cs) {
   if (!gc_cuda_head_supported(N, positions, C, K)) return (int)cudaErrorInvalidValue;
   unsigned int* ticket = static_cast<unsigned int*>(scratch);
   float* per_sample = reinterpret_cast<float*>(static_cast<uint8_t*>(scratch) + 256);
   head_fwd_kernel<<<N, HEAD_THREADS, 0, (cudaStream_t)cs>>>(x, positions, C, W, bias, K, labels, N, pooled, logits, dlogits, per_sample,
-                                                            ticket, out3);
+                                                            ticket, out3, loss);
   return (int)cudaGetLastError();
 }
 

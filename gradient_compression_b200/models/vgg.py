@@ -5,7 +5,7 @@ from __future__ import annotations
 
 import torch.nn as nn
 
-from ..ops.bn import defer_batch_counters, flush_batch_counters
+from ..ops.bn import defer_batch_counters, flush_batch_counters, hooked
 from ..ops.conv import conv_bn_act
 from ..ops.head import head_loss
 from .layers import bn, conv, head, linear
@@ -60,6 +60,9 @@ class VGG(nn.Module):
                         and x.shape[2] % 2 == 0 and x.shape[3] % 2 == 0)
                 x = conv_bn_act(m, mods[i + 1], x, pool=pool)
                 i += 4 if pool else 3
+            elif (type(m) is nn.AvgPool2d and not hooked(m) and m.kernel_size in (1, (1, 1)) and m.stride in (1, (1, 1)) and m.padding in (0, (0, 0))
+                  and m.divisor_override in (None, 1)):
+                i += 1                            # the mean over one pixel
             else:
                 x = m(x)
                 i += 1

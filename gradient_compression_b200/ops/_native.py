@@ -144,7 +144,7 @@ def cuda():
         _declare(lib, "gc_cuda_head_scratch_bytes", c_i64, [c_int])
         _declare(lib, "gc_cuda_head_eval", c_int, [P, c_int, c_int, c_int, P, P, c_int, P, P])
         _declare(lib, "gc_cuda_logit_metrics", c_int, [P, P, c_int, c_int, P, P])
-        _declare(lib, "gc_cuda_head_forward", c_int, [P, c_int, c_int, c_int, P, P, c_int, P, P, P, P, P, P, P])
+        _declare(lib, "gc_cuda_head_forward", c_int, [P, c_int, c_int, c_int, P, P, c_int, P, P, P, P, P, P, P, P])
         _declare(lib, "gc_cuda_head_backward", c_int, [P, P, P, P, c_int, c_int, c_int, c_int, P, P, P, P])
         _declare(lib, "gc_cuda_psgd_max_rank", c_int, [])
         _declare(lib, "gc_cuda_psgd_p", c_int, [c_int, P, P, P, c_int, c_i64, P, P, P, c_int, c_i64, P])

@@ -51,19 +51,23 @@ class _HeadCE(torch.autograd.Function):
         logits = torch.empty(n, k, dtype=torch.float32, device=dev)
         dlogits = torch.empty(n, k, dtype=torch.float32, device=dev)
         out3 = torch.empty(3, dtype=torch.float32, device=dev)
+        loss = torch.empty((), dtype=torch.float32, device=dev)
         wc = weight.contiguous()
         with torch.cuda.device(dev):
             nat.check(nat.cuda().gc_cuda_head_forward(x.data_ptr(), n, h * w, c, wc.data_ptr(), nat.ptr(bias), k, labels.data_ptr(),
                                                       pooled.data_ptr(), logits.data_ptr(), dlogits.data_ptr(),
-                                                      _scratch_for(dev, n).data_ptr(), out3.data_ptr(), nat.stream_ptr()),
+                                                      _scratch_for(dev, n).data_ptr(), out3.data_ptr(), loss.data_ptr(), nat.stream_ptr()),
                       "head_forward")
         ctx.save_for_backward(pooled, dlogits, wc)
         ctx.shape, ctx.has_bias = (n, c, h, w), bias is not None
         ctx.mark_non_differentiable(logits, out3)
-        return out3[0].clone(), logits, out3
+        ctx.set_materialize_grads(False)      # (no zeros for the logits and the metrics)
+        return loss, logits, out3
 
     @staticmethod
     def backward(ctx, gloss, _glogits, _gmetrics):
+        if gloss is None:
+            return None, None, None, None
         pooled, dlogits, wc = ctx.saved_tensors
         n, c, h, w = ctx.shape
         k = wc.shape[0]

@@ -75,6 +75,15 @@ class _StatusMirror:
         self.event = None
 
 
+def _side_by_side(scalars):
+    """The scalars as one vector: the tensor they are the elements of, where there is one (the fused head's), else a new one."""
+    base = scalars[0]._base
+    if base is not None and base.shape == (len(scalars),) and base.dtype == torch.float32 and all(
+            v._base is base and v.dim() == 0 and v.data_ptr() == base.data_ptr() + i * base.stride(0) * 4 for i, v in enumerate(scalars)):
+        return base
+    return torch.stack([v.reshape(()).float() for v in scalars])
+
+
 class GraphedStep:
     """``step(batch) -> loss`` (a device scalar); ``step.metrics`` holds the batch's cross-entropy / top-1 / top-5 as
     device scalars after every call.
@@ -142,8 +151,7 @@ class GraphedStep:
                 m = task.evaluate_predictions(pred.detach(), y, loss)
             self.metrics = {k: (v if torch.is_tensor(v) else torch.as_tensor(v)) for k, v in m.items()}
             # the three scalars side by side: one device-to-host copy reads a step's result
-            self.metrics_vec = torch.stack([self.metrics[k].reshape(()).float() for k in
-                                            ("cross_entropy_loss", "top1_accuracy", "top5_accuracy")])
+            self.metrics_vec = _side_by_side([self.metrics[k] for k in ("cross_entropy_loss", "top1_accuracy", "top5_accuracy")])
         return loss
 
     def _graph_safe(self):

@@ -1,0 +1,27 @@
+"""Small things a captured step leaves out: a vector of metrics that exists already is not stacked again, VGG's pooling of one pixel is not run unless
+it does something."""
+import torch
+
+from gradient_compression_b200 import models
+from gradient_compression_b200.parallel.graph import _side_by_side
+
+
+def test_side_by_side():
+    base = torch.tensor([1.0, 2.0, 3.0])
+    assert _side_by_side([base[0], base[1], base[2]]) is base
+    for scalars in ([base[0], base[2], base[1]], [base[0], base[1]], [base[0].clone(), base[1], base[2]], list(torch.ones(3, dtype=torch.float64)), [torch.ones(1)] * 3):
+        got = _side_by_side(scalars)
+        assert got is not base and got.dtype == torch.float32 and got.tolist() == [float(v) for v in scalars]
+
+
+def test_pooling_of_one_pixel():
+    torch.manual_seed(0)
+    net, x = models.VGG11().eval(), torch.randn(2, 3, 32, 32)
+    want = net.features(x)
+    assert torch.equal(net._features(x), want)
+    seen = []
+    handle = net.features[-1].register_forward_hook(lambda *_: seen.append(1))
+    net._features(x)
+    handle.remove()
+    net.features[-1].divisor_override = 2
+    assert seen == [1] and torch.equal(net._features(x), want / 2)
