@@ -32,12 +32,11 @@ __device__ __forceinline__ void st4(float* p, const float4& v) { *reinterpret_ca
 
 struct PoolGeom { int H, W, Hp, Wp; };
 
-// Rows (in units of C floats) of the four pixels of pooled pixel r.
+// Rows (in units of C floats) of the four pixels of pooled pixel r.  (32-bit divisions: 2^31 rows of 32 channels are 256 GB, and the host refuses them.)
 __device__ __forceinline__ void pool_rows(const PoolGeom& g, int64_t r, int64_t (&row)[4]) {
-  const int64_t n = r / (g.Hp * g.Wp);
-  const int rem = (int)(r - n * (g.Hp * g.Wp));
-  const int hp = rem / g.Wp, wp = rem - hp * g.Wp;
-  row[0] = (n * g.H + 2 * hp) * g.W + 2 * wp;
+  const uint32_t line = (uint32_t)r / (uint32_t)g.Wp, n = line / (uint32_t)g.Hp;       // the pooled line, its image
+  const uint32_t wp = (uint32_t)r - line * (uint32_t)g.Wp, hp = line - n * (uint32_t)g.Hp;
+  row[0] = ((int64_t)n * g.H + 2 * hp) * g.W + 2 * wp;
   row[1] = row[0] + 1;
   row[2] = row[0] + g.W;
   row[3] = row[2] + 1;
@@ -322,7 +321,8 @@ __device__ __forceinline__ float4 keep_bits(const float4& d, uint32_t m) {
 // from the saved output; pass 1 leaves it in shared memory, a byte per pair of rows and thread, so that the output is read once.
 //
 // KEEP: no thread has more than two rows, and what pass 1 read of dy and x stays in registers for pass 2 (8x8x256 at batch 31: 6.4 -> 6.1 us, 4x4x512
-// at 128: 6.5 -> 6.1; four and six rows in shared memory gained nothing: 8x8x256 at batch 128 8.0 -> 8.3).
+// at 128: 6.5 -> 6.1; four and six rows in shared memory gained nothing: 8x8x256 at batch 128 8.0 -> 8.3).  With a pool: no more than one pooled row, its four
+// pixels and the winners stay (with 32-bit divisions and a row per thread instead of two: 4x4x512 at batch 128 12.3 -> 7.5 us, forward 5.4 -> 4.4).
 template <bool POOL, bool KEEP>
 __global__ void __launch_bounds__(THREADS, 1) bn_fused_bwd_kernel(const Shape s, const BwdArgs a) {
   extern __shared__ uint8_t masks[];       // [a.masks][THREADS]
@@ -338,9 +338,31 @@ __global__ void __launch_bounds__(THREADS, 1) bn_fused_bwd_kernel(const Shape s,
   const Channels ch{ld4(a.stats + c4), ld4(a.stats + C + c4), ld4(a.gamma + c4), ld4(a.beta + c4)};
   const bool from_y = a.relu && a.y != nullptr;
   float4 sg = make_float4(0.f, 0.f, 0.f, 0.f), sx = sg;
+  float4 kw[4] = {sg, sg, sg, sg};                     // KEEP with a pool: the window's pixels normalised, the winner's index per channel (-1: none)
+  int kwin[4] = {-1, -1, -1, -1};
   float4 kd0 = sg, kd1 = sg, kv0 = sg, kv1 = sg;       // KEEP: dy behind the ReLU and x normalised of both rows, zeros beyond the last one
 
-  if (POOL) {
+  if (POOL && KEEP) {
+    const int64_t i = lo + rl;
+    if (i < hi) {
+      int64_t row[4];
+      pool_rows(s.pool, i, row);
+      kd0 = ld4_last(a.dy + i * C + c4);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) kw[j] = ld4_last(a.x + row[j] * C + c4);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) kw[j] = normalized(kw[j], ch);
+      float xh;
+      kwin[0] = pool_route(kw[0].x, kw[1].x, kw[2].x, kw[3].x, ch.gm.x, ch.bt.x, a.relu, xh);
+      if (kwin[0] >= 0) { sg.x = kd0.x; sx.x = kd0.x * xh; }
+      kwin[1] = pool_route(kw[0].y, kw[1].y, kw[2].y, kw[3].y, ch.gm.y, ch.bt.y, a.relu, xh);
+      if (kwin[1] >= 0) { sg.y = kd0.y; sx.y = kd0.y * xh; }
+      kwin[2] = pool_route(kw[0].z, kw[1].z, kw[2].z, kw[3].z, ch.gm.z, ch.bt.z, a.relu, xh);
+      if (kwin[2] >= 0) { sg.z = kd0.z; sx.z = kd0.z * xh; }
+      kwin[3] = pool_route(kw[0].w, kw[1].w, kw[2].w, kw[3].w, ch.gm.w, ch.bt.w, a.relu, xh);
+      if (kwin[3] >= 0) { sg.w = kd0.w; sx.w = kd0.w * xh; }
+    }
+  } else if (POOL) {
     for (int64_t i = lo + rl; i < hi; i += LANES) {
       int64_t row[4];
       pool_rows(s.pool, i, row);
@@ -417,6 +439,16 @@ __global__ void __launch_bounds__(THREADS, 1) bn_fused_bwd_kernel(const Shape s,
     return make_float4(ch.gm.x * ch.rs.x * (d.x - mb.x - xh.x * dg.x * inv_m), ch.gm.y * ch.rs.y * (d.y - mb.y - xh.y * dg.y * inv_m),
                        ch.gm.z * ch.rs.z * (d.z - mb.z - xh.z * dg.z * inv_m), ch.gm.w * ch.rs.w * (d.w - mb.w - xh.w * dg.w * inv_m));
   };
+  if (POOL && KEEP) {
+    const int64_t i = lo + rl;
+    if (i >= hi) return;
+    int64_t row[4];
+    pool_rows(s.pool, i, row);
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      st4(a.dx + row[j] * C + c4, input_gradient(make_float4(kwin[0] == j ? kd0.x : 0.f, kwin[1] == j ? kd0.y : 0.f, kwin[2] == j ? kd0.z : 0.f, kwin[3] == j ? kd0.w : 0.f), kw[j]));
+    return;
+  }
   if (POOL) {
     for (int64_t i = hi - 1 - rl; i >= lo; i -= LANES) {
       int64_t row[4];
@@ -489,10 +521,12 @@ int sm_count() {
 // Blocks of a launch: one per SM, and no more than the scratch has partial sums for, whatever the chip's size.
 int block_limit(int sms) { return sms < MAX_BLOCKS ? sms : MAX_BLOCKS; }
 
-// Runs of rows per channel group: as many as blocks allow, two hundred and some rows each at least (two per thread).
-void plan(Shape& s, int sms) {
+// Runs of rows per channel group: as many as blocks allow, two hundred and some rows each at least (two per thread; one where a row is a
+// pooled one with its four pixels).
+void plan(Shape& s, int sms, int pool) {
   s.G = s.C / CH;
-  int64_t most = block_limit(sms) / s.G, want = (s.M + 2 * LANES - 1) / (2 * LANES);
+  const int64_t least = pool ? LANES : 2 * LANES;
+  int64_t most = block_limit(sms) / s.G, want = (s.M + least - 1) / least;
   if (most < 1) most = 1;
   int64_t r = want < most ? want : most;
   s.per = (s.M + r - 1) / r;
@@ -524,7 +558,7 @@ int gc_cuda_bn_fused_blocks(int64_t M, int C, int sms) {
   Shape s{};
   s.M = M;
   s.C = C;
-  plan(s, sms);
+  plan(s, sms, 0);
   return s.G * s.R;
 }
 
@@ -540,12 +574,12 @@ int gc_cuda_bn_fused_forward(const float* x, int N, int H, int W, int C, int poo
   Shape s{};
   s.M = (int64_t)N * H * W / (pool ? 4 : 1);
   s.C = C;
-  if (!shape_ok(s.M, C, sm_count()) || (pool && ((H | W) & 1 || residual != nullptr))) return (int)cudaErrorInvalidValue;
+  if (!shape_ok(s.M, C, sm_count()) || (pool && ((H | W) & 1 || residual != nullptr || s.M > 0x3fffffff))) return (int)cudaErrorInvalidValue;
   s.pool = PoolGeom{H, W, H / 2, W / 2};
   s.sync = (GroupSync*)scratch;
   s.parts = (float*)((uint8_t*)scratch + sizeof(GroupSync));
   s.error_flag = error_flag;
-  plan(s, sm_count());
+  plan(s, sm_count(), pool);
   const FwdArgs a{x, partials, nparts, gamma, beta, residual, relu, running_mean, running_var, momentum, eps, stats, y};
   const void* k = partials != nullptr ? (pool ? (const void*)bn_fused_fwd_kernel<true, false> : (const void*)bn_fused_fwd_kernel<false, false>)
                                       : (pool ? (const void*)bn_fused_fwd_kernel<true, true> : (const void*)bn_fused_fwd_kernel<false, true>);
@@ -559,19 +593,19 @@ int gc_cuda_bn_fused_backward(const float* dy, const float* x, const float* y, i
   Shape s{};
   s.M = (int64_t)N * H * W / (pool ? 4 : 1);
   s.C = C;
-  if (!shape_ok(s.M, C, sm_count()) || (pool && ((H | W) & 1 || dres != nullptr))) return (int)cudaErrorInvalidValue;
+  if (!shape_ok(s.M, C, sm_count()) || (pool && ((H | W) & 1 || dres != nullptr || s.M > 0x3fffffff))) return (int)cudaErrorInvalidValue;
   s.pool = PoolGeom{H, W, H / 2, W / 2};
   s.sync = (GroupSync*)scratch;
   s.parts = (float*)((uint8_t*)scratch + sizeof(GroupSync));
   s.error_flag = error_flag;
-  plan(s, sm_count());
+  plan(s, sm_count(), pool);
   const int64_t pairs = (s.per + 2 * LANES - 1) / (2 * LANES);
-  const bool keep = !pool && pairs == 1;
+  const bool keep = s.per <= (pool ? 1 : 2) * LANES;
   // masks of as many row pairs as shared memory holds (192 KB: 49 K rows of 32 channels a block)
   constexpr int most = 192;
   const int masks = y == nullptr || pool || keep ? 0 : (int)(pairs < most ? pairs : most);
   const BwdArgs a{dy, x, y, stats, gamma, beta, relu, sums, dx, dres, masks};
-  const void* k = pool ? (const void*)bn_fused_bwd_kernel<true, false> : keep ? (const void*)bn_fused_bwd_kernel<false, true> : (const void*)bn_fused_bwd_kernel<false, false>;
+  const void* k = pool ? (keep ? (const void*)bn_fused_bwd_kernel<true, true> : (const void*)bn_fused_bwd_kernel<true, false>) : keep ? (const void*)bn_fused_bwd_kernel<false, true> : (const void*)bn_fused_bwd_kernel<false, false>;
   if (masks * THREADS > 24 * 1024) {
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, most * THREADS);
     if (e != cudaSuccess) return (int)e;
