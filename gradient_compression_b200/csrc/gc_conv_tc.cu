@@ -173,7 +173,9 @@ bool wgrad_ok(const Shape& s) {
 }
 
 // A[p][k] = x[n, h + r - pad, w + s - pad, c] with k = (r * R + s) * Cin + c (zero outside the image and for
-// k >= R*R*Cin), stride 1; wpad[co][k] = w[co][k] padded to Kp columns.  One thread per (position, 4 columns).
+// k >= R*R*Cin), stride 1; wpad[co][k] = w[co][k] padded to Kp columns.  One thread per (position, 4 columns); a thread keeps its columns from one
+// position to the next, so that their taps are looked up once (bound by instructions; 32x32x3, 9.5 -> 7.7 us
+// at 128 images, 15.3 -> 11.0 at 256).
 constexpr int IM2COL_MAX_KP = 128;
 
 __global__ void __launch_bounds__(256) im2col_small_kernel(const float* __restrict__ x, float* __restrict__ A, int N, int H, int W,
@@ -190,20 +192,28 @@ __global__ void __launch_bounds__(256) im2col_small_kernel(const float* __restri
     tap_dw[k] = tap % R - pad;
   }
   __syncthreads();
-  const uint32_t uq = (uint32_t)quads, uqpr = (uint32_t)qpr, uW = (uint32_t)W, uH = (uint32_t)H;      // host: quads < 2^31
-  for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < uq; q += gridDim.x * blockDim.x) {
-    const uint32_t p = q / uqpr;
-    const int k0 = (int)(q - p * uqpr) * 4;
+  const uint32_t uqpr = (uint32_t)qpr, uW = (uint32_t)W, uH = (uint32_t)H, positions = (uint32_t)quads / uqpr;      // host: quads < 2^31
+  const uint32_t thread = blockIdx.x * blockDim.x + threadIdx.x, together = gridDim.x * blockDim.x / uqpr;            // positions at once
+  const int k0 = (int)(thread % uqpr) * 4;
+  int dh[4], dw[4], from[4];                                        // of this thread's columns; a padding column is never inside
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const int c = tap_c[k0 + j];
+    dh[j] = c >= 0 ? tap_dh[k0 + j] : -H - R;
+    dw[j] = tap_dw[k0 + j];
+    from[j] = (tap_dh[k0 + j] * W + dw[j]) * Cin + c;
+  }
+  for (uint32_t p = thread / uqpr; p < positions && thread < together * uqpr; p += together) {
     const uint32_t row = p / uW;
     const int wo = (int)(p - row * uW);
     const uint32_t n = row / uH;
     const int ho = (int)(row - n * uH);
+    const float* xp = x + (int64_t)p * Cin;                         // the position's own pixel (stride 1)
     float v[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      const int k = k0 + j;
-      const int c = tap_c[k], hi = ho + tap_dh[k], wi = wo + tap_dw[k];
-      v[j] = (c >= 0 && hi >= 0 && hi < H && wi >= 0 && wi < W) ? x[(((int64_t)n * H + hi) * W + wi) * Cin + c] : 0.f;
+      const int hi = ho + dh[j], wi = wo + dw[j];
+      v[j] = ((uint32_t)hi < uH && (uint32_t)wi < uW) ? xp[from[j]] : 0.f;
     }
     *reinterpret_cast<float4*>(A + (int64_t)p * Kp + k0) = make_float4(v[0], v[1], v[2], v[3]);
   }

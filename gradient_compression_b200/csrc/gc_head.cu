@@ -41,7 +41,7 @@ __device__ __forceinline__ void pooled_logits(HeadShared& sh, const float* __res
   const float inv_pos = 1.0f / (float)positions;
   for (int q = threadIdx.x; q < (C >> 2); q += HEAD_THREADS) {
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 8
+#pragma unroll 16
     for (int p = 0; p < positions; ++p) {
       const float4 v = *reinterpret_cast<const float4*>(xn + (int64_t)p * C + 4 * q);
       acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
@@ -146,11 +146,13 @@ __global__ void __launch_bounds__(HEAD_THREADS) head_fwd_kernel(const float* __r
   __shared__ HeadShared sh;
   __shared__ int last;
   const int n = blockIdx.x;
+  pdl_wait();
+  pdl_launch_dependents();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int label = warp == 0 ? (int)labels[n] : 0;                // on its way while the block pools
   pooled_logits(sh, x, n, positions, C, W, bias, K, pooled, logits);
   __syncthreads();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (warp == 0) {
-    const int label = (int)labels[n];
     const float z = lane < K ? sh.logit[lane] : -INFINITY;
     const float zmax = warp_max(z);
     const float e = lane < K ? __expf(z - zmax) : 0.f;
@@ -189,6 +191,8 @@ __global__ void __launch_bounds__(HEAD_THREADS) head_bwd_dx_kernel(const float* 
                                                                    float* __restrict__ dx) {
   __shared__ float sd[HEAD_MAX_CLASSES];
   const int n = blockIdx.y;
+  pdl_wait();
+  pdl_launch_dependents();
   if (threadIdx.x < K) sd[threadIdx.x] = dlogits[(int64_t)n * K + threadIdx.x] * (g != nullptr ? *g : 1.f) / (float)positions;
   __syncthreads();
   const int q = blockIdx.x * HEAD_THREADS + threadIdx.x;
@@ -204,13 +208,17 @@ __global__ void __launch_bounds__(HEAD_THREADS) head_bwd_dx_kernel(const float* 
 }
 
 // One block per 32 channels: warp w sums the samples w, w + 8, ... for its lane's channel and all classes, the eight partial
-// sums meet in shared memory.
-constexpr int HEAD_DW_CHANNELS = 32;
+// sums meet in shared memory.  Bound by latency: eight samples' values are loaded together (128 samples of 512 channels, one at a time: 11 us).
+// beside: the launch in front is head_bwd_dx_kernel, which writes nothing that is read here and let this one start only when the kernels before it
+// were complete; the two run side by side and this one ends after the other.
+constexpr int HEAD_DW_CHANNELS = 32, HEAD_DW_AHEAD = 8;
 
 __global__ void __launch_bounds__(HEAD_THREADS) head_bwd_dw_kernel(const float* __restrict__ dlogits, const float* __restrict__ pooled,
                                                                    const float* __restrict__ g, int N, int C, int K,
-                                                                   float* __restrict__ dW, float* __restrict__ db) {
+                                                                   float* __restrict__ dW, float* __restrict__ db, int beside) {
   extern __shared__ float sdl[];                 // dlogits [N, K], then partial sums [8 warps][K][32 channels]
+  if (!beside) pdl_wait();
+  pdl_launch_dependents();
   float* part = sdl + N * K;
   for (int i = threadIdx.x; i < N * K; i += HEAD_THREADS) sdl[i] = dlogits[i];
   __syncthreads();
@@ -221,11 +229,21 @@ __global__ void __launch_bounds__(HEAD_THREADS) head_bwd_dw_kernel(const float* 
 #pragma unroll
   for (int k = 0; k < HEAD_MAX_CLASSES; ++k) acc[k] = 0.f;
   if (c < C) {
-    for (int n = warp; n < N; n += HEAD_THREADS / 32) {
-      const float pv = pooled[(int64_t)n * C + c];
+    for (int n0 = warp; n0 < N; n0 += HEAD_DW_AHEAD * (HEAD_THREADS / 32)) {
+      float pv[HEAD_DW_AHEAD];
 #pragma unroll
-      for (int k = 0; k < HEAD_MAX_CLASSES; ++k)
-        if (k < K) acc[k] = fmaf(sdl[n * K + k], pv, acc[k]);
+      for (int u = 0; u < HEAD_DW_AHEAD; ++u) {
+        const int n = n0 + u * (HEAD_THREADS / 32);
+        pv[u] = n < N ? pooled[(int64_t)n * C + c] : 0.f;
+      }
+#pragma unroll
+      for (int u = 0; u < HEAD_DW_AHEAD; ++u) {
+        const int n = n0 + u * (HEAD_THREADS / 32);
+        if (n >= N) break;
+#pragma unroll
+        for (int k = 0; k < HEAD_MAX_CLASSES; ++k)
+          if (k < K) acc[k] = fmaf(sdl[n * K + k], pv[u], acc[k]);
+      }
     }
   }
 #pragma unroll
@@ -241,9 +259,11 @@ __global__ void __launch_bounds__(HEAD_THREADS) head_bwd_dw_kernel(const float* 
   }
   if (blockIdx.x == 0 && threadIdx.x < K && db != nullptr) {
     float sum = 0.f;
+#pragma unroll 8
     for (int n = 0; n < N; ++n) sum += sdl[n * K + threadIdx.x];
     db[threadIdx.x] = sum * gs;
   }
+  if (beside) pdl_wait();
 }
 
 }  // namespace
@@ -283,8 +303,8 @@ int gc_cuda_head_forward(const float* x, int N, int positions, int C, const floa
   if (!gc_cuda_head_supported(N, positions, C, K)) return (int)cudaErrorInvalidValue;
   unsigned int* ticket = static_cast<unsigned int*>(scratch);
   float* per_sample = reinterpret_cast<float*>(static_cast<uint8_t*>(scratch) + 256);
-  head_fwd_kernel<<<N, HEAD_THREADS, 0, (cudaStream_t)cs>>>(x, positions, C, W, bias, K, labels, N, pooled, logits, dlogits, per_sample,
-                                                            ticket, out3, loss);
+  launch_pdl(head_fwd_kernel, dim3((unsigned)N), dim3(HEAD_THREADS), 0, (cudaStream_t)cs, x, positions, C, W, bias, K, labels, N, pooled, logits, dlogits, per_sample,
+             ticket, out3, loss);
   return (int)cudaGetLastError();
 }
 
@@ -295,7 +315,7 @@ int gc_cuda_head_backward(const float* dlogits, const float* pooled, const float
   cudaStream_t st = (cudaStream_t)cs;
   if (dx != nullptr) {
     dim3 grid((unsigned)(((C >> 2) + HEAD_THREADS - 1) / HEAD_THREADS), (unsigned)N);
-    head_bwd_dx_kernel<<<grid, HEAD_THREADS, 0, st>>>(dlogits, W, g, positions, C, K, dx);
+    launch_pdl(head_bwd_dx_kernel, grid, dim3(HEAD_THREADS), 0, st, dlogits, W, g, positions, C, K, dx);
   }
   if (dW != nullptr) {
     static bool configured = false;
@@ -304,8 +324,8 @@ int gc_cuda_head_backward(const float* dlogits, const float* pooled, const float
       configured = true;
     }
     const size_t smem = (size_t)N * K * 4 + (size_t)(HEAD_THREADS / 32) * K * HEAD_DW_CHANNELS * 4;
-    head_bwd_dw_kernel<<<(unsigned)((C + HEAD_DW_CHANNELS - 1) / HEAD_DW_CHANNELS), HEAD_THREADS, smem, st>>>(dlogits, pooled, g, N, C, K,
-                                                                                                        dW, db);
+    launch_pdl(head_bwd_dw_kernel, dim3((unsigned)((C + HEAD_DW_CHANNELS - 1) / HEAD_DW_CHANNELS)), dim3(HEAD_THREADS), smem, st, dlogits, pooled, g, N, C, K, dW, db,
+               dx != nullptr ? 1 : 0);
   }
   return (int)cudaGetLastError();
 }
