@@ -292,6 +292,7 @@ struct BwdArgs {
   const float *stats, *gamma, *beta;
   int relu;
   float *sums, *dx, *dres;
+  int64_t stream;          // rows of a block (whole pairs of rows of all threads) whose first reading leaves no trace in L2
   int masks;               // pairs of rows per thread whose ReLU masks fit the dynamic shared memory
 };
 
@@ -320,10 +321,15 @@ __device__ __forceinline__ float4 keep_bits(const float4& d, uint32_t m) {
 // A thread's rows are lo + rl + 128 k; pass 1 takes k upwards in pairs, pass 2 downwards.  Behind a residual the ReLU's mask comes
 // from the saved output; pass 1 leaves it in shared memory, a byte per pair of rows and thread, so that the output is read once.
 //
+// STREAM: dy and x are more than L2 keeps between the passes.  Pass 2 starts with the rows that pass 1 read last, and finds them only if neither the rows in
+// front of them nor its own results push them out: the first a.stream rows of a block are read, and everything is stored, with evict-first priority.
+// 32x32x256 at batch 128 106.7 -> 101.5 us, behind a residual 162.0 -> 153.0, 16x16x512 50.4 -> 47.2 and 76.5 -> 72.4; ResNet-50's step 5760 -> 5724 us with
+// 64 MB of both left to stay, 5729 with 96, 5739 with 128, 5736 with 48, 5760 with 32 (of 126 MB of L2; the next kernels read the results).
+//
 // KEEP: no thread has more than two rows, and what pass 1 read of dy and x stays in registers for pass 2 (8x8x256 at batch 31: 6.4 -> 6.1 us, 4x4x512
 // at 128: 6.5 -> 6.1; four and six rows in shared memory gained nothing: 8x8x256 at batch 128 8.0 -> 8.3).  With a pool: no more than one pooled row, its four
 // pixels and the winners stay (with 32-bit divisions and a row per thread instead of two: 4x4x512 at batch 128 12.3 -> 7.5 us, forward 5.4 -> 4.4).
-template <bool POOL, bool KEEP>
+template <bool POOL, bool KEEP, bool STREAM>
 __global__ void __launch_bounds__(THREADS, 1) bn_fused_bwd_kernel(const Shape s, const BwdArgs a) {
   extern __shared__ uint8_t masks[];       // [a.masks][THREADS]
   __shared__ float warp_part[THREADS / 32][VALUES];
@@ -405,17 +411,21 @@ __global__ void __launch_bounds__(THREADS, 1) bn_fused_bwd_kernel(const Shape s,
     };
     int64_t i = lo + rl;
     int pair = 0;
-    for (; i + LANES < hi; i += 2 * LANES, ++pair) {
-      const int64_t at = i * C + c4, next = at + (int64_t)LANES * C;
-      const float4 d0 = ld4(a.dy + at), v0 = ld4(a.x + at), d1 = ld4(a.dy + next), v1 = ld4(a.x + next);
-      uint32_t m = 0;
-      if (from_y) {
-        m = positive_bits(ld4_last(a.y + at)) | positive_bits(ld4_last(a.y + next)) << 4;
-        if (pair < a.masks) masks[pair * THREADS + threadIdx.x] = (uint8_t)m;
+    auto pairs_until = [&](int64_t end, auto load) {
+      for (; i + LANES < end; i += 2 * LANES, ++pair) {
+        const int64_t at = i * C + c4, next = at + (int64_t)LANES * C;
+        const float4 d0 = load(a.dy + at), v0 = load(a.x + at), d1 = load(a.dy + next), v1 = load(a.x + next);
+        uint32_t m = 0;
+        if (from_y) {
+          m = positive_bits(ld4_last(a.y + at)) | positive_bits(ld4_last(a.y + next)) << 4;
+          if (pair < a.masks) masks[pair * THREADS + threadIdx.x] = (uint8_t)m;
+        }
+        add(d0, v0, m);
+        add(d1, v1, m >> 4);
       }
-      add(d0, v0, m);
-      add(d1, v1, m >> 4);
-    }
+    };
+    if (STREAM) pairs_until(lo + a.stream < hi ? lo + a.stream : hi, [](const float* p) { return ld4_last(p); });
+    pairs_until(hi, [](const float* p) { return ld4(p); });
     if (i < hi) {
       const int64_t at = i * C + c4;
       uint32_t m = 0;
@@ -481,11 +491,15 @@ __global__ void __launch_bounds__(THREADS, 1) bn_fused_bwd_kernel(const Shape s,
     }
     return;
   }
+  auto store = [](float* p, const float4& v) {
+    if (STREAM) __stcs(reinterpret_cast<float4*>(p), v);
+    else st4(p, v);
+  };
   auto finish = [&](float4 d, const float4& v, uint32_t m, int64_t at) {
     const float4 xh = normalized(v, ch);
     if (a.relu) d = from_y ? keep_bits(d, m) : keep_positive(d, affine(xh, ch));
-    if (a.dres != nullptr) st4(a.dres + at, d);
-    st4(a.dx + at, input_gradient(d, xh));
+    if (a.dres != nullptr) store(a.dres + at, d);
+    store(a.dx + at, input_gradient(d, xh));
   };
   const int rows = hi - lo > rl ? (int)((hi - lo - rl + LANES - 1) / LANES) : 0;       // this thread's
   auto mask_of = [&](int pair, int64_t at, int64_t next, bool two) {
@@ -604,8 +618,12 @@ int gc_cuda_bn_fused_backward(const float* dy, const float* x, const float* y, i
   // masks of as many row pairs as shared memory holds (192 KB: 49 K rows of 32 channels a block)
   constexpr int most = 192;
   const int masks = y == nullptr || pool || keep ? 0 : (int)(pairs < most ? pairs : most);
-  const BwdArgs a{dy, x, y, stats, gamma, beta, relu, sums, dx, dres, masks};
-  const void* k = pool ? (keep ? (const void*)bn_fused_bwd_kernel<true, true> : (const void*)bn_fused_bwd_kernel<true, false>) : keep ? (const void*)bn_fused_bwd_kernel<false, true> : (const void*)bn_fused_bwd_kernel<false, false>;
+  // dy and x together beyond 64 MB: what exceeds it, the first rows of every block, is read the first time as data that is not needed again
+  const int64_t both = s.M * C * 8, stay = (int64_t)64 << 20;
+  const int64_t stream = pool || both <= stay ? 0 : (int64_t)((double)s.per * (double)(both - stay) / (double)both) / (2 * LANES) * (2 * LANES);
+  const BwdArgs a{dy, x, y, stats, gamma, beta, relu, sums, dx, dres, stream, masks};
+  const void* k = pool ? (keep ? (const void*)bn_fused_bwd_kernel<true, true, false> : (const void*)bn_fused_bwd_kernel<true, false, false>) : keep ? (const void*)bn_fused_bwd_kernel<false, true, false> :
+                  stream > 0 ? (const void*)bn_fused_bwd_kernel<false, false, true> : (const void*)bn_fused_bwd_kernel<false, false, false>;
   if (masks * THREADS > 24 * 1024) {
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, most * THREADS);
     if (e != cudaSuccess) return (int)e;
