@@ -188,7 +188,7 @@ __device__ __forceinline__ uint32_t ld_acquire_gpu(const uint32_t* p) {
 // memory (the wait returns once the previous kernel has completed and its writes are visible; it returns at once
 // in a kernel launched the ordinary way), and pdl_launch_dependents() to let its own successor be scheduled.
 // GCB200_PDL=0 turns it off.  Who takes part: the tensor-core kernels (their barriers, TMEM and tensor maps are ready when the previous
-// kernel ends: 1.7 us from launch to launch and 0.5-1.1 us of set-up a launch otherwise), and the small batch-norm kernels.  The fused batch-norm kernels release
+// kernel ends: 1.7 us from launch to launch and 0.5-1.1 us of set-up a launch otherwise), the small batch-norm and the head's kernels.  The fused batch-norm kernels release
 // their successors but are launched the ordinary way (gc_bn_fused.cu says why).  Every kernel releases its successors at its start, behind its own wait: steps of
 // ResNet-50 / VGG-16 / ResNet-18 at batch 31 in us, and an evaluation batch of ResNet-50: 6086 / 1051 / 1056 / 2843 without, 5881 / 1029 / 1012 / 2733 with it;
 // released when the last tile is accumulated instead 5913 / 1030 / 1015 / 2706.

@@ -290,7 +290,7 @@ struct TapCols {
 };
 
 // Where the rows of the OUTPUT go when it is not a matrix but a strided sub-grid of an NHWC tensor read through a 4-D map
-// {C, W', H', N} (the input gradient of a stride-2 convolution: one launch per parity class of input pixels): row
+// {C, W', H', N} (the input gradient of a stride-2 convolution where a parity class of input pixels is a launch of its own; all classes in one: a 5-D map): row
 // p = (n, i, j) of the result is stored at coordinates (column, j, i, n).  hw == 0: a plain 2-D matrix.
 // nh: the map's dimensions are {C, W', N, H'}, for tiles whose rows run (h, image, w).
 struct ConvC {

@@ -17,8 +17,8 @@ whose taps the kernel addresses rotated by 180 degrees (for shapes that path doe
 that one batched kernel refreshes after every optimiser step); in residual blocks the product is added straight onto the
 skip connection's or projection shortcut's gradient (``GradLink``); weight gradient ``dY^T X`` on the split-K kernel with
 MN-major operands, per filter tap from shifted boxes, added straight into the owner's flat gradient buffer.  The input
-gradient of a stride-2 convolution is four launches of the forward kernel, one per parity class of input pixels, each
-writing its pixels through a strided 4-D store map.  Grouped convolutions and shapes the tilings exclude use cuDNN
+gradient of a stride-2 convolution is four products of the forward kernel, one per parity class of input pixels, in one
+launch, each writing its pixels through a strided store map.  Grouped convolutions and shapes the tilings exclude use cuDNN
 through ``bn_act(bn, conv(x))`` or ``aten.convolution_backward``.
 
 The reference builds the same layers from ``nn.Conv2d`` + ``nn.BatchNorm2d`` + ``F.relu`` module calls
@@ -513,8 +513,7 @@ class _ConvBNAct(torch.autograd.Function):
                         dx += acc
                 elif (mode == "conv" and stride == 2 and "dgrad_s2" in PATHS and _filter_in_place_ok(w)
                       and lib.gc_cuda_conv_dgrad_s2_supported(n, x.shape[2], x.shape[3], cin, cout, r, pad)):
-                    # one launch per parity class of input pixels, each a stride-1 convolution of dY written through a
-                    # strided 4-D store map
+                    # one product per parity class of input pixels, each a stride-1 convolution of dY written through a strided store map
                     dx = torch.empty_like(x)
                     nat.check(lib.gc_cuda_conv_dgrad_s2(dconv.data_ptr(), w.data_ptr(), dx.data_ptr(), n,
                                                         x.shape[2], x.shape[3], cin, cout, r, pad, _err(x.device), st()),
