@@ -16,12 +16,30 @@ then clears the status, switches the reducer to its ``torch.distributed`` backen
 """
 from __future__ import annotations
 
+import contextlib
 import ctypes
 
 import torch
 
 from ..ops import _native as nat
 from . import comm
+
+
+class _InFlight:
+    """A host buffer that the device may still write to, and the event behind that."""
+
+    def __init__(self, event, host):
+        self.event, self.host = event, host
+
+
+_in_flight = []      # buffers of mirrors that are gone, until their last copy has landed
+
+
+def _release_landed():
+    for entry in list(_in_flight):
+        if entry.event.query():
+            with contextlib.suppress(ValueError):           # (another thread has)
+                _in_flight.remove(entry)
 
 
 class _StatusMirror:
@@ -36,10 +54,19 @@ class _StatusMirror:
     def watch(self, arenas):
         ctxs = [c for a in arenas for c in a.ctxs]
         if [c.handle.value for c in ctxs] != [c.handle.value for c in self.ctxs]:
+            self._let_go()
+            _release_landed()
             self.ctxs = ctxs
             self.host = torch.zeros(max(len(ctxs), 1), 2, dtype=torch.int32).pin_memory()
+
+    def _let_go(self):
+        """The buffer is not to be used for something else before the copy on its way has landed."""
+        if self.event is not None:
+            _in_flight.append(_InFlight(self.event, self.host))
             self.event = None
 
+    def __del__(self):
+        self._let_go()
 
     def check(self):
         """Raise for what the last completed copy shows (nothing is waited for: a copy still in flight is looked at by

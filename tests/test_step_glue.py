@@ -3,6 +3,7 @@ it does something."""
 import torch
 
 from gradient_compression_b200 import models
+from gradient_compression_b200.parallel import graph
 from gradient_compression_b200.parallel.graph import _side_by_side
 
 
@@ -25,3 +26,20 @@ def test_pooling_of_one_pixel():
     handle.remove()
     net.features[-1].divisor_override = 2
     assert seen == [1] and torch.equal(net._features(x), want / 2)
+
+
+def test_status_buffer_outlives_its_mirror_until_the_copy_has_landed():
+    class Event:
+        done = False
+
+        def query(self):
+            return self.done
+
+    mirror, event, before = graph._StatusMirror(torch.device("cpu")), Event(), len(graph._in_flight)
+    mirror.host, mirror.event = torch.zeros(1, 2), event
+    del mirror
+    graph._release_landed()
+    assert [e.event for e in graph._in_flight[before:]] == [event]
+    event.done = True
+    graph._release_landed()
+    assert len(graph._in_flight) == before
