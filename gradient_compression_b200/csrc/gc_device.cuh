@@ -93,7 +93,8 @@ __device__ __forceinline__ float round_level(float g, float scale, float s, uint
 __device__ __forceinline__ float signed_value(float g, float level, float dq) {
   return __fmaf_rn(dq, g < 0.0f ? -level : level, 0.0f);
 }
-// The same where g is no NaN (a negative one would count as negative here): one instruction less.
+// The same where g is a number and its scale finite (a negative NaN, and a -0.0 whose level is not zero, would count as negative here): one
+// instruction less.
 __device__ __forceinline__ float signed_value_of_number(float g, float level, float dq) {
   return __fmaf_rn(dq, __uint_as_float(__float_as_uint(level) | (__float_as_uint(g) & 0x80000000u)), 0.0f);
 }

@@ -135,7 +135,8 @@ __device__ __forceinline__ float solo_grid_max(Waiter& w, SoloSync& sync, float 
 }
 
 // Pass 2 for any input: infinities and NaN (norm = inf), more quads than 32 bits count, a fine scale with no more levels than the coarse
-// one or (norms below 1e-35) of infinite size.  Plain loads; a function of its own, as its registers cost the usual path its own.
+// one, a scale of infinite size (levels / norm overflows: norms below 7.5e-37 at 8 bits, 1.9e-34 at 16; zero times infinity is given the last
+// level, without the sign of the zero).  Plain loads; a function of its own, as its registers cost the usual path its own.
 template <bool TWO, int CAP>
 __device__ __noinline__ void pass2_any(const SegTable<CAP>& t, const SoloParams& p, float norm, uint32_t step, uint32_t first, int iters, int kept, const float4* slots) {
   const float s_lo = (float)p.s_lo, s_hi = (float)p.s_hi;
@@ -232,7 +233,7 @@ __global__ void __launch_bounds__(THREADS, 1) solo_maxnorm_kernel(const __grid_c
   const float sc_lo = norm > 0.0f ? s_lo / norm : 0.0f, dq_lo = dequant_scale(norm, p.s_lo, 1);
   const float sc_hi = TWO && norm > 0.0f ? s_hi / norm : 0.0f, dq_hi = TWO ? dequant_scale(norm, p.s_hi, 1) : 0.0f;
 
-  // From here on: finite numbers, quads of 32-bit index, and a fine scale with more levels than the coarse one.
+  // From here on: finite numbers and scales, quads of 32-bit index, and a fine scale with more levels than the coarse one.
   PhiloxHead head_one;
   if (TWO) {
     if (threadIdx.x == 0) {
@@ -269,7 +270,8 @@ __global__ void __launch_bounds__(THREADS, 1) solo_maxnorm_kernel(const __grid_c
 
   // pass 2, last tile first: the ring still holds the last RING tiles
   if (iters == 0) return;
-  if (!(norm < __int_as_float(0x7f800000)) || (uint64_t)t.start[t.n] >= (1ull << 34) || (TWO && (p.s_hi <= p.s_lo || !(sc_hi < __int_as_float(0x7f800000))))) {
+  const float inf = __int_as_float(0x7f800000);
+  if (!(norm < inf) || !((TWO ? sc_hi : sc_lo) < inf) || (uint64_t)t.start[t.n] >= (1ull << 34) || (TWO && p.s_hi <= p.s_lo)) {
     pass2_any<TWO, CAP>(t, p, norm, step, first, iters, kept, slots);
     return;
   }

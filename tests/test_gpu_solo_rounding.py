@@ -50,3 +50,13 @@ def test_special_values(name, config, value):
         long = torch.randn(148 * 4096 * 14 + 3, generator=torch.Generator().manual_seed(2)) * (1e-37 if abs(value) < 1e-30 else 1.0)
         long[::100003] = value
         compare(name, config, [long])
+
+
+@pytest.mark.parametrize("n", [4096 * 3 + 5, 148 * 4096 * 14 + 9])
+@pytest.mark.parametrize("norm", [1e-34, 1e-36, 1e-37])
+@pytest.mark.parametrize("name,config", CONFIGS)
+def test_zeros_of_both_signs_at_tiny_norms(name, config, norm, n):
+    """Where levels / norm overflows, zero times infinity is given the last level, and the sign of a zero does not count."""
+    x = torch.rand(n, generator=torch.Generator().manual_seed(n)) * (2 * norm) - norm
+    x[::7], x[3::7], x[1] = 0.0, -0.0, -norm
+    compare(name, config, [x])
