@@ -11,6 +11,8 @@ CONFIGS = [("QSGDMaxNormReducer", {"quantization_level": 1}), ("QSGDMaxNormReduc
            ("QSGDMaxNormTwoScaleReducer", {"quantization_level": 2, "higher_quantization_level": 6}),
            ("QSGDMaxNormTwoScaleReducer", {"quantization_level": 6, "higher_quantization_level": 10}),
            ("QSGDMaxNormTwoScaleReducer", {"quantization_level": 6, "higher_quantization_level": 6})]
+RANDK = [("GlobalRandKMaxNormReducer", {"K": 3000, "quantization_level": 8}),
+         ("GlobalRandKMaxNormTwoScaleReducer", {"K": 3000, "quantization_level": 6, "higher_quantization_level": 10})]
 NAN = float("nan")
 
 
@@ -53,10 +55,11 @@ def test_special_values(name, config, value):
 
 
 @pytest.mark.parametrize("n", [4096 * 3 + 5, 148 * 4096 * 14 + 9])
-@pytest.mark.parametrize("norm", [1e-34, 1e-36, 1e-37])
-@pytest.mark.parametrize("name,config", CONFIGS)
+@pytest.mark.parametrize("norm", [1e-34, 1e-36, 1e-37, 1e-44])
+@pytest.mark.parametrize("name,config", CONFIGS + RANDK)
 def test_zeros_of_both_signs_at_tiny_norms(name, config, norm, n):
-    """Where levels / norm overflows, zero times infinity is given the last level, and the sign of a zero does not count."""
+    """Where levels / norm overflows, zero times infinity is given the last level, and the sign of a zero does not count; where the value of a level
+    underflows to zero (1e-44 and more than thirteen levels), negative elements become -0.0."""
     x = torch.rand(n, generator=torch.Generator().manual_seed(n)) * (2 * norm) - norm
     x[::7], x[3::7], x[1] = 0.0, -0.0, -norm
     compare(name, config, [x])
