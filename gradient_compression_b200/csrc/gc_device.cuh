@@ -191,9 +191,14 @@ __device__ __forceinline__ uint32_t ld_acquire_gpu(const uint32_t* p) {
 // in a kernel launched the ordinary way), and pdl_launch_dependents() to let its own successor be scheduled.
 // GCB200_PDL=0 turns it off.  Who takes part: the tensor-core kernels (their barriers, TMEM and tensor maps are ready when the previous
 // kernel ends: 1.7 us from launch to launch and 0.5-1.1 us of set-up a launch otherwise), the small batch-norm and the head's kernels.  The fused batch-norm kernels release
-// their successors but are launched the ordinary way (gc_bn_fused.cu says why).  Every kernel releases its successors at its start, behind its own wait: steps of
+// their successors but are launched the ordinary way (gc_bn_fused.cu says why).  Kernels release their successors at their start, behind their own wait: steps of
 // ResNet-50 / VGG-16 / ResNet-18 at batch 31 in us, and an evaluation batch of ResNet-50: 6086 / 1051 / 1056 / 2843 without, 5881 / 1029 / 1012 / 2733 with it;
 // released when the last tile is accumulated instead 5913 / 1030 / 1015 / 2706.
+// Who may read before its predecessor is complete: a kernel that is told to wait late (wait_late, beside) -- because that predecessor is named by
+// its caller, writes nothing it reads or adds to, and released it behind a wait of its own, so that everything in front of that is complete.
+// The exceptions to that release are not named by any such caller: zero_kernel (gc_tc.cuh) releases first and then waits; Top-K's fold and the
+// Philox fill, launched the ordinary way, begin when all in front is complete and never wait; the late waiters themselves release first.
+// Whatever follows one of those waits at its start.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

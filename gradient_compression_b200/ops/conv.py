@@ -304,13 +304,14 @@ def conv_forward(x, w, bias=None, stride=1, pad=1, col_partials=None, out=None, 
 
 def conv_wgrad(dy, x, r, stride, pad, out=None, beside=False):
     """Weight gradient ``[Cout, R*R*Cin]`` (channels-last filter order) of ``conv2d(x, w, stride, pad)`` given the
-    channels-last output gradient ``dy``; added onto ``out`` when given."""
+    channels-last output gradient ``dy``; added onto ``out`` when given.  ``beside``: as in ``gemm.gemm_tn_tf32``, where ``out``
+    is given (otherwise the launch in front is the zeroing of the result, which the kernel waits for)."""
     n, cin, h, wd = x.shape
     cout = dy.shape[1]
     dw = out if out is not None else torch.zeros(cout, r * r * cin, dtype=torch.float32, device=x.device)
     with torch.cuda.device(x.device):
         nat.check(nat.cuda().gc_cuda_conv_wgrad(dy.data_ptr(), x.data_ptr(), dw.data_ptr(), n, h, wd, cin, cout, r, stride, pad,
-                                                _err(x.device), nat.stream_ptr(), int(beside)), "conv_wgrad")
+                                                _err(x.device), nat.stream_ptr(), int(beside and out is not None)), "conv_wgrad")
     return dw
 
 
@@ -543,11 +544,11 @@ class _ConvBNAct(torch.autograd.Function):
                 slot = _slot_of(w) if WGRAD_ENABLED else None       # the owner's gradient storage, or None: return a tensor
                 if mode == "gemm" and WGRAD_ENABLED and cout % 32 == 0 and cin % 32 == 0:
                     # dW[Cout, Cin] = dY^T X over all positions: split-K GEMM with MN-major tcgen05 operands
-                    dw2d = gemm.gemm_tn_tf32(_as_2d(dconv), _as_2d(x), out=slot, accumulate=slot is not None, beside=beside and slot is not None)
+                    dw2d = gemm.gemm_tn_tf32(_as_2d(dconv), _as_2d(x), out=slot, accumulate=slot is not None, beside=beside)
                     dw = None if slot is not None else dw2d.view(cout, cin, 1, 1).contiguous(memory_format=torch.channels_last)
                 elif mode == "conv" and WGRAD_ENABLED and lib.gc_cuda_conv_wgrad_supported(n, x.shape[2], x.shape[3], cin, cout, r,
                                                                                            stride, pad):
-                    dw2d = conv_wgrad(dconv, x, r, stride, pad, out=slot, beside=beside and slot is not None)
+                    dw2d = conv_wgrad(dconv, x, r, stride, pad, out=slot, beside=beside)
                     dw = None if slot is not None else dw2d.view(cout, r, r, cin).permute(0, 3, 1, 2)
                 elif mode == "stem" and WGRAD_ENABLED and cout % 32 == 0:
                     dwp = gemm.gemm_tn_tf32(_as_2d(dconv), gathered)                       # [Cout, STEM_K]

@@ -113,7 +113,7 @@ def gemm_tn_tf32(a_pm, b_pn, out=None, accumulate=False, beside=False):
     operands are MN-major tcgen05 operands and the contraction is split over CTAs whose partial tiles are added onto
     ``out`` by TMA reduce stores (so the summation order of the partials is not fixed).  ``beside``: the launch in front on this
     stream is the input gradient of the same layer; the two then run side by side (``out`` and the operands must not come
-    from that launch)."""
+    from that launch).  Without ``accumulate`` the launch in front is the zeroing of ``out``, and the product waits for it."""
     if out is None:
         assert not accumulate
         out = torch.zeros(a_pm.shape[1], b_pn.shape[1], dtype=torch.float32, device=a_pm.device)
@@ -125,7 +125,7 @@ def gemm_tn_tf32(a_pm, b_pn, out=None, accumulate=False, beside=False):
     with torch.cuda.device(a_pm.device):
         nat.check(nat.cuda().gc_cuda_gemm_tn_tf32(a_pm.data_ptr(), b_pn.data_ptr(), out.data_ptr(), a_pm.shape[0], a_pm.shape[1],
                                                   b_pn.shape[1], a_pm.stride(0), b_pn.stride(0), out.stride(0),
-                                                  _error_flag(a_pm.device).data_ptr(), nat.stream_ptr(), int(beside)), "gemm_tn_tf32")
+                                                  _error_flag(a_pm.device).data_ptr(), nat.stream_ptr(), int(beside and accumulate)), "gemm_tn_tf32")
     return out
 
 
