@@ -32,7 +32,9 @@ class _InFlight:
         self.event, self.host = event, host
 
 
-_in_flight = []      # buffers of mirrors that are gone, until their last copy has landed
+# Buffers of mirrors that are gone, until their last copy has landed: looked at by every later step of the process (not when a mirror goes: that may
+# be in the middle of a capture, which a query would end).  Without a later step the last one's stays, eight bytes an arena.
+_in_flight = []
 
 
 def _release_landed():
@@ -55,7 +57,6 @@ class _StatusMirror:
         ctxs = [c for a in arenas for c in a.ctxs]
         if [c.handle.value for c in ctxs] != [c.handle.value for c in self.ctxs]:
             self._let_go()
-            _release_landed()
             self.ctxs = ctxs
             self.host = torch.zeros(max(len(ctxs), 1), 2, dtype=torch.int32).pin_memory()
 
@@ -71,6 +72,8 @@ class _StatusMirror:
     def check(self):
         """Raise for what the last completed copy shows (nothing is waited for: a copy still in flight is looked at by
         a later call)."""
+        if _in_flight:
+            _release_landed()
         if self.event is None or not self.event.query():
             return
         self.event = None

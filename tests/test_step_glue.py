@@ -43,3 +43,16 @@ def test_status_buffer_outlives_its_mirror_until_the_copy_has_landed():
     event.done = True
     graph._release_landed()
     assert len(graph._in_flight) == before
+
+
+def test_a_later_step_gives_back_the_status_buffer_of_one_that_is_gone():
+    class Event:
+        def query(self):
+            return True
+
+    mirror, other, before = graph._StatusMirror(torch.device("cpu")), graph._StatusMirror(torch.device("cpu")), len(graph._in_flight)
+    mirror.host, mirror.event = torch.zeros(1, 2), Event()
+    del mirror
+    assert len(graph._in_flight) == before + 1
+    other.check()                                   # its arenas stay as they are
+    assert len(graph._in_flight) == before
