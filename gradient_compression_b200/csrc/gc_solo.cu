@@ -2,6 +2,7 @@
 // straight from the gradient tensors into the gradient tensors.
 //
 //   solo_maxnorm_kernel  QSGD-MaxNorm and its two-scale variant: one persistent block of 1024 threads per SM.
+//   solo_maxnorm_one_kernel  the same of up to 16 K elements, which one block holds.
 //   solo_randk_kernel    GlobalRandK-MaxNorm and its two-scale variant.
 //   solo_copy_kernel     AllReduce-SGD: the mean over one worker.
 //
@@ -32,7 +33,7 @@ constexpr int THREADS = SEG_TILE;
 constexpr int SLOTS = 13;                  // tiles of shared memory
 constexpr int RING = 4;                    // ... of which the copies in flight take these ...
 constexpr int KEPT = SLOTS - RING;         // ... when a block has more tiles than slots; the rest stay there between the passes
-constexpr int ONE_BLOCK_TILES = 4;         // up to this many tiles run on one block: no grid barrier, an ordinary launch
+constexpr int ONE_BLOCK_TILES = 4;         // up to this many tiles run on one block: no grid barrier, an ordinary launch of a kernel of its own
 
 struct SoloParams {
   ArenaHeader* hdr;
@@ -134,39 +135,80 @@ __device__ __forceinline__ float solo_grid_max(Waiter& w, SoloSync& sync, float 
   return m;
 }
 
-// Pass 2 for any input: infinities and NaN (norm = inf), more quads than 32 bits count, a fine scale with no more levels than the coarse
-// one, a scale of infinite size (levels / norm overflows: norms below 7.5e-37 at 8 bits, 1.9e-34 at 16; zero times infinity is given the last
-// level, without the sign of the zero).  Plain loads; a function of its own, as its registers cost the usual path its own.
+// What becomes of one quad, for any input: infinities and NaN (norm = inf), quads beyond 32 bits, a fine scale with no more levels than the
+// coarse one, a scale of infinite size (levels / norm overflows: norms below 7.5e-37 at 8 bits, 1.9e-34 at 16; zero times infinity is given the
+// last level, without the sign of the zero).
+template <bool TWO>
+struct AnyValue {
+  float s_lo, s_hi, sc_lo, sc_hi, dq_lo, dq_hi;
+  __device__ __forceinline__ AnyValue(const SoloParams& p, float norm)
+      : s_lo((float)p.s_lo), s_hi((float)p.s_hi), sc_lo(norm > 0.0f ? s_lo / norm : 0.0f), sc_hi(TWO && norm > 0.0f ? s_hi / norm : 0.0f),
+        dq_lo(dequant_scale(norm, p.s_lo, 1)), dq_hi(TWO ? dequant_scale(norm, p.s_hi, 1) : 0.0f) {}
+  __device__ __forceinline__ float4 operator()(const SoloParams& p, const float4& x, uint64_t quad, uint32_t step) const {
+    if (!TWO) {
+      const U4 r = solo_philox(p, quad, step, PURPOSE_ROUND);
+      return make_float4(signed_value(x.x, round_level(x.x, sc_lo, s_lo, r.x), dq_lo), signed_value(x.y, round_level(x.y, sc_lo, s_lo, r.y), dq_lo),
+                         signed_value(x.z, round_level(x.z, sc_lo, s_lo, r.z), dq_lo), signed_value(x.w, round_level(x.w, sc_lo, s_lo, r.w), dq_lo));
+    }
+    // the fine scale where its level fits the coarse range, else the coarse scale; its noise is only drawn where it is used
+    const U4 r = solo_philox(p, quad, step, PURPOSE_ROUND_HI);
+    const float h0 = round_level(x.x, sc_hi, s_hi, r.x), h1 = round_level(x.y, sc_hi, s_hi, r.y);
+    const float h2 = round_level(x.z, sc_hi, s_hi, r.z), h3 = round_level(x.w, sc_hi, s_hi, r.w);
+    float4 y = make_float4(signed_value(x.x, h0, dq_hi), signed_value(x.y, h1, dq_hi), signed_value(x.z, h2, dq_hi), signed_value(x.w, h3, dq_hi));
+    if (fmaxf(fmaxf(h0, h1), fmaxf(h2, h3)) > s_lo) {
+      const U4 w = solo_philox(p, quad, step, PURPOSE_ROUND);
+      if (h0 > s_lo) y.x = signed_value(x.x, round_level(x.x, sc_lo, s_lo, w.x), dq_lo);
+      if (h1 > s_lo) y.y = signed_value(x.y, round_level(x.y, sc_lo, s_lo, w.y), dq_lo);
+      if (h2 > s_lo) y.z = signed_value(x.z, round_level(x.z, sc_lo, s_lo, w.z), dq_lo);
+      if (h3 > s_lo) y.w = signed_value(x.w, round_level(x.w, sc_lo, s_lo, w.w), dq_lo);
+    }
+    return y;
+  }
+};
+
+// Pass 2 with it.  Plain loads; a function of its own, as its registers cost the usual path its own.
 template <bool TWO, int CAP>
 __device__ __noinline__ void pass2_any(const SegTable<CAP>& t, const SoloParams& p, float norm, uint32_t step, uint32_t first, int iters, int kept, const float4* slots) {
-  const float s_lo = (float)p.s_lo, s_hi = (float)p.s_hi;
-  const float sc_lo = norm > 0.0f ? s_lo / norm : 0.0f, dq_lo = dequant_scale(norm, p.s_lo, 1);
-  const float sc_hi = TWO && norm > 0.0f ? s_hi / norm : 0.0f, dq_hi = TWO ? dequant_scale(norm, p.s_hi, 1) : 0.0f;
+  const AnyValue<TWO> value(p, norm);
   SegCursor<CAP, -1> c(t, first + iters - 1);
   for (int it = iters - 1; it >= 0; --it, c.step(t)) {
     if (c.empty(t)) continue;
     const float4 x = it < kept ? slots[it * THREADS + threadIdx.x] : c.load(t);
-    const uint64_t quad = c.quad;
-    float4 y;
-    if (TWO) {
-      // the fine scale where its level fits the coarse range, else the coarse scale; its noise is only drawn where it is used
-      const U4 r = solo_philox(p, quad, step, PURPOSE_ROUND_HI);
-      const float h0 = round_level(x.x, sc_hi, s_hi, r.x), h1 = round_level(x.y, sc_hi, s_hi, r.y);
-      const float h2 = round_level(x.z, sc_hi, s_hi, r.z), h3 = round_level(x.w, sc_hi, s_hi, r.w);
-      y = make_float4(signed_value(x.x, h0, dq_hi), signed_value(x.y, h1, dq_hi), signed_value(x.z, h2, dq_hi), signed_value(x.w, h3, dq_hi));
-      if (fmaxf(fmaxf(h0, h1), fmaxf(h2, h3)) > s_lo) {
-        const U4 w = solo_philox(p, quad, step, PURPOSE_ROUND);
-        if (h0 > s_lo) y.x = signed_value(x.x, round_level(x.x, sc_lo, s_lo, w.x), dq_lo);
-        if (h1 > s_lo) y.y = signed_value(x.y, round_level(x.y, sc_lo, s_lo, w.y), dq_lo);
-        if (h2 > s_lo) y.z = signed_value(x.z, round_level(x.z, sc_lo, s_lo, w.z), dq_lo);
-        if (h3 > s_lo) y.w = signed_value(x.w, round_level(x.w, sc_lo, s_lo, w.w), dq_lo);
-      }
-    } else {
-      const U4 r = solo_philox(p, quad, step, PURPOSE_ROUND);
-      y = make_float4(signed_value(x.x, round_level(x.x, sc_lo, s_lo, r.x), dq_lo), signed_value(x.y, round_level(x.y, sc_lo, s_lo, r.y), dq_lo),
-                      signed_value(x.z, round_level(x.z, sc_lo, s_lo, r.z), dq_lo), signed_value(x.w, round_level(x.w, sc_lo, s_lo, r.w), dq_lo));
+    c.store(t, value(p, x, c.quad, step));
+  }
+}
+
+// Up to ONE_BLOCK_TILES tiles: one block, which keeps them in registers.  Such a call is a launch and little more: no ring, no dynamic shared memory,
+// no barrier but that of the norm, every load in flight at once.  The kernel below, run with one block, had its ring's prologue and a called function in
+// the way (us a call back to back / in a graph; 1024 elements 5.84 / 3.43, before it had that function 5.60 / 3.39, here 4.80 / 2.87, which
+// is the host's time; 16384 elements 8.21 / 6.56 -> 7.29 / 5.53, two scales 10.26 / 8.88 -> 10.25 / 8.32).
+template <bool TWO, int CAP>
+__global__ void __launch_bounds__(THREADS, 1) solo_maxnorm_one_kernel(const __grid_constant__ SegTable<CAP> t, const __grid_constant__ SoloParams p) {
+  __shared__ float smem[32];
+  const uint32_t epoch = next_epoch(p.hdr);
+  const uint32_t step = p.step + (p.step_from_device ? launch_calls(p.hdr) : 0u);
+  const int iters = (int)t.tile0[t.n];
+  float4 x[ONE_BLOCK_TILES];
+  float m = 0.0f;
+  {
+    SegCursor<CAP, 1> c(t, 0);
+#pragma unroll
+    for (int u = 0; u < ONE_BLOCK_TILES; ++u) {
+      x[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (u < iters) { x[u] = c.load(t); c.step(t); }
     }
-    c.store(t, y);
+  }
+#pragma unroll
+  for (int u = 0; u < ONE_BLOCK_TILES; ++u) m = max_nan(max_nan(max_nan(max_nan(m, x[u].x), x[u].y), x[u].z), x[u].w);
+  const float norm = block_max(abs_for_max(m), smem);
+  commit_epoch(p.hdr, epoch, 0);
+  const AnyValue<TWO> value(p, norm);
+  SegCursor<CAP, 1> c(t, 0);
+#pragma unroll
+  for (int u = 0; u < ONE_BLOCK_TILES; ++u) {
+    if (u >= iters) break;
+    if (!c.empty(t)) c.store(t, value(p, x[u], c.quad, step));
+    c.step(t);
   }
 }
 
@@ -415,6 +457,11 @@ __global__ void __launch_bounds__(THREADS) solo_randk_kernel(const __grid_consta
 
 template <bool TWO, int CAP>
 int launch_maxnorm(const SegTable<CAP>& t, const SoloParams& p, int sm_count, int max_blocks, cudaStream_t st) {
+  const uint32_t tiles = t.tile0[t.n];
+  if (tiles <= ONE_BLOCK_TILES) {
+    solo_maxnorm_one_kernel<TWO, CAP><<<1, THREADS, 0, st>>>(t, p);
+    return (int)cudaGetLastError();
+  }
   auto kernel = solo_maxnorm_kernel<TWO, CAP>;
   static bool ready[64] = {};              // per device: the shared-memory limit has been raised
   int dev = 0;
@@ -425,8 +472,7 @@ int launch_maxnorm(const SegTable<CAP>& t, const SoloParams& p, int sm_count, in
     if (e != cudaSuccess) return (int)e;
     ready[dev] = true;
   }
-  const uint32_t tiles = t.tile0[t.n];
-  uint32_t blocks = tiles <= ONE_BLOCK_TILES ? 1u : (tiles < (uint32_t)sm_count ? tiles : (uint32_t)sm_count);
+  uint32_t blocks = tiles < (uint32_t)sm_count ? tiles : (uint32_t)sm_count;
   if (max_blocks > 0 && blocks > (uint32_t)max_blocks) blocks = (uint32_t)max_blocks;
   const int iters = (int)((tiles + blocks - 1) / blocks);
   void* args[2] = {(void*)&t, (void*)&p};

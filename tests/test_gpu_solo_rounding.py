@@ -63,3 +63,11 @@ def test_zeros_of_both_signs_at_tiny_norms(name, config, norm, n):
     x = torch.rand(n, generator=torch.Generator().manual_seed(n)) * (2 * norm) - norm
     x[::7], x[3::7], x[1] = 0.0, -0.0, -norm
     compare(name, config, [x])
+
+
+@pytest.mark.parametrize("sizes", [[1], [4095], [4097], [8193], [12288], [16383], [16384], [16385], [1, 4090, 3, 4000], [5, 0, 7], [4096, 1, 2, 3], [1, 4097, 1, 2]])
+@pytest.mark.parametrize("name,config", CONFIGS)
+def test_one_block(name, config, sizes):
+    """Up to four tiles of 4096 elements have a kernel of their own; a tensor that starts inside a tile begins another."""
+    gen = torch.Generator().manual_seed(sum(sizes))
+    compare(name, config, [torch.randn(n, generator=gen) for n in sizes])
