@@ -567,14 +567,16 @@ extern "C" {
 int gc_cuda_bn_fused_supported(int64_t M, int C) { return shape_ok(M, C, sm_count()) ? 1 : 0; }
 
 // Blocks a launch on M rows of C channels takes on a chip of `sms` SMs, each of which has a row of partial sums (0: not taken).
-int gc_cuda_bn_fused_blocks(int64_t M, int C, int sms) {
+static int planned_blocks(int64_t M, int C, int sms, int pool) {
   if (!shape_ok(M, C, sms)) return 0;
   Shape s{};
   s.M = M;
   s.C = C;
-  plan(s, sms, 0);
+  plan(s, sms, pool);
   return s.G * s.R;
 }
+int gc_cuda_bn_fused_blocks(int64_t M, int C, int sms) { return planned_blocks(M, C, sms, 0); }
+int gc_cuda_bn_fused_pool_blocks(int64_t M, int C, int sms) { return planned_blocks(M, C, sms, 1); }      // M pooled rows
 
 // Scratch of both directions: barrier counts (zeroed once when allocated; every launch leaves them ready) and partial sums.
 int64_t gc_cuda_bn_fused_scratch_bytes() { return (int64_t)sizeof(GroupSync) + (int64_t)MAX_BLOCKS * VALUES * 4; }

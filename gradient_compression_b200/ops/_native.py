@@ -186,6 +186,7 @@ def cuda():
         _declare(lib, "gc_cuda_tc_taps_config", None, [c_int])
         _declare(lib, "gc_cuda_bn_fused_supported", c_int, [c_i64, c_int])
         _declare(lib, "gc_cuda_bn_fused_blocks", c_int, [c_i64, c_int, c_int])
+        _declare(lib, "gc_cuda_bn_fused_pool_blocks", c_int, [c_i64, c_int, c_int])
         _declare(lib, "gc_cuda_bn_fused_scratch_bytes", c_i64, [])
         _declare(lib, "gc_cuda_bn_fused_forward", c_int, [P] + [c_int] * 5 + [P, c_int, P, P, P, c_int, P, P, c_float, c_float, P, P, P, P, P])
         _declare(lib, "gc_cuda_bn_fused_backward", c_int, [P, P, P] + [c_int] * 5 + [P, P, P, c_int, P, P, P, P, P, P])
