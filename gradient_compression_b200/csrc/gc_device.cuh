@@ -80,7 +80,8 @@ __device__ __forceinline__ float max_nan(float m, float x) {
 //   subtracts it times 2^125.  Rounding that up keeps the ceiling: integers are floats, so no rounding up passes one.
 //   ceil: adding 1.5 * 2^23 rounding up leaves it in the last mantissa bits (-1 < l - u < 2^16 where it matters).
 // Six instructions with the clamp, two of them on the ALU, which Philox keeps busy.  (Flooring, then comparing the fraction with u as
-// integers, takes nine and five: 140 against 81 instructions a quad in the second pass of a single worker's reduce.)
+// integers, takes nine and five.  With it and what else a quad was spared, the second pass of a single worker's reduce executes 107 instructions
+// a quad instead of 126, with two scales 184 instead of 281.)
 constexpr float ROUND_BASE = 12582912.0f;
 __device__ __forceinline__ float round_up_base(float g, float scale, uint32_t rnd) {      // ROUND_BASE + level, not clamped
   const float l = __fmul_rn(fabsf(g), scale);
@@ -189,8 +190,9 @@ __device__ __forceinline__ uint32_t ld_acquire_gpu(const uint32_t* p) {
 // draining, which hides its launch latency and prologue.  Such a kernel calls pdl_wait() before it touches
 // memory (the wait returns once the previous kernel has completed and its writes are visible; it returns at once
 // in a kernel launched the ordinary way), and pdl_launch_dependents() to let its own successor be scheduled.
-// GCB200_PDL=0 turns it off.  Who takes part: the tensor-core kernels (their barriers, TMEM and tensor maps are ready when the previous
-// kernel ends: 1.7 us from launch to launch and 0.5-1.1 us of set-up a launch otherwise), the small batch-norm and the head's kernels.  The fused batch-norm kernels release
+// GCB200_PDL=0 turns it off.  Who takes part: the persistent and the transposed tensor-core kernels (their barriers, TMEM and tensor maps are ready
+// when the previous kernel ends: 1.7 us from launch to launch and 0.5-1.1 us of set-up a launch otherwise), zero_kernel, the small and the separate-pass batch norms, the
+// head's training kernels, PowerSGD's and, behind the fold, Top-K's, the status copy.  The fused batch-norm kernels release
 // their successors but are launched the ordinary way (gc_bn_fused.cu says why).  Kernels release their successors at their start, behind their own wait: steps of
 // ResNet-50 / VGG-16 / ResNet-18 at batch 31 in us, and an evaluation batch of ResNet-50: 6086 / 1051 / 1056 / 2843 without, 5881 / 1029 / 1012 / 2733 with it;
 // released when the last tile is accumulated instead 5913 / 1030 / 1015 / 2706.

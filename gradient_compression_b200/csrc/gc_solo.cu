@@ -11,11 +11,12 @@
 // tiles of every block stay in shared memory (KEPT x 16 KB per SM, 22 MB over the chip), and the rest is read again in
 // falling order, last tile first, so that what was read most recently comes out of L2 (stores are streaming, so that
 // they push out each other and not the tiles still to come).  Both passes load through a ring of
-// asynchronous copies, RING tiles (64 KB per SM) ahead.  The second pass is otherwise bound by instruction issue: ten Philox
-// rounds per quad plus the rounding of four elements.  Rounding is therefore written without int <-> float conversions,
+// asynchronous copies, RING tiles (64 KB per SM) ahead.  The second pass is held up by its arithmetic and its stores, which overlap by half: ten
+// Philox rounds per quad plus the rounding of four elements, and 4 n bytes out (ResNet-50's arena: 24 of 54 us for the first pass; the second's 29 are 20 without
+// Philox, 24 without stores, 12 without both; 64 M floats, of which the chip keeps little: 49 of 145 us, then 96, 87, 62 and 35).  Rounding is therefore written without int <-> float conversions,
 // which run at a quarter of the rate of the rest (see round_level), the round keys come with the parameters, what a launch's blocks have in
 // common is taken out of the first three rounds, and infinities and NaN, which only a norm of infinity can mean, have a pass of their own.
-// Two scales, 33.5 M floats: 309 -> 219 instructions a quad, 125 -> 103 us; one scale, ResNet-50's arena: 45.8 -> 41.2 us.  Two quads side by side in
+// 33.5 M floats, instructions of both passes a quad: two scales 309 -> 212, 127 -> 106 us; one scale 154 -> 135, 83.5 -> 80 us.  Two quads side by side in
 // a thread spill (50 -> 57 us on VGG-16's tensors), both scales' noise drawn at once, too, took longer (59 us).
 #include <cuda_runtime.h>
 #include <stdint.h>

@@ -1576,7 +1576,7 @@ inline Plan pick_classes(int M, int N, int K, int t0, int t1) {
 
 // C[M, N] = 0 in front of a split contraction, which adds its partial tiles.  A kernel of its own instead of a memset node: a programmatic dependent
 // itself, and the product behind it can be one, too (it sets up its barriers and TMEM meanwhile):
-// ResNet-18's step at batch 31, with 13 of them, 971 -> 949 us, ResNet-50's with eight 5821 -> 5812.
+// ResNet-18's step at batch 31, with 11 of them, 947 -> 942 us, VGG-16's at 128, with 11, 1020 -> 1017, ResNet-50's, with eight, 5804 -> 5808 (no difference).
 __global__ void __launch_bounds__(512) zero_kernel(float4* __restrict__ p, int64_t quads) {
   gc::pdl_launch_dependents();
   gc::pdl_wait();
